@@ -297,7 +297,7 @@ __device__ void pull_chunk(const BArgs& a, uint32_t q, uint32_t ch, uint32_t* he
         v[0] = NONE64;
         if (valid) {
             const unsigned long long d = qq.prop[s];
-            const unsigned long long wt = G.w[p];
+            const unsigned long long wt = G.w8 ? (unsigned long long)G.w8[p] : G.w[p];
             if (G.weight_kind == WEDGE_WEIGHTS_F64)
                 v[0] = (unsigned long long)__double_as_longlong(
                     __dadd_rn(__longlong_as_double((long long)d), __longlong_as_double((long long)wt)));

@@ -75,6 +75,13 @@ int track(wedge_graph* h, void* p)
     return WEDGE_OK;
 }
 
+static void untrack(wedge_graph* h, void* p)
+{
+    for (int i = 0; i < h->nallocs; ++i)
+        if (h->allocs[i] == p)
+            h->allocs[i] = h->allocs[--h->nallocs];
+}
+
 static int track_state(wedge_graph* h, void* p)
 {
     if (h->nstate >= (int)(sizeof(h->state_allocs) / sizeof(h->state_allocs[0])))
@@ -303,9 +310,9 @@ __global__ void max_weight_kernel(const unsigned long long* w, uint64_t E, unsig
         atomicMax(out, m);
 }
 
-__global__ void narrow_weights_kernel(const unsigned long long* w, uint64_t Epad, uint8_t* w8)
+__global__ void narrow_weights_kernel(const unsigned long long* w, uint64_t E, uint8_t* w8)
 {
-    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < Epad; e += (uint64_t)gridDim.x * blockDim.x)
+    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x)
         w8[e] = (uint8_t)w[e];
 }
 
@@ -351,18 +358,50 @@ __global__ void permutation_kernel(const unsigned long long* sorted_key, uint64_
     }
 }
 
-__global__ void relabel_edges_kernel(const uint32_t* src, const uint32_t* dst, uint64_t E, const uint32_t* old2new,
-                                     unsigned long long* key)
-{
-    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x)
-        key[e] = ((unsigned long long)old2new[dst[e]] << 32) | old2new[src[e]];
-}
-
-__global__ void unpack_edges_kernel(const unsigned long long* key, uint64_t E, uint32_t* src, uint32_t* dst)
+// Sort keys of the relabelled edges: destination | source | weight byte, from
+// the top, in vbits, vbits and 8 bits (no weight bits where w is null)
+__global__ void relabel_edges_kernel(const uint32_t* src, const uint32_t* dst, const unsigned long long* w, uint64_t E,
+                                     const uint32_t* old2new, int vbits, unsigned long long* key)
 {
     for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x) {
-        src[e] = (uint32_t)(key[e] & 0xffffffffull);
-        dst[e] = (uint32_t)(key[e] >> 32);
+        const unsigned long long k = ((unsigned long long)old2new[dst[e]] << vbits) | old2new[src[e]];
+        key[e] = w ? (k << 8) | (w[e] & 0xFFull) : k;
+    }
+}
+
+__global__ void unpack_edges_kernel(const unsigned long long* key, uint64_t E, int vbits, uint32_t* src, uint32_t* dst,
+                                    uint8_t* w8)
+{
+    const unsigned long long mask = (1ull << vbits) - 1ull;
+    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x) {
+        unsigned long long k = key[e];
+        if (w8) {
+            w8[e] = (uint8_t)k;
+            k >>= 8;
+        }
+        src[e] = (uint32_t)(k & mask);
+        dst[e] = (uint32_t)(k >> vbits);
+    }
+}
+
+// destination | source | weight keys -> destination | weight | source keys
+__global__ void weight_key_kernel(unsigned long long* key, uint64_t E, int vbits)
+{
+    const unsigned long long mask = (1ull << vbits) - 1ull;
+    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x) {
+        const unsigned long long k = key[e];
+        key[e] = ((k >> (vbits + 8)) << (vbits + 8)) | ((k & 0xFFull) << vbits) | ((k >> 8) & mask);
+    }
+}
+
+// the sorted destination | weight | source keys, and the padding past the last in-edge
+__global__ void weight_unpack_kernel(const unsigned long long* key, uint64_t E, uint64_t Epad, int vbits, uint32_t* wsrc,
+                                     uint8_t* ww8)
+{
+    const unsigned long long mask = (1ull << vbits) - 1ull;
+    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < Epad; e += (uint64_t)gridDim.x * blockDim.x) {
+        wsrc[e] = e < E ? (uint32_t)(key[e] & mask) : NONE32;
+        ww8[e] = e < E ? (uint8_t)(key[e] >> vbits) : (uint8_t)0xFFu;
     }
 }
 
@@ -370,10 +409,18 @@ __global__ void unpack_edges_kernel(const unsigned long long* key, uint64_t E, u
 // by id), so the sources gathered most often are the lowest ids and share cache
 // lines; edges are renumbered and re-sorted by (destination, source).  The
 // permutations stay on the device: roots are mapped in, results mapped back.
+// Byte-wide weights travel inside the 64-bit sort keys where those have room
+// (*w8 receives them; 8 + 8 bytes per in-edge and pass instead of 16 + 16 with
+// the 64-bit weights as a payload), and the same keys, sorted once more by
+// (destination, weight), give the in-edges a second time, each destination's
+// by ascending weight (*wsrc, *ww8: 5 bytes per in-edge; null where the device
+// has no room for them, and on shards).
 static int relabel_by_degree(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_src, uint32_t* d_dst,
-                             unsigned long long* d_w, uint32_t** new2old, uint32_t** old2new,
-                             const uint32_t* global_outdeg)
+                             unsigned long long* d_w, bool byte_weights, uint32_t** new2old, uint32_t** old2new,
+                             uint8_t** w8, uint32_t** wsrc, uint8_t** ww8, const uint32_t* global_outdeg)
 {
+    *w8 = *ww8 = nullptr;
+    *wsrc = nullptr;
     cudaStream_t st = h->stream;
     const uint32_t cap = (uint32_t)h->num_sms * 16u;
     int rc;
@@ -410,28 +457,51 @@ static int relabel_by_degree(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d
     int vbits = 1;
     while (vbits < 32 && (1ull << vbits) < V)
         ++vbits;
+    const bool in_key = byte_weights && 2 * vbits + 8 <= 64;
+    const uint64_t Epad = (E + MAX_TILE_E - 1) / MAX_TILE_E * MAX_TILE_E;
     unsigned long long *ek = nullptr, *ek2 = nullptr, *w2 = nullptr;
     WEDGE_CHECK(cudaMallocAsync((void**)&ek, E * sizeof(unsigned long long), st));
     WEDGE_CHECK(cudaMallocAsync((void**)&ek2, E * sizeof(unsigned long long), st));
-    relabel_edges_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, d_dst, E, *old2new, ek);
+    const uint32_t grid = grid_for(E, AUX_THREADS, cap);
+    relabel_edges_kernel<<<grid, AUX_THREADS, 0, st>>>(d_src, d_dst, in_key ? d_w : nullptr, E, *old2new, vbits, ek);
     cub::DoubleBuffer<unsigned long long> kb(ek, ek2);
     size_t tb = 0;
     void* tmp = nullptr;
-    if (d_w) {
+    if (d_w && !in_key) {
         WEDGE_CHECK(cudaMallocAsync((void**)&w2, E * sizeof(unsigned long long), st));
         cub::DoubleBuffer<unsigned long long> vb(d_w, w2);
-        WEDGE_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, tb, kb, vb, (long long)E, 0, 32 + vbits, st));
+        WEDGE_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, tb, kb, vb, (long long)E, 0, 2 * vbits, st));
         WEDGE_CHECK(cudaMallocAsync(&tmp, tb ? tb : 1, st));
-        WEDGE_CHECK(cub::DeviceRadixSort::SortPairs(tmp, tb, kb, vb, (long long)E, 0, 32 + vbits, st));
+        WEDGE_CHECK(cub::DeviceRadixSort::SortPairs(tmp, tb, kb, vb, (long long)E, 0, 2 * vbits, st));
         if (vb.Current() != d_w)
             WEDGE_CHECK(cudaMemcpyAsync(d_w, vb.Current(), E * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, st));
     } else {
-        WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(nullptr, tb, kb, (long long)E, 0, 32 + vbits, st));
+        const int b0 = in_key ? 8 : 0;
+        WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(nullptr, tb, kb, (long long)E, b0, b0 + 2 * vbits, st));
         WEDGE_CHECK(cudaMallocAsync(&tmp, tb ? tb : 1, st));
-        WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tb, kb, (long long)E, 0, 32 + vbits, st));
+        WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tb, kb, (long long)E, b0, b0 + 2 * vbits, st));
     }
-    unpack_edges_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(kb.Current(), E, d_src, d_dst);
+    if (in_key && (rc = dalloc(h, w8, Epad)))
+        return rc;
+    unpack_edges_kernel<<<grid, AUX_THREADS, 0, st>>>(kb.Current(), E, vbits, d_src, d_dst, *w8);
+    if (in_key)
+        WEDGE_CHECK(cudaMemsetAsync(*w8 + E, 0, Epad - E, st));
     cudaFreeAsync(tmp, st);
+    if (in_key && !global_outdeg && Epad < (1ull << 32)) { /* 32-bit in-edge positions */
+        if (dalloc(h, wsrc, Epad) == WEDGE_OK && dalloc(h, ww8, Epad) == WEDGE_OK) {
+            weight_key_kernel<<<grid, AUX_THREADS, 0, st>>>(kb.Current(), E, vbits);
+            WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(nullptr, tb, kb, (long long)E, vbits, 2 * vbits + 8, st));
+            WEDGE_CHECK(cudaMallocAsync(&tmp, tb ? tb : 1, st));
+            WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tb, kb, (long long)E, vbits, 2 * vbits + 8, st));
+            cudaFreeAsync(tmp, st);
+            weight_unpack_kernel<<<grid_for(Epad, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(kb.Current(), E, Epad, vbits,
+                                                                                         *wsrc, *ww8);
+        } else {
+            cudaGetLastError(); /* no room: the SSSP pulls go without (one of the two stays the handle's, unused) */
+            *wsrc = nullptr;
+            *ww8 = nullptr;
+        }
+    }
     cudaFreeAsync(ek, st);
     cudaFreeAsync(ek2, st);
     if (w2)
@@ -469,26 +539,47 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
     g.w = d_w;
     const uint32_t cap = (uint32_t)h->num_sms * 16u;
 
-    int* d_err = nullptr;
-    WEDGE_CHECK(cudaMallocAsync((void**)&d_err, sizeof(int), st));
-    WEDGE_CHECK(cudaMemsetAsync(d_err, 0, sizeof(int), st));
+    // input errors and the largest uint64 weight
+    unsigned long long *d_chk = nullptr, chk[2] = {0ull, 0ull};
+    WEDGE_CHECK(cudaMallocAsync((void**)&d_chk, sizeof(chk), st));
+    WEDGE_CHECK(cudaMemsetAsync(d_chk, 0, sizeof(chk), st));
     if (E)
-        validate_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, d_dst, E, V, d_err);
-    int herr = 0;
-    WEDGE_CHECK(cudaMemcpyAsync(&herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+        validate_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, d_dst, E, V, (int*)d_chk);
+    if (E && d_w && weight_kind == WEDGE_WEIGHTS_U64)
+        max_weight_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_w, E, d_chk + 1);
+    WEDGE_CHECK(cudaMemcpyAsync(chk, d_chk, sizeof(chk), cudaMemcpyDeviceToHost, st));
     WEDGE_CHECK(cudaStreamSynchronize(st));
-    cudaFreeAsync(d_err, st);
-    if (herr) {
+    cudaFreeAsync(d_chk, st);
+    // weights in one byte each where every uint64 weight is below 256: the pulls
+    // stream 1 byte per in-edge instead of 8
+    const bool byte_weights = E && d_w && weight_kind == WEDGE_WEIGHTS_U64 && chk[1] < 256ull;
+    if (chk[0]) {
         cudaFreeAsync(d_dst, st);
         return WEDGE_ERR_FORMAT;
     }
     {
         uint32_t *n2o = nullptr, *o2n = nullptr;
-        int rc = relabel_by_degree(h, V, E, d_src, d_dst, d_w, &n2o, &o2n, d_global_outdeg);
+        uint8_t *w8 = nullptr, *ww8 = nullptr;
+        uint32_t* wsrc = nullptr;
+        int rc = relabel_by_degree(h, V, E, d_src, d_dst, d_w, byte_weights, &n2o, &o2n, &w8, &wsrc, &ww8, d_global_outdeg);
         if (rc)
             return rc;
         g.new2old = n2o;
         g.old2new = o2n;
+        if (w8) { /* the 64-bit words are not read any more */
+            WEDGE_CHECK(cudaStreamSynchronize(st));
+            untrack(h, d_w);
+            cudaFree(d_w);
+            g.w = d_w = nullptr;
+        } else if (byte_weights) {
+            if ((rc = dalloc(h, &w8, g.Epad)))
+                return rc;
+            narrow_weights_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_w, E, w8);
+            WEDGE_CHECK(cudaMemsetAsync(w8 + E, 0, g.Epad - E, st));
+        }
+        g.w8 = w8;
+        g.wsrc = wsrc;
+        g.ww8 = ww8;
     }
 
     // compressed destinations
@@ -588,27 +679,6 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
     WEDGE_CHECK(cudaGetLastError());
     g.nsplit = nsplit[0];
     g.nwide = nsplit[1];
-    // SSSP weights in one byte each where every uint64 weight is below 256: the
-    // pulls stream 1 byte per in-edge instead of 8 (same arithmetic, 64-bit sums)
-    g.w8 = nullptr;
-    if (d_w && weight_kind == WEDGE_WEIGHTS_U64 && E) {
-        unsigned long long* d_max = nullptr;
-        unsigned long long wmax = 0;
-        WEDGE_CHECK(cudaMallocAsync((void**)&d_max, sizeof(unsigned long long), st));
-        WEDGE_CHECK(cudaMemsetAsync(d_max, 0, sizeof(unsigned long long), st));
-        max_weight_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_w, E, d_max);
-        WEDGE_CHECK(cudaMemcpyAsync(&wmax, d_max, sizeof(wmax), cudaMemcpyDeviceToHost, st));
-        WEDGE_CHECK(cudaStreamSynchronize(st));
-        cudaFreeAsync(d_max, st);
-        if (wmax < 256ull) {
-            uint8_t* w8 = nullptr;
-            if ((rc = dalloc(h, &w8, g.Epad)))
-                return rc;
-            narrow_weights_kernel<<<grid_for(g.Epad, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_w, g.Epad, w8);
-            WEDGE_CHECK(cudaGetLastError());
-            g.w8 = w8;
-        }
-    }
     g.dst_ident = (Vne && last_dst == Vne - 1) ? 1u : 0u;
     g.sym = h_asym ? 0u : 1u;
     g.dst_id = dst_id;
@@ -840,6 +910,8 @@ __host__ __device__ constexpr uint32_t pull_launches_of(int app)
 {
     return app == WEDGE_APP_PR ? 1u : app == WEDGE_APP_CC ? 4u : 2u;
 }
+// SSSP with weight-ordered in-edges: Wedge pulls and 64-bit dense ones, sssp_wo_kernel, sssp_wo_long_kernel
+constexpr uint32_t SSSP_WO_LAUNCHES = 3u;
 // dst_kernel launches of one pull
 __host__ __device__ constexpr uint32_t dst_launches_of(int app)
 {
@@ -866,6 +938,12 @@ __device__ __forceinline__ void dist32_put(const DevState& s, uint32_t v, unsign
         s.dist32[v] = (uint32_t)d;
     else
         atomicMin(&s.dist32[v], (uint32_t)d);
+}
+
+// the weight-ordered kernels run this pull: dense and filtered pulls while every distance fits the 32-bit copy
+__device__ __forceinline__ bool sssp_wo_runs(const DevState& s, const Ctrl* c)
+{
+    return s.wo && c->mode != MODE_WEDGE && !c->narrow_ovf;
 }
 
 // The Wedge pull of SSSP over in-edge positions: every vertex the last pull
@@ -1005,6 +1083,11 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
     }
     if (APP == WEDGE_APP_SSSP && mode == MODE_WEDGE && s.push) {
         sssp_push_pull(g, s, c, block_cnt);
+        return;
+    }
+    if (APP == WEDGE_APP_SSSP && sssp_wo_runs(s, c)) { /* the next two launches are this pull */
+        if (threadIdx.x < NCNT)
+            block_cnt[NCNT * blockIdx.x + threadIdx.x] = 0ull;
         return;
     }
     /* the in-edge stream is read once per pull: it should not push the gathered array out of L2 */
@@ -1367,33 +1450,23 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
 }
 
 // SSSP dense and source-filtered pulls over 512-edge tiles, for graphs with
-// byte-wide weights and in-edge positions in the CSRI (Wedge pulls relax the
-// activated sources' in-edges, sssp_push_pull).  Lane l loads its 16 sources
-// (two 256-bit loads) and 16 weight bytes (one 128-bit load), gathers the
-// sources' distances (hub cache or global memory) and adds the weights; the
-// warp takes the per-destination minimum with the segmented reduction.  The
-// minima of the tile's first complete destinations (256 with 32-bit sums, 128
-// with 64-bit ones) are staged
-// in the warp's slice of shared memory and compared, written and activated by
-// the warp's lanes together over consecutive destinations; spanning
-// destinations take atomicMin.  While the distances fit the 32-bit copy the
-// candidates are 32-bit sums (a sum at or above the copy's limit is dropped,
-// Ctrl::narrow_ovf and Ctrl::ovf_redo are set, and the next pull is a dense
-// 64-bit one, which relaxes every in-edge again).  Two instantiations run
-// each launch, the 64-bit one first: SUMS32 for dense and filtered pulls while
-// the distances fit the copy, the other for the rest (and the Wedge pulls);
-// each returns at once where the other runs (the 32-bit one may set
-// Ctrl::narrow_ovf, so it runs second).  Two launches as pull_kernel's (hub
-// destinations' tiles first).  Dynamic shared memory: hub cache | staged minima.
+// byte-wide weights and in-edge positions in the CSRI but without the
+// weight-ordered in-edges of sssp_wo_kernel (shards), whose Wedge pulls relax
+// the activated sources' in-edges (sssp_push_pull).  Lane l loads its 16
+// sources (two 256-bit loads) and 16 weight bytes (one 128-bit load), gathers
+// the sources' distances (hub cache or global memory; the 32-bit copy while
+// it is exact) and adds the weights in 64 bits; the warp takes the
+// per-destination minimum with the segmented reduction.  The minima of the
+// tile's first complete destinations are staged in the warp's slice of shared
+// memory and compared, written and activated by the warp's lanes together over
+// consecutive destinations; the spanning ones are left to sssp_split_kernel.
+// Two launches as pull_kernel's (hub destinations' tiles first).  Dynamic
+// shared memory: hub cache | staged minima.
 constexpr int SSSP_EPL = 16;
 constexpr uint32_t SSSP_TILE = 32u * SSSP_EPL;
-constexpr uint32_t SSSP_SLOTS = 128;   /* staged 64-bit minima per warp (64-bit instantiation) */
-constexpr uint32_t SSSP_SLOTS32 = 256; /* staged 32-bit minima per warp: the tiles with more destinations
-                                          (R-MAT scale 22: 7% of the complete ones, 25% past 128 slots) */
-constexpr uint32_t SSSP_WARP_STAGE = SSSP_SLOTS * 8u > SSSP_SLOTS32 * 4u ? SSSP_SLOTS * 8u : SSSP_SLOTS32 * 4u;
-constexpr uint32_t SSSP_STAGE_BYTES = (PULL_THREADS / 32) * SSSP_WARP_STAGE;
+constexpr uint32_t SSSP_SLOTS = 128; /* staged minima per warp */
+constexpr uint32_t SSSP_STAGE_BYTES = (PULL_THREADS / 32) * SSSP_SLOTS * 8u;
 
-template <bool SUMS32>
 __global__ void __launch_bounds__(PULL_THREADS, 1)
     sssp_pull_kernel(DevGraph g, DevState s, unsigned long long* block_cnt, uint32_t phase)
 {
@@ -1408,8 +1481,6 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
     if (c->done)
         return;
     const uint32_t mode = c->mode;
-    if ((mode != MODE_WEDGE && s.dist32 && !c->narrow_ovf && s.narrow_sums) != SUMS32)
-        return; /* the other instantiation's launch */
     if (mode == MODE_WEDGE) {
         if (phase == PHASE_HUBS)
             sssp_push_pull(g, s, c, block_cnt);
@@ -1428,18 +1499,16 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
     uint32_t* nxt = next_front(s, c->parity);
     const bool filtered = mode == MODE_FILTERED;
     const uint32_t hub_bytes = s.hub_bytes;
-    const bool narrow = s.dist32 && !c->narrow_ovf; /* gathers from the 32-bit copy (and, SUMS32, sums) */
+    const bool narrow = s.dist32 && !c->narrow_ovf; /* gathers from the 32-bit copy */
     const uint32_t lim = s.narrow_lim;
-    bool dropped = false;                           /* a 32-bit sum reached the limit */
     const unsigned long long pol = l2_evict_first_policy(); /* for the in-edge and weight streams */
     const unsigned char* hub_src = narrow ? reinterpret_cast<const unsigned char*>(s.dist32)
                                           : reinterpret_cast<const unsigned char*>(s.prop64);
     uint32_t* hub32 = reinterpret_cast<uint32_t*>(sssp_smem);
     unsigned long long* hub64 = reinterpret_cast<unsigned long long*>(sssp_smem);
-    constexpr uint32_t SLOTS = SUMS32 ? SSSP_SLOTS32 : SSSP_SLOTS;
-    unsigned char* stage = sssp_smem + hub_bytes + (uint32_t)wib * SSSP_WARP_STAGE;
-    uint32_t* my_min32 = reinterpret_cast<uint32_t*>(stage);
-    unsigned long long* my_min64 = reinterpret_cast<unsigned long long*>(stage);
+    constexpr uint32_t SLOTS = SSSP_SLOTS;
+    unsigned long long* my_min64 =
+        reinterpret_cast<unsigned long long*>(sssp_smem + hub_bytes + (uint32_t)wib * SSSP_SLOTS * 8u);
     unsigned long long mass = 0, edges = 0, tiles = 0, dsts = 0, act = 0, occ = 0;
     if (threadIdx.x < 3)
         sh_deg[threadIdx.x] = 0u;
@@ -1573,64 +1642,31 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
                 activate(vtx);
             }
         };
-        if constexpr (SUMS32) {
-            uint32_t v[EPL];
+        unsigned long long v[EPL];
 #pragma unroll
-            for (int q = 0; q < EPL; ++q) {
-                const uint32_t x = sa[q];
-                bool on = x != NONE32;
-                if (filtered && on)
-                    on = (ld_ro_u32(cur + (x >> 5)) >> (x & 31u)) & 1u; /* changed by the previous pull */
-                // global memory only for sources past the hub cache, behind a
-                // branch (measured 7% faster per dense pull than a select of
-                // the two loads)
-                uint32_t gy = NONE32;
-                if (on && x >= hub_lim)
-                    gy = ld_gather_u32(s.dist32 + x);
-                const uint32_t y = on ? ((x < hub_lim) ? hub32[x] : gy) : NONE32;
-                const uint32_t w = (wword[q >> 2] >> (8 * (q & 3))) & 0xFFu;
-                uint32_t sum = y + w; /* phase_edge_pull_sssp.c:136-137 */
-                if (y != NONE32 && (sum < y || sum >= lim)) {
-                    dropped = true;
-                    sum = NONE32;
-                }
-                v[q] = (y == NONE32) ? NONE32 : sum;
+        for (int q = 0; q < EPL; ++q) {
+            const uint32_t x = sa[q];
+            bool on = x != NONE32;
+            if (filtered && on)
+                on = (ld_ro_u32(cur + (x >> 5)) >> (x & 31u)) & 1u; /* changed by the previous pull */
+            unsigned long long d = NONE64;
+            if (on && narrow) {
+                const uint32_t y = (x < hub_lim) ? hub32[x] : ld_gather_u32(s.dist32 + x);
+                d = (y == NONE32) ? NONE64 : (unsigned long long)y;
+            } else if (on) {
+                d = (x < hub_lim) ? hub64[x] : s.prop64[x];
             }
-            tile_geometry_bits<EPL>(g, base, t + 1u >= T, k0, kend, lane, tg);
-            seg_reduce<EPL>(v, tg, lane, MinU32(), [&](uint32_t k, uint32_t val, int kind) {
-                const uint32_t slot = k - tg.k0;
-                if (kind == EMIT_COMPLETE && slot < SLOTS)
-                    my_min32[slot] = val;
-                else
-                    apply(k, val == NONE32 ? NONE64 : (unsigned long long)val, kind);
-            });
-        } else {
-            unsigned long long v[EPL];
-#pragma unroll
-            for (int q = 0; q < EPL; ++q) {
-                const uint32_t x = sa[q];
-                bool on = x != NONE32;
-                if (filtered && on)
-                    on = (ld_ro_u32(cur + (x >> 5)) >> (x & 31u)) & 1u; /* changed by the previous pull */
-                unsigned long long d = NONE64;
-                if (on && narrow) {
-                    const uint32_t y = (x < hub_lim) ? hub32[x] : ld_gather_u32(s.dist32 + x);
-                    d = (y == NONE32) ? NONE64 : (unsigned long long)y;
-                } else if (on) {
-                    d = (x < hub_lim) ? hub64[x] : s.prop64[x];
-                }
-                const unsigned long long w = (wword[q >> 2] >> (8 * (q & 3))) & 0xFFu;
-                v[q] = (d == NONE64) ? NONE64 : d + w; /* phase_edge_pull_sssp.c:136-137 */
-            }
-            tile_geometry_bits<EPL>(g, base, t + 1u >= T, k0, kend, lane, tg);
-            seg_reduce<EPL>(v, tg, lane, MinU64(), [&](uint32_t k, unsigned long long val, int kind) {
-                const uint32_t slot = k - tg.k0;
-                if (kind == EMIT_COMPLETE && slot < SLOTS)
-                    my_min64[slot] = val;
-                else
-                    apply(k, val, kind);
-            });
+            const unsigned long long w = (wword[q >> 2] >> (8 * (q & 3))) & 0xFFu;
+            v[q] = (d == NONE64) ? NONE64 : d + w; /* phase_edge_pull_sssp.c:136-137 */
         }
+        tile_geometry_bits<EPL>(g, base, t + 1u >= T, k0, kend, lane, tg);
+        seg_reduce<EPL>(v, tg, lane, MinU64(), [&](uint32_t k, unsigned long long val, int kind) {
+            const uint32_t slot = k - tg.k0;
+            if (kind == EMIT_COMPLETE && slot < SLOTS)
+                my_min64[slot] = val;
+            else
+                apply(k, val, kind);
+        });
         dsts += tg.ndst;
         __syncwarp();
         const uint32_t nd = tg.ndst;
@@ -1642,14 +1678,8 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
         for (uint32_t j0 = 0; j0 < jhi; j0 += 32u) { /* warp-uniform rounds */
             const uint32_t j = j0 + (uint32_t)lane;
             unsigned long long val = NONE64;
-            if (j >= jlo && j < jhi) {
-                if constexpr (SUMS32) {
-                    const uint32_t x = my_min32[j];
-                    val = x == NONE32 ? NONE64 : (unsigned long long)x;
-                } else {
-                    val = my_min64[j];
-                }
-            }
+            if (j >= jlo && j < jhi)
+                val = my_min64[j];
             bool chg = false;
             uint32_t vtx = 0u, od = 0u;
             if (val != NONE64) {
@@ -1680,10 +1710,6 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
     if (use_hub && threadIdx.x == 0 && !mbar_wait_bounded(&hub_bar, 0u, HUB_WAIT_TRIES)) {
         atomicOr(&c->error, ERR_HUB_TIMEOUT);
         mbar_wait_bounded(&hub_bar, 0u, HUB_WAIT_TRIES);
-    }
-    if (__any_sync(FULL, dropped) && lane == 0) {
-        atomicOr(&c->narrow_ovf, 1u);
-        atomicOr(&c->ovf_redo, 1u);
     }
     {
         const unsigned long long d0 = warp_sum_u64(degs & 0x1FFFFFull);
@@ -1797,6 +1823,263 @@ __global__ void sssp_split_kernel(DevGraph g, DevState s, unsigned long long* bl
         atomicAdd(&bc[CNT_DEG1], d1);
         atomicAdd(&bc[CNT_DEG2], d2);
     }
+}
+
+// SSSP dense and source-filtered pulls over weight-ordered in-edges, 32-bit
+// sums.  Distances are not negative, so an in-edge whose weight alone is not
+// below its destination's distance cannot lower it, and neither can the ones
+// after it: a destination reads its in-edges by ascending weight and stops at
+// the first such weight.  On R-MAT graphs with weights 1..255 the first dense
+// pull reads 15% of the in-edges and the later ones 5-6% (scales 20 and 22),
+// where a tile pull streams and gathers them all: 4.95 / 4.90 / 4.64 ms for
+// the three dense pulls at scale 26 before.  Bound by the latency of a
+// destination's chain (offsets, distance, weights and sources, distances of
+// the sources): one destination per lane, four in-edges a step (one word of
+// weights, one 128-bit load of sources, up to four gathers in flight), 64
+// warps per SM.  A destination that has not stopped after SSSP_WO_WINDOW
+// in-edges leaves the others to sssp_wo_long_kernel, in pieces of
+// SSSP_WO_PIECE up to the first weight that cannot lower it.
+//
+// A sum at or above the 32-bit copy's limit that would have lowered its
+// destination is dropped, Ctrl::narrow_ovf and Ctrl::ovf_redo are set, and the
+// next pull is a dense 64-bit one, which relaxes every in-edge again.
+constexpr uint32_t SSSP_WO_WINDOW = 32;
+constexpr uint32_t SSSP_WO_PIECE = 4096;
+
+// four weight-ordered in-edges at position p (a multiple of 4), of which those
+// in [lo, hi) are the destination's: lowers dist, counts the in-edges read
+struct WoStep {
+    uint32_t last;    // weight of position p + 3
+    bool dropped;     // a sum past the limit would have lowered dist
+};
+
+__device__ __forceinline__ WoStep sssp_wo_step(const DevGraph& g, const DevState& s, const uint32_t* filter, uint32_t p,
+                                               uint32_t lo, uint32_t hi, uint32_t& dist, uint32_t& edges)
+{
+    const uint32_t ww = ld_ro_u32(reinterpret_cast<const uint32_t*>(g.ww8 + p));
+    const uint4 xs = __ldg(reinterpret_cast<const uint4*>(g.wsrc + p));
+    const uint32_t x[4] = {xs.x, xs.y, xs.z, xs.w};
+    uint32_t y[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+        bool on = p + j >= lo && p + j < hi && ((ww >> (8 * j)) & 0xFFu) < dist;
+        edges += on ? 1u : 0u;
+        if (filter && on)
+            on = (ld_ro_u32(filter + (x[j] >> 5)) >> (x[j] & 31u)) & 1u; /* changed by the previous pull */
+        y[j] = NONE32;
+        if (on)
+            y[j] = ld_gather_u32(s.dist32 + x[j]);
+    }
+    WoStep r{ww >> 24, false};
+    uint32_t m = dist;
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+        const uint32_t sum = y[j] + ((ww >> (8 * j)) & 0xFFu); /* phase_edge_pull_sssp.c:136-137 */
+        if (y[j] != NONE32) {
+            if (sum < y[j] || sum >= s.narrow_lim)
+                r.dropped = true;
+            else
+                m = min(m, sum);
+        }
+    }
+    r.dropped = r.dropped && m == NONE32;
+    dist = m;
+    return r;
+}
+
+// a block's counters, per lane in 32 bits except the mass (in-edge positions fit 32 bits here)
+__device__ __forceinline__ void sssp_wo_counters(unsigned long long* block_cnt, unsigned long long mass, uint32_t edges,
+                                                 uint32_t dsts, uint32_t act, uint32_t occ, const uint32_t (&deg)[3])
+{
+    constexpr int WARPS = PULL_THREADS / 32;
+    __shared__ unsigned long long sh_cnt[WARPS][NCNT];
+    const unsigned long long v[NCNT] = {warp_sum_u64(mass),   warp_sum_u64(edges),  0ull,
+                                        warp_sum_u64(dsts),   warp_sum_u64(act),    warp_sum_u64(deg[0]),
+                                        warp_sum_u64(deg[1]), warp_sum_u64(deg[2]), warp_sum_u64(occ)};
+    if ((threadIdx.x & 31) == 0)
+        for (uint32_t j = 0; j < NCNT; ++j)
+            sh_cnt[threadIdx.x >> 5][j] = v[j];
+    __syncthreads();
+    if (threadIdx.x < NCNT) {
+        unsigned long long a = 0;
+        for (int w = 0; w < WARPS; ++w)
+            a += sh_cnt[w][threadIdx.x];
+        block_cnt[NCNT * blockIdx.x + threadIdx.x] = a;
+    }
+}
+
+__global__ void __launch_bounds__(PULL_THREADS, 2) sssp_wo_kernel(DevGraph g, DevState s, unsigned long long* block_cnt)
+{
+    __shared__ uint32_t runs; /* one answer per block: another block may set Ctrl::narrow_ovf meanwhile */
+    Ctrl* c = s.ctrl;
+    if (c->done)
+        return;
+    if (threadIdx.x == 0)
+        runs = sssp_wo_runs(s, c) ? 1u : 0u;
+    __syncthreads();
+    if (!runs) {
+        if (threadIdx.x < NCNT)
+            block_cnt[NCNT * blockIdx.x + threadIdx.x] = 0ull;
+        return;
+    }
+    const int lane = threadIdx.x & 31;
+    const uint32_t nthr = gridDim.x * blockDim.x;
+    const uint32_t* filter = c->mode == MODE_FILTERED ? cur_front(s, c->parity) : nullptr;
+    uint32_t* nxt = next_front(s, c->parity);
+    unsigned long long mass = 0;
+    uint32_t edges = 0, dsts = 0, act = 0, occ = 0, deg[3] = {0u, 0u, 0u};
+    bool dropped = false;
+    // the next group's offsets and vertices are loaded while this one is pulled
+    uint32_t plo = 0u, phi = 0u, pd = 0u;
+    auto prefetch = [&](uint32_t b) {
+        const uint32_t kk = b + (uint32_t)lane;
+        if (kk < g.Vne) {
+            plo = (uint32_t)g.dst_off[kk];
+            phi = (uint32_t)g.dst_off[kk + 1u];
+            pd = g.dst_ident ? kk : g.dst_id[kk];
+        }
+    };
+    const uint32_t b0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
+    prefetch(b0);
+    for (uint32_t base = b0; base < g.Vne; base += nthr) {
+        const uint32_t k = base + (uint32_t)lane;
+        const uint32_t lo = plo, hi = phi, d = pd;
+        prefetch(base + nthr);
+        const bool mine = k < g.Vne;
+        bool chg = false;
+        uint32_t npiece = 0u, rest = 0u;
+        uint32_t word = NONE32, od = 0u;
+        if (mine) {
+            ++dsts;
+            const uint32_t before = s.dist32[d];
+            uint32_t dist = before, p = lo & ~3u;
+            bool more = true;
+            do {
+                const WoStep r = sssp_wo_step(g, s, filter, p, lo, hi, dist, edges);
+                dropped = dropped || r.dropped;
+                p += 4u;
+                more = p < hi && r.last < dist;
+            } while (more && p - lo < SSSP_WO_WINDOW);
+            if (more) {
+                rest = p;
+                uint32_t end = hi;
+                if (hi - p > SSSP_WO_PIECE) { /* first weight that cannot lower the destination */
+                    uint32_t a = p;
+                    while (a < end) {
+                        const uint32_t mid = a + (end - a) / 2u;
+                        if (g.ww8[mid] < dist)
+                            a = mid + 1u;
+                        else
+                            end = mid;
+                    }
+                }
+                npiece = (end - p + SSSP_WO_PIECE - 1u) / SSSP_WO_PIECE;
+            }
+            chg = dist < before;
+            if (chg) { /* the destination's only writer in this launch */
+                s.dist32[d] = dist;
+                s.prop64[d] = dist;
+                od = g.outdeg[d];
+                word = d >> 5;
+                mass += od;
+                ++act;
+                const uint32_t bk = degree_bucket(od);
+#pragma unroll
+                for (uint32_t b = 0; b < 3u; ++b)
+                    deg[b] += bk == b ? 1u : 0u;
+            }
+        }
+        // frontier bits: one atomicOr per distinct word of the 32 destinations
+        const uint32_t grp = __match_any_sync(FULL, word);
+        const uint32_t bits = __reduce_or_sync(grp, chg ? 1u << (d & 31u) : 0u);
+        if (chg && (uint32_t)lane == (uint32_t)(__ffs(grp) - 1)) {
+            atomicOr(&nxt[word], bits);
+            ++occ;
+        }
+        if (__any_sync(FULL, npiece != 0u)) {
+            uint32_t incl = npiece;
+#pragma unroll
+            for (int q = 1; q < 32; q <<= 1) {
+                const uint32_t v = __shfl_up_sync(FULL, incl, q);
+                if (lane >= q)
+                    incl += v;
+            }
+            uint32_t at = 0u;
+            if (lane == 31)
+                at = atomicAdd(&c->need_n, incl);
+            at = __shfl_sync(FULL, at, 31) + incl - npiece;
+            for (uint32_t i = 0; i < npiece; ++i)
+                s.wo_items[at + i] = make_uint2(k, rest + i * SSSP_WO_PIECE);
+        }
+    }
+    if (dropped) {
+        atomicOr(&c->narrow_ovf, 1u);
+        atomicOr(&c->ovf_redo, 1u);
+    }
+    sssp_wo_counters(block_cnt, mass, edges, dsts, act, occ, deg);
+}
+
+// the long destinations' other in-edges, one piece per warp: 128 in-edges a
+// step.  Several pieces of a destination combine with atomicMin.  Runs when
+// sssp_wo_kernel ran, also where that set Ctrl::narrow_ovf (the copy's sums
+// stay exact: sums past the limit are dropped here too).
+__global__ void __launch_bounds__(PULL_THREADS, 2)
+    sssp_wo_long_kernel(DevGraph g, DevState s, unsigned long long* block_cnt)
+{
+    Ctrl* c = s.ctrl;
+    if (c->done)
+        return;
+    const uint32_t n = c->need_n; /* 0 unless sssp_wo_kernel listed pieces */
+    if (n == 0u) {
+        if (threadIdx.x < NCNT)
+            block_cnt[NCNT * blockIdx.x + threadIdx.x] = 0ull;
+        return;
+    }
+    const int lane = threadIdx.x & 31;
+    const uint32_t* filter = c->mode == MODE_FILTERED ? cur_front(s, c->parity) : nullptr;
+    uint32_t* nxt = next_front(s, c->parity);
+    unsigned long long mass = 0;
+    uint32_t edges = 0, act = 0, occ = 0, deg[3] = {0u, 0u, 0u};
+    bool dropped = false;
+    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nw) {
+        const uint2 it = s.wo_items[i];
+        const uint32_t d = g.dst_ident ? it.x : g.dst_id[it.x];
+        const uint32_t end = (uint32_t)g.dst_off[it.x + 1u];
+        const uint32_t hi = end - it.y > SSSP_WO_PIECE ? it.y + SSSP_WO_PIECE : end;
+        const uint32_t before = s.dist32[d];
+        uint32_t dist = before;
+        for (uint32_t p = it.y; p < hi; p += 128u) { /* it.y is a multiple of 4 */
+            const uint32_t q = p + 4u * (uint32_t)lane;
+            WoStep r{0xFFFFFFFFu, false};
+            if (q < hi)
+                r = sssp_wo_step(g, s, filter, q, it.y, hi, dist, edges);
+            dropped = dropped || r.dropped;
+            dist = __reduce_min_sync(FULL, dist);
+            if (__shfl_sync(FULL, r.last, 31) >= dist)
+                break; /* the step's largest weight; past the end: none */
+        }
+        if (lane == 0 && dist < before && dist < atomicMin(&s.dist32[d], dist)) {
+            atomicMin(&s.prop64[d], (unsigned long long)dist);
+            const uint32_t b = 1u << (d & 31u);
+            const uint32_t o = atomicOr(&nxt[d >> 5], b);
+            occ += o == 0u ? 1u : 0u;
+            if (!(o & b)) {
+                const uint32_t od = g.outdeg[d];
+                mass += od;
+                ++act;
+                const uint32_t bk = degree_bucket(od);
+#pragma unroll
+                for (uint32_t j = 0; j < 3u; ++j)
+                    deg[j] += bk == j ? 1u : 0u;
+            }
+        }
+    }
+    if (dropped) {
+        atomicOr(&c->narrow_ovf, 1u);
+        atomicOr(&c->ovf_redo, 1u);
+    }
+    sssp_wo_counters(block_cnt, mass, edges, 0u, act, occ, deg);
 }
 
 // The per-destination work of a dense pull, one destination per lane, launched
@@ -2358,7 +2641,7 @@ __device__ __forceinline__ void log_iteration(DevState& s, Ctrl* c, const unsign
     c->tiles_scanned += cnt[CNT_TILES];
     c->dsts_scanned += cnt[CNT_DSTS];
     c->activated += cnt[CNT_ACT];
-    c->pull_launches += pull_launches_of((int)s.app);
+    c->pull_launches += s.wo ? SSSP_WO_LAUNCHES : pull_launches_of((int)s.app);
     if (c->iter < LOG_CAP) {
         IterRec& r = s.log[c->iter];
         r.mass_in = c->last_mass;
@@ -3769,12 +4052,13 @@ static uint64_t knob_value(const wedge_graph* h, int k)
         e = getenv("WEDGE_PROBE_EDGES");
         break;
     case WEDGE_KNOB_SSSP_TILE: {
-        // default: 512-edge tiles from 2^23 in-edges; below, the extra launches of
-        // the 512-edge pull (two instantiations and a finish per launch) cost more
-        // than its faster tiles save (batched workload, scales 12-20: 181 against
-        // 156 ms one query at a time)
+        // default: the weight-ordered pulls on every graph that has them (R-MAT
+        // scale 18: 0.55 ms per SSSP against 0.59 ms in 256-edge tiles, scale
+        // 22: 1.40 against 2.10, scale 26: 4.76 against 21.7); else 512-edge
+        // tiles from 2^23 in-edges: below, the extra launches of the 512-edge
+        // pull cost more than its faster tiles save
         const char* t = getenv("WEDGE_SSSP_TILES512");
-        return (t && t[0] == '0') ? 256u : (t && t[0] == '1') ? 512u : h->g.E >= (1ull << 23) ? 512u : 256u;
+        return (t && t[0] == '0') ? 256u : (t && t[0] == '1') ? 512u : (h->g.wsrc || h->g.E >= (1ull << 23)) ? 512u : 256u;
     }
     case WEDGE_KNOB_SSSP_NARROW:
         e = getenv("WEDGE_SSSP_NARROW");
@@ -3789,20 +4073,29 @@ static uint64_t knob_value(const wedge_graph* h, int k)
     return (end && *end == '\0' && knob_ok(k, v)) ? v : defaults[k];
 }
 
-// SSSP runs sssp_pull_kernel (512-edge tiles) where the knob asks for it and
-// the graph has byte-wide weights and in-edge positions, else pull_kernel
+// SSSP pulls the weight-ordered in-edges (sssp_wo_kernel) where the graph has
+// them, the distances have a 32-bit copy and the tile knob does not ask for
+// the 256-edge tiles
+static bool sssp_wo(const wedge_graph* h)
+{
+    return h->s.push && h->g.wsrc && knob_value(h, WEDGE_KNOB_SSSP_NARROW) != 0u &&
+           knob_value(h, WEDGE_KNOB_SSSP_TILE) == 512u;
+}
+
+// else sssp_pull_kernel (512-edge tiles) where the knob asks for it and the
+// graph has byte-wide weights and in-edge positions, else pull_kernel
 // (256-edge tiles; 20.6 against 23.2 ms per SSSP at R-MAT scale 26 with
 // 64-bit distance gathers)
 static bool sssp_tiles512(const wedge_graph* h)
 {
-    return h->s.push && h->g.w8 && knob_value(h, WEDGE_KNOB_SSSP_TILE) == 512u;
+    return h->s.push && h->g.w8 && !sssp_wo(h) && knob_value(h, WEDGE_KNOB_SSSP_TILE) == 512u;
 }
 static uint32_t sssp_split_grid(wedge_graph* h);
 
 static const void* pull_fn(const wedge_graph* h, int app)
 {
     if (app == WEDGE_APP_SSSP && sssp_tiles512(h))
-        return (const void*)sssp_pull_kernel<false>;
+        return (const void*)sssp_pull_kernel;
     switch (app) {
     case WEDGE_APP_BFS:
         return (const void*)pull_kernel<WEDGE_APP_BFS, PullEpl<WEDGE_APP_BFS>::value>;
@@ -3841,22 +4134,16 @@ static uint32_t pull_tile_e(const wedge_graph* h, int app)
 static int setup_hub(wedge_graph* h, int app, int precision)
 {
     const void* fn = pull_fn(h, app);
-    /* the 512-edge SSSP pull runs as two instantiations with one shared-memory layout */
-    const void* fn2 = (app == WEDGE_APP_SSSP && sssp_tiles512(h)) ? (const void*)sssp_pull_kernel<true> : nullptr;
     cudaFuncAttributes fa;
     WEDGE_CHECK(cudaFuncGetAttributes(&fa, fn));
-    if (fn2) {
-        cudaFuncAttributes fb;
-        WEDGE_CHECK(cudaFuncGetAttributes(&fb, fn2));
-        fa.sharedSizeBytes = fa.sharedSizeBytes > fb.sharedSizeBytes ? fa.sharedSizeBytes : fb.sharedSizeBytes;
-    }
     int optin = 0;
     WEDGE_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
     const uint64_t elem = (app == WEDGE_APP_SSSP) ? (h->s.dist32 ? 4 : 8)
                           : (app == WEDGE_APP_PR && precision != WEDGE_PREC_FP32C) ? 8 : 4;
     const uint64_t stage = (app == WEDGE_APP_SSSP && sssp_tiles512(h)) ? SSSP_STAGE_BYTES : 0u; /* after the cache */
     uint64_t avail = (uint64_t)optin > fa.sharedSizeBytes + stage + 64u ? (uint64_t)optin - fa.sharedSizeBytes - stage - 64u : 0u;
-    const uint64_t want = knob_value(h, WEDGE_KNOB_HUB_BYTES);
+    /* the weight-ordered SSSP pulls gather through L1; the 64-bit pulls after an overflow use no cache */
+    const uint64_t want = (app == WEDGE_APP_SSSP && sssp_wo(h)) ? 0u : knob_value(h, WEDGE_KNOB_HUB_BYTES);
     if (want < avail)
         avail = want;
     const uint64_t have = (app == WEDGE_APP_BFS) ? (h->g.V + 31) / 32 : h->g.V;
@@ -3871,8 +4158,6 @@ static int setup_hub(wedge_graph* h, int app, int precision)
     h->s.hub_bytes = h->hub_bytes;
     h->pull_smem = h->hub_bytes + (uint32_t)stage;
     WEDGE_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->pull_smem));
-    if (fn2)
-        WEDGE_CHECK(cudaFuncSetAttribute(fn2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->pull_smem));
     if (two_phase_app(app) && n) {
         uint32_t* d = (uint32_t*)(h->s.block_part + h->pull_grid); /* counters: scratch until the first pull */
         hub_split_kernel<<<1, 1, 0, h->stream>>>(h->g, (uint32_t)n, pull_tile_e(h, app), d);
@@ -4093,9 +4378,13 @@ static int ensure_state(wedge_graph* h, int app, int precision)
             if (g.weight_kind != WEDGE_WEIGHTS_F64 && nk && (rc = dalloc(h, &s.dist32, V, true)))
                 return rc;
             s.narrow_lim = nk > 1u ? (uint32_t)nk : NONE32; /* a limit below 2^32-1 tests the switch to 64 bits */
-            s.narrow_sums = g.shard ? 0u : 1u;
             if (sssp_tiles512(h) && (rc = sssp_split_state(h)))
                 return rc;
+            if (sssp_wo(h)) {
+                s.wo = 1u;
+                if ((rc = dalloc(h, &s.wo_items, g.E / (SSSP_WO_WINDOW + 1u) + g.E / SSSP_WO_PIECE + 2, true)))
+                    return rc;
+            }
         } else if ((rc = dalloc(h, &s.prop32, V, true))) {
             return rc;
         }
@@ -4139,6 +4428,8 @@ static unsigned long long* counters(wedge_graph* h) { return (unsigned long long
 // counter slots the pulls of one iteration fill (two launches for CC/SSSP)
 static uint32_t pull_slots(wedge_graph* h, int app)
 {
+    if (app == WEDGE_APP_SSSP && h->s.wo)
+        return h->pull_grid + 2u * h->dst_grid;
     return h->dst_grid * dst_launches_of(app) + h->pull_grid * (pull_launches_of(app) - dst_launches_of(app));
 }
 
@@ -4160,15 +4451,16 @@ static void launch_pull_app(wedge_graph* h)
             cnt += (uint64_t)NCNT * dgrid;
         }
     }
-    if (APP == WEDGE_APP_SSSP && sssp_tiles512(h)) {
+    if (APP == WEDGE_APP_SSSP && h->s.wo) {
+        pull_kernel<APP, EPL><<<grid, PULL_THREADS, h->hub_bytes, h->stream>>>(h->g, h->s, cnt, PHASE_ALL);
+        cnt += (uint64_t)NCNT * grid;
+        sssp_wo_kernel<<<h->dst_grid, PULL_THREADS, 0, h->stream>>>(h->g, h->s, cnt);
+        sssp_wo_long_kernel<<<h->dst_grid, PULL_THREADS, 0, h->stream>>>(h->g, h->s, cnt + (uint64_t)NCNT * h->dst_grid);
+    } else if (APP == WEDGE_APP_SSSP && sssp_tiles512(h)) {
         const uint32_t sgrid = sssp_split_grid(h);
-        sssp_pull_kernel<false><<<grid, PULL_THREADS, h->pull_smem, h->stream>>>(h->g, h->s, cnt, PHASE_HUBS);
-        sssp_pull_kernel<true><<<grid, PULL_THREADS, h->pull_smem, h->stream>>>(h->g, h->s, cnt, PHASE_HUBS);
+        sssp_pull_kernel<<<grid, PULL_THREADS, h->pull_smem, h->stream>>>(h->g, h->s, cnt, PHASE_HUBS);
         sssp_split_kernel<<<sgrid, AUX_THREADS, 0, h->stream>>>(h->g, h->s, cnt, grid, PHASE_HUBS);
-        sssp_pull_kernel<false><<<grid, PULL_THREADS, h->pull_smem, h->stream>>>(h->g, h->s, cnt + NCNT * grid,
-                                                                                 PHASE_REST);
-        sssp_pull_kernel<true><<<grid, PULL_THREADS, h->pull_smem, h->stream>>>(h->g, h->s, cnt + NCNT * grid,
-                                                                                PHASE_REST);
+        sssp_pull_kernel<<<grid, PULL_THREADS, h->pull_smem, h->stream>>>(h->g, h->s, cnt + NCNT * grid, PHASE_REST);
         sssp_split_kernel<<<sgrid, AUX_THREADS, 0, h->stream>>>(h->g, h->s, cnt + NCNT * grid, grid, PHASE_REST);
     } else if (two_phase_app(APP)) {
         pull_kernel<APP, EPL><<<grid, PULL_THREADS, h->hub_bytes, h->stream>>>(h->g, h->s, cnt, PHASE_HUBS);
@@ -4207,9 +4499,9 @@ static uint64_t build_launches(const wedge_graph* h)
 
 static uint64_t iteration_launches(const wedge_graph* h, int app)
 {
-    /* decide, the build, the pull (the 512-edge SSSP pull: two instantiations per launch and a
-       split-destination finish after each) */
-    const uint64_t pulls = pull_launches_of(app) * ((app == WEDGE_APP_SSSP && sssp_tiles512(h)) ? 3ull : 1ull);
+    /* decide, the build, the pull (the 512-edge SSSP pull: a split-destination finish after each launch) */
+    const uint64_t pulls = (app == WEDGE_APP_SSSP && h->s.wo) ? SSSP_WO_LAUNCHES
+                           : pull_launches_of(app) * ((app == WEDGE_APP_SSSP && sssp_tiles512(h)) ? 2ull : 1ull);
     return 1ull + build_launches(h) + pulls;
 }
 

@@ -3,7 +3,10 @@
 // Device layout of a loaded graph (all resident in HBM):
 //   src[Epad]      uint32 in-edge sources, grouped by destination in file order,
 //                  padded to a multiple of TILE with NONE32
-//   w[Epad]        64-bit weight words (SSSP only; uint64 or IEEE double)
+//   w[Epad]        64-bit weight words (SSSP only; uint64 or IEEE double), or
+//   w8[Epad]       one byte each where every uint64 weight is below 256; then also
+//   wsrc[Epad], ww8[Epad]  sources and weights once more, each destination's by
+//                  ascending weight (the SSSP dense pulls)
 //   dst_id[Vne]    vertex id of compressed destination k (only vertices with
 //                  in-degree > 0 are listed, ascending)
 //   dst_off[Vne+1] first edge of compressed destination k
@@ -84,7 +87,7 @@ struct Ctrl {
     unsigned long long dsts_scanned;   // destinations in visited tiles
     unsigned long long activated;      // vertices activated by pulls
     unsigned int items;                // Wedge-build work items appended by the last pull
-    unsigned int need_n;               // tiles the probe listed for the dense tile pull (tile_list)
+    unsigned int need_n;               // tiles the probe listed for the dense tile pull (tile_list); SSSP: wo_items
     unsigned int cand_n;               // BFS: candidate destinations the last Wedge build listed
     unsigned int tiles;                // length of the Wedge tile list
     unsigned int mode;                 // MODE_DENSE / MODE_WEDGE for the next pull
@@ -127,6 +130,8 @@ struct DevGraph {
     const uint32_t* src;
     const unsigned long long* w;
     const uint8_t* w8;         // the same weights in one byte each, when every weight is a uint64 below 256
+    const uint32_t* wsrc;      // [Epad] with byte-wide weights: every destination's sources by ascending weight
+    const uint8_t* ww8;        // [Epad] and those weights (dst_off holds for both orders); or null
     const uint32_t* dst_id;
     const unsigned long long* dst_off;
     const uint32_t* tile_dst0;
@@ -150,7 +155,8 @@ struct DevState {
                                    // unreached or not below the limit), the array the pulls gather while
                                    // Ctrl::narrow_ovf is 0; or null
     uint32_t narrow_lim;           // distances the 32-bit copy holds: below this (2^32-1, or a smaller test limit)
-    uint32_t narrow_sums;          // the 512-edge SSSP pull may sum in 32 bits (not on shards: see ovf_redo)
+    uint32_t wo;                   // SSSP dense pulls run over the weight-ordered in-edges (sssp_wo_kernel)
+    uint2* wo_items;               // (compressed destination, first in-edge) left to sssp_wo_long_kernel
     double* rank;                  // PageRank FP64: rank / outdegree'
     double* acc;                   // PageRank accumulators (graph_vertex_accumulators)
     double* inv_od;                // PageRank 1 / outdegree' (outdegree, or N for dangling vertices)
@@ -235,7 +241,7 @@ struct wedge_graph {
     uint32_t pull_smem;                // dynamic shared memory of the tile pulls (hub cache + staged minima)
     float* net;                        // device copy of the scheduler network (wedge_cuda_set_scheduler)
     // allocations owned by the handle
-    void* allocs[32];
+    void* allocs[40];
     int nallocs;
     void* state_allocs[32];
     int nstate;
