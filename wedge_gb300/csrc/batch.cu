@@ -5,8 +5,8 @@
 //   build   Wedge frontier of the queries whose next pull is sparse: the
 //           out-edge chunks of the vertices the last pull activated are
 //           marked (wedge.c:63-155), and newly marked chunks are appended to
-//           the query's chunk list -- or, on graphs whose CSRI holds in-edge
-//           positions, every activated vertex's out-list becomes PIECE-entry
+//           the query's chunk list -- or, on graphs whose CSRI holds
+//           destinations, every activated vertex's out-list becomes PIECE-entry
 //           items whose in-edges the pull relaxes one by one (as the single-
 //           query engine's SSSP Wedge pulls); the previous frontier bitmaps
 //           are cleared
@@ -43,18 +43,18 @@ struct BGraph {
     const uint32_t* dst_id;
     const unsigned long long* dst_off;
     const uint32_t* chunk_dst0;  // [nchunks+1] compressed destination owning edge 32*c (Vne past the end)
-    const uint32_t* dst_start;   // destination-start bitmap and 128-edge tile index of the graph handle
-    const uint32_t* tile_dst0;
+    const uint32_t* dst_start;   // destination-start bitmap of the graph handle
     const uint8_t* w8;           // byte-wide weights, or null
     const uint32_t* outdeg;
     const unsigned long long* csri_off;
     const uint32_t* csri;
-    uint32_t csri_shift;  // chunk of a CSRI entry: entry >> csri_shift (5: positions, 0: chunk ids)
+    const uint8_t* cw8;          // out-edge weights (push): byte-wide, or
+    const unsigned long long* cw; // 64-bit words
     const uint32_t* new2old;
     const uint32_t* old2new;
     uint64_t V, E;
     uint32_t Vne, nchunks, weight_kind;
-    uint32_t push;               // sparse pulls relax in-edge positions (CSRI of positions)
+    uint32_t push;               // sparse pulls relax out-edges (CSRI of destinations)
 };
 
 struct BQuery {
@@ -64,7 +64,7 @@ struct BQuery {
     uint32_t* list[2];        // [V] the same vertices as lists
     uint32_t* chunk_bits;     // [nchunks/32+1] Wedge frontier
     uint32_t* chunk_list;     // [nchunks] its marked chunks
-    uint2* vitems;            // [V + E/PIECE + 1] (vertex, piece) items of a sparse pull over in-edge positions
+    uint2* vitems;            // [V + E/PIECE + 1] (vertex, piece) items of a sparse pull over out-edges
 };
 
 struct BCtl {
@@ -176,7 +176,7 @@ __device__ void phase_build(const BArgs& a)
             start = G.csri_off[v];
             len = G.csri_off[v + 1] - start;
         }
-        // sparse pulls over in-edge positions: PIECE-entry items of each out-list
+        // sparse pulls over out-edges: PIECE-entry items of each out-list
         if (valid && a.graphs[a.q[q].graph].push) {
             const uint32_t np = (uint32_t)((len + PIECE - 1) / PIECE);
             if (np) {
@@ -190,7 +190,7 @@ __device__ void phase_build(const BArgs& a)
         if (valid && len <= a.split) {
             const BGraph& G = a.graphs[a.q[q].graph];
             for (unsigned long long j = 0; j < len; ++j)
-                mark_batch_chunk(a.q[q], a.ctl[q], G.csri[start + j] >> G.csri_shift);
+                mark_batch_chunk(a.q[q], a.ctl[q], G.csri[start + j]);
         }
         // long lists: the whole warp, one list at a time
         uint32_t longs = __ballot_sync(FULL, valid && len > a.split && !a.graphs[a.q[q].graph].push);
@@ -201,7 +201,7 @@ __device__ void phase_build(const BArgs& a)
             const unsigned long long ls = __shfl_sync(FULL, start, l), ll = __shfl_sync(FULL, len, l);
             const BGraph& G = a.graphs[a.q[lq].graph];
             for (unsigned long long j = lane; j < ll; j += 32)
-                mark_batch_chunk(a.q[lq], a.ctl[lq], G.csri[ls + j] >> G.csri_shift);
+                mark_batch_chunk(a.q[lq], a.ctl[lq], G.csri[ls + j]);
         }
     }
     // clear the previous frontier bits (their list is exact)
@@ -404,7 +404,7 @@ __device__ void pull_tile(const BArgs& a, uint32_t q, uint32_t t, unsigned long 
     }
 }
 
-// A sparse pull over in-edge positions: the in-edges of one PIECE of an
+// A sparse pull over out-edges: the in-edges of one PIECE of an
 // activated vertex's out-list are relaxed by the warp's lanes (BFS: an
 // unvisited destination takes the vertex as its parent; SSSP: min-plus)
 __device__ void push_piece(const BArgs& a, uint32_t q, uint2 it, unsigned long long& mass)
@@ -429,13 +429,12 @@ __device__ void push_piece(const BArgs& a, uint32_t q, uint2 it, unsigned long l
     const unsigned long long du = qq.prop[it.x];
     const bool f64 = G.weight_kind == WEDGE_WEIGHTS_F64;
     for (unsigned long long j = lo + (unsigned long long)lane; j < hi; j += 32u) {
-        const uint32_t p = G.csri[j];
-        const uint32_t vtx = G.dst_id[dst_of_pos(G.dst_start, G.tile_dst0, p)];
+        const uint32_t vtx = G.csri[j];
         if (qq.app == WEDGE_APP_BFS) {
             if (qq.prop[vtx] == NONE64 && atomicCAS(&qq.prop[vtx], NONE64, (unsigned long long)it.x) == NONE64)
                 activate(vtx);
         } else {
-            const unsigned long long wt = G.w8 ? (unsigned long long)G.w8[p] : G.w[p];
+            const unsigned long long wt = G.cw8 ? (unsigned long long)G.cw8[j] : G.cw[j];
             const unsigned long long nd =
                 f64 ? (unsigned long long)__double_as_longlong(
                           __dadd_rn(__longlong_as_double((long long)du), __longlong_as_double((long long)wt)))
@@ -759,10 +758,10 @@ extern "C" int wedge_cuda_batch_create(wedge_graph_t* const* graphs, uint32_t nu
         G.outdeg = g.outdeg;
         G.csri_off = g.csri_off;
         G.csri = g.csri;
-        G.csri_shift = g.csri_pos ? 5u : 0u;
-        G.push = g.csri_pos ? 1u : 0u;
+        G.cw8 = g.cw8;
+        G.cw = g.cw;
+        G.push = g.csr;
         G.dst_start = g.dst_start;
-        G.tile_dst0 = g.tile_dst0;
         G.w8 = g.w8;
         G.new2old = g.new2old;
         G.old2new = g.old2new;

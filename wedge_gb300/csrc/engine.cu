@@ -164,13 +164,13 @@ static uint32_t grid_for(uint64_t work, uint32_t threads, uint32_t cap)
 
 /* ================================================================= build */
 
-__global__ void validate_kernel(const uint32_t* src, const uint32_t* dst, uint64_t E, uint64_t V, int* err)
+__global__ void validate_kernel(const uint32_t* src, const uint32_t* dst, uint64_t E, uint64_t V, bool grouped, int* err)
 {
     for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t d = dst[e];
         if (src[e] >= V || d >= V)
             atomicOr(err, 1);
-        if (e > 0 && dst[e - 1] > d)
+        if (grouped && e > 0 && dst[e - 1] > d)
             atomicOr(err, 2);
     }
 }
@@ -217,15 +217,13 @@ __global__ void widen_kernel(const uint32_t* in, unsigned long long* out, uint64
         out[i] = in[i];
 }
 
-// CSRI fill (graphdata.c:535-569), grouped by source: the in-edge position of
-// every out-edge (its chunk is position / 32), or, on graphs whose padded
-// in-edges do not fit 32 bits, its chunk id
-__global__ void csri_fill_kernel(const uint32_t* src, uint64_t E, unsigned long long* cursor, uint32_t* csri,
-                                 uint32_t positions)
+// CSRI fill (graphdata.c:535-569) of graphs whose padded in-edges do not fit 32
+// bits, grouped by source: the 32-edge chunk of every out-edge
+__global__ void csri_fill_kernel(const uint32_t* src, uint64_t E, unsigned long long* cursor, uint32_t* csri)
 {
     for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x) {
         const unsigned long long pos = atomicAdd(&cursor[src[e]], 1ull);
-        csri[pos] = (uint32_t)(positions ? e : e / CHUNK);
+        csri[pos] = (uint32_t)(e / CHUNK);
     }
 }
 
@@ -265,12 +263,31 @@ __global__ void dst_index_kernel(const uint32_t* dst_id, uint32_t Vne, uint32_t*
         inv[dst_id[k]] = k;
 }
 
+// A graph whose in-lists and out-lists are the same arrays holds every edge's
+// reverse as often as the edge: symmetric, without a search (R-MAT scale 24,
+// symmetrised: 77 ms of searches at load).  *differ is set where they are not.
+__global__ void list_compare_kernel(const uint32_t* in_src, const uint32_t* out_dst, const unsigned long long* in_off,
+                                    const unsigned long long* out_off, const uint32_t* dst_id, uint32_t Vne, uint64_t E,
+                                    unsigned int* differ)
+{
+    bool bad = false;
+    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x)
+        bad = bad || in_src[e] != out_dst[e];
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < Vne; k += gridDim.x * blockDim.x)
+        bad = bad || in_off[k] != out_off[dst_id[k]] || in_off[k + 1u] != out_off[dst_id[k] + 1u];
+    if (bad)
+        atomicOr(differ, 1u);
+}
+
 // Symmetry: the reverse of every edge s -> d is an edge, i.e. d is among the
 // in-neighbours of s (ascending within a destination: a binary search).  Sets
-// *asym at the first edge without its reverse; the others then stop early.
+// asym[0] at the first edge without its reverse; the others then stop early.
+// asym[1]: the searches are needed.
 __global__ void sym_check_kernel(const uint32_t* src, const uint32_t* dst, uint64_t E, const uint32_t* inv,
                                  const unsigned long long* dst_off, unsigned int* asym)
 {
+    if (asym[1] == 0u)
+        return; /* list_compare_kernel found the lists alike */
     uint32_t n = 0;
     for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x) {
         if ((++n & 63u) == 0u && *(volatile unsigned int*)asym)
@@ -394,6 +411,16 @@ __global__ void weight_key_kernel(unsigned long long* key, uint64_t E, int vbits
     }
 }
 
+// out-edges from keys sorted by source: the destination above `shift` bits, the weight byte at `wshift`
+__global__ void csr_unpack_kernel(const unsigned long long* key, uint64_t E, int shift, int wshift, uint32_t* nbr, uint8_t* w8)
+{
+    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x) {
+        nbr[e] = (uint32_t)(key[e] >> shift);
+        if (w8)
+            w8[e] = (uint8_t)(key[e] >> wshift);
+    }
+}
+
 // the sorted destination | weight | source keys, and the padding past the last in-edge
 __global__ void weight_unpack_kernel(const unsigned long long* key, uint64_t E, uint64_t Epad, int vbits, uint32_t* wsrc,
                                      uint8_t* ww8)
@@ -405,6 +432,21 @@ __global__ void weight_unpack_kernel(const unsigned long long* key, uint64_t E, 
     }
 }
 
+__global__ void permute_degrees_kernel(const uint32_t* global_outdeg, const uint32_t* new2old, uint64_t V, uint32_t* outdeg)
+{
+    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x)
+        outdeg[v] = global_outdeg[new2old[v]];
+}
+
+// The CSRI holds every out-edge's destination; on graphs beyond 2^32 padded
+// in-edges its 32-edge chunk, the unit their Wedge frontiers mark
+// (WEDGE_CSRI_CHUNKS=1 selects that form on any graph)
+static bool csri_chunks(uint64_t Epad)
+{
+    const char* force = getenv("WEDGE_CSRI_CHUNKS");
+    return Epad >= (1ull << 32) || (force && force[0] == '1');
+}
+
 // Degree relabelling: vertices are renumbered by descending out-degree (ties
 // by id), so the sources gathered most often are the lowest ids and share cache
 // lines; edges are renumbered and re-sorted by (destination, source).  The
@@ -414,13 +456,18 @@ __global__ void weight_unpack_kernel(const unsigned long long* key, uint64_t E, 
 // the 64-bit weights as a payload), and the same keys, sorted once more by
 // (destination, weight), give the in-edges a second time, each destination's
 // by ascending weight (*wsrc, *ww8: 5 bytes per in-edge; null where the device
-// has no room for them, and on shards).
+// has no room for them, and on shards).  A last sort by source gives the
+// out-edges: every source's destinations (*csri) and weights (*cw8 or *cw);
+// with radix passes over the source bits alone that is 3-4 passes, where
+// filling them through atomic cursors took as long as nine (R-MAT scale 24).
 static int relabel_by_degree(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_src, uint32_t* d_dst,
                              unsigned long long* d_w, bool byte_weights, uint32_t** new2old, uint32_t** old2new,
-                             uint8_t** w8, uint32_t** wsrc, uint8_t** ww8, const uint32_t* global_outdeg)
+                             uint8_t** w8, uint32_t** wsrc, uint8_t** ww8, uint32_t** csri, uint8_t** cw8,
+                             unsigned long long** cw, uint32_t* outdeg, const uint32_t* global_outdeg)
 {
-    *w8 = *ww8 = nullptr;
-    *wsrc = nullptr;
+    *w8 = *ww8 = *cw8 = nullptr;
+    *wsrc = *csri = nullptr;
+    *cw = nullptr;
     cudaStream_t st = h->stream;
     const uint32_t cap = (uint32_t)h->num_sms * 16u;
     int rc;
@@ -449,6 +496,7 @@ static int relabel_by_degree(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d
         cudaFreeAsync(tmp, st);
         permutation_kernel<<<grid_for(V, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(db.Current(), V, *new2old, *old2new);
     }
+    permute_degrees_kernel<<<grid_for(V, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(deg, *new2old, V, outdeg);
     cudaFreeAsync(deg, st);
     cudaFreeAsync(vk, st);
     cudaFreeAsync(vk2, st);
@@ -502,6 +550,29 @@ static int relabel_by_degree(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d
             *ww8 = nullptr;
         }
     }
+    if (!csri_chunks(Epad)) {
+        if ((rc = dalloc(h, csri, E)) || (in_key && (rc = dalloc(h, cw8, E))) || (d_w && !in_key && (rc = dalloc(h, cw, E))))
+            return rc;
+        /* the keys hold the source in bits [0, vbits) after the weight order, else above the weight byte */
+        const int s0 = (in_key && !*wsrc) ? 8 : 0;
+        const int shift = in_key ? vbits + 8 : vbits;
+        const int wshift = *wsrc ? vbits : 0;
+        if (d_w && !in_key) {
+            WEDGE_CHECK(cudaMemcpyAsync(*cw, d_w, E * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, st));
+            cub::DoubleBuffer<unsigned long long> vb(*cw, w2);
+            WEDGE_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, tb, kb, vb, (long long)E, s0, s0 + vbits, st));
+            WEDGE_CHECK(cudaMallocAsync(&tmp, tb ? tb : 1, st));
+            WEDGE_CHECK(cub::DeviceRadixSort::SortPairs(tmp, tb, kb, vb, (long long)E, s0, s0 + vbits, st));
+            if (vb.Current() != *cw)
+                WEDGE_CHECK(cudaMemcpyAsync(*cw, vb.Current(), E * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, st));
+        } else {
+            WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(nullptr, tb, kb, (long long)E, s0, s0 + vbits, st));
+            WEDGE_CHECK(cudaMallocAsync(&tmp, tb ? tb : 1, st));
+            WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tb, kb, (long long)E, s0, s0 + vbits, st));
+        }
+        cudaFreeAsync(tmp, st);
+        csr_unpack_kernel<<<grid, AUX_THREADS, 0, st>>>(kb.Current(), E, shift, wshift, *csri, *cw8);
+    }
     cudaFreeAsync(ek, st);
     cudaFreeAsync(ek2, st);
     if (w2)
@@ -510,21 +581,15 @@ static int relabel_by_degree(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d
     return WEDGE_OK;
 }
 
-// Builds the device CSC from destination-sorted device edge arrays.  d_src and
-// d_w (if any) must hold roundup(E, TILE) entries and become owned by the
-// handle; d_dst is consumed and freed.
-__global__ void permute_degrees_kernel(const uint32_t* global_outdeg, const uint32_t* new2old, uint64_t V, uint32_t* outdeg)
-{
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x)
-        outdeg[v] = global_outdeg[new2old[v]];
-}
-
-// Builds the device CSC.  A shard (d_global_outdeg given: the whole graph's
+// Builds the device CSC from device edge arrays, grouped by ascending
+// destination (checked) unless `grouped` is false.  d_src and d_w (if any) must
+// hold roundup(E, TILE) entries and become owned by the handle; d_dst is
+// consumed and freed.  A shard (d_global_outdeg given: the whole graph's
 // out-degrees, caller numbering) numbers vertices by those degrees, so all
 // shards share one numbering, and keeps them as its out-degrees (the changed
 // mass and PageRank's divisor), while its CSRI indexes its own in-edges.
 int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_src, uint32_t* d_dst,
-                            unsigned long long* d_w, int weight_kind, const uint32_t* d_global_outdeg)
+                            unsigned long long* d_w, int weight_kind, const uint32_t* d_global_outdeg, bool grouped)
 {
     cudaStream_t st = h->stream;
     DevGraph& g = h->g;
@@ -544,7 +609,8 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
     WEDGE_CHECK(cudaMallocAsync((void**)&d_chk, sizeof(chk), st));
     WEDGE_CHECK(cudaMemsetAsync(d_chk, 0, sizeof(chk), st));
     if (E)
-        validate_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, d_dst, E, V, (int*)d_chk);
+        validate_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, d_dst, E, V, grouped,
+                                                                                 (int*)d_chk);
     if (E && d_w && weight_kind == WEDGE_WEIGHTS_U64)
         max_weight_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_w, E, d_chk + 1);
     WEDGE_CHECK(cudaMemcpyAsync(chk, d_chk, sizeof(chk), cudaMemcpyDeviceToHost, st));
@@ -557,13 +623,20 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
         cudaFreeAsync(d_dst, st);
         return WEDGE_ERR_FORMAT;
     }
+    uint32_t *outdeg = nullptr, *csri = nullptr;
     {
         uint32_t *n2o = nullptr, *o2n = nullptr;
-        uint8_t *w8 = nullptr, *ww8 = nullptr;
+        uint8_t *w8 = nullptr, *ww8 = nullptr, *cw8 = nullptr;
         uint32_t* wsrc = nullptr;
-        int rc = relabel_by_degree(h, V, E, d_src, d_dst, d_w, byte_weights, &n2o, &o2n, &w8, &wsrc, &ww8, d_global_outdeg);
+        unsigned long long* cw = nullptr;
+        int rc = dalloc(h, &outdeg, V);
+        if (!rc)
+            rc = relabel_by_degree(h, V, E, d_src, d_dst, d_w, byte_weights, &n2o, &o2n, &w8, &wsrc, &ww8, &csri, &cw8, &cw,
+                                   outdeg, d_global_outdeg);
         if (rc)
             return rc;
+        g.cw8 = cw8;
+        g.cw = cw;
         g.new2old = n2o;
         g.old2new = o2n;
         if (w8) { /* the 64-bit words are not read any more */
@@ -595,56 +668,63 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
         WEDGE_CHECK(cudaStreamSynchronize(st));
     }
     g.Vne = Vne;
-    uint32_t *dst_id, *tile_dst0, *outdeg, *csri;
+    uint32_t *dst_id, *tile_dst0;
     unsigned long long *dst_off, *csri_off;
+    const bool chunks = csri_chunks(g.Epad);
     int rc;
     if ((rc = dalloc(h, &dst_id, Vne)) || (rc = dalloc(h, &dst_off, (uint64_t)Vne + 1)) ||
-        (rc = dalloc(h, &tile_dst0, (uint64_t)g.T + 1)) || (rc = dalloc(h, &outdeg, V)) ||
-        (rc = dalloc(h, &csri_off, V + 1)) || (rc = dalloc(h, &csri, E)))
+        (rc = dalloc(h, &tile_dst0, (uint64_t)g.T + 1)) || (rc = dalloc(h, &csri_off, V + 1)) ||
+        ((chunks || !csri) && (rc = dalloc(h, &csri, E))))
         return rc;
     if (E) {
         compress_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_dst, kidx, E, dst_id, dst_off);
     }
     tile_index_kernel<<<grid_for((uint64_t)g.T + 1, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(kidx, E, g.T, Vne,
                                                                                                tile_dst0, dst_off);
-    // symmetry (CC's label space)
-    unsigned int h_asym = 1u;
-    if (E) {
-        uint32_t* inv = nullptr;
-        unsigned int* d_asym = nullptr;
-        WEDGE_CHECK(cudaMallocAsync((void**)&inv, V * sizeof(uint32_t), st));
-        WEDGE_CHECK(cudaMallocAsync((void**)&d_asym, sizeof(unsigned int), st));
-        WEDGE_CHECK(cudaMemsetAsync(d_asym, 0, sizeof(unsigned int), st));
-        WEDGE_CHECK(cudaMemsetAsync(inv, 0xFF, V * sizeof(uint32_t), st));
-        dst_index_kernel<<<grid_for(Vne, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(dst_id, Vne, inv);
-        sym_check_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, d_dst, E, inv, dst_off, d_asym);
-        WEDGE_CHECK(cudaMemcpyAsync(&h_asym, d_asym, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
-        cudaFreeAsync(d_asym, st);
-        cudaFreeAsync(inv, st);
-    }
     cudaFreeAsync(kidx, st);
-    cudaFreeAsync(d_dst, st);
 
-    // out-degrees and CSRI: in-edge positions where they fit 32 bits
-    // (WEDGE_CSRI_CHUNKS=1 selects chunk ids on any graph: the encoding, and
-    // the chunk Wedge pulls, of graphs beyond 2^32 padded in-edges)
-    const char* force_chunks = getenv("WEDGE_CSRI_CHUNKS");
-    const uint32_t csri_pos = (g.Epad < (1ull << 32) && !(force_chunks && force_chunks[0] == '1')) ? 1u : 0u;
-    WEDGE_CHECK(cudaMemsetAsync(outdeg, 0, V * sizeof(uint32_t), st));
-    if (E)
-        outdeg_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, E, outdeg);
+    // CSRI offsets: the out-degrees' prefix sums (a shard's CSRI indexes its own in-edges)
+    uint32_t* own = outdeg;
+    if (d_global_outdeg) {
+        WEDGE_CHECK(cudaMallocAsync((void**)&own, V * sizeof(uint32_t), st));
+        WEDGE_CHECK(cudaMemsetAsync(own, 0, V * sizeof(uint32_t), st));
+        if (E)
+            outdeg_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, E, own);
+    }
     unsigned long long* wide = nullptr;
     WEDGE_CHECK(cudaMallocAsync((void**)&wide, (V + 1) * sizeof(unsigned long long), st));
-    widen_kernel<<<grid_for(V, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(outdeg, wide, V);
+    widen_kernel<<<grid_for(V, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(own, wide, V);
     WEDGE_CHECK(cudaMemsetAsync(wide + V, 0, sizeof(unsigned long long), st));
     if ((rc = device_scan(h, wide, csri_off, V + 1, false)))
         return rc;
-    WEDGE_CHECK(cudaMemcpyAsync(wide, csri_off, (V + 1) * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, st));
-    if (E)
-        csri_fill_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, E, wide, csri, csri_pos);
+    if (chunks && E) {
+        WEDGE_CHECK(cudaMemcpyAsync(wide, csri_off, (V + 1) * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, st));
+        csri_fill_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, E, wide, csri);
+    }
     cudaFreeAsync(wide, st);
-    if (d_global_outdeg) /* the shard's own counts built the CSRI; the graph's degrees from here on */
-        permute_degrees_kernel<<<grid_for(V, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_global_outdeg, g.new2old, V, outdeg);
+    if (own != outdeg)
+        cudaFreeAsync(own, st);
+
+    // symmetry (CC's label space); inv stays: a vertex's compressed destination
+    unsigned int h_asym = 1u;
+    uint32_t* inv = nullptr;
+    if (E) {
+        unsigned int* d_asym = nullptr; /* [0] an edge without its reverse, [1] the searches are needed */
+        if ((rc = dalloc(h, &inv, V)))
+            return rc;
+        WEDGE_CHECK(cudaMallocAsync((void**)&d_asym, 2 * sizeof(unsigned int), st));
+        WEDGE_CHECK(cudaMemsetAsync(d_asym, 0, sizeof(unsigned int), st));
+        WEDGE_CHECK(cudaMemsetAsync(d_asym + 1, chunks ? 0xFF : 0, sizeof(unsigned int), st));
+        WEDGE_CHECK(cudaMemsetAsync(inv, 0xFF, V * sizeof(uint32_t), st));
+        dst_index_kernel<<<grid_for(Vne, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(dst_id, Vne, inv);
+        if (!chunks)
+            list_compare_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, csri, dst_off, csri_off, dst_id,
+                                                                                     Vne, E, d_asym + 1);
+        sym_check_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, d_dst, E, inv, dst_off, d_asym);
+        WEDGE_CHECK(cudaMemcpyAsync(&h_asym, d_asym, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
+        cudaFreeAsync(d_asym, st);
+    }
+    cudaFreeAsync(d_dst, st);
 
     // destination starts, one bit per in-edge (the pulls' tile geometry)
     uint32_t* dst_start = nullptr;
@@ -688,7 +768,12 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
     g.outdeg = outdeg;
     g.csri_off = csri_off;
     g.csri = csri;
-    g.csri_pos = csri_pos;
+    g.csr = chunks ? 0u : 1u;
+    g.dst_index = g.dst_ident ? nullptr : inv;
+    if (g.dst_ident && inv) {
+        untrack(h, inv);
+        cudaFree(inv);
+    }
     g.split_k = split_k;
     g.split_t0 = split_t0;
     g.split_t1 = split_t1;
@@ -946,15 +1031,18 @@ __device__ __forceinline__ bool sssp_wo_runs(const DevState& s, const Ctrl* c)
     return s.wo && c->mode != MODE_WEDGE && !c->narrow_ovf;
 }
 
-// The Wedge pull of SSSP over in-edge positions: every vertex the last pull
+// The Wedge pull of SSSP over the out-edges: every vertex the last pull
 // activated relaxes exactly the in-edges its out-edges are (the CSRI holds
-// their positions), where the chunk form pulls the whole 32-edge chunks
-// holding them (phase_edge_pull_sssp.c:171-306 over the chunks
-// wedge_generate_frontier marks).  Both reach the same fixed point, the least
-// dist[d] = min over in-edges of dist[s] + w, by monotone relaxations; only
-// the iteration counts may differ.  Vertices with at most BIG_LIST out-edges
-// take a thread each; expand_kernel split the longer lists into PIECE-entry
-// items, which take a warp each.  block_cnt as pull_kernel's.
+// their destinations, cw8 or cw their weights, both read in order), where the
+// chunk form pulls the whole 32-edge chunks holding them
+// (phase_edge_pull_sssp.c:171-306 over the chunks wedge_generate_frontier
+// marks).  Both reach the same fixed point, the least dist[d] = min over
+// in-edges of dist[s] + w, by monotone relaxations; only the iteration counts
+// may differ.  Vertices with at most BIG_LIST out-edges take a thread each;
+// expand_kernel split the longer lists into PIECE-entry items, which take a
+// warp each.  While the 32-bit copy is exact a sum below its limit is compared
+// with and lowered in the copy (half the bytes of the one random access an
+// out-edge needs).  block_cnt as pull_kernel's.
 __device__ __forceinline__ void sssp_push_pull(const DevGraph& g, const DevState& s, const Ctrl* c,
                                                unsigned long long* block_cnt)
 {
@@ -968,16 +1056,24 @@ __device__ __forceinline__ void sssp_push_pull(const DevGraph& g, const DevState
     if (threadIdx.x < 3)
         sh_pdeg[threadIdx.x] = 0u;
     __syncthreads();
-    auto relax = [&](unsigned long long du, uint32_t pos) {
-        const unsigned long long wv = g.w8 ? (unsigned long long)g.w8[pos] : g.w[pos];
+    const bool narrow = s.dist32 && !c->narrow_ovf;
+    auto relax = [&](unsigned long long du, uint32_t vtx, unsigned long long wv) {
         const unsigned long long nd =
             f64 ? (unsigned long long)__double_as_longlong(__dadd_rn(__longlong_as_double((long long)du),
                                                                      __longlong_as_double((long long)wv)))
                 : du + wv; /* phase_edge_pull_sssp.c:136-137; an activated source is reached */
-        const uint32_t k = dst_of_pos(g, pos);
-        const uint32_t vtx = g.dst_ident ? k : g.dst_id[k];
-        if (nd < s.prop64[vtx] && nd < atomicMin(&s.prop64[vtx], nd)) {
-            dist32_put(s, vtx, nd, false);
+        bool lower;
+        if (narrow && nd < (unsigned long long)s.narrow_lim) {
+            const uint32_t n32 = (uint32_t)nd;
+            lower = n32 < s.dist32[vtx] && n32 < atomicMin(&s.dist32[vtx], n32);
+            if (lower)
+                atomicMin(&s.prop64[vtx], nd);
+        } else {
+            lower = nd < s.prop64[vtx] && nd < atomicMin(&s.prop64[vtx], nd);
+            if (lower)
+                dist32_put(s, vtx, nd, false);
+        }
+        if (lower) {
             const uint32_t b = 1u << (vtx & 31u);
             const uint32_t o = atomicOr(&nxt[vtx >> 5], b);
             occ += o == 0u ? 1u : 0u;
@@ -991,6 +1087,7 @@ __device__ __forceinline__ void sssp_push_pull(const DevGraph& g, const DevState
             }
         }
     };
+    auto weight = [&](unsigned long long j) -> unsigned long long { return g.cw8 ? (unsigned long long)g.cw8[j] : g.cw[j]; };
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t nthr = gridDim.x * blockDim.x;
     const uint32_t n = c->alist_n;
@@ -1000,14 +1097,14 @@ __device__ __forceinline__ void sssp_push_pull(const DevGraph& g, const DevState
         if (len > BIG_LIST)
             continue; /* an item of expand_kernel's */
         const unsigned long long du = s.prop64[u];
-        uint32_t pos[BIG_LIST];
+        uint32_t to[BIG_LIST];
 #pragma unroll
         for (uint32_t j = 0; j < BIG_LIST; ++j)
-            pos[j] = (j < len) ? g.csri[lo + j] : 0u;
+            to[j] = (j < len) ? g.csri[lo + j] : 0u;
 #pragma unroll
         for (uint32_t j = 0; j < BIG_LIST; ++j)
             if (j < len)
-                relax(du, pos[j]);
+                relax(du, to[j], weight(lo + j));
         edges += len;
     }
     const uint32_t ni = c->items;
@@ -1018,7 +1115,7 @@ __device__ __forceinline__ void sssp_push_pull(const DevGraph& g, const DevState
         const unsigned long long hi = (lo + PIECE < end) ? lo + PIECE : end;
         const unsigned long long du = s.prop64[it.x];
         for (unsigned long long j = lo + (unsigned long long)lane; j < hi; j += 32u) {
-            relax(du, g.csri[j]);
+            relax(du, g.csri[j], weight(j));
             ++edges;
         }
     }
@@ -1450,7 +1547,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
 }
 
 // SSSP dense and source-filtered pulls over 512-edge tiles, for graphs with
-// byte-wide weights and in-edge positions in the CSRI but without the
+// byte-wide weights and destinations in the CSRI but without the
 // weight-ordered in-edges of sssp_wo_kernel (shards), whose Wedge pulls relax
 // the activated sources' in-edges (sssp_push_pull).  Lane l loads its 16
 // sources (two 256-bit loads) and 16 weight bytes (one 128-bit load), gathers
@@ -2162,6 +2259,8 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
     // destinations are consecutive, so most of their tiles share a word: one
     // atomic per distinct word.  Called by all lanes.
     auto mark_open = [&](uint32_t ta, uint32_t tb) {
+        if (!s.tile_open)
+            return;
         const bool one = ta <= tb && (ta >> 5) == (tb >> 5);
         if (ta <= tb && !one)
             mark_tiles(s.tile_open, ta, tb);
@@ -2739,9 +2838,6 @@ __global__ void decide_kernel(DevGraph g, DevState s, const unsigned long long* 
     }
 }
 
-// chunk of a CSRI entry (an in-edge position, or a chunk id on graphs too large for 32-bit positions)
-__device__ __forceinline__ uint32_t csri_chunk(const DevGraph& g, uint32_t x) { return g.csri_pos ? x / CHUNK : x; }
-
 // chunks per pull tile of an application, as a shift (tile = 32 * EPL in-edges)
 __device__ __forceinline__ uint32_t chunk_tile_shift(uint32_t app)
 {
@@ -2750,20 +2846,16 @@ __device__ __forceinline__ uint32_t chunk_tile_shift(uint32_t app)
 }
 
 
-// Wedge build over in-edge positions (BFS, CC): the destination of in-edge
-// pos, if unfinished (BFS unvisited, CC label not 0), becomes a candidate of
-// the next pull, listed once (its cand bit).
+// Wedge build over out-edges (BFS, CC): the destination d of one, if unfinished
+// (BFS unvisited, CC label not 0), becomes a candidate of the next pull, listed
+// once (its cand bit).
 // Warp-collective: every lane calls it, with valid false where it has no edge.
-__device__ __forceinline__ void add_candidate(const DevGraph& g, const DevState& s, uint32_t pos, bool valid)
+__device__ __forceinline__ void add_candidate(const DevGraph& g, const DevState& s, uint32_t d, bool valid)
 {
     uint32_t k = 0;
     bool add = false;
-    if (valid && s.tile_open) { /* a closed tile has no unfinished destination */
-        const uint32_t t = pos >> (5u + chunk_tile_shift(s.app));
-        valid = (s.tile_open[t >> 5] >> (t & 31u)) & 1u;
-    }
     if (valid) {
-        k = dst_of_pos(g, pos);
+        k = g.dst_ident ? d : g.dst_index[d];
         const uint32_t b = 1u << (k & 31u);
         if (!(s.vis_c[k >> 5] & b) && !(s.cand[k >> 5] & b))
             add = !(atomicOr(&s.cand[k >> 5], b) & b);
@@ -2821,7 +2913,7 @@ __device__ __forceinline__ void advance_body(const DevGraph& g, const DevState& 
         const uint64_t twords = (uint64_t)g.T / 32 + 2;
         for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < twords; i += (uint64_t)gridDim.x * blockDim.x) {
             s.tile_need[i] = 0u;
-            if (dense)
+            if (dense && s.tile_open)
                 s.tile_open[i] = 0u;
         }
     }
@@ -2899,7 +2991,7 @@ __global__ void expand_kernel(DevGraph g, DevState s)
                 len = 0;
             }
             if (s.push)
-                len = 0; /* SSSP over in-edge positions: the pull relaxes the short lists itself */
+                len = 0; /* SSSP over out-edges: the pull relaxes the short lists itself */
         }
         // a short list's entries are loaded together, then marked
         uint32_t ch[BIG_LIST];
@@ -2913,7 +3005,7 @@ __global__ void expand_kernel(DevGraph g, DevState s)
         } else {
 #pragma unroll
             for (uint32_t j = 0; j < BIG_LIST; ++j)
-                mark_chunk(s, csri_chunk(g, ch[j]), j < len);
+                mark_chunk(s, ch[j], j < len);
         }
         uint32_t incl = np;
 #pragma unroll
@@ -2937,7 +3029,7 @@ __global__ void expand_kernel(DevGraph g, DevState s)
 __global__ void wedge_build_kernel(DevGraph g, DevState s)
 {
     Ctrl* c = s.ctrl;
-    if (c->done || c->mode != MODE_WEDGE || s.push) /* SSSP over in-edge positions: the pull takes the items */
+    if (c->done || c->mode != MODE_WEDGE || s.push) /* SSSP over out-edges: the pull takes the items */
         return;
     const int lane = threadIdx.x & 31;
     const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -2955,7 +3047,7 @@ __global__ void wedge_build_kernel(DevGraph g, DevState s)
             if (s.cand)
                 add_candidate(g, s, x, valid);
             else
-                mark_chunk(s, csri_chunk(g, x), valid);
+                mark_chunk(s, x, valid);
         }
     }
 }
@@ -2972,7 +3064,7 @@ __global__ void compact_kernel(DevGraph g, DevState s)
     constexpr uint32_t TPW = 32 / EPL;
     constexpr uint32_t MASK = (EPL >= 32) ? FULL : ((1u << EPL) - 1u);
     Ctrl* c = s.ctrl;
-    if (c->done || c->mode != MODE_WEDGE || s.cand || s.push) /* over in-edge positions: no tiles */
+    if (c->done || c->mode != MODE_WEDGE || s.cand || s.push) /* over out-edges: no tiles */
         return;
     const int lane = threadIdx.x & 31;
     const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -4083,7 +4175,7 @@ static bool sssp_wo(const wedge_graph* h)
 }
 
 // else sssp_pull_kernel (512-edge tiles) where the knob asks for it and the
-// graph has byte-wide weights and in-edge positions, else pull_kernel
+// graph has byte-wide weights and a CSRI of destinations, else pull_kernel
 // (256-edge tiles; 20.6 against 23.2 ms per SSSP at R-MAT scale 26 with
 // 64-bit distance gathers)
 static bool sssp_tiles512(const wedge_graph* h)
@@ -4355,7 +4447,7 @@ static int ensure_state(wedge_graph* h, int app, int precision)
     s.block_part = bp; /* [grid] doubles, then the counters */
     WEDGE_CHECK(cudaMemset(bp, 0, sizeof(double) * (grid + slots * NCNT)));
     s.app = (uint32_t)app;
-    s.push = (app == WEDGE_APP_SSSP && g.csri_pos) ? 1u : 0u;
+    s.push = (app == WEDGE_APP_SSSP && g.csr) ? 1u : 0u;
     s.probe_edges = (uint32_t)knob_value(h, WEDGE_KNOB_PROBE_EDGES);
     if (app == WEDGE_APP_PR && precision == WEDGE_PREC_FP32C) {
         if ((rc = pr32_state(h)))
@@ -4402,7 +4494,7 @@ static int ensure_state(wedge_graph* h, int app, int precision)
             if ((rc = dalloc(h, &s.cc_best, V, true)))
                 return rc;
         }
-        if (app == WEDGE_APP_BFS || app == WEDGE_APP_CC) {
+        if ((app == WEDGE_APP_BFS || app == WEDGE_APP_CC) && !g.csr) { /* chunk frontiers leave out closed tiles */
             if ((rc = dalloc(h, &s.tile_open, (uint64_t)g.T / 32 + 2, true)))
                 return rc;
         }
@@ -4410,7 +4502,7 @@ static int ensure_state(wedge_graph* h, int app, int precision)
             if ((rc = dalloc(h, &s.tile_need, (uint64_t)g.T / 32 + 2, true)))
                 return rc;
         }
-        if ((app == WEDGE_APP_BFS || app == WEDGE_APP_CC) && g.csri_pos) { /* Wedge pulls over candidate destinations */
+        if ((app == WEDGE_APP_BFS || app == WEDGE_APP_CC) && g.csr) { /* Wedge pulls over candidate destinations */
             if ((rc = dalloc(h, &s.cand, (uint64_t)g.Vne / 32 + 2, true)) ||
                 (rc = dalloc(h, &s.cand_list, (uint64_t)g.Vne + 1, true)))
                 return rc;
@@ -4491,7 +4583,7 @@ static void launch_pull(wedge_graph* h, int app)
 
 // kernels one iteration launches: the pull(s) and the five of the tail
 // the Wedge build's launches: collect, expand, build (not for SSSP over
-// in-edge positions), compact (chunk frontiers only)
+// out-edges), compact (chunk frontiers only)
 static uint64_t build_launches(const wedge_graph* h)
 {
     return 2ull + (h->s.push ? 0ull : 1ull) + ((h->s.cand || h->s.push) ? 0ull : 1ull);
@@ -4549,9 +4641,9 @@ static void launch_wedge_build(wedge_graph* h, const DevGraph& g, int app)
 {
     collect_kernel<<<aux_grid(h, (g.V + 31) / 32), AUX_THREADS, 0, h->stream>>>(g, h->s, (uint32_t)app);
     expand_kernel<<<h->build_grid, AUX_THREADS, 0, h->stream>>>(g, h->s);
-    if (!h->s.push) /* SSSP over in-edge positions: the pull takes expand_kernel's items */
+    if (!h->s.push) /* SSSP over out-edges: the pull takes expand_kernel's items */
         wedge_build_kernel<<<h->build_grid, AUX_THREADS, 0, h->stream>>>(g, h->s);
-    if (!h->s.cand && !h->s.push) /* over in-edge positions the build lists candidates or items, not tiles */
+    if (!h->s.cand && !h->s.push) /* over out-edges the build lists candidates or items, not tiles */
         launch_compact(h, app);
 }
 

@@ -14,9 +14,10 @@
 //   tile_dst0[T+1] compressed destination owning edge 128*t (Vne where that
 //                  edge is padding); pull tiles of 32*EPL edges index it with a stride
 //   outdeg[V]      out-degree (graphdata.c:430-490)
-//   csri_off[V+1], csri[E]  for every source, the in-edge position of each of
-//                  its out-edges (its Wedge chunk of 32 in-edges = position / 32;
-//                  chunk ids where Epad >= 2^32): the CSRI of graphdata.c:493-585
+//   csri_off[V+1], csri[E]  for every source, the destination of each of its
+//                  out-edges, by ascending id (the Wedge chunk of 32 in-edges that
+//                  holds it where Epad >= 2^32): the CSRI of graphdata.c:493-585;
+//                  cw8[E] or cw[E] the out-edges' weights
 // A tile (128 consecutive in-edges) is the unit of work of one warp; a chunk
 // (32 in-edges, one 128-byte line of sources) is the unit the Wedge frontier
 // marks, i.e. the GPU form of the reference's frontier element of 4 edge
@@ -125,7 +126,7 @@ struct DevGraph {
     uint32_t dst_ident;        // dst_id[k] == k for every k (the vertices with in-edges are [0, Vne))
     uint32_t nwide;            // destinations spanning more than SPLIT_SERIAL tile boundaries (back of the split lists)
     uint32_t sym;              // every edge's reverse is an edge too: CC propagates engine ids (see cc_best_kernel)
-    uint32_t csri_pos;         // csri holds in-edge positions (Epad < 2^32), else chunk ids
+    uint32_t csr;              // csri holds destinations (Epad < 2^32), else chunk ids
     uint32_t shard;            // a destination-range shard (wedge_cuda_load_shard)
     const uint32_t* src;
     const unsigned long long* w;
@@ -139,6 +140,9 @@ struct DevGraph {
     const uint32_t* outdeg;
     const unsigned long long* csri_off;
     const uint32_t* csri;
+    const uint8_t* cw8;        // [E] with csr: the out-edges' weights, in one byte each beside w8, or
+    const unsigned long long* cw; // [E] 64-bit words beside w; null without weights
+    const uint32_t* dst_index; // [V] compressed destination of a vertex (NONE32: no in-edges); null where dst_ident
     const uint32_t* split_k;   // compressed destinations whose in-edges span tiles ([T]: nsplit short
                                // ones from the front, nwide long ones from the back)
     const uint32_t* split_t0;  // their first tile
@@ -208,7 +212,7 @@ struct DevState {
     uint32_t hub_tile;             // CC/SSSP: first tile whose destinations all have ids >= hub_n
     uint32_t hub_k;                // CC/SSSP: compressed destinations with ids < hub_n
     const float* net;              // scheduler network blob (WEDGE_SCHED_LEARNED), or null
-    uint32_t push;                 // SSSP over in-edge positions: Wedge pulls relax the activated sources' out-edges
+    uint32_t push;                 // SSSP over out-edges: Wedge pulls relax the activated sources' out-edges
     uint32_t probe_edges;          // default BFS/CC probe window
 };
 
@@ -262,7 +266,8 @@ struct wedge_graph {
 namespace wedge {
 // implemented in engine.cu, used by loaders in graph.cu
 int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_src, uint32_t* d_dst,
-                            unsigned long long* d_w, int weight_kind, const uint32_t* d_global_outdeg = nullptr);
+                            unsigned long long* d_w, int weight_kind, const uint32_t* d_global_outdeg = nullptr,
+                            bool grouped = true);
 int new_handle(wedge_graph** out);
 void free_handle(wedge_graph* h);
 int track(wedge_graph* h, void* p);

@@ -252,19 +252,12 @@ static uint32_t bits_for(uint64_t V)
     return b;
 }
 
-// sorts the (dst, src) keys, unpacks them into edge arrays and builds the CSC
+// unpacks the (dst, src) keys into edge arrays and builds the CSC (whose
+// relabelling sorts them: the generator's order does not matter)
 static int build_from_keys(wedge_graph* h, uint64_t V, uint64_t E, unsigned long long* keys, uint32_t sbits,
                            int weight_kind)
 {
     cudaStream_t st = h->stream;
-    unsigned long long* alt = nullptr;
-    WEDGE_CHECK(cudaMalloc((void**)&alt, (E ? E : 1) * sizeof(unsigned long long)));
-    cub::DoubleBuffer<unsigned long long> db(keys, alt);
-    size_t tb = 0;
-    WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(nullptr, tb, db, (long long)E, 0, (int)(2 * sbits), st));
-    void* tmp = nullptr;
-    WEDGE_CHECK(cudaMalloc(&tmp, tb ? tb : 1));
-    WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tb, db, (long long)E, 0, (int)(2 * sbits), st));
     uint32_t *d_src, *d_dst;
     unsigned long long* d_w;
     int rc = alloc_edges(E, weight_kind != WEDGE_WEIGHTS_NONE, &d_src, &d_dst, &d_w);
@@ -273,14 +266,11 @@ static int build_from_keys(wedge_graph* h, uint64_t V, uint64_t E, unsigned long
     if ((rc = track(h, d_src)) || (d_w && (rc = track(h, d_w))))
         return rc;
     if (E)
-        unpack_keys_kernel<<<grid_of(E, h->num_sms), 256, 0, st>>>(db.Current(), E, sbits, weight_kind, d_src, d_dst,
-                                                                     d_w);
+        unpack_keys_kernel<<<grid_of(E, h->num_sms), 256, 0, st>>>(keys, E, sbits, weight_kind, d_src, d_dst, d_w);
     WEDGE_CHECK(cudaStreamSynchronize(st));
-    cudaFree(tmp);
-    cudaFree(alt);
     cudaFree(keys);
     WEDGE_CHECK(cudaGetLastError());
-    return build_from_device_edges(h, V, E, d_src, d_dst, d_w, weight_kind);
+    return build_from_device_edges(h, V, E, d_src, d_dst, d_w, weight_kind, nullptr, false);
 }
 
 }  // namespace wedge
