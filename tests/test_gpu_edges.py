@@ -52,3 +52,83 @@ def test_weight_ordered_pull(engine_lib, n, weights):
             for sched in (W.SCHED_DENSE, W.SCHED_FILTERED, W.SCHED_PLAIN):
                 g.run(W.APP_SSSP, W.Params(sched=sched, flags=W.FLAG_GRAPH))
                 assert np.array_equal(g.read_results(), expect), (limit, sched)
+
+
+def fan_in_out(n, seed):
+    """0 -> n vertices -> n + 1 -> n vertices again, each with a few random edges:
+    out-lists of n destinations, and vertices of one"""
+    rng = np.random.default_rng(seed)
+    V = 2 * n + 3
+    first, hub, second = np.arange(1, n + 1), n + 1, np.arange(n + 2, 2 * n + 2)
+    s = [np.zeros(n, np.int64), first, np.full(n, hub), rng.integers(0, V - 1, 2 * n)]
+    d = [first, np.full(n, hub), second, rng.integers(0, V - 1, 2 * n)]
+    s, d = np.concatenate(s), np.concatenate(d)
+    order = np.lexsort((s, d))
+    s, d = s[order].astype(np.uint32), d[order].astype(np.uint32)
+    return V, s, d, rng.integers(0, 256, len(s)).astype(np.uint64)
+
+
+def least_labels(V, src, dst):
+    x = np.arange(V)
+    while True:
+        y = x.copy()
+        np.minimum.at(y, dst, x[src])
+        if np.array_equal(x, y):
+            return x.astype(np.float64)
+        x = y
+
+
+def check_traversals(W, V, s, d, w, scheds, flags_list):
+    import helpers
+
+    levels = helpers.bfs_levels(V, s, d, 0)
+    labels = least_labels(V, s.astype(np.int64), d.astype(np.int64))
+    dist = bellman_ford(V, s, d, w, 0)
+    fw = (w.astype(np.float64) + 0.25).view(np.uint64)
+    with W.Graph.from_edges(V, s, d, w) as g, W.Graph.from_edges(V, s, d, fw, W.WEIGHTS_F64) as gf:
+        fdist = None
+        parents = None
+        for sched in scheds:
+            for flags in flags_list:
+                p = W.Params(sched=sched, flags=flags)
+                g.run(W.APP_BFS, p)
+                got = g.read_results()
+                helpers.check_bfs(got, V, s, d, 0, levels)
+                assert parents is None or np.array_equal(got, parents), "parents differ between schedules"
+                parents = got
+                g.run(W.APP_CC, p)
+                assert np.array_equal(g.read_results().view(np.float64), labels)
+                g.run(W.APP_SSSP, p)
+                assert np.array_equal(g.read_results(), dist)
+                gf.run(W.APP_SSSP, p)
+                got = gf.read_results()
+                assert fdist is None or np.array_equal(got, fdist), "FP64 distances differ between schedules"
+                fdist = got
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 63, 127, 128, 129, 255, 257, 1023, 5000])
+def test_out_lists_of_the_loop(engine_lib, n):
+    """out-lists around what a warp takes at once (32 vertices, 128 out-edges), the
+    whole traversal in one launch, iteration by iteration and host-driven"""
+    W = engine_lib
+    V, s, d, w = fan_in_out(n, n)
+    check_traversals(W, V, s, d, w, (W.SCHED_PLAIN, W.SCHED_DENSE, W.SCHED_WEDGE, W.SCHED_FILTERED),
+                     (0, W.FLAG_GRAPH, W.FLAG_TIMING))
+
+
+@pytest.mark.parametrize("edges", [(1 << 20) - 513, 1 << 20, (1 << 20) + 1, (1 << 20) + 700])
+def test_largest_whole_traversal(engine_lib, edges):
+    """graphs around the size up to which a traversal is one launch; past it the dense
+    iterations take their own launches"""
+    W = engine_lib
+    rng = np.random.default_rng(edges)
+    V = 70_001
+    # a short-diameter core and a long tail of vertices, so that every strategy runs
+    core = rng.integers(0, 4000, (2, edges - 20_000))
+    tail = np.arange(4000, 24_000)
+    s = np.concatenate([core[0], np.where(tail % 50 == 0, tail % 4000, tail - 1)])
+    d = np.concatenate([core[1], tail])
+    order = np.lexsort((s, d))
+    s, d = s[order].astype(np.uint32), d[order].astype(np.uint32)
+    w = rng.integers(0, 256, len(s)).astype(np.uint64)
+    check_traversals(W, V, s, d, w, (W.SCHED_PLAIN, W.SCHED_FILTERED), (0, W.FLAG_GRAPH, W.FLAG_TIMING))

@@ -801,15 +801,15 @@ __device__ __forceinline__ double warp_sum_f64(double x)
 
 __device__ __forceinline__ const uint32_t* cur_front(const DevState& s, uint32_t parity)
 {
-    return parity ? s.front1 : s.front0;
+    return s.front + parity * s.front_stride;
 }
 
-// pull output bitmap: the other half of the double buffer.  The pull reads the
+// pull output bitmap: the next of the three in turn.  The pull reads the
 // vertices the previous pull activated (BFS frontier; CC/SSSP changed
 // vertices, read by the source-filtered pull) and writes the ones it activates.
 __device__ __forceinline__ uint32_t* next_front(const DevState& s, uint32_t parity)
 {
-    return parity ? s.front0 : s.front1;
+    return s.front + (parity == 2u ? 0u : parity + 1u) * s.front_stride;
 }
 
 // in-edges per lane of each application's pull (tile = 32 * EPL in-edges)
@@ -2674,8 +2674,8 @@ __device__ __forceinline__ uint32_t choose_mode(uint32_t sched, unsigned long lo
 // reduced counters) and the traversal so far.  Every feature is O(1) in size.
 // Single-precision arithmetic: one thread computes them after every pull, and
 // the FP64 units of this GPU are slow.
-__device__ void sched_features(const DevGraph& g, const Ctrl* c, uint32_t app, const unsigned long long (&cnt)[NCNT],
-                               float* f)
+__device__ void sched_features(const DevGraph& g, unsigned long long activated, uint32_t iter, uint32_t app,
+                               const unsigned long long (&cnt)[NCNT], float* f)
 {
     const float V = (float)(g.V ? g.V : 1), E = (float)(g.E ? g.E : 1);
     const float m = (float)cnt[CNT_MASS], act = (float)cnt[CNT_ACT];
@@ -2694,8 +2694,8 @@ __device__ void sched_features(const DevGraph& g, const Ctrl* c, uint32_t app, c
     f[6] = b1 / a;
     f[7] = b2 / a;
     f[8] = (act - b0 - b1 - b2) / a;
-    f[9] = (float)c->activated / V;         // activated so far (BFS: visited fraction)
-    f[10] = log2f(1.0f + (float)c->iter) / 8.0f;
+    f[9] = (float)activated / V;         // activated so far (BFS: visited fraction)
+    f[10] = log2f(1.0f + (float)iter) / 8.0f;
     f[11] = log2f(E) / 40.0f;
     f[12] = app == WEDGE_APP_BFS ? 1.0f : 0.0f;
     f[13] = app == WEDGE_APP_CC ? 1.0f : 0.0f;
@@ -2703,9 +2703,7 @@ __device__ void sched_features(const DevGraph& g, const Ctrl* c, uint32_t app, c
     f[15] = log2f(E / V) / 8.0f;            // average degree
 }
 
-// After a pull: reduce the block counters, count the iteration, stop when no
-// edge was activated (execution_bfs.c:239-251) or at the cap, choose the next
-// pull (execution_bfs.c:141, execution_cc.c:103).
+// the sum of a pull's per-block counters (one block, all threads)
 __device__ __forceinline__ void reduce_counters(const unsigned long long* block_cnt, uint32_t nblocks,
                                                 unsigned long long (&out)[NCNT])
 {
@@ -2734,13 +2732,14 @@ __device__ __forceinline__ void reduce_counters(const unsigned long long* block_
     }
 }
 
-__device__ __forceinline__ void log_iteration(DevState& s, Ctrl* c, const unsigned long long (&cnt)[NCNT])
+__device__ __forceinline__ void log_iteration(DevState& s, Ctrl* c, const unsigned long long (&cnt)[NCNT],
+                                              uint32_t pull_launches)
 {
     c->edges_scanned += cnt[CNT_EDGES];
     c->tiles_scanned += cnt[CNT_TILES];
     c->dsts_scanned += cnt[CNT_DSTS];
     c->activated += cnt[CNT_ACT];
-    c->pull_launches += s.wo ? SSSP_WO_LAUNCHES : pull_launches_of((int)s.app);
+    c->pull_launches += pull_launches;
     if (c->iter < LOG_CAP) {
         IterRec& r = s.log[c->iter];
         r.mass_in = c->last_mass;
@@ -2755,66 +2754,51 @@ __device__ __forceinline__ void log_iteration(DevState& s, Ctrl* c, const unsign
     c->iter += 1u;
 }
 
-// After a pull: reduce the block counters, count the iteration, stop when no
-// edge was activated (execution_bfs.c:239-251) or at the cap, choose the next
-// pull (execution_bfs.c:141, execution_cc.c:103).
-__global__ void decide_kernel(DevGraph g, DevState s, const unsigned long long* block_cnt, uint32_t nblocks, uint32_t app)
+// the counters of sparse_loop_kernel, before its next launch
+__device__ __forceinline__ void loop_reset(Ctrl* c)
 {
-    Ctrl* c = s.ctrl;
-    if (c->done)
-        return;
-    const uint32_t nsum = ((g.T + TILES_PER_REGION - 1) / TILES_PER_REGION + 31) / 32;
-    for (uint32_t i = threadIdx.x; i < nsum; i += blockDim.x)
-        s.summary[i] = 0u; /* the pull has cleared every chunk word it walked */
-    unsigned long long cnt[NCNT];
-    reduce_counters(block_cnt, nblocks, cnt);
-    __shared__ float feat[NF], xs[NF], h1[NH], h2[NH], pred[NO];
-    __shared__ uint32_t go;
-    if (threadIdx.x == 0) {
-        const unsigned long long m = cnt[CNT_MASS];
-        if (c->mode == MODE_WEDGE)
-            c->wedge_iters += 1u;
-        log_iteration(s, c, cnt);
-        c->last_mass = m;
-        c->mass = m;
-        c->parity ^= 1u;
-        c->need_n = 0u;
-        c->cand_n = 0u;
-        c->tiles = 0u;
-        c->items = 0u;
-        c->alist_n = 0u;
-        go = 0u;
-        // SSSP: a pull dropped 32-bit sums that reached the copy's limit; the
-        // next pull is dense and 64-bit, and relaxes every in-edge again
-        const bool redo = c->ovf_redo != 0u;
-        c->ovf_redo = 0u;
-        if (m == 0ull && !redo) {
-            c->done = 1u;
-            c->loop = 0u;
-        } else if (c->iter >= c->max_iter) {
-            c->done = 1u;
-            c->not_converged = 1u;
-            c->loop = 0u;
-        } else {
-            c->mode = choose_mode(c->sched, m, c->threshold);
-            if (c->sched == WEDGE_SCHED_PROBE && c->iter == c->probe_iter)
-                c->mode = c->probe_mode;
-            sched_features(g, c, app, cnt, feat);
-            if (c->iter < LOG_CAP) {
-                for (int i = 0; i < NF; ++i)
-                    s.log[c->iter].feat[i] = feat[i];
-                s.log[c->iter].learned = 0u;
-            }
-            go = (c->sched == WEDGE_SCHED_LEARNED && s.net) ? 1u : 0u;
-            if (redo) {
-                c->mode = MODE_DENSE;
-                go = 0u;
-            }
-        }
+    c->bar = 0u;
+    for (int i = 0; i < 3; ++i) {
+        c->ln[i] = 0u;
+        c->li[i] = 0u;
+        for (uint32_t j = 0; j < NCNT; ++j)
+            c->lacc[i][j] = 0ull;
     }
-    __syncthreads();
-    if (!go)
-        return;
+}
+
+__global__ void loop_reset_kernel(DevState s)
+{
+    loop_reset(s.ctrl);
+}
+
+// what follows a pull that changed `mass` out-edges
+struct NextPull {
+    bool done, capped;
+    uint32_t mode;
+};
+
+__device__ __forceinline__ NextPull next_pull(uint32_t sched, unsigned long long mass, bool redo, uint32_t iter,
+                                              uint32_t max_iter, unsigned long long thr, uint32_t probe_iter,
+                                              uint32_t probe_mode)
+{
+    NextPull n{false, false, MODE_DENSE};
+    if (mass == 0ull && !redo) {
+        n.done = true;
+    } else if (iter >= max_iter) {
+        n.done = n.capped = true;
+    } else if (!redo) {
+        n.mode = choose_mode(sched, mass, thr);
+        if (sched == WEDGE_SCHED_PROBE && iter == probe_iter)
+            n.mode = probe_mode;
+    }
+    return n;
+}
+
+// The scheduler network's choice in place of the plain one in Ctrl::mode, for
+// the next iteration's features `feat` in shared memory (one block, all threads)
+__device__ __forceinline__ void ask_network(DevState& s, Ctrl* c, uint32_t app, const float* feat)
+{
+    __shared__ float xs[NF], h1[NH], h2[NH], pred[NO];
     // the scheduler network: predicted log2 cost of each strategy
     sched_forward_block(s.net, feat, xs, h1, h2, pred);
     if (threadIdx.x == 0) {
@@ -2835,6 +2819,94 @@ __global__ void decide_kernel(DevGraph g, DevState s, const unsigned long long* 
             if (c->iter < LOG_CAP)
                 s.log[c->iter].learned = 1u;
         }
+    }
+}
+
+// the same with the features from the iteration's log record, or none past the log's end
+__device__ __forceinline__ void ask_network(DevState& s, Ctrl* c, uint32_t app, uint32_t iter)
+{
+    __shared__ float feat[NF];
+    if (iter >= LOG_CAP)
+        return; /* the plain rule */
+    __syncthreads();
+    if (threadIdx.x < NF)
+        feat[threadIdx.x] = s.log[iter].feat[threadIdx.x];
+    __syncthreads();
+    ask_network(s, c, app, feat);
+}
+
+// The control block after a pull whose reduced counters are cnt (one block, all
+// threads): the iteration's record, convergence and the next pull.
+__device__ __forceinline__ void decide_block(const DevGraph& g, DevState& s, Ctrl* c, uint32_t app,
+                                             const unsigned long long (&cnt)[NCNT], uint32_t pull_launches)
+{
+    __shared__ float feat[NF];
+    __shared__ uint32_t go;
+    if (threadIdx.x == 0) {
+        const unsigned long long m = cnt[CNT_MASS];
+        if (c->mode == MODE_WEDGE)
+            c->wedge_iters += 1u;
+        log_iteration(s, c, cnt, pull_launches);
+        c->last_mass = m;
+        c->mass = m;
+        c->parity = c->parity == 2u ? 0u : c->parity + 1u;
+        c->need_n = 0u;
+        c->cand_n = 0u;
+        c->tiles = 0u;
+        c->items = 0u;
+        c->alist_n = 0u;
+        go = 0u;
+        // SSSP: a pull dropped 32-bit sums that reached the copy's limit; the
+        // next pull is dense and 64-bit, and relaxes every in-edge again
+        const bool redo = c->ovf_redo != 0u;
+        c->ovf_redo = 0u;
+        const NextPull n = next_pull(c->sched, m, redo, c->iter, c->max_iter, c->threshold, c->probe_iter, c->probe_mode);
+        if (n.done) {
+            c->done = 1u;
+            c->not_converged = n.capped ? 1u : 0u;
+            c->loop = 0u;
+        } else {
+            c->mode = n.mode;
+            sched_features(g, c->activated, c->iter, app, cnt, feat);
+            if (c->iter < LOG_CAP) {
+                for (int i = 0; i < NF; ++i)
+                    s.log[c->iter].feat[i] = feat[i];
+                s.log[c->iter].learned = 0u;
+            }
+            go = (c->sched == WEDGE_SCHED_LEARNED && s.net && !redo) ? 1u : 0u;
+        }
+    }
+    __syncthreads();
+    if (go)
+        ask_network(s, c, app, feat);
+}
+
+// After a pull: reduce the block counters, count the iteration, stop when no
+// edge was activated (execution_bfs.c:239-251) or at the cap, choose the next
+// pull (execution_bfs.c:141, execution_cc.c:103).  With `fused` (the loops
+// whose Wedge iterations sparse_loop_kernel runs) there was a pull unless that
+// kernel ended the traversal, its counters are cleared for its next launch,
+// and in a captured loop (`captured`) the loop's condition is set.
+__global__ void decide_kernel(DevGraph g, DevState s, const unsigned long long* block_cnt, uint32_t nblocks, uint32_t app,
+                              uint32_t fused, uint32_t captured, cudaGraphConditionalHandle handle)
+{
+    Ctrl* c = s.ctrl;
+    if (!c->done) {
+        const uint32_t nsum = ((g.T + TILES_PER_REGION - 1) / TILES_PER_REGION + 31) / 32;
+        for (uint32_t i = threadIdx.x; i < nsum && !fused; i += blockDim.x)
+            s.summary[i] = 0u; /* the pull has cleared every chunk word it walked */
+        unsigned long long cnt[NCNT];
+        reduce_counters(block_cnt, nblocks, cnt);
+        decide_block(g, s, c, app, cnt, s.wo ? SSSP_WO_LAUNCHES : pull_launches_of((int)app));
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (fused) {
+            loop_reset(c);
+            c->bodies += 1u;
+        }
+        if (captured)
+            cudaGraphSetConditional(handle, c->loop);
     }
 }
 
@@ -3147,9 +3219,10 @@ __global__ void init_kernel(DevGraph g, DevState s, uint32_t app, uint32_t topen
     }
     const uint64_t nwords = (g.V + 31) / 32;
     for (uint64_t i = tid; i < nwords; i += stride) {
-        s.front0[i] = 0u;
-        if (s.front1)
-            s.front1[i] = 0u;
+        for (uint32_t b = 0; b < 3u; ++b)
+            s.front[b * s.front_stride + i] = 0u;
+        if (s.visv)
+            s.visv[i] = 0u;
     }
     const uint64_t cwords = ((uint64_t)g.T + 7) / 8;
     for (uint64_t i = tid; i < cwords; i += stride)
@@ -3235,6 +3308,8 @@ __global__ void init_root_kernel(DevGraph g, DevState s, uint32_t app, uint64_t 
         c->probe_edges = s.probe_edges;
         c->narrow_ovf = 0;
         c->ovf_redo = 0;
+        c->bodies = 0;
+        loop_reset(c);
         if (app == WEDGE_APP_CC) {
             c->last_mass = g.E;
             c->mode = MODE_DENSE; /* first CC pull is always dense, execution_cc.c:103 */
@@ -3244,7 +3319,7 @@ __global__ void init_root_kernel(DevGraph g, DevState s, uint32_t app, uint64_t 
                 if (s.dist32)
                     s.dist32[root] = 0u;
             }
-            s.front0[root >> 5] |= 1u << (root & 31u);
+            s.front[root >> 5] |= 1u << (root & 31u);
             c->last_mass = g.outdeg[root];
             c->mode = choose_mode(sched, g.outdeg[root], thr);
             if (sched == WEDGE_SCHED_PROBE && probe_iter == 0u)
@@ -3259,6 +3334,537 @@ __global__ void init_root_kernel(DevGraph g, DevState s, uint32_t app, uint64_t 
             c->done = 1;
             c->loop = 0;
         }
+    }
+}
+
+/* ------------------------------------------------ sparse iterations in one launch */
+//
+// A Wedge iteration of a traversal changes little: as separate launches (pull,
+// decide, collect, expand, build) it took 35-50 us whatever its size, 132 of
+// the 158 iterations of SSSP on the 4096^2 grid and every iteration of a small
+// graph.  sparse_loop_kernel runs all consecutive Wedge iterations in one
+// cooperative launch, one grid barrier each: the vertices the last iteration
+// changed relax their out-edges (every one of them is an in-edge of the
+// reference's Wedge pull; BFS: an unvisited destination takes the least
+// frontier source, CC and SSSP: min) and the changed destinations are listed
+// for the next iteration as they change.  The out-edges of up to 32 listed
+// vertices are spread over a warp's lanes by a prefix sum, four per lane in
+// flight; lists above LOOP_LONG are cut into items.  Bound by the latency of
+// the chain list -> offsets -> out-edge -> destination -> atomic -> list, about
+// 7 us an iteration with few changed vertices, and by the random access per
+// out-edge with many.
+//
+// What the phases share: three frontier bitmaps in turn (read, written,
+// cleared), two lists, three sets of counters (the one two iterations back is
+// cleared while no block reads it).  Every block takes the iteration's
+// decision for itself from the summed counters; the last one writes it down.
+// Graphs of at most LOOP_SMALL_EDGES in-edges run whole in the launch: there a
+// dense iteration is no more work than a Wedge one, and the launches were all
+// the time (BFS at scale 12: 182 us).
+constexpr uint32_t LOOP_LONG = 128;   // out-edges of one vertex a warp takes at once: one round of four per lane
+constexpr uint32_t LOOP_BUF = 128;    // listed vertices a warp keeps in shared memory
+constexpr uint32_t BARRIER_TRIES = 1u << 22;
+enum : uint32_t { ERR_BARRIER_TIMEOUT = 4u };
+
+// all blocks of a cooperative launch; false when it did not complete within
+// the probes (Ctrl::error is set).  target: this block's running arrival count
+// (thread 0).  Writes before it are visible after it to plain loads.
+__device__ __forceinline__ bool grid_barrier(Ctrl* c, uint32_t& target, uint32_t* ok)
+{
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        target += gridDim.x;
+        __threadfence();
+        atomicAdd(&c->bar, 1u);
+        uint32_t v, tries = 0;
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&c->bar) : "memory");
+        } while ((int)(v - target) < 0 && ++tries < BARRIER_TRIES);
+        *ok = (int)(v - target) >= 0 ? 1u : 0u;
+        if (!*ok) { /* the traversal ends with an error */
+            atomicOr(&c->error, ERR_BARRIER_TIMEOUT);
+            atomicExch(&c->loop, 0u);
+            atomicExch(&c->done, 1u);
+        }
+        __threadfence();
+    }
+    __syncthreads();
+    return *ok != 0u;
+}
+
+// The running totals of a traversal while sparse_loop_kernel iterates (one
+// thread): decide_block's record, without a read of device memory.
+struct LoopBook {
+    unsigned long long edges, dsts, activated, last_mass;
+    uint32_t wedge_iters, pull_launches;
+
+    __device__ void open(const Ctrl* c)
+    {
+        edges = c->edges_scanned;
+        dsts = c->dsts_scanned;
+        activated = c->activated;
+        last_mass = c->last_mass;
+        wedge_iters = c->wedge_iters;
+        pull_launches = c->pull_launches + 1u;
+    }
+
+    // after iteration `iter`, run in `mode`
+    __device__ void note(const DevGraph& g, const DevState& s, uint32_t app, const unsigned long long (&cnt)[NCNT],
+                         const NextPull& next, uint32_t mode, uint32_t iter)
+    {
+        edges += cnt[CNT_EDGES];
+        dsts += cnt[CNT_DSTS];
+        activated += cnt[CNT_ACT];
+        wedge_iters += mode == MODE_WEDGE ? 1u : 0u;
+        if (iter < LOG_CAP) {
+            IterRec& r = s.log[iter];
+            r.mass_in = last_mass;
+            r.mass_out = cnt[CNT_MASS];
+            r.edges = cnt[CNT_EDGES];
+            r.tiles = 0ull;
+            r.dsts = cnt[CNT_DSTS];
+            r.activated = cnt[CNT_ACT];
+            r.mode = mode;
+            r.iter = iter;
+        }
+        if (!next.done && iter + 1u < LOG_CAP) {
+            sched_features(g, activated, iter + 1u, app, cnt, s.log[iter + 1u].feat);
+            s.log[iter + 1u].learned = 0u;
+        }
+        last_mass = cnt[CNT_MASS];
+    }
+
+    // into the control block: before another launch or block reads it
+    __device__ void close(Ctrl* c, unsigned long long mass, const NextPull& next, uint32_t iter, uint32_t parity) const
+    {
+        c->edges_scanned = edges;
+        c->dsts_scanned = dsts;
+        c->activated = activated;
+        c->last_mass = mass;
+        c->mass = mass;
+        c->wedge_iters = wedge_iters;
+        c->pull_launches = pull_launches;
+        c->iter = iter;
+        c->parity = parity;
+        if (next.done) {
+            c->done = 1u;
+            c->not_converged = next.capped ? 1u : 0u;
+            c->loop = 0u;
+        } else {
+            c->mode = next.mode;
+        }
+    }
+};
+
+template <int APP>
+__global__ void __launch_bounds__(PULL_THREADS, 1)
+    sparse_loop_kernel(DevGraph g, DevState s, uint32_t small, uint32_t max_steps)
+{
+    constexpr int WARPS = PULL_THREADS / 32;
+    using val_t = typename CurT<APP>::type;
+    __shared__ uint32_t sh_pre[WARPS][32], sh_beg[WARPS][32], sh_buf[WARPS][LOOP_BUF];
+    __shared__ val_t sh_val[WARPS][32];
+    __shared__ unsigned long long sh_acc[NCNT];
+    __shared__ uint32_t sh_ok, sh_n[3];
+    Ctrl* c = s.ctrl;
+    if (c->done)
+        return;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
+    const uint32_t nw = nthr >> 5;
+    const uint32_t gw = (uint32_t)wib * gridDim.x + blockIdx.x; /* few warps' work goes to as many SMs */
+    const uint32_t nwords = (uint32_t)((g.V + 31) / 32);
+    uint32_t mode = c->mode, parity = c->parity, iter = c->iter;
+    const uint32_t sched = c->sched, max_iter = c->max_iter, probe_iter = c->probe_iter, probe_mode = c->probe_mode;
+    const unsigned long long thr = c->threshold;
+    const bool loop = small != 0u || mode == MODE_WEDGE;
+    const bool f64 = g.weight_kind == WEDGE_WEIGHTS_F64;
+    uint32_t* my_buf = sh_buf[wib];
+    uint32_t* my_pre = sh_pre[wib];
+    uint32_t* my_beg = sh_beg[wib];
+    val_t* my_val = sh_val[wib];
+    uint32_t target = 0u, kept = 0u; /* kept: listed vertices in my_buf */
+    uint32_t* out_list = s.alist;
+    uint2* out_items = s.items;
+    uint32_t *out_n = &c->ln[0], *out_i = &c->li[0];
+    auto flush = [&]() {
+        __syncwarp();
+        if (kept) {
+            uint32_t b = 0u;
+            if (lane == 0)
+                b = atomicAdd(out_n, kept);
+            b = __shfl_sync(FULL, b, 0);
+            for (uint32_t i = (uint32_t)lane; i < kept; i += 32u)
+                out_list[b + i] = my_buf[i];
+        }
+        kept = 0u;
+        __syncwarp();
+    };
+    // vertex v (of out-degree od) to the next iteration's list or items; called by all lanes
+    auto append = [&](bool on, uint32_t v, uint32_t od) {
+        const bool shrt = on && od <= LOOP_LONG;
+        const uint32_t m = __ballot_sync(FULL, shrt);
+        if (m) {
+            if (kept + 32u > LOOP_BUF)
+                flush();
+            if (shrt)
+                my_buf[kept + (uint32_t)__popc(m & ((1u << lane) - 1u))] = v;
+            kept += (uint32_t)__popc(m);
+        }
+        if (__any_sync(FULL, on && !shrt)) { /* the lanes write the long vertices' items together */
+            const uint32_t np = on && !shrt ? (od + LOOP_LONG - 1u) / LOOP_LONG : 0u;
+            uint32_t incl = np;
+#pragma unroll
+            for (int q = 1; q < 32; q <<= 1) {
+                const uint32_t y = __shfl_up_sync(FULL, incl, q);
+                if (lane >= q)
+                    incl += y;
+            }
+            const uint32_t excl = incl - np, total = __shfl_sync(FULL, incl, 31);
+            uint32_t at = 0u;
+            if (lane == 0)
+                at = atomicAdd(out_i, total);
+            at = __shfl_sync(FULL, at, 0);
+            for (uint32_t t0 = 0; t0 < total; t0 += 32u) { /* item t0 + lane is one of the last lane's that begins at or before it */
+                const uint32_t q = t0 + (uint32_t)lane;
+                uint32_t o = 0u;
+#pragma unroll
+                for (uint32_t h = 16u; h > 0u; h >>= 1)
+                    if (__shfl_sync(FULL, excl, (int)(o + h)) <= q)
+                        o += h;
+                const uint32_t ov = __shfl_sync(FULL, v, (int)o), first = __shfl_sync(FULL, excl, (int)o);
+                if (q < total)
+                    out_items[at + q] = make_uint2(ov, q - first);
+            }
+        }
+    };
+
+    // ---- the bitmap of the vertices the last iteration changed -> the list;
+    // the next bitmap and the tile list's bits are cleared
+    {
+        const uint32_t* cur = cur_front(s, parity);
+        uint32_t* nxt = next_front(s, parity);
+        const bool all = APP == WEDGE_APP_CC && iter == 0u; /* every vertex is active before CC's first pull */
+        /* whole sectors of 8 words, four of them far apart: the vertices of many
+           out-edges have neighbouring ids */
+        for (uint32_t base = 0u; base < nwords; base += nw * 32u) {
+            const uint32_t i = base + (gw + ((uint32_t)lane >> 3) * nw) * 8u + ((uint32_t)lane & 7u);
+            uint32_t word = 0u;
+            if (i < nwords) {
+                word = cur[i];
+                nxt[i] = 0u;
+                if (APP == WEDGE_APP_BFS)
+                    s.visv[i] |= word;
+                if (all)
+                    word = (uint64_t)i * 32u + 32u <= g.V ? FULL : (1u << (g.V & 31u)) - 1u;
+            }
+            if (!loop)
+                continue;
+            uint32_t busy = __ballot_sync(FULL, word != 0u);
+            while (busy) { /* one word's vertices a round */
+                const int l = __ffs(busy) - 1;
+                busy &= busy - 1u;
+                const uint32_t w = __shfl_sync(FULL, word, l);
+                const uint32_t v = __shfl_sync(FULL, i, l) * 32u + (uint32_t)lane;
+                const bool on = (w >> lane) & 1u;
+                append(on, v, on ? g.outdeg[v] : 0u);
+            }
+        }
+        if (s.tile_need)
+            for (uint32_t i = tid; i < g.T / 32u + 2u; i += nthr)
+                s.tile_need[i] = 0u;
+        if (!loop)
+            return;
+        flush();
+    }
+    // The record of the iterations is kept by one thread of the last block, which
+    // has work last: in registers, so that the loop does not wait for it
+    const bool scribe = blockIdx.x + 1u == gridDim.x && threadIdx.x == 0;
+    LoopBook book;
+    if (scribe)
+        book.open(c);
+    if (!grid_barrier(c, target, &sh_ok))
+        return;
+
+    for (uint32_t step = 0;; ++step) {
+        const uint32_t a = step % 3u, b = (step + 1u) % 3u;
+        /* one warp of the block reads what all blocks read at once */
+        if (threadIdx.x < 3)
+            sh_n[threadIdx.x] = __ldcg(threadIdx.x == 0 ? &c->ln[a] : threadIdx.x == 1 ? &c->li[a] : &c->narrow_ovf);
+        __syncthreads();
+        const uint32_t n = sh_n[0], ni = sh_n[1];
+        const uint32_t half = step & 1u;
+        const uint32_t* list = s.alist + (half ? s.alist_stride : 0ull);
+        const uint2* items = s.items + (half ? s.item_stride : 0ull);
+        out_list = s.alist + (half ? 0ull : s.alist_stride);
+        out_items = s.items + (half ? 0ull : s.item_stride);
+        out_n = &c->ln[b];
+        out_i = &c->li[b];
+        const uint32_t* cur = cur_front(s, parity);
+        uint32_t* nxt = next_front(s, parity);
+        uint32_t* old = next_front(s, (parity + 1u) % 3u);
+        const bool narrow = APP == WEDGE_APP_SSSP && s.dist32 && !sh_n[2];
+        unsigned long long mass = 0, degs = 0; /* degs: activated vertices per out-degree bucket 0..2, 21 bits each */
+        uint32_t edges = 0, act = 0, occ = 0, dsts = 0;
+        if (tid == 0u) { /* counters no block reads any more */
+            c->ln[(step + 2u) % 3u] = 0u;
+            c->li[(step + 2u) % 3u] = 0u;
+        }
+        if (blockIdx.x == 0 && threadIdx.x < NCNT)
+            c->lacc[b][threadIdx.x] = 0ull;
+        for (uint32_t i = tid; i < nwords; i += nthr)
+            old[i] = 0u;
+
+        // Four out-edges per lane (of vertices with values x), in stages, so that
+        // the four chains are in flight together: destinations; their present
+        // state; the atomics that lower it; the new frontier bits and
+        // out-degrees; the list.
+        auto relax4 = [&](const bool (&on)[4], const val_t (&x)[4], const uint32_t (&e)[4]) {
+            uint32_t d[4], od[4], o[4];
+            bool low[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                d[u] = on[u] ? g.csri[e[u]] : 0u;
+            if constexpr (APP == WEDGE_APP_BFS) {
+                uint32_t seen[4], p[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    seen[u] = on[u] ? s.visv[d[u] >> 5] | cur[d[u] >> 5] : FULL;
+                    p[u] = on[u] ? s.prop32[d[u]] : 0u;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) { /* unvisited before this iteration, and not yet a lesser parent's */
+                    low[u] = !((seen[u] >> (d[u] & 31u)) & 1u) && p[u] > x[u];
+                    if (low[u])
+                        p[u] = atomicMin(&s.prop32[d[u]], x[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    low[u] = low[u] && p[u] == NONE32; /* the first to reach it lists it */
+            } else if constexpr (APP == WEDGE_APP_CC) {
+                uint32_t p[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    p[u] = on[u] ? s.prop32[d[u]] : 0u;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    low[u] = x[u] < p[u];
+                    if (low[u])
+                        p[u] = atomicMin(&s.prop32[d[u]], x[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    low[u] = low[u] && x[u] < p[u];
+            } else {
+                unsigned long long nd[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const unsigned long long wv = !on[u] ? 0ull : g.cw8 ? (unsigned long long)g.cw8[e[u]] : g.cw[e[u]];
+                    nd[u] = f64 ? (unsigned long long)__double_as_longlong(__dadd_rn(__longlong_as_double((long long)x[u]),
+                                                                                     __longlong_as_double((long long)wv)))
+                                : x[u] + wv; /* phase_edge_pull_sssp.c:136-137; an activated source is reached */
+                }
+                if (narrow) {
+                    uint32_t p[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        p[u] = on[u] ? s.dist32[d[u]] : 0u;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        low[u] = nd[u] < (unsigned long long)p[u] && nd[u] < (unsigned long long)s.narrow_lim;
+                        if (low[u])
+                            p[u] = atomicMin(&s.dist32[d[u]], (uint32_t)nd[u]);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        if (on[u] && nd[u] >= (unsigned long long)s.narrow_lim) { /* past the 32-bit copy */
+                            low[u] = nd[u] < s.prop64[d[u]] && nd[u] < atomicMin(&s.prop64[d[u]], nd[u]);
+                            if (low[u])
+                                dist32_put(s, d[u], nd[u], false);
+                        } else {
+                            low[u] = low[u] && nd[u] < (unsigned long long)p[u];
+                            if (low[u])
+                                atomicMin(&s.prop64[d[u]], nd[u]);
+                        }
+                    }
+                } else {
+                    unsigned long long p[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        p[u] = on[u] ? s.prop64[d[u]] : 0ull;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        low[u] = nd[u] < p[u];
+                        if (low[u])
+                            p[u] = atomicMin(&s.prop64[d[u]], nd[u]);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        low[u] = low[u] && nd[u] < p[u];
+                        if (low[u])
+                            dist32_put(s, d[u], nd[u], false);
+                    }
+                }
+            }
+            if (!__any_sync(FULL, low[0] || low[1] || low[2] || low[3]))
+                return;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                o[u] = FULL;
+                od[u] = 0u;
+                if (low[u]) {
+                    o[u] = atomicOr(&nxt[d[u] >> 5], 1u << (d[u] & 31u));
+                    od[u] = g.outdeg[d[u]];
+                    if (APP == WEDGE_APP_BFS || (APP == WEDGE_APP_CC && x[u] == 0u)) { /* visited; label 0 is final */
+                        const uint32_t k = g.dst_ident ? d[u] : g.dst_index[d[u]];
+                        atomicOr(&s.vis_c[k >> 5], 1u << (k & 31u));
+                    }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                occ += o[u] == 0u ? 1u : 0u;
+                const bool first = low[u] && !((o[u] >> (d[u] & 31u)) & 1u);
+                if (first) {
+                    mass += od[u];
+                    ++act;
+                    const uint32_t bk = degree_bucket(od[u]);
+                    if (bk < 3u)
+                        degs += 1ull << (21u * bk);
+                }
+                append(first, d[u], od[u]);
+            }
+        };
+        auto value = [&](uint32_t v) -> val_t {
+            if constexpr (APP == WEDGE_APP_BFS)
+                return v;
+            else if constexpr (APP == WEDGE_APP_CC)
+                return s.prop32[v];
+            else
+                return s.prop64[v];
+        };
+        // LOOP_LONG out-edges of a long list
+        for (uint32_t i = gw; i < ni; i += nw) {
+            const uint2 it = items[i];
+            const uint32_t lo = (uint32_t)g.csri_off[it.x] + it.y * LOOP_LONG, end = (uint32_t)g.csri_off[it.x + 1u];
+            const uint32_t hi = end - lo > LOOP_LONG ? lo + LOOP_LONG : end;
+            const val_t x0 = value(it.x);
+            if (APP == WEDGE_APP_BFS && it.y == 0u && lane == 0)
+                atomicOr(&s.visv[it.x >> 5], 1u << (it.x & 31u));
+            const val_t x[4] = {x0, x0, x0, x0};
+            for (uint32_t t = lo; t < hi; t += 128u) {
+                bool on[4];
+                uint32_t e[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    e[u] = t + 32u * u + (uint32_t)lane;
+                    on[u] = e[u] < hi;
+                }
+                relax4(on, x, e);
+            }
+            if (lane == 0)
+                edges += hi - lo;
+        }
+        // up to 32 listed vertices a warp, fewer while that leaves warps without any
+        const uint32_t chunk = min(32u, max(1u, (n + nw - 1u) / nw));
+        for (uint32_t i0 = gw * chunk; i0 < n; i0 += nw * chunk) {
+            const uint32_t i = i0 + (uint32_t)lane;
+            uint32_t lo = 0u, len = 0u;
+            __syncwarp();
+            if ((uint32_t)lane < chunk && i < n) {
+                const uint32_t v = list[i];
+                lo = (uint32_t)g.csri_off[v];
+                len = (uint32_t)g.csri_off[v + 1u] - lo;
+                my_val[lane] = value(v);
+                if (APP == WEDGE_APP_BFS)
+                    atomicOr(&s.visv[v >> 5], 1u << (v & 31u));
+                ++dsts;
+            }
+            uint32_t incl = len;
+#pragma unroll
+            for (int q = 1; q < 32; q <<= 1) {
+                const uint32_t y = __shfl_up_sync(FULL, incl, q);
+                if (lane >= q)
+                    incl += y;
+            }
+            const uint32_t total = __shfl_sync(FULL, incl, 31);
+            my_pre[lane] = incl - len;
+            my_beg[lane] = lo - (incl - len);
+            __syncwarp();
+            if (lane == 0)
+                edges += total;
+            for (uint32_t t0 = 0; t0 < total; t0 += 128u) {
+                bool on[4];
+                uint32_t e[4];
+                val_t x[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const uint32_t t = t0 + 32u * u + (uint32_t)lane;
+                    on[u] = t < total;
+                    uint32_t o = 0u; /* the vertex: the last one whose out-edges begin at or before t */
+#pragma unroll
+                    for (uint32_t h = 16u; h > 0u; h >>= 1)
+                        if (my_pre[o + h] <= t)
+                            o += h;
+                    e[u] = my_beg[o] + t;
+                    x[u] = my_val[o];
+                }
+                relax4(on, x, e);
+            }
+        }
+        flush();
+        // the iteration's counters
+        __syncthreads(); /* cnt of the last iteration is read */
+        if (threadIdx.x < NCNT)
+            sh_acc[threadIdx.x] = 0ull;
+        __syncthreads();
+        if (__any_sync(FULL, (edges | dsts) != 0u)) {
+            const unsigned long long v[NCNT] = {
+                warp_sum_u64(mass), __reduce_add_sync(FULL, edges), 0ull, __reduce_add_sync(FULL, dsts),
+                __reduce_add_sync(FULL, act), warp_sum_u64(degs & 0x1FFFFFull), warp_sum_u64((degs >> 21) & 0x1FFFFFull),
+                warp_sum_u64(degs >> 42), __reduce_add_sync(FULL, occ)};
+            if (lane == 0)
+#pragma unroll
+                for (uint32_t j = 0; j < NCNT; ++j)
+                    if (v[j])
+                        atomicAdd(&sh_acc[j], v[j]);
+        }
+        __syncthreads();
+        if (threadIdx.x < NCNT && sh_acc[threadIdx.x])
+            atomicAdd(&c->lacc[a][threadIdx.x], sh_acc[threadIdx.x]);
+        if (!grid_barrier(c, target, &sh_ok))
+            return;
+        // the decision, the same in every block; block 0 writes it down
+        if (threadIdx.x < NCNT)
+            sh_acc[threadIdx.x] = __ldcg(&c->lacc[a][threadIdx.x]);
+        __syncthreads();
+        unsigned long long cnt[NCNT];
+#pragma unroll
+        for (uint32_t j = 0; j < NCNT; ++j)
+            cnt[j] = sh_acc[j];
+        const NextPull next = next_pull(sched, cnt[CNT_MASS], false, iter + 1u, max_iter, thr, probe_iter, probe_mode);
+        if (scribe)
+            book.note(g, s, (uint32_t)APP, cnt, next, mode, iter);
+        if (scribe && (next.done || step + 1u == max_steps || (!small && next.mode != MODE_WEDGE) ||
+                       sched == WEDGE_SCHED_LEARNED))
+            book.close(c, cnt[CNT_MASS], next, iter + 1u, (parity + 1u) % 3u);
+        if (!next.done && sched == WEDGE_SCHED_LEARNED && s.net && blockIdx.x + 1u == gridDim.x)
+            ask_network(s, c, (uint32_t)APP, iter + 1u);
+        mode = next.mode;
+        ++iter;
+        parity = (parity + 1u) % 3u;
+        if (!next.done && sched == WEDGE_SCHED_LEARNED && s.net) { /* the last block asked the network */
+            if (!grid_barrier(c, target, &sh_ok))
+                return;
+            mode = *(volatile unsigned int*)&c->mode;
+        }
+        if (!next.done && !small && mode != MODE_WEDGE && APP == WEDGE_APP_BFS) { /* a dense pull takes over */
+            cur = cur_front(s, parity);
+            for (uint32_t i = tid; i < nwords; i += nthr)
+                s.visv[i] |= cur[i];
+        }
+        if (next.done || step + 1u == max_steps || (!small && mode != MODE_WEDGE))
+            return;
     }
 }
 
@@ -3402,7 +4008,7 @@ __global__ void pr_finish_kernel(DevGraph g, DevState s, uint32_t nblocks, const
         reduce_counters(block_cnt, nblocks, cnt); /* contains __syncthreads */
         if (threadIdx.x == 0) {
             c->last_mass = 0;
-            log_iteration(s, c, cnt);
+            log_iteration(s, c, cnt, 1u);
         }
     }
     merge_splits(g, s.acc, g.split_k, g.split_t0, g.split_t1, g.nsplit, g.nwide, g.T, [&](uint32_t t) { return s.tail_part[t]; },
@@ -3899,7 +4505,7 @@ __global__ void pr32_total_kernel(DevState s, uint32_t nparts, const unsigned lo
         c->pr_total = S;
         if (nblocks) {
             c->last_mass = 0;
-            log_iteration(s, c, cnt);
+            log_iteration(s, c, cnt, 1u);
         }
     }
 }
@@ -4249,7 +4855,8 @@ static int setup_hub(wedge_graph* h, int app, int precision)
     h->hub_bytes = (uint32_t)(n * elem);
     h->s.hub_bytes = h->hub_bytes;
     h->pull_smem = h->hub_bytes + (uint32_t)stage;
-    WEDGE_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->pull_smem));
+    /* the function's limit, not this handle's size: handles with larger caches may be alive */
+    WEDGE_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
     if (two_phase_app(app) && n) {
         uint32_t* d = (uint32_t*)(h->s.block_part + h->pull_grid); /* counters: scratch until the first pull */
         hub_split_kernel<<<1, 1, 0, h->stream>>>(h->g, (uint32_t)n, pull_tile_e(h, app), d);
@@ -4289,7 +4896,7 @@ static int pr32_setup_hub(wedge_graph* h)
     h->s.hub_bytes = (uint32_t)(n * 4u);
     h->hub_bytes = h->s.hub_bytes;
     WEDGE_CHECK(cudaFuncSetAttribute(pr32_pull_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(h->hub_bytes + PR32_STAGE_BYTES)));
+                                     optin - (int)fa.sharedSizeBytes));
     return WEDGE_OK;
 }
 
@@ -4423,6 +5030,11 @@ static int sssp_split_state(wedge_graph* h)
     return WEDGE_OK;
 }
 
+// The traversal loops run their Wedge iterations in sparse_loop_kernel where
+// the CSRI holds destinations (and the vertices' out-degrees are its lists'
+// lengths); the phase API and chunk frontiers take the separate launches.
+static bool fused_loop(const wedge_graph* h) { return h->g.csr && !h->g.shard && h->g.E != 0; }
+
 static int ensure_state(wedge_graph* h, int app, int precision)
 {
     if (h->built_app == app && (app != WEDGE_APP_PR || h->last_precision == precision))
@@ -4480,11 +5092,17 @@ static int ensure_state(wedge_graph* h, int app, int precision)
         } else if ((rc = dalloc(h, &s.prop32, V, true))) {
             return rc;
         }
-        if ((rc = dalloc(h, &s.front0, nwords, true)) || (rc = dalloc(h, &s.front1, nwords, true)) ||
+        s.front_stride = nwords;
+        s.alist_stride = V + 1;
+        s.item_stride = g.E / (LOOP_LONG / 2u) + 2;
+        const uint64_t build_items = V + g.E / PIECE + 2, loop_items = fused_loop(h) ? 2 * s.item_stride : 0;
+        const uint64_t nitems = build_items > loop_items ? build_items : loop_items;
+        if ((rc = dalloc(h, &s.front, 3 * nwords, true)) ||
+            (app == WEDGE_APP_BFS && g.csr && (rc = dalloc(h, &s.visv, nwords, true))) ||
             (rc = dalloc(h, &s.chunk_bits, (uint64_t)g.T / TILES_PER_WORD + REGION_WORDS + 2, true)) ||
             (rc = dalloc(h, &s.summary, (uint64_t)g.T / TILES_PER_REGION / 32 + 2, true)) ||
             (rc = dalloc(h, &s.tile_list, (uint64_t)g.T + 1, true)) ||
-            (rc = dalloc(h, &s.items, V + g.E / PIECE + 2, true)) || (rc = dalloc(h, &s.alist, V + 1, true)))
+            (rc = dalloc(h, &s.items, nitems, true)) || (rc = dalloc(h, &s.alist, 2 * (V + 1), true)))
             return rc;
         if (app == WEDGE_APP_BFS || app == WEDGE_APP_CC) {
             if ((rc = dalloc(h, &s.vis_c, (uint64_t)g.Vne / 32 + 2, true)))
@@ -4597,6 +5215,12 @@ static uint64_t iteration_launches(const wedge_graph* h, int app)
     return 1ull + build_launches(h) + pulls;
 }
 
+// a round of the fused loop: the Wedge iterations' launch, the dense pull's and the decision
+static uint64_t fused_launches(const wedge_graph* h, int app)
+{
+    return iteration_launches(h, app) - build_launches(h) + 1ull;
+}
+
 // sssp_split_kernel: a thread per short split, a warp per long one
 static uint32_t sssp_split_grid(wedge_graph* h)
 {
@@ -4647,15 +5271,54 @@ static void launch_wedge_build(wedge_graph* h, const DevGraph& g, int app)
         launch_compact(h, app);
 }
 
+static void launch_decide(wedge_graph* h, int app, bool fused, bool captured = false, cudaGraphConditionalHandle handle = 0)
+{
+    decide_kernel<<<1, AUX_THREADS, 0, h->stream>>>(h->g, h->s, counters(h), pull_slots(h, app), (uint32_t)app,
+                                                    fused ? 1u : 0u, captured ? 1u : 0u, handle);
+}
+
+// whole traversals in one launch up to this many in-edges
+constexpr uint64_t LOOP_SMALL_EDGES = 1ull << 20;
+static bool small_loop(const wedge_graph* h) { return h->g.E <= LOOP_SMALL_EDGES; }
+
+// one block per SM, fewer on graphs that leave most of them without work (a
+// barrier of few blocks is faster)
+static int launch_sparse_loop(wedge_graph* h, int app, uint32_t max_steps)
+{
+    const uint64_t want = h->g.E / 2048u + 8u;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((uint32_t)(want < (uint64_t)h->num_sms ? want : (uint64_t)h->num_sms));
+    cfg.blockDim = dim3(PULL_THREADS);
+    cfg.stream = h->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative; /* the blocks wait for one another */
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const uint32_t small = small_loop(h) ? 1u : 0u;
+    switch (app) {
+    case WEDGE_APP_BFS:
+        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, sparse_loop_kernel<WEDGE_APP_BFS>, h->g, h->s, small, max_steps));
+        break;
+    case WEDGE_APP_CC:
+        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, sparse_loop_kernel<WEDGE_APP_CC>, h->g, h->s, small, max_steps));
+        break;
+    default:
+        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, sparse_loop_kernel<WEDGE_APP_SSSP>, h->g, h->s, small, max_steps));
+        break;
+    }
+    return WEDGE_OK;
+}
+
 // iteration tail after a pull: mass/convergence, Wedge frontier, bitmap reset
 static void launch_tail(wedge_graph* h, int app)
 {
-    decide_kernel<<<1, AUX_THREADS, 0, h->stream>>>(h->g, h->s, counters(h), pull_slots(h, app), (uint32_t)app);
+    launch_decide(h, app, false);
     launch_wedge_build(h, h->g, app); /* collect_kernel clears the bitmaps for the next pull */
 }
 
 static void launch_init(wedge_graph* h, int app, uint64_t root, uint32_t sched, unsigned long long thr, uint32_t max_iter,
-                        uint32_t probe_iter = 0xFFFFFFFFu, uint32_t probe_mode = MODE_DENSE)
+                        uint32_t probe_iter = 0xFFFFFFFFu, uint32_t probe_mode = MODE_DENSE, bool build = true)
 {
     const uint64_t work = h->g.V > h->g.T ? h->g.V : h->g.T;
     const uint32_t tile_e = pull_tile_e(h, app);
@@ -4664,7 +5327,8 @@ static void launch_init(wedge_graph* h, int app, uint64_t root, uint32_t sched, 
     init_root_kernel<<<1, 32, 0, h->stream>>>(h->g, h->s, (uint32_t)app, root, sched, thr,
                                                                            max_iter, probe_iter, probe_mode);
     h->cc_pending = (app == WEDGE_APP_CC && h->s.cc_best) ? 1 : 0;
-    launch_wedge_build(h, h->g, app); /* collect_kernel clears the bitmaps for the first pull */
+    if (build)
+        launch_wedge_build(h, h->g, app); /* collect_kernel clears the bitmaps for the first pull */
 }
 
 // CC on a symmetric graph, once the labels converged: caller-id labels in
@@ -4730,13 +5394,22 @@ static int build_graph(wedge_graph* h, int app)
     const cudaStream_t run_stream = h->stream;
     h->stream = h->own_stream;
     WEDGE_CHECK(cudaStreamBeginCaptureToGraph(h->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    launch_pull(h, app);
-    launch_tail(h, app);
-    loop_cond_kernel<<<1, 1, 0, h->stream>>>(h->s, handle);
+    int rc = WEDGE_OK;
+    if (fused_loop(h)) { /* Wedge iterations, a dense pull, the decision and the loop condition */
+        rc = launch_sparse_loop(h, app, 0xFFFFFFFFu);
+        launch_pull(h, app);
+        launch_decide(h, app, true, true, handle);
+    } else {
+        launch_pull(h, app);
+        launch_tail(h, app);
+        loop_cond_kernel<<<1, 1, 0, h->stream>>>(h->s, handle);
+    }
     cudaGraph_t captured;
     const cudaError_t ce = cudaStreamEndCapture(h->stream, &captured);
     h->stream = run_stream;
     WEDGE_CHECK(ce);
+    if (rc)
+        return rc;
     WEDGE_CHECK(cudaGraphInstantiate(&h->graph_exec, graph, 0));
     cudaGraphDestroy(graph);
     h->graph_app = app;
@@ -4770,7 +5443,10 @@ static int traversal_stats(wedge_graph* h, int app, uint64_t launches, bool use_
         st->edges_scanned = c.edges_scanned;
         st->tiles_scanned = c.tiles_scanned;
         st->pull_launches = c.pull_launches;
-        st->kernel_launches = use_graph ? launches + (iteration_launches(h, app) + 1ull) * c.iter : launches;
+        /* the device loop's launches: per iteration, or per round of the fused loop */
+        st->kernel_launches = !use_graph ? launches
+                              : c.bodies ? launches + fused_launches(h, app) * c.bodies
+                                         : launches + (iteration_launches(h, app) + 1ull) * c.iter;
     }
     if (c.error)
         return WEDGE_ERR_CUDA;
@@ -4790,7 +5466,9 @@ static int run_traversal(wedge_graph* h, int app, const wedge_params_t* p, wedge
     if (cap > 0x7fffffffull)
         cap = 0x7fffffffull;
     const bool timing = (p->flags & WEDGE_FLAG_TIMING) != 0;
-    const bool use_graph = (p->flags & WEDGE_FLAG_GRAPH) != 0 && !timing;
+    const bool fused = fused_loop(h);
+    const bool one = fused && small_loop(h) && !timing; /* the whole traversal in one launch */
+    const bool use_graph = (p->flags & WEDGE_FLAG_GRAPH) != 0 && !timing && !one;
     uint64_t launches = 0;
     double t_pull_dense = 0, t_pull_wedge = 0, t_wedge = 0;
     if (use_graph) {
@@ -4799,10 +5477,15 @@ static int run_traversal(wedge_graph* h, int app, const wedge_params_t* p, wedge
             return rc;
     }
     WEDGE_CHECK(cudaEventRecord(h->ev[0], h->stream));
-    launch_init(h, app, root, (uint32_t)p->sched, thr, (uint32_t)cap, p->probe_iter, (uint32_t)p->probe_mode);
-    launches += 2ull + build_launches(h); /* init, root, the Wedge build */
+    launch_init(h, app, root, (uint32_t)p->sched, thr, (uint32_t)cap, p->probe_iter, (uint32_t)p->probe_mode, !fused);
+    launches += 2ull + (fused ? 0ull : build_launches(h)); /* init, root, the Wedge build */
     Ctrl c;
-    if (use_graph) {
+    if (one) {
+        int rc = launch_sparse_loop(h, app, 0xFFFFFFFFu);
+        if (rc)
+            return rc;
+        launches += 1ull;
+    } else if (use_graph) {
         WEDGE_CHECK(cudaGraphLaunch(h->graph_exec, h->stream));
     } else if (timing) {
         for (;;) {
@@ -4812,12 +5495,21 @@ static int run_traversal(wedge_graph* h, int app, const wedge_params_t* p, wedge
             if (c.done)
                 break;
             const uint32_t mode = c.mode;
+            const bool sparse = fused && (mode == MODE_WEDGE || small_loop(h));
             WEDGE_CHECK(cudaEventRecord(h->ev[2], h->stream));
-            launch_pull(h, app);
+            if (fused && (rc = launch_sparse_loop(h, app, 1u))) /* one Wedge iteration, or the bitmaps' clearing */
+                return rc;
+            if (!sparse)
+                launch_pull(h, app);
             WEDGE_CHECK(cudaEventRecord(h->ev[3], h->stream));
-            launch_tail(h, app);
+            if (sparse)
+                loop_reset_kernel<<<1, 1, 0, h->stream>>>(h->s);
+            else if (fused)
+                launch_decide(h, app, true);
+            else
+                launch_tail(h, app);
             WEDGE_CHECK(cudaEventRecord(h->ev[4], h->stream));
-            launches += iteration_launches(h, app);
+            launches += sparse ? 2ull : fused ? fused_launches(h, app) : iteration_launches(h, app);
             WEDGE_CHECK(cudaEventSynchronize(h->ev[4]));
             float a = 0, b = 0;
             cudaEventElapsedTime(&a, h->ev[2], h->ev[3]);
@@ -4836,9 +5528,17 @@ static int run_traversal(wedge_graph* h, int app, const wedge_params_t* p, wedge
         // speculative batches: kernels are no-ops once Ctrl::done is set
         for (;;) {
             for (int b = 0; b < 3; ++b) {
+                if (fused) {
+                    int rc = launch_sparse_loop(h, app, 0xFFFFFFFFu);
+                    if (rc)
+                        return rc;
+                }
                 launch_pull(h, app);
-                launch_tail(h, app);
-                launches += iteration_launches(h, app);
+                if (fused)
+                    launch_decide(h, app, true);
+                else
+                    launch_tail(h, app);
+                launches += fused ? fused_launches(h, app) : iteration_launches(h, app);
             }
             int rc = read_ctrl(h, &c);
             if (rc)
@@ -4854,9 +5554,10 @@ static int run_traversal(wedge_graph* h, int app, const wedge_params_t* p, wedge
     WEDGE_CHECK(cudaEventRecord(h->ev[1], h->stream));
     WEDGE_CHECK(cudaGetLastError());
     h->last_app = app;
-    if (!wait && use_graph) {
+    if (!wait && (use_graph || one)) {
         h->pend_app = app;
         h->pend_launches = launches;
+        h->pend_graph = use_graph;
         return WEDGE_OK;
     }
     return traversal_stats(h, app, launches, use_graph, timing, t_pull_dense, t_pull_wedge, t_wedge, st);
@@ -5189,7 +5890,7 @@ int wedge_cuda_wait(wedge_graph_t* g, wedge_stats_t* stats)
     if (g->pend_app == WEDGE_APP_PR)
         rc = pr_stats(g, g->pend_iters, g->pend_launches != 0, false, 0.0, 0.0, stats);
     else if (g->pend_app >= 0)
-        rc = traversal_stats(g, g->pend_app, g->pend_launches, true, false, 0.0, 0.0, 0.0, stats);
+        rc = traversal_stats(g, g->pend_app, g->pend_launches, g->pend_graph != 0, false, 0.0, 0.0, 0.0, stats);
     else if (stats)
         memset(stats, 0, sizeof(*stats));
     g->pend_app = -1;
@@ -5307,7 +6008,7 @@ int wedge_cuda_shard_state(wedge_graph_t* g, int which, void* host, uint64_t byt
         int rc = read_ctrl(g, &c);
         if (rc)
             return rc;
-        dev = (void*)(c.parity ? g->s.front1 : g->s.front0); /* the bitmap the last pull wrote */
+        dev = (void*)(g->s.front + c.parity * g->s.front_stride); /* the bitmap the last pull wrote */
         need = (g->g.V + 31) / 32 * 4ull;
     }
     if (bytes < need)
@@ -5394,7 +6095,7 @@ int wedge_cuda_run_phase(wedge_graph_t* g, int app, int phase, const wedge_param
             launch_pr_total(g);
         } else {
             launch_pull(g, app);
-            decide_kernel<<<1, AUX_THREADS, 0, g->stream>>>(dg, g->s, counters(g), pull_slots(g, app), (uint32_t)app);
+            launch_decide(g, app, false);
         }
         break;
     }

@@ -98,7 +98,7 @@ struct Ctrl {
     unsigned int not_converged;        // iteration cap reached
     unsigned int max_iter;
     unsigned int sched;                // enum wedge_sched
-    unsigned int parity;               // BFS frontier double-buffer parity
+    unsigned int parity;               // which of the three frontier bitmaps the next pull reads
     unsigned int loop;                 // 1 while the traversal continues (CUDA-graph loop condition)
     unsigned int error;                // kernel-detected error (bounds)
     unsigned int pull_launches;
@@ -112,6 +112,10 @@ struct Ctrl {
                                        // 64-bit distances from then on
     unsigned int ovf_redo;             // SSSP: a pull dropped sums its 32-bit arithmetic could not hold: the next
                                        // pull is dense (64-bit) and the traversal does not stop before it
+    unsigned int bodies;               // rounds of the fused traversal loop
+    unsigned int bar;                  // sparse_loop_kernel: grid-barrier arrivals, and per step modulo 3
+    unsigned int ln[3], li[3];         // vertices and items listed for it,
+    unsigned long long lacc[3][NCNT];  // and its counters
     double pr_total;                   // sum of all accumulators (phase_vertex_pr.c:161); compensated FP32:
                                        // the total the next iteration uses
     double pr_prev;                    // compensated FP32: the total the last iteration used
@@ -187,8 +191,9 @@ struct DevState {
     uint32_t* ovf_list;            // complete destinations past the staged slots of their tile (tile order)
     uint32_t novf;
     double* block_part;            // [grid] per-block sums of tile sums
-    uint32_t* front0;              // V-bit frontier bitmaps (active / snapshot)
-    uint32_t* front1;
+    uint32_t* front;               // [3][front_stride] V-bit frontier bitmaps in turn: read, written, spare
+    uint64_t front_stride;
+    uint32_t* visv;                // V-bit, BFS: visited before this iteration's frontier (sparse_loop_kernel)
     uint32_t* vis_c;               // Vne-bit: destination finished (BFS visited; CC label 0, the least label)
     uint32_t* tile_open;           // T-bit: tile still has an unfinished destination (BFS, CC)
     uint32_t* tile_need;           // T-bit: BFS tiles with in-edges the probe left to the tile pull
@@ -197,8 +202,10 @@ struct DevState {
     uint32_t* chunk_bits;          // Wedge frontier: one bit per chunk
     uint32_t* summary;             // one bit per region of REGION_WORDS chunk words (any chunk marked)
     unsigned long long* tile_list; // (tile << 32 | chunk mask) of the next Wedge pull
-    uint2* items;                  // (vertex, piece) Wedge-build work items
-    uint32_t* alist;               // vertices the last pull activated (Wedge build)
+    uint2* items;                  // (vertex, piece) work items of long out-lists: Wedge build, or two
+                                   // buffers item_stride apart (sparse_loop_kernel)
+    uint32_t* alist;               // vertices the last pull activated: Wedge build, or two buffers alist_stride apart
+    uint64_t alist_stride, item_stride;
     uint32_t* cc_best;             // CC on a symmetric graph: least caller id of the component a label represents
     const uint32_t* cc_map;        // results only: CC labels are looked up here (engine ids not yet converted)
     Ctrl* ctrl;
@@ -231,6 +238,7 @@ struct wedge_graph {
     unsigned long long* xbuf;          // device staging of asynchronous exports (8 bytes per vertex, on first use)
     int pend_app;                      // run queued by wedge_cuda_run_async, reported by wedge_cuda_wait (-1 none)
     uint64_t pend_launches;
+    int pend_graph;                    // it runs as the captured loop
     uint32_t pend_iters;
     int device;
     int num_sms;
