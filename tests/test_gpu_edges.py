@@ -132,3 +132,32 @@ def test_largest_whole_traversal(engine_lib, edges):
     s, d = s[order].astype(np.uint32), d[order].astype(np.uint32)
     w = rng.integers(0, 256, len(s)).astype(np.uint64)
     check_traversals(W, V, s, d, w, (W.SCHED_PLAIN, W.SCHED_FILTERED), (0, W.FLAG_GRAPH, W.FLAG_TIMING))
+
+
+@pytest.mark.parametrize("weights", ["bytes", "zeros", "words", "beyond32", "f64"])
+def test_near_vertices_first(engine_lib, weights):
+    """long SSSPs with many changed vertices, where far ones wait: the distances are
+    those of all-dense pulls, whatever interrupts the loop (schedules, one
+    iteration at a time), with zero weights, wide ones and 32-bit overflow"""
+    W = engine_lib
+    side, rng = 700, np.random.default_rng(5)
+    v = np.arange(side * side).reshape(side, side)
+    s = np.concatenate([v[:, :-1].ravel(), v[:, 1:].ravel(), v[:-1].ravel(), v[1:].ravel(), rng.integers(0, side * side, 9000)])
+    d = np.concatenate([v[:, 1:].ravel(), v[:, :-1].ravel(), v[1:].ravel(), v[:-1].ravel(), rng.integers(0, side * side, 9000)])
+    order = np.lexsort((s, d))
+    s, d = s[order].astype(np.uint32), d[order].astype(np.uint32)
+    n = len(s)
+    kind = W.WEIGHTS_U64
+    if weights == "f64":
+        w, kind = rng.random(n).view(np.uint64), W.WEIGHTS_F64
+    else:
+        w = {"bytes": rng.integers(1, 256, n), "zeros": rng.integers(0, 2, n) * rng.integers(1, 256, n),
+             "words": rng.integers(0, 100_000, n), "beyond32": rng.integers(0, 1 << 31, n)}[weights].astype(np.uint64)
+    with W.Graph.from_edges(side * side, s, d, w, kind) as g:
+        g.run(W.APP_SSSP, W.Params(sched=W.SCHED_DENSE))
+        expect = g.read_results().copy()
+        for sched in (W.SCHED_PLAIN, W.SCHED_WEDGE):
+            for flags in (0, W.FLAG_GRAPH, W.FLAG_TIMING):
+                st = g.run(W.APP_SSSP, W.Params(sched=sched, flags=flags))
+                assert st["iterations"] > 32
+                assert np.array_equal(g.read_results(), expect), (sched, flags)

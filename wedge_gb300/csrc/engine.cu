@@ -313,18 +313,28 @@ __global__ void sym_check_kernel(const uint32_t* src, const uint32_t* dst, uint6
     }
 }
 
-// largest weight word (uint64 weights; the byte-wide copy applies below 256)
-__global__ void max_weight_kernel(const unsigned long long* w, uint64_t E, unsigned long long* out)
+// out[0]: largest weight word (uint64 weights; the byte-wide copy applies below
+// 256); out[1]: the sum of the weights as a double's bits, for their mean (any
+// order of addition: it scales SSSP's near bound)
+__global__ void weight_stats_kernel(const unsigned long long* w, uint64_t E, int f64, unsigned long long* out)
 {
     unsigned long long m = 0;
-    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x)
-        m = w[e] > m ? w[e] : m;
+    double sum = 0.0;
+    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x) {
+        const unsigned long long x = w[e];
+        m = x > m ? x : m;
+        sum += f64 ? __longlong_as_double((long long)x) : (double)x;
+    }
     for (int d = 16; d > 0; d >>= 1) {
         const unsigned long long y = __shfl_xor_sync(FULL, m, d);
         m = y > m ? y : m;
+        sum += __shfl_xor_sync(FULL, sum, d);
     }
-    if ((threadIdx.x & 31) == 0 && m)
-        atomicMax(out, m);
+    if ((threadIdx.x & 31) == 0) {
+        if (m)
+            atomicMax(out, m);
+        atomicAdd((double*)(out + 1), sum);
+    }
 }
 
 __global__ void narrow_weights_kernel(const unsigned long long* w, uint64_t E, uint8_t* w8)
@@ -605,20 +615,24 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
     const uint32_t cap = (uint32_t)h->num_sms * 16u;
 
     // input errors and the largest uint64 weight
-    unsigned long long *d_chk = nullptr, chk[2] = {0ull, 0ull};
+    unsigned long long *d_chk = nullptr, chk[3] = {0ull, 0ull, 0ull};
     WEDGE_CHECK(cudaMallocAsync((void**)&d_chk, sizeof(chk), st));
     WEDGE_CHECK(cudaMemsetAsync(d_chk, 0, sizeof(chk), st));
     if (E)
         validate_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, d_dst, E, V, grouped,
                                                                                  (int*)d_chk);
-    if (E && d_w && weight_kind == WEDGE_WEIGHTS_U64)
-        max_weight_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_w, E, d_chk + 1);
+    if (E && d_w)
+        weight_stats_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_w, E, weight_kind == WEDGE_WEIGHTS_F64,
+                                                                                 d_chk + 1);
     WEDGE_CHECK(cudaMemcpyAsync(chk, d_chk, sizeof(chk), cudaMemcpyDeviceToHost, st));
     WEDGE_CHECK(cudaStreamSynchronize(st));
     cudaFreeAsync(d_chk, st);
     // weights in one byte each where every uint64 weight is below 256: the pulls
     // stream 1 byte per in-edge instead of 8
     const bool byte_weights = E && d_w && weight_kind == WEDGE_WEIGHTS_U64 && chk[1] < 256ull;
+    double wsum;
+    memcpy(&wsum, &chk[2], sizeof(wsum));
+    g.wmean = E && wsum > 0.0 ? wsum / (double)E : 0.0; /* 0 for sums that are no number too */
     if (chk[0]) {
         cudaFreeAsync(d_dst, st);
         return WEDGE_ERR_FORMAT;
@@ -2761,6 +2775,9 @@ __device__ __forceinline__ void loop_reset(Ctrl* c)
     for (int i = 0; i < 3; ++i) {
         c->ln[i] = 0u;
         c->li[i] = 0u;
+        c->lf[i] = 0u;
+        c->lmin[i] = NONE64;
+        c->lfar[i] = 0ull;
         for (uint32_t j = 0; j < NCNT; ++j)
             c->lacc[i][j] = 0ull;
     }
@@ -3223,6 +3240,8 @@ __global__ void init_kernel(DevGraph g, DevState s, uint32_t app, uint32_t topen
             s.front[b * s.front_stride + i] = 0u;
         if (s.visv)
             s.visv[i] = 0u;
+        if (s.far)
+            s.far[i] = 0u;
     }
     const uint64_t cwords = ((uint64_t)g.T + 7) / 8;
     for (uint64_t i = tid; i < cwords; i += stride)
@@ -3358,11 +3377,26 @@ __global__ void init_root_kernel(DevGraph g, DevState s, uint32_t app, uint64_t 
 // cleared), two lists, three sets of counters (the one two iterations back is
 // cleared while no block reads it).  Every block takes the iteration's
 // decision for itself from the summed counters; the last one writes it down.
+// A long SSSP (past NEAR_ITER iterations: grids and roads; an R-MAT graph takes
+// 10-15 and would only take more) visits the near vertices first: while its
+// changed vertices have more than NEAR_MASS out-edges (fewer cost no more than
+// the barrier), those whose distance is above a bound wait in a far list.
+// When the near ones have fewer, the bound rises by NEAR_STEP mean weights, at
+// least from the least distance waiting, and the far list is gone through.  A
+// far vertex's distance is often lowered before its turn, so its out-edges are
+// relaxed once or twice instead of 13 times (4096^2 grid: 78 M out-edges
+// relaxed for 1.9 G; 16.1 -> 6.6 ms.  Steps of 1/2, 2 and 4 mean weights: 7.4,
+// 6.9, 9.1 ms; masses of 2^14, 2^17, 2^18: 6.8, 6.6, 7.1 ms).  Before a dense
+// pull the waiting vertices join the frontier bitmap.
+//
 // Graphs of at most LOOP_SMALL_EDGES in-edges run whole in the launch: there a
 // dense iteration is no more work than a Wedge one, and the launches were all
 // the time (BFS at scale 12: 182 us).
 constexpr uint32_t LOOP_LONG = 128;   // out-edges of one vertex a warp takes at once: one round of four per lane
-constexpr uint32_t LOOP_BUF = 128;    // listed vertices a warp keeps in shared memory
+constexpr uint32_t LOOP_BUF = 96;     // listed vertices a warp keeps in shared memory (each list)
+constexpr unsigned long long NEAR_MASS = 1ull << 16;
+constexpr double NEAR_STEP = 1.0;
+constexpr uint32_t NEAR_ITER = 16;
 constexpr uint32_t BARRIER_TRIES = 1u << 22;
 enum : uint32_t { ERR_BARRIER_TIMEOUT = 4u };
 
@@ -3391,6 +3425,11 @@ __device__ __forceinline__ bool grid_barrier(Ctrl* c, uint32_t& target, uint32_t
     __syncthreads();
     return *ok != 0u;
 }
+
+template <bool B>
+struct BoolTag {
+    static constexpr bool value = B;
+};
 
 // The running totals of a traversal while sparse_loop_kernel iterates (one
 // thread): decide_block's record, without a read of device memory.
@@ -3464,8 +3503,16 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
     using val_t = typename CurT<APP>::type;
     __shared__ uint32_t sh_pre[WARPS][32], sh_beg[WARPS][32], sh_buf[WARPS][LOOP_BUF];
     __shared__ val_t sh_val[WARPS][32];
+    __shared__ uint32_t sh_fbuf[APP == WEDGE_APP_SSSP ? WARPS : 1][LOOP_BUF]; /* for the far list */
     __shared__ unsigned long long sh_acc[NCNT];
-    __shared__ uint32_t sh_ok, sh_n[3];
+    __shared__ uint32_t sh_ok, sh_n[4];
+    // SSSP: what every block knows of the sorting-out, computed by thread 0
+    __shared__ struct {
+        unsigned long long bound, listed, waiting, far_min; /* far_min: the least distance waiting (none waiting: the
+                                                               least one the last iteration changed) */
+        uint32_t release, nfar;                             /* far lists begun; vertices of the one whose turn it is */
+    } so;
+    __shared__ unsigned long long sh_far[2];
     Ctrl* c = s.ctrl;
     if (c->done)
         return;
@@ -3484,6 +3531,14 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
     uint32_t* my_beg = sh_beg[wib];
     val_t* my_val = sh_val[wib];
     uint32_t target = 0u, kept = 0u; /* kept: listed vertices in my_buf */
+    if (threadIdx.x == 0) {
+        so.bound = NONE64;
+        so.listed = c->mass;
+        so.waiting = 0ull;
+        so.far_min = NONE64;
+        so.release = 0u;
+        so.nfar = 0u;
+    }
     uint32_t* out_list = s.alist;
     uint2* out_items = s.items;
     uint32_t *out_n = &c->ln[0], *out_i = &c->li[0];
@@ -3589,10 +3644,43 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
     for (uint32_t step = 0;; ++step) {
         const uint32_t a = step % 3u, b = (step + 1u) % 3u;
         /* one warp of the block reads what all blocks read at once */
-        if (threadIdx.x < 3)
-            sh_n[threadIdx.x] = __ldcg(threadIdx.x == 0 ? &c->ln[a] : threadIdx.x == 1 ? &c->li[a] : &c->narrow_ovf);
+        if (threadIdx.x < 4)
+            sh_n[threadIdx.x] = __ldcg(threadIdx.x == 0   ? &c->ln[a]
+                                       : threadIdx.x == 1 ? &c->li[a]
+                                       : threadIdx.x == 2 ? &c->narrow_ovf
+                                                          : &c->lf[APP == WEDGE_APP_SSSP ? so.release % 3u : 0u]);
         __syncthreads();
         const uint32_t n = sh_n[0], ni = sh_n[1];
+        /* from one iteration before distances may be sorted out: that one finds the least */
+        const bool sorting = APP == WEDGE_APP_SSSP && iter + 1u >= NEAR_ITER && (so.waiting != 0ull || so.listed > NEAR_MASS / 4u);
+        if (APP == WEDGE_APP_SSSP && !sorting && threadIdx.x == 0)
+            so.far_min = NONE64;
+        if (sorting) {
+            if (threadIdx.x == 0) {
+                auto beyond = [&](unsigned long long from) { /* a step past a distance; the nearest vertex is never beyond it */
+                    const unsigned long long to =
+                        f64 ? (unsigned long long)__double_as_longlong(__longlong_as_double((long long)from) + NEAR_STEP * g.wmean)
+                            : from + (unsigned long long)(NEAR_STEP * g.wmean);
+                    return max(from, to);
+                };
+                const bool now = iter >= NEAR_ITER && mode == MODE_WEDGE && so.listed > NEAR_MASS;
+                if (!now)
+                    so.bound = NONE64; /* every vertex is near */
+                so.nfar = 0u;
+                if (so.waiting != 0ull && (!now || so.listed - so.waiting < NEAR_MASS)) {
+                    so.nfar = sh_n[3];
+                    ++so.release; /* from here on far vertices go to the other buffer */
+                    if (now)
+                        so.bound = beyond(max(so.bound, so.far_min));
+                    so.far_min = NONE64;
+                } else if (so.waiting == 0ull) {
+                    if (now && so.bound == NONE64 && so.far_min != NONE64)
+                        so.bound = beyond(so.far_min);
+                    so.far_min = NONE64;
+                }
+            }
+            __syncthreads();
+        }
         const uint32_t half = step & 1u;
         const uint32_t* list = s.alist + (half ? s.alist_stride : 0ull);
         const uint2* items = s.items + (half ? s.item_stride : 0ull);
@@ -3609,18 +3697,53 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
         if (tid == 0u) { /* counters no block reads any more */
             c->ln[(step + 2u) % 3u] = 0u;
             c->li[(step + 2u) % 3u] = 0u;
+            if (sorting && so.nfar)
+                c->lf[(so.release + 1u) % 3u] = 0u;
+            c->lmin[b] = NONE64;
+            c->lfar[b] = 0ull;
         }
         if (blockIdx.x == 0 && threadIdx.x < NCNT)
             c->lacc[b][threadIdx.x] = 0ull;
         for (uint32_t i = tid; i < nwords; i += nthr)
             old[i] = 0u;
 
+        unsigned long long far_mass = 0ull, least = NONE64; /* sorting: change of the waiting out-edges, least distance */
+        auto work = [&](auto tag) {
+        constexpr bool FAR = decltype(tag)::value;
+        const unsigned long long bound = FAR ? so.bound : NONE64;
+        const uint32_t release = FAR ? so.release : 0u, nfar = FAR ? so.nfar : 0u;
+        const uint32_t* far_src = s.far_list + ((release & 1u) ? 0ull : s.alist_stride); /* release - 1 */
+        uint32_t* far_dst = s.far_list + ((release & 1u) ? s.alist_stride : 0ull);
+        // vertex v to the far list; called by all lanes
+        uint32_t far_kept = 0u;
+        auto flush_far = [&]() {
+            __syncwarp();
+            uint32_t at = 0u;
+            if (lane == 0)
+                at = atomicAdd(&c->lf[release % 3u], far_kept);
+            at = __shfl_sync(FULL, at, 0);
+            for (uint32_t q = (uint32_t)lane; q < far_kept; q += 32u)
+                far_dst[at + q] = sh_fbuf[APP == WEDGE_APP_SSSP ? wib : 0][q];
+            far_kept = 0u;
+            __syncwarp();
+        };
+        auto put_far = [&](bool on, uint32_t v) {
+            const uint32_t m = __ballot_sync(FULL, on);
+            if (m) {
+                if (far_kept + 32u > LOOP_BUF)
+                    flush_far();
+                if (on)
+                    sh_fbuf[APP == WEDGE_APP_SSSP ? wib : 0][far_kept + (uint32_t)__popc(m & ((1u << lane) - 1u))] = v;
+                far_kept += (uint32_t)__popc(m);
+            }
+        };
         // Four out-edges per lane (of vertices with values x), in stages, so that
         // the four chains are in flight together: destinations; their present
         // state; the atomics that lower it; the new frontier bits and
         // out-degrees; the list.
         auto relax4 = [&](const bool (&on)[4], const val_t (&x)[4], const uint32_t (&e)[4]) {
             uint32_t d[4], od[4], o[4];
+            val_t nd[4]; /* SSSP: the new distances */
             bool low[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u)
@@ -3656,7 +3779,6 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
                 for (int u = 0; u < 4; ++u)
                     low[u] = low[u] && x[u] < p[u];
             } else {
-                unsigned long long nd[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     const unsigned long long wv = !on[u] ? 0ull : g.cw8 ? (unsigned long long)g.cw8[e[u]] : g.cw[e[u]];
@@ -3708,12 +3830,14 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
             }
             if (!__any_sync(FULL, low[0] || low[1] || low[2] || low[3]))
                 return;
+            bool wait[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 o[u] = FULL;
                 od[u] = 0u;
+                wait[u] = FAR && low[u] && (unsigned long long)nd[u] > bound;
                 if (low[u]) {
-                    o[u] = atomicOr(&nxt[d[u] >> 5], 1u << (d[u] & 31u));
+                    o[u] = atomicOr(&(wait[u] ? s.far : nxt)[d[u] >> 5], 1u << (d[u] & 31u));
                     od[u] = g.outdeg[d[u]];
                     if (APP == WEDGE_APP_BFS || (APP == WEDGE_APP_CC && x[u] == 0u)) { /* visited; label 0 is final */
                         const uint32_t k = g.dst_ident ? d[u] : g.dst_index[d[u]];
@@ -3723,16 +3847,30 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                occ += o[u] == 0u ? 1u : 0u;
-                const bool first = low[u] && !((o[u] >> (d[u] & 31u)) & 1u);
+                const uint32_t bit = 1u << (d[u] & 31u);
+                const bool first = low[u] && !(o[u] & bit);
                 if (first) {
-                    mass += od[u];
                     ++act;
                     const uint32_t bk = degree_bucket(od[u]);
                     if (bk < 3u)
                         degs += 1ull << (21u * bk);
                 }
-                append(first, d[u], od[u]);
+                if constexpr (FAR) {
+                    if (low[u] && (wait[u] || bound == NONE64))
+                        least = min(least, (unsigned long long)nd[u]);
+                    if (wait[u]) {
+                        if (first)
+                            far_mass += od[u];
+                    } else if (low[u] && (s.far[d[u] >> 5] & bit) && (atomicAnd(&s.far[d[u] >> 5], ~bit) & bit)) {
+                        far_mass -= od[u]; /* it waits no longer */
+                    }
+                    put_far(first && wait[u], d[u]);
+                }
+                const bool list_it = first && !wait[u];
+                occ += o[u] == 0u && list_it ? 1u : 0u;
+                if (list_it)
+                    mass += od[u];
+                append(list_it, d[u], od[u]);
             }
         };
         auto value = [&](uint32_t v) -> val_t {
@@ -3765,20 +3903,55 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
             if (lane == 0)
                 edges += hi - lo;
         }
-        // up to 32 listed vertices a warp, fewer while that leaves warps without any
-        const uint32_t chunk = min(32u, max(1u, (n + nw - 1u) / nw));
-        for (uint32_t i0 = gw * chunk; i0 < n; i0 += nw * chunk) {
+        // up to 32 listed vertices a warp, fewer while that leaves warps without any;
+        // the far list after the near one
+        const uint32_t both = n + nfar, chunk = min(32u, max(1u, (both + nw - 1u) / nw));
+        for (uint32_t i0 = gw * chunk; i0 < both; i0 += nw * chunk) {
             const uint32_t i = i0 + (uint32_t)lane;
-            uint32_t lo = 0u, len = 0u;
+            uint32_t lo = 0u, len = 0u, v = 0u, od = 0u;
+            bool wait = false, later = false;
             __syncwarp();
-            if ((uint32_t)lane < chunk && i < n) {
-                const uint32_t v = list[i];
+            if ((uint32_t)lane < chunk && i < both) {
+                const bool from_far = i >= n;
+                v = from_far ? far_src[i - n] : list[i];
                 lo = (uint32_t)g.csri_off[v];
                 len = (uint32_t)g.csri_off[v + 1u] - lo;
-                my_val[lane] = value(v);
+                const val_t x = value(v);
+                my_val[lane] = x;
+                if constexpr (FAR) {
+                    const uint32_t bit = 1u << (v & 31u);
+                    if (from_far) {
+                        /* a vertex listed twice is taken once: its bit says that its out-edges are in `waiting` */
+                        if (!(atomicAnd(&s.far[v >> 5], ~bit) & bit)) { /* taken meanwhile, as a near vertex */
+                            len = 0u;
+                        } else if (x <= bound) {
+                            far_mass -= len;
+                            if (len > LOOP_LONG) { /* as items, next */
+                                later = !(atomicOr(&nxt[v >> 5], bit) & bit);
+                                od = len;
+                                mass += later ? od : 0u;
+                                len = 0u;
+                            }
+                        } else { /* waits on; listed by another warp meanwhile: counted twice */
+                            wait = !(atomicOr(&s.far[v >> 5], bit) & bit);
+                            far_mass -= wait ? 0u : len;
+                            least = min(least, (unsigned long long)x);
+                            len = 0u;
+                        }
+                    } else if (x > bound) { /* the first step's list is not sorted out yet */
+                        wait = !(atomicOr(&s.far[v >> 5], bit) & bit);
+                        least = min(least, (unsigned long long)x);
+                        far_mass += wait ? len : 0u;
+                        len = 0u;
+                    }
+                }
                 if (APP == WEDGE_APP_BFS)
                     atomicOr(&s.visv[v >> 5], 1u << (v & 31u));
                 ++dsts;
+            }
+            if constexpr (FAR) {
+                put_far(wait, v);
+                append(later, v, od);
             }
             uint32_t incl = len;
 #pragma unroll
@@ -3812,11 +3985,26 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
                 relax4(on, x, e);
             }
         }
+        if (FAR && far_kept)
+            flush_far();
+        };
+        if constexpr (APP == WEDGE_APP_SSSP) {
+            if (sorting)
+                work(BoolTag<true>{});
+            else
+                work(BoolTag<false>{});
+        } else {
+            work(BoolTag<false>{});
+        }
         flush();
         // the iteration's counters
         __syncthreads(); /* cnt of the last iteration is read */
         if (threadIdx.x < NCNT)
             sh_acc[threadIdx.x] = 0ull;
+        if (threadIdx.x == 32) {
+            sh_far[0] = NONE64;
+            sh_far[1] = 0ull;
+        }
         __syncthreads();
         if (__any_sync(FULL, (edges | dsts) != 0u)) {
             const unsigned long long v[NCNT] = {
@@ -3828,16 +4016,43 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
                 for (uint32_t j = 0; j < NCNT; ++j)
                     if (v[j])
                         atomicAdd(&sh_acc[j], v[j]);
+            if (sorting) {
+                far_mass = warp_sum_u64(far_mass);
+                for (int q = 16; q > 0; q >>= 1)
+                    least = min(least, __shfl_xor_sync(FULL, least, q));
+                if (lane == 0 && far_mass)
+                    atomicAdd(&sh_far[1], far_mass); /* modulo 2^64: it may be negative */
+                if (lane == 0 && least != NONE64)
+                    atomicMin(&sh_far[0], least);
+            }
         }
         __syncthreads();
         if (threadIdx.x < NCNT && sh_acc[threadIdx.x])
             atomicAdd(&c->lacc[a][threadIdx.x], sh_acc[threadIdx.x]);
+        if (sorting && threadIdx.x == 32) {
+            if (sh_far[0] != NONE64)
+                atomicMin(&c->lmin[a], sh_far[0]);
+            if (sh_far[1])
+                atomicAdd(&c->lfar[a], sh_far[1]);
+        }
         if (!grid_barrier(c, target, &sh_ok))
             return;
         // the decision, the same in every block; block 0 writes it down
         if (threadIdx.x < NCNT)
             sh_acc[threadIdx.x] = __ldcg(&c->lacc[a][threadIdx.x]);
+        if (sorting && threadIdx.x >= 32 && threadIdx.x < 34)
+            sh_far[threadIdx.x - 32] = __ldcg(threadIdx.x == 32 ? &c->lmin[a] : &c->lfar[a]);
         __syncthreads();
+        if (APP == WEDGE_APP_SSSP && threadIdx.x == 0) {
+            if (sorting) { /* the waiting vertices are active too */
+                so.far_min = min(so.far_min, sh_far[0]);
+                so.waiting += sh_far[1];
+                sh_acc[CNT_MASS] += so.waiting;
+            }
+            so.listed = sh_acc[CNT_MASS];
+        }
+        if (APP == WEDGE_APP_SSSP)
+            __syncthreads();
         unsigned long long cnt[NCNT];
 #pragma unroll
         for (uint32_t j = 0; j < NCNT; ++j)
@@ -3858,12 +4073,20 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
                 return;
             mode = *(volatile unsigned int*)&c->mode;
         }
-        if (!next.done && !small && mode != MODE_WEDGE && APP == WEDGE_APP_BFS) { /* a dense pull takes over */
-            cur = cur_front(s, parity);
-            for (uint32_t i = tid; i < nwords; i += nthr)
-                s.visv[i] |= cur[i];
+        const bool leave = step + 1u == max_steps || (!small && mode != MODE_WEDGE);
+        if (!next.done && leave && (APP == WEDGE_APP_BFS || (sorting && so.release + so.waiting != 0ull))) {
+            /* another launch takes over: the waiting vertices join the frontier */
+            uint32_t* fr = s.front + parity * s.front_stride; /* this iteration's bitmap */
+            for (uint32_t i = tid; i < nwords; i += nthr) {
+                if (APP == WEDGE_APP_BFS) {
+                    s.visv[i] |= fr[i];
+                } else {
+                    fr[i] |= s.far[i];
+                    s.far[i] = 0u;
+                }
+            }
         }
-        if (next.done || step + 1u == max_steps || (!small && mode != MODE_WEDGE))
+        if (next.done || leave)
             return;
     }
 }
@@ -5099,6 +5322,8 @@ static int ensure_state(wedge_graph* h, int app, int precision)
         const uint64_t nitems = build_items > loop_items ? build_items : loop_items;
         if ((rc = dalloc(h, &s.front, 3 * nwords, true)) ||
             (app == WEDGE_APP_BFS && g.csr && (rc = dalloc(h, &s.visv, nwords, true))) ||
+            (app == WEDGE_APP_SSSP && fused_loop(h) &&
+             ((rc = dalloc(h, &s.far, nwords, true)) || (rc = dalloc(h, &s.far_list, 2 * (V + 1), true)))) ||
             (rc = dalloc(h, &s.chunk_bits, (uint64_t)g.T / TILES_PER_WORD + REGION_WORDS + 2, true)) ||
             (rc = dalloc(h, &s.summary, (uint64_t)g.T / TILES_PER_REGION / 32 + 2, true)) ||
             (rc = dalloc(h, &s.tile_list, (uint64_t)g.T + 1, true)) ||

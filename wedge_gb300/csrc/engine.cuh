@@ -115,7 +115,9 @@ struct Ctrl {
     unsigned int bodies;               // rounds of the fused traversal loop
     unsigned int bar;                  // sparse_loop_kernel: grid-barrier arrivals, and per step modulo 3
     unsigned int ln[3], li[3];         // vertices and items listed for it,
-    unsigned long long lacc[3][NCNT];  // and its counters
+    unsigned long long lacc[3][NCNT];  // its counters; SSSP: the least distance it sorted out and by how many
+    unsigned long long lmin[3], lfar[3]; // out-edges it changed the waiting ones; by far list modulo 3:
+    unsigned int lf[3];                // vertices listed
     double pr_total;                   // sum of all accumulators (phase_vertex_pr.c:161); compensated FP32:
                                        // the total the next iteration uses
     double pr_prev;                    // compensated FP32: the total the last iteration used
@@ -131,6 +133,7 @@ struct DevGraph {
     uint32_t nwide;            // destinations spanning more than SPLIT_SERIAL tile boundaries (back of the split lists)
     uint32_t sym;              // every edge's reverse is an edge too: CC propagates engine ids (see cc_best_kernel)
     uint32_t csr;              // csri holds destinations (Epad < 2^32), else chunk ids
+    double wmean;              // mean weight (0: none)
     uint32_t shard;            // a destination-range shard (wedge_cuda_load_shard)
     const uint32_t* src;
     const unsigned long long* w;
@@ -206,6 +209,8 @@ struct DevState {
                                    // buffers item_stride apart (sparse_loop_kernel)
     uint32_t* alist;               // vertices the last pull activated: Wedge build, or two buffers alist_stride apart
     uint64_t alist_stride, item_stride;
+    uint32_t* far;                 // V-bit, SSSP: changed vertices that wait (sparse_loop_kernel), and
+    uint32_t* far_list;            // two lists of them alist_stride apart
     uint32_t* cc_best;             // CC on a symmetric graph: least caller id of the component a label represents
     const uint32_t* cc_map;        // results only: CC labels are looked up here (engine ids not yet converted)
     Ctrl* ctrl;
