@@ -499,10 +499,11 @@ static int relabel_by_degree(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d
     {
         cub::DoubleBuffer<unsigned long long> db(vk, vk2);
         size_t tb = 0;
-        WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(nullptr, tb, db, (long long)V, 0, 64, st));
+        /* by the degree alone: the sort is stable, and the keys start in id order */
+        WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(nullptr, tb, db, (long long)V, 32, 64, st));
         void* tmp = nullptr;
         WEDGE_CHECK(cudaMallocAsync(&tmp, tb ? tb : 1, st));
-        WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tb, db, (long long)V, 0, 64, st));
+        WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tb, db, (long long)V, 32, 64, st));
         cudaFreeAsync(tmp, st);
         permutation_kernel<<<grid_for(V, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(db.Current(), V, *new2old, *old2new);
     }
