@@ -161,3 +161,49 @@ def test_near_vertices_first(engine_lib, weights):
                 st = g.run(W.APP_SSSP, W.Params(sched=sched, flags=flags))
                 assert st["iterations"] > 32
                 assert np.array_equal(g.read_results(), expect), (sched, flags)
+
+
+def plain_pagerank(V, src, dst, iterations, damping):
+    outdeg = np.bincount(src, minlength=V).astype(np.float64)
+    outdeg[outdeg == 0] = V
+    outdeg = outdeg.astype(np.longdouble)
+    rank = (np.longdouble(1.0) / V) / outdeg
+    for _ in range(iterations):
+        acc = np.zeros(V, np.longdouble)  # a plain double sum of a hub's in-edges is off by more than the engine's
+        np.add.at(acc, dst, rank[src])
+        rank = ((acc + (1.0 - acc.sum()) / V) * damping + (1.0 - damping) / V) / outdeg
+    return rank.astype(np.float64)
+
+
+@pytest.mark.parametrize("iterations", [1, 2, 5])
+@pytest.mark.parametrize("degrees", ["one", "tile", "hub", "mixed"])
+def test_pagerank_in_one_launch(engine_lib, iterations, degrees):
+    """in-degrees around the tiles (256 and 512 in-edges): a tile of 256 or more
+    destinations, destinations that end with a tile, that span two, nine and more;
+    vertices without in-edges, without out-edges and without both; odd and even
+    iteration counts (double-buffered ranks), and the phases after a run"""
+    W = engine_lib
+    rng = np.random.default_rng(iterations)
+    ind = {"one": np.ones(1500, np.int64), "tile": np.array([256, 512, 255, 1, 257, 511, 513, 256, 3, 253]),
+           "hub": np.array([5, 700, 4607, 4608, 20_000, 1, 2560]), "mixed": rng.integers(0, 60, 900)}[degrees]
+    V = len(ind) + 700
+    d = np.repeat(np.arange(len(ind)), ind)
+    s = rng.integers(len(ind) // 2, V - 50, len(d))
+    order = np.lexsort((s, d))
+    s, d = s[order].astype(np.uint32), d[order].astype(np.uint32)
+    expect = plain_pagerank(V, s.astype(np.int64), d.astype(np.int64), iterations, 0.85)
+    with W.Graph.from_edges(V, s, d) as g:
+        for prec, tol in ((W.PREC_FP64, 1e-13), (W.PREC_FP32C, 1e-6)):
+            for flags in (0, W.FLAG_GRAPH, W.FLAG_TIMING):
+                p = W.Params(num_iterations=iterations, damping=0.85, precision=prec, flags=flags)
+                st = g.run(W.APP_PR, p)
+                got = g.read_results().view(np.float64).copy()
+                assert np.abs(got - expect).sum() <= tol * np.abs(expect).sum()
+                assert abs(st["pr_sum"] - 1.0) < 1e-6 and st["iterations"] == iterations
+            # one more iteration by phases from the FP64 run's ranks
+        g.run(W.APP_PR, W.Params(num_iterations=iterations, damping=0.85))
+        p = W.Params(damping=0.85)
+        g.run_phase(W.APP_PR, W.PHASE_PULL_DENSE, p)
+        g.run_phase(W.APP_PR, W.PHASE_VERTEX_PR, p)
+        more = plain_pagerank(V, s.astype(np.int64), d.astype(np.int64), iterations + 1, 0.85)
+        assert np.abs(g.read_results().view(np.float64) - more).sum() <= 1e-13 * np.abs(more).sum()

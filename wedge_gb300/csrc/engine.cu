@@ -104,10 +104,7 @@ static void free_state(wedge_graph* h)
         h->graph_exec = nullptr;
         h->graph_app = -1;
     }
-    if (h->pr_exec) {
-        cudaGraphExecDestroy(h->pr_exec);
-        h->pr_exec = nullptr;
-    }
+    h->pr_flip = 0;
 }
 
 void free_handle(wedge_graph* h)
@@ -254,6 +251,76 @@ __global__ void split_kernel(const unsigned long long* dst_off, uint32_t Vne, ui
             split_t1[i] = t1;
         }
     }
+}
+
+// The same lists in ascending order of the destinations (PageRank's FP32 total
+// and pr_loop_kernel add up ranks in list order: an order that atomics decide
+// would change their last bits from load to load).  Every tile boundary that a
+// destination crosses first is one split: its flag (1, or 1 << 32 for a long
+// one), by an exclusive scan its place.
+__device__ __forceinline__ unsigned long long split_at(const uint32_t* tile_dst0, const unsigned long long* dst_off, uint32_t t,
+                                                       uint32_t T, uint64_t E, uint32_t tile_e, uint32_t& k, uint32_t& t1)
+{
+    const uint64_t p = (uint64_t)(t + 1u) * tile_e; /* the boundary after tile t */
+    if (t + 1u >= T || p >= E)
+        return 0ull;
+    k = tile_dst0[(uint64_t)(t + 1u) * (tile_e / TILE)];
+    const unsigned long long lo = dst_off[k];
+    if (lo >= p || lo < p - tile_e)
+        return 0ull; /* starts there, or crossed an earlier boundary */
+    t1 = (uint32_t)((dst_off[k + 1u] - 1u) / tile_e);
+    return t1 - t <= SPLIT_SERIAL ? 1ull : 1ull << 32;
+}
+
+__global__ void split_flag_kernel(const uint32_t* tile_dst0, const unsigned long long* dst_off, uint32_t T, uint64_t E,
+                                  uint32_t tile_e, unsigned long long* flag)
+{
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t <= T; t += gridDim.x * blockDim.x) {
+        uint32_t k, t1;
+        flag[t] = t < T ? split_at(tile_dst0, dst_off, t, T, E, tile_e, k, t1) : 0ull;
+    }
+}
+
+__global__ void split_fill_kernel(const uint32_t* tile_dst0, const unsigned long long* dst_off, uint32_t T, uint64_t E,
+                                  uint32_t tile_e, const unsigned long long* pos, uint32_t* split_k, uint32_t* split_t0,
+                                  uint32_t* split_t1)
+{
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
+        uint32_t k, t1;
+        const unsigned long long f = split_at(tile_dst0, dst_off, t, T, E, tile_e, k, t1);
+        if (f) {
+            const uint32_t i = f == 1ull ? (uint32_t)pos[t] : T - 1u - (uint32_t)(pos[t] >> 32);
+            split_k[i] = k;
+            split_t0[i] = t;
+            split_t1[i] = t1;
+        }
+    }
+}
+
+// out[0]: vertices with out-edges, ids [0, out[0]) in the descending degree
+// order; out[1]: destinations among them
+__global__ void dangling_kernel(const uint32_t* outdeg, uint64_t V, const uint32_t* dst_id, uint32_t Vne, unsigned int* out)
+{
+    uint32_t lo = 0, hi = (uint32_t)V;
+    while (lo < hi) {
+        const uint32_t mid = lo + (hi - lo) / 2u;
+        if (outdeg[mid] != 0u)
+            lo = mid + 1u;
+        else
+            hi = mid;
+    }
+    out[0] = lo;
+    const uint32_t Vout = lo;
+    lo = 0;
+    hi = Vne;
+    while (lo < hi) {
+        const uint32_t mid = lo + (hi - lo) / 2u;
+        if (dst_id[mid] < Vout)
+            lo = mid + 1u;
+        else
+            hi = mid;
+    }
+    out[1] = lo;
 }
 
 // vertex -> compressed destination index (preset to NONE32: no in-edges)
@@ -755,13 +822,14 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
     if ((rc = dalloc(h, &split_k, g.T)) || (rc = dalloc(h, &split_t0, g.T)) || (rc = dalloc(h, &split_t1, g.T)))
         return rc;
     unsigned int* d_cnt = nullptr;
-    WEDGE_CHECK(cudaMallocAsync((void**)&d_cnt, 2 * sizeof(unsigned int), st));
-    WEDGE_CHECK(cudaMemsetAsync(d_cnt, 0, 2 * sizeof(unsigned int), st));
+    WEDGE_CHECK(cudaMallocAsync((void**)&d_cnt, 4 * sizeof(unsigned int), st));
+    WEDGE_CHECK(cudaMemsetAsync(d_cnt, 0, 4 * sizeof(unsigned int), st));
     if (Vne)
         split_kernel<<<grid_for(Vne, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(dst_off, Vne, g.T, TILE, split_k, split_t0,
                                                                              split_t1, d_cnt);
-    unsigned int nsplit[2] = {0, 0};
-    WEDGE_CHECK(cudaMemcpyAsync(nsplit, d_cnt, 2 * sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
+    dangling_kernel<<<1, 1, 0, st>>>(outdeg, V, dst_id, Vne, d_cnt + 2);
+    unsigned int nsplit[4] = {0, 0, 0, 0};
+    WEDGE_CHECK(cudaMemcpyAsync(nsplit, d_cnt, 4 * sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
     // dst_id ascends, so it is the identity when its last entry is Vne-1 (symmetric
     // graphs after the degree relabelling: in-degree > 0 exactly for ids < Vne)
     uint32_t last_dst = 0;
@@ -774,6 +842,8 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
     WEDGE_CHECK(cudaGetLastError());
     g.nsplit = nsplit[0];
     g.nwide = nsplit[1];
+    g.Vout = nsplit[2];
+    g.Viso = (uint32_t)(V - nsplit[2]) - (Vne - nsplit[3]);
     g.dst_ident = (Vne && last_dst == Vne - 1) ? 1u : 0u;
     g.sym = h_asym ? 0u : 1u;
     g.dst_id = dst_id;
@@ -4184,19 +4254,25 @@ __global__ void pr_init_kernel(DevGraph g, DevState s, uint32_t max_iter)
 // counterpart of the ordered merge of phases.c:71-114).  A thread sums each of
 // the nshort splits at the front of the lists serially (most span one tile
 // boundary); a warp sums each of the nwide at the back (hubs).
-template <class Tail, class Head>
-__device__ __forceinline__ void merge_splits(const DevGraph& g, double* acc, const uint32_t* split_k,
-                                             const uint32_t* split_t0, const uint32_t* split_t1, uint32_t nshort,
-                                             uint32_t nwide, uint32_t cap, Tail tail, Head head)
+// put(k, sum) takes each one's sum, on one lane.  tid: this thread's number of nthreads.
+template <class Tail, class Head, class Put>
+__device__ __forceinline__ void merge_splits(const uint32_t* split_k, const uint32_t* split_t0, const uint32_t* split_t1,
+                                             uint32_t nshort, uint32_t nwide, uint32_t cap, uint32_t tid, uint32_t nthreads, Tail tail,
+                                             Head head, Put put)
 {
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t nthreads = gridDim.x * blockDim.x;
     for (uint32_t i = tid; i < nshort; i += nthreads) {
         const uint32_t t0 = split_t0[i], t1 = split_t1[i], k = split_k[i];
+        double p[SPLIT_SERIAL]; /* all loads in flight together */
+#pragma unroll
+        for (uint32_t j = 0; j < SPLIT_SERIAL; ++j)
+            p[j] = t0 + j < t1 ? tail(t0 + j) : 0.0;
+        const double h = head(t1);
         double x = 0.0;
-        for (uint32_t t = t0; t < t1; ++t)
-            x = __dadd_rn(x, tail(t));
-        acc[g.dst_ident ? k : g.dst_id[k]] = __dadd_rn(x, head(t1));
+#pragma unroll
+        for (uint32_t j = 0; j < SPLIT_SERIAL; ++j)
+            if (t0 + j < t1)
+                x = __dadd_rn(x, p[j]);
+        put(k, __dadd_rn(x, h));
     }
     const int lane = threadIdx.x & 31;
     for (uint32_t j = tid >> 5; j < nwide; j += nthreads >> 5) {
@@ -4214,10 +4290,8 @@ __device__ __forceinline__ void merge_splits(const DevGraph& g, double* acc, con
         for (; t < b; t += 32u)
             x0 = __dadd_rn(x0, tail(t));
         const double x = warp_sum_f64(__dadd_rn(__dadd_rn(x0, x1), __dadd_rn(x2, x3)));
-        if (lane == 0) {
-            const uint32_t k = split_k[i];
-            acc[g.dst_ident ? k : g.dst_id[k]] = __dadd_rn(x, head(b));
-        }
+        if (lane == 0)
+            put(split_k[i], __dadd_rn(x, head(b)));
     }
 }
 
@@ -4235,8 +4309,9 @@ __global__ void pr_finish_kernel(DevGraph g, DevState s, uint32_t nblocks, const
             log_iteration(s, c, cnt, 1u);
         }
     }
-    merge_splits(g, s.acc, g.split_k, g.split_t0, g.split_t1, g.nsplit, g.nwide, g.T, [&](uint32_t t) { return s.tail_part[t]; },
-                 [&](uint32_t t) { return s.head_part[t]; });
+    merge_splits(g.split_k, g.split_t0, g.split_t1, g.nsplit, g.nwide, g.T, blockIdx.x * blockDim.x + threadIdx.x,
+                 gridDim.x * blockDim.x, [&](uint32_t t) { return s.tail_part[t]; }, [&](uint32_t t) { return s.head_part[t]; },
+                 [&](uint32_t k, double x) { s.acc[g.dst_ident ? k : g.dst_id[k]] = x; });
 }
 
 // perform_vertex_phase_pr (phase_vertex_pr.c:26-77):
@@ -4639,39 +4714,32 @@ __global__ void __launch_bounds__(PULL_THREADS, 1) pr32_pull_kernel(DevGraph g, 
     }
 }
 
-// Destinations whose in-edges span tiles: the (sum, compensation) partials of
-// the tiles they continue through, then of the tile they end in, combined by
-// two-sum in tile order (the counterpart of the ordered merge of
-// phases.c:71-114), then their vertex phase; and the vertices with out-edges
-// but no in-edges, whose sum is 0.  Short splits take a thread each, long ones
-// (hubs) a warp each.  s.pmass[part0 + b] = the block's sum of new non-dangling ranks.
-__global__ void pr32_finish_kernel(DevGraph g, DevState s, uint32_t part0)
+// The destinations spanning the 512-edge tiles and those past a tile's staged
+// slots: put(k, sum) once for each.  Short splits take a thread, long ones (hubs)
+// a warp.  FLIGHT partials of a short split are loaded together: all of them in
+// pr_loop_kernel, which waits for the last; one in pr32_finish_kernel, where
+// most splits span one boundary and threads are plenty (8: 0.45 ms more per
+// PageRank at scale 26).
+template <uint32_t FLIGHT, class Put>
+__device__ __forceinline__ void pr32_splits(const DevState& s, uint32_t tid, uint32_t nthr, Put put)
 {
-    const Ctrl* c = s.ctrl;
-    float* nxt = s.rank32 + ((c->iter & 1u) ? 0ull : s.rstride);
-    const Pr32K K = pr32_constants(g, s, c->pr_total);
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t nthr = gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
-    F2 mass{0.0f, 0.0f};
-    auto finish = [&](uint32_t k, F2 sum) {
-        const uint32_t vtx = g.dst_ident ? k : g.dst_id[k];
-        const float inv = s.inv32[vtx];
-        const float r = pr32_rank(K, __fadd_rn(sum.s, sum.c));
-        nxt[vtx] = __fmul_rn(r, fabsf(inv));
-        if (inv > 0.0f)
-            mass = f2_add(mass, r);
-    };
     const AddF2 add;
     for (uint32_t i = tid; i < s.pnsplit; i += nthr) {
         const uint32_t t0 = s.psplit_t0[i], t1 = s.psplit_t1[i];
-        F2 x{0.0f, 0.0f};
-        for (uint32_t tt = t0; tt < t1; ++tt) {
-            const float2 p = s.ptail[tt];
-            x = add(x, F2{p.x, p.y});
-        }
         const float2 h = s.phead[t1];
-        finish(s.psplit_k[i], add(x, F2{h.x, h.y}));
+        F2 x{0.0f, 0.0f};
+        for (uint32_t tt = t0; tt < t1; tt += FLIGHT) {
+            float2 p[FLIGHT];
+#pragma unroll
+            for (uint32_t j = 0; j < FLIGHT; ++j)
+                p[j] = tt + j < t1 ? s.ptail[tt + j] : make_float2(0.0f, 0.0f);
+#pragma unroll
+            for (uint32_t j = 0; j < FLIGHT; ++j)
+                if (tt + j < t1)
+                    x = add(x, F2{p[j].x, p[j].y});
+        }
+        put(s.psplit_k[i], add(x, F2{h.x, h.y}));
     }
     for (uint32_t j = tid >> 5; j < s.pnwide; j += nthr >> 5) {
         const uint32_t i = s.pT - 1u - j;
@@ -4686,13 +4754,38 @@ __global__ void pr32_finish_kernel(DevGraph g, DevState s, uint32_t part0)
             x = add(x, F2{__shfl_xor_sync(FULL, x.s, d), __shfl_xor_sync(FULL, x.c, d)});
         if (lane == 0) {
             const float2 h = s.phead[b];
-            finish(s.psplit_k[i], add(x, F2{h.x, h.y}));
+            put(s.psplit_k[i], add(x, F2{h.x, h.y}));
         }
     }
     for (uint32_t i = tid; i < s.novf; i += nthr) { /* complete destinations past a tile's staged slots */
         const uint32_t k = s.ovf_list[i];
-        finish(k, F2{s.ovf_sum[k], 0.0f});
+        put(k, F2{s.ovf_sum[k], 0.0f});
     }
+}
+
+// Destinations whose in-edges span tiles: the (sum, compensation) partials of
+// the tiles they continue through, then of the tile they end in, combined by
+// two-sum in tile order (the counterpart of the ordered merge of
+// phases.c:71-114), then their vertex phase; and the vertices with out-edges
+// but no in-edges, whose sum is 0.  Short splits take a thread each, long ones
+// (hubs) a warp each.  s.pmass[part0 + b] = the block's sum of new non-dangling ranks.
+__global__ void pr32_finish_kernel(DevGraph g, DevState s, uint32_t part0)
+{
+    const Ctrl* c = s.ctrl;
+    float* nxt = s.rank32 + ((c->iter & 1u) ? 0ull : s.rstride);
+    const Pr32K K = pr32_constants(g, s, c->pr_total);
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t nthr = gridDim.x * blockDim.x;
+    F2 mass{0.0f, 0.0f};
+    auto finish = [&](uint32_t k, F2 sum) {
+        const uint32_t vtx = g.dst_ident ? k : g.dst_id[k];
+        const float inv = s.inv32[vtx];
+        const float r = pr32_rank(K, __fadd_rn(sum.s, sum.c));
+        nxt[vtx] = __fmul_rn(r, fabsf(inv));
+        if (inv > 0.0f)
+            mass = f2_add(mass, r);
+    };
+    pr32_splits<1>(s, tid, nthr, finish);
     const float r0 = pr32_rank(K, 0.0f);
     for (uint32_t i = tid; i < s.nz; i += nthr) {
         const uint32_t v = s.zlist[i];
@@ -4750,10 +4843,337 @@ __global__ void pr32_iso_kernel(DevGraph g, DevState s)
     }
 }
 
-// condition of the captured PageRank iteration loop
-__global__ void pr_loop_cond_kernel(DevState s, cudaGraphConditionalHandle handle)
+/* ------------------------------------------ PageRank iterations in one launch */
+//
+// pr_loop_kernel runs a whole PageRank in one cooperative launch: the initial
+// ranks, then per iteration the edge pull with the vertex phase of the
+// destinations inside one tile, a grid barrier, the destinations spanning
+// tiles, a second barrier, and the next total rank, which every block adds up
+// from the per-block sums in the same order.  As in the compensated-FP32
+// kernels above the total an iteration uses is the sum of the non-dangling
+// ranks it reads (S(i) = sum of acc(i)), so it is known before the pull and no
+// accumulator array is written.  Per iteration, before -> now: FP64 R-MAT scale
+// 16 31 -> 20 us, scale 22 489 -> 339 us; FP32 scale 16 37 -> 16 us, scale 20 72
+// -> 49 us.  Of the 20 us the two barriers take 3, the rest is this GPU's FP64
+// adds (a warp's occupies the SM's FP64 units for 16 cycles): tiles of 256
+// in-edges need fewer scan steps per in-edge than 128, the divisions are one
+// thread's, warps without a rank to sum leave the sum out.  Vertices are
+// numbered by descending out-degree, so the dangling ones are the ids from
+// g.Vout on.
+template <bool F64>
+struct PrPrec;
+template <>
+struct PrPrec<true> {
+    using rank_t = double;
+    using sum_t = double;
+    using add_t = AddF64;
+    static constexpr int epl = 8;
+    static constexpr uint32_t slots = 256; /* staged sums per warp: all of a tile's destinations */
+    struct K {
+        double corr, d, omd;
+    };
+    static __device__ __forceinline__ K constants(const DevGraph& g, const DevState& s, double total)
+    {
+        const double N = (double)g.V;
+        return K{__ddiv_rn(__dsub_rn(1.0, total), N), s.damping, __ddiv_rn(__dsub_rn(1.0, s.damping), N)};
+    }
+    /* phase_vertex_pr.c:57-72 */
+    static __device__ __forceinline__ double rank(const K& k, double sum)
+    {
+        return __dadd_rn(__dmul_rn(__dadd_rn(sum, k.corr), k.d), k.omd);
+    }
+    static __device__ __forceinline__ double scale(double r, double inv) { return __dmul_rn(r, inv); }
+    static __device__ __forceinline__ double value(double x) { return x; }
+    static __device__ __forceinline__ double first(const DevGraph& g) { return __ddiv_rn(1.0, (double)g.V); }
+    static __device__ __forceinline__ double add(double a, double x) { return __dadd_rn(a, x); }
+    static __device__ __forceinline__ double zero() { return 0.0; }
+    static __device__ __forceinline__ double total(double x) { return x; }
+};
+template <>
+struct PrPrec<false> {
+    using rank_t = float;
+    using sum_t = F2;
+    using add_t = AddF2;
+    static constexpr int epl = PR32_EPL;
+    static constexpr uint32_t slots = PR32_SLOTS; /* the others are finished from ovf_sum */
+    using K = Pr32K;
+    static __device__ __forceinline__ K constants(const DevGraph& g, const DevState& s, double total)
+    {
+        return pr32_constants(g, s, total);
+    }
+    static __device__ __forceinline__ float rank(const K& k, F2 sum) { return pr32_rank(k, __fadd_rn(sum.s, sum.c)); }
+    static __device__ __forceinline__ float rank(const K& k, float sum) { return pr32_rank(k, sum); }
+    static __device__ __forceinline__ float scale(float r, float inv) { return __fmul_rn(r, fabsf(inv)); }
+    static __device__ __forceinline__ float value(F2 x) { return __fadd_rn(x.s, x.c); }
+    static __device__ __forceinline__ float first(const DevGraph& g) { return __double2float_rn(__ddiv_rn(1.0, (double)g.V)); }
+    static __device__ __forceinline__ F2 add(F2 a, float x) { return f2_add(a, x); }
+    static __device__ __forceinline__ F2 zero() { return F2{0.0f, 0.0f}; }
+    static __device__ __forceinline__ double total(F2 x) { return __dadd_rn((double)x.s, (double)x.c); }
+};
+
+// bytes of the warps' staged sums
+template <bool F64>
+constexpr uint32_t pr_stage_bytes()
 {
-    cudaGraphSetConditional(handle, s.ctrl->iter < s.ctrl->max_iter ? 1u : 0u);
+    return (PULL_THREADS / 32) * PrPrec<F64>::slots * (uint32_t)sizeof(typename PrPrec<F64>::rank_t);
+}
+
+// a rank this launch writes in other iterations (no .nc), kept in L1
+__device__ __forceinline__ float ld_rank(const float* p)
+{
+    float r;
+    asm volatile("ld.global.L1::evict_last.f32 %0, [%1];" : "=f"(r) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ double ld_rank(const double* p)
+{
+    double r;
+    asm volatile("ld.global.L1::evict_last.f64 %0, [%1];" : "=d"(r) : "l"(p));
+    return r;
+}
+
+template <bool F64>
+__global__ void __launch_bounds__(PULL_THREADS, 1) pr_loop_kernel(DevGraph g, DevState s, uint32_t iters)
+{
+    using P = PrPrec<F64>;
+    using rank_t = typename P::rank_t;
+    using sum_t = typename P::sum_t;
+    constexpr int EPL = P::epl;
+    constexpr uint32_t TILE_E = 32u * EPL, Q = TILE_E / TILE, PR_SLOTS = P::slots;
+    __shared__ unsigned long long hub_bar;
+    __shared__ double sh_part[PULL_THREADS / 32];
+    __shared__ typename P::K sh_k; /* one thread's FP64 divisions: this GPU's FP64 units are slow */
+    __shared__ uint32_t sh_ok, sh_dsts;
+    extern __shared__ __align__(16) unsigned char pr_smem[];
+    Ctrl* c = s.ctrl;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
+    const uint32_t nw = nthr >> 5;
+    const uint32_t T = (uint32_t)((g.E + TILE_E - 1) / TILE_E);
+    // few tiles go to as many SMs; of many, an SM takes neighbouring ones (their gathers share its L1)
+    const uint32_t spread = (uint32_t)wib * gridDim.x + blockIdx.x, gw = T < 4u * nw ? spread : tid >> 5;
+    const uint32_t hub_bytes = s.hub_bytes;
+    const uint64_t stride = s.rstride;
+    rank_t* rank = F64 ? reinterpret_cast<rank_t*>(s.rank) : reinterpret_cast<rank_t*>(s.rank32);
+    const rank_t* inv = F64 ? reinterpret_cast<const rank_t*>(s.inv_od) : reinterpret_cast<const rank_t*>(s.inv32);
+    const rank_t* hub = reinterpret_cast<const rank_t*>(pr_smem);
+    rank_t* my_sum = reinterpret_cast<rank_t*>(pr_smem + hub_bytes) + (uint32_t)wib * PR_SLOTS;
+    uint32_t target = 0u, phase = 0u;
+    if (threadIdx.x == 0) {
+        sh_dsts = 0u;
+        if (hub_bytes)
+            mbar_init(&hub_bar, 1u);
+    }
+    // execution_initialize_pr (execution_pr.c:380-392)
+    if (threadIdx.x == 0)
+        sh_part[0] = (double)P::first(g);
+    __syncthreads();
+    const rank_t r0 = (rank_t)sh_part[0];
+    for (uint64_t v = tid; v < g.V; v += nthr)
+        rank[v] = P::scale(r0, inv[v]);
+    double total = __dmul_rn((double)g.Vout, (double)r0), before = total;
+    if (!grid_barrier(c, target, &sh_ok))
+        return;
+    const unsigned long long pol = l2_evict_first_policy();
+    for (uint32_t it = 0; it < iters; ++it) {
+        const rank_t* cur = rank + ((it & 1u) ? stride : 0ull);
+        rank_t* nxt = rank + ((it & 1u) ? 0ull : stride);
+        if (threadIdx.x == 32)
+            sh_k = P::constants(g, s, total);
+        // ---- hub cache: ranks [0, hub_n) of the current buffer
+        if (hub_bytes && threadIdx.x == 0) {
+            asm volatile("fence.proxy.async;" ::: "memory"); /* the ranks were written by plain stores */
+            mbar_arrive_expect_tx(&hub_bar, hub_bytes);
+            for (uint32_t off = 0; off < hub_bytes; off += 32768u)
+                bulk_g2s(pr_smem + off, reinterpret_cast<const unsigned char*>(cur) + off, min(32768u, hub_bytes - off),
+                         &hub_bar);
+        }
+        __syncthreads();
+        const typename P::K K = sh_k;
+        uint32_t hub_lim = 0; /* cache entries this warp reads: 0 until the copy completed */
+        sum_t mass = P::zero();   /* new ranks of the non-dangling vertices */
+        uint32_t dsts = 0;
+        auto put = [&](uint32_t vtx, rank_t r) {
+            nxt[vtx] = P::scale(r, inv[vtx]);
+            if (vtx < g.Vout)
+                mass = P::add(mass, r);
+        };
+        uint32_t t = gw;
+        uint32_t k0n = 0, kendn = 0;
+        if (t < T) {
+            k0n = g.tile_dst0[(uint64_t)t * Q];
+            kendn = g.tile_dst0[((uint64_t)t + 1u) * Q];
+        }
+        for (; t < T; t += nw) {
+            const uint32_t k0 = k0n, kend = kendn;
+            if (t + nw < T) { /* the next tile's bounds, one tile ahead */
+                k0n = g.tile_dst0[(uint64_t)(t + nw) * Q];
+                kendn = g.tile_dst0[((uint64_t)(t + nw) + 1u) * Q];
+            }
+            if (hub_bytes && hub_lim == 0u) {
+                uint32_t ready = 0u;
+                if (lane == 0)
+                    ready = mbar_test_wait(&hub_bar, phase) ? 1u : 0u;
+                if (__shfl_sync(FULL, ready, 0))
+                    hub_lim = hub_bytes / (uint32_t)sizeof(rank_t);
+            }
+            const uint64_t base = (uint64_t)t * TILE_E;
+            uint32_t sa[EPL];
+            load_sources<EPL>(g, base, FULL, lane, sa, pol);
+            sum_t v[EPL];
+#pragma unroll
+            for (int q = 0; q < EPL; ++q) {
+                const uint32_t x = sa[q];
+                const rank_t y = (x < hub_lim) ? hub[x] : (x != NONE32) ? ld_rank(cur + x) : (rank_t)0;
+                if constexpr (F64)
+                    v[q] = y;
+                else
+                    v[q] = F2{y, 0.0f};
+            }
+            TileGeo<EPL> tg;
+            tile_geometry_bits<EPL>(g, base, t + 1u >= T, k0, kend, lane, tg);
+            dsts += tg.ndst;
+            seg_reduce<EPL>(v, tg, lane, typename P::add_t(), [&](uint32_t k, sum_t val, int kind) {
+                if (kind == EMIT_COMPLETE) {
+                    const uint32_t slot = k - tg.k0;
+                    if (slot < PR_SLOTS)
+                        my_sum[slot] = P::value(val);
+                    else if constexpr (!F64)
+                        s.ovf_sum[k] = P::value(val);
+                } else if constexpr (F64) {
+                    (kind == EMIT_HEAD ? s.head_part : s.tail_part)[t] = val;
+                } else {
+                    (kind == EMIT_HEAD ? s.phead : s.ptail)[t] = make_float2(val.s, val.c);
+                }
+            });
+            __syncwarp();
+            const uint32_t nd = tg.ndst;
+            const uint32_t jlo = tg.k0_fresh ? 0u : 1u;                      /* slot 0 began in an earlier tile */
+            const uint32_t jhi = min(tg.tail_cont ? nd - 1u : nd, PR_SLOTS); /* the last slot may continue */
+            for (uint32_t j = jlo + (uint32_t)lane; j < jhi; j += 32u) {
+                const uint32_t k = tg.k0 + j;
+                put(g.dst_ident ? k : g.dst_id[k], P::rank(K, my_sum[j]));
+            }
+            __syncwarp(); /* my_sum is rewritten by the next tile */
+        }
+        // vertices with out-edges and no in-edges: the sum is 0
+        {
+            const rank_t rz = P::rank(K, (rank_t)0);
+            for (uint32_t v = tid; v < g.Vout; v += nthr)
+                if (!((s.has_in[v >> 5] >> (v & 31u)) & 1u))
+                    put(v, rz);
+        }
+        // the cache is filled again after the barriers: its copy has landed by then
+        if (hub_bytes && threadIdx.x == 0 && !mbar_wait_bounded(&hub_bar, phase, HUB_WAIT_TRIES)) {
+            atomicOr(&c->error, ERR_HUB_TIMEOUT);
+            mbar_wait_bounded(&hub_bar, phase, HUB_WAIT_TRIES);
+        }
+        phase ^= 1u;
+        if (it == 0u && lane == 0)
+            atomicAdd(&sh_dsts, dsts);
+        if (!grid_barrier(c, target, &sh_ok))
+            return;
+        // ---- destinations whose in-edges span tiles, in tile order (phases.c:71-114)
+        if constexpr (F64) {
+            merge_splits(s.psplit_k, s.psplit_t0, s.psplit_t1, s.pnsplit, s.pnwide, s.pT, spread * 32u + (uint32_t)lane, nthr,
+                         [&](uint32_t tt) { return s.tail_part[tt]; }, [&](uint32_t tt) { return s.head_part[tt]; },
+                         [&](uint32_t k, double x) { put(g.dst_ident ? k : g.dst_id[k], P::rank(K, x)); });
+        } else {
+            pr32_splits<SPLIT_SERIAL>(s, spread * 32u + (uint32_t)lane, nthr, [&](uint32_t k, F2 x) { put(g.dst_ident ? k : g.dst_id[k], P::rank(K, x)); });
+        }
+        // ---- the block's sums of the new ranks, then the grid's
+        {
+            double m = 0.0;
+            if (__any_sync(FULL, P::value(mass) != (rank_t)0)) /* idle warps leave the FP64 units to the others */
+                m = warp_sum_f64(P::total(mass));
+            if (lane == 0)
+                sh_part[wib] = m;
+            __syncthreads();
+            if (wib == 0) {
+                m = warp_sum_f64(sh_part[lane]);
+                if (lane == 0)
+                    s.pmass[blockIdx.x] = m;
+            }
+        }
+        if (it == 0u && threadIdx.x == 0)
+            atomicAdd(&c->lacc[0][CNT_DSTS], (unsigned long long)sh_dsts);
+        if (!grid_barrier(c, target, &sh_ok))
+            return;
+        before = total;
+        if (wib == 0) { /* the sum of all blocks' parts, the same in every block */
+            double x = 0.0;
+            for (uint32_t i = (uint32_t)lane; i < gridDim.x; i += 32u)
+                x = __dadd_rn(x, __ldcg(&s.pmass[i]));
+            x = warp_sum_f64(x);
+            if (lane == 0)
+                sh_part[0] = x;
+        }
+        __syncthreads();
+        total = sh_part[0];
+        __syncthreads();
+    }
+    // vertices with neither in- nor out-edges: the last iteration's constant, once
+    if (threadIdx.x == 0)
+        sh_k = P::constants(g, s, before);
+    __syncthreads();
+    const rank_t ri = P::rank(sh_k, (rank_t)0);
+    rank_t* last = rank + ((iters & 1u) ? stride : 0ull);
+    sum_t dangling = P::zero(); /* for PageRank Sum: the dangling vertices' ranks, times V again */
+    for (uint64_t v = (uint64_t)g.Vout + tid; v < g.V; v += nthr) {
+        if ((s.has_in[v >> 5] >> (v & 31u)) & 1u)
+            dangling = P::add(dangling, P::scale(last[v], (rank_t)g.V));
+        else
+            last[v] = P::scale(ri, inv[v]);
+    }
+    {
+        const double x = warp_sum_f64(P::total(dangling));
+        if (lane == 0)
+            sh_part[wib] = x;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double y = 0.0;
+            for (int w = 0; w < PULL_THREADS / 32; ++w)
+                y = __dadd_rn(y, sh_part[w]);
+            s.pmass[gridDim.x + blockIdx.x] = y;
+        }
+        if (!grid_barrier(c, target, &sh_ok))
+            return;
+    }
+    // ---- statistics and the per-iteration records
+    if (blockIdx.x == 0) {
+        const unsigned long long dsts = __ldcg(&c->lacc[0][CNT_DSTS]);
+        for (uint32_t i = threadIdx.x; i < iters && i < LOG_CAP; i += blockDim.x) {
+            IterRec& r = s.log[i];
+            r.mass_in = 0ull;
+            r.mass_out = 0ull;
+            r.edges = g.E;
+            r.tiles = T;
+            r.dsts = dsts;
+            r.activated = 0ull;
+            r.mode = MODE_DENSE;
+            r.iter = i;
+        }
+        if (threadIdx.x == 0) {
+            c->iter = iters;
+            c->max_iter = iters;
+            c->wedge_iters = 0;
+            c->edges_scanned = g.E * iters;
+            c->tiles_scanned = (unsigned long long)T * iters;
+            c->dsts_scanned = dsts * iters;
+            c->activated = 0;
+            c->pull_launches = 1;
+            c->last_mass = 0;
+            c->done = 0;
+            c->mode = MODE_DENSE;
+            c->parity = 0;
+            c->pr_prev = before;
+            c->pr_total = total;
+            double all = __dadd_rn(total, __dmul_rn((double)g.Viso, (double)ri));
+            for (uint32_t b = 0; b < gridDim.x; ++b)
+                all = __dadd_rn(all, __ldcg(&s.pmass[gridDim.x + b]));
+            c->pr_sum = all;
+        }
+    }
 }
 
 // PageRank Sum (execution_pr.c:63-71): sum of rank' * outdegree' over all vertices
@@ -5124,6 +5544,51 @@ static int pr32_setup_hub(wedge_graph* h)
     return WEDGE_OK;
 }
 
+// Split lists of tiles of tile_e in-edges (destinations spanning tiles: short
+// ones from the front, long ones from the back)
+static int split_state(wedge_graph* h, uint32_t tile_e)
+{
+    DevGraph& g = h->g;
+    DevState& s = h->s;
+    cudaStream_t st = h->stream;
+    const uint32_t cap = (uint32_t)h->num_sms * 8u;
+    int rc;
+    s.pT = (uint32_t)(g.Epad / tile_e);
+    if ((rc = dalloc(h, &s.psplit_k, (uint64_t)s.pT + 1, true)) || (rc = dalloc(h, &s.psplit_t0, (uint64_t)s.pT + 1, true)) ||
+        (rc = dalloc(h, &s.psplit_t1, (uint64_t)s.pT + 1, true)))
+        return rc;
+    unsigned long long *flag = nullptr, n = 0ull;
+    WEDGE_CHECK(cudaMallocAsync((void**)&flag, ((uint64_t)s.pT + 1) * sizeof(unsigned long long), st));
+    const uint32_t grid = grid_for((uint64_t)s.pT + 1, AUX_THREADS, cap);
+    split_flag_kernel<<<grid, AUX_THREADS, 0, st>>>(g.tile_dst0, g.dst_off, s.pT, g.E, tile_e, flag);
+    if ((rc = device_scan(h, flag, flag, (uint64_t)s.pT + 1, false)))
+        return rc;
+    split_fill_kernel<<<grid, AUX_THREADS, 0, st>>>(g.tile_dst0, g.dst_off, s.pT, g.E, tile_e, flag, s.psplit_k, s.psplit_t0,
+                                                   s.psplit_t1);
+    WEDGE_CHECK(cudaGetLastError());
+    WEDGE_CHECK(cudaMemcpyAsync(&n, flag + s.pT, sizeof(n), cudaMemcpyDeviceToHost, st));
+    WEDGE_CHECK(cudaStreamSynchronize(st));
+    cudaFreeAsync(flag, st);
+    s.pnsplit = (uint32_t)n;
+    s.pnwide = (uint32_t)(n >> 32);
+    return WEDGE_OK;
+}
+
+// the vertices with in-edges, one bit each
+static int has_in_state(wedge_graph* h)
+{
+    const uint64_t words = (h->g.V + 31) / 32 + 1;
+    const int rc = dalloc(h, &h->s.has_in, words, true);
+    if (rc)
+        return rc;
+    WEDGE_CHECK(cudaMemsetAsync(h->s.has_in, 0, words * sizeof(uint32_t), h->stream));
+    if (h->g.Vne)
+        mark_has_in_kernel<<<grid_for(h->g.Vne, AUX_THREADS, (uint32_t)h->num_sms * 8u), AUX_THREADS, 0, h->stream>>>(
+            h->g, h->s.has_in);
+    WEDGE_CHECK(cudaGetLastError());
+    return WEDGE_OK;
+}
+
 // State of the compensated-FP32 PageRank: the double-buffered FP32 ranks,
 // FP32 1/outdegree', the split lists of its PR32_TILE-edge tiles, the lists of
 // vertices without in-edges, and the per-block sums of the total rank.
@@ -5136,23 +5601,12 @@ static int pr32_state(wedge_graph* h)
     const uint32_t cap = (uint32_t)h->num_sms * 8u;
     int rc;
     s.rstride = (V + 31) & ~31ull;
-    s.pT = (uint32_t)(g.Epad / PR32_TILE);
-    if ((rc = dalloc(h, &s.rank32, 2 * s.rstride, true)) || (rc = dalloc(h, &s.inv32, V, true)) ||
+    if ((rc = split_state(h, PR32_TILE)) || (rc = dalloc(h, &s.rank32, 2 * s.rstride, true)) || (rc = dalloc(h, &s.inv32, V, true)) ||
         (rc = dalloc(h, &s.pmass, (uint64_t)h->pull_grid + cap + 8, true)) ||
-        (rc = dalloc(h, &s.psplit_k, (uint64_t)s.pT + 1, true)) || (rc = dalloc(h, &s.psplit_t0, (uint64_t)s.pT + 1, true)) ||
-        (rc = dalloc(h, &s.psplit_t1, (uint64_t)s.pT + 1, true)) || (rc = dalloc(h, &s.phead, (uint64_t)s.pT + 1, true)) ||
+        (rc = dalloc(h, &s.phead, (uint64_t)s.pT + 1, true)) ||
         (rc = dalloc(h, &s.ptail, (uint64_t)s.pT + 1, true)))
         return rc;
     pr32_inv_kernel<<<grid_for(V, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(g, s.inv32);
-    // destinations spanning the pull's tiles
-    unsigned int* d_cnt = nullptr;
-    WEDGE_CHECK(cudaMallocAsync((void**)&d_cnt, 2 * sizeof(unsigned int), st));
-    WEDGE_CHECK(cudaMemsetAsync(d_cnt, 0, 2 * sizeof(unsigned int), st));
-    if (g.Vne)
-        split_kernel<<<grid_for(g.Vne, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(g.dst_off, g.Vne, s.pT, PR32_TILE, s.psplit_k,
-                                                                               s.psplit_t0, s.psplit_t1, d_cnt);
-    unsigned int nsplit[2] = {0, 0};
-    WEDGE_CHECK(cudaMemcpyAsync(nsplit, d_cnt, sizeof(nsplit), cudaMemcpyDeviceToHost, st));
     // complete destinations past a tile's staged slots, in tile order
     const uint32_t T = (uint32_t)((g.E + PR32_TILE - 1) / PR32_TILE);
     s.novf = 0;
@@ -5179,22 +5633,17 @@ static int pr32_state(wedge_graph* h)
     // vertices without in-edges, in id order: with out-edges (gathered, so written every
     // iteration) and without (written once at the end)
     if (V == 0) {
-        s.pnsplit = s.pnwide = s.nz = s.ni = 0;
-        WEDGE_CHECK(cudaStreamSynchronize(st));
-        cudaFree(d_cnt);
+        s.nz = s.ni = 0;
         return WEDGE_OK;
     }
-    const uint64_t words = (V + 31) / 32;
-    uint32_t *has_in = nullptr, *fz = nullptr, *fi = nullptr, *pz = nullptr, *pi = nullptr;
-    WEDGE_CHECK(cudaMallocAsync((void**)&has_in, words * sizeof(uint32_t), st));
+    uint32_t *fz = nullptr, *fi = nullptr, *pz = nullptr, *pi = nullptr;
+    if ((rc = has_in_state(h)))
+        return rc;
     WEDGE_CHECK(cudaMallocAsync((void**)&fz, V * sizeof(uint32_t), st));
     WEDGE_CHECK(cudaMallocAsync((void**)&fi, V * sizeof(uint32_t), st));
     WEDGE_CHECK(cudaMallocAsync((void**)&pz, V * sizeof(uint32_t), st));
     WEDGE_CHECK(cudaMallocAsync((void**)&pi, V * sizeof(uint32_t), st));
-    WEDGE_CHECK(cudaMemsetAsync(has_in, 0, words * sizeof(uint32_t), st));
-    if (g.Vne)
-        mark_has_in_kernel<<<grid_for(g.Vne, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(g, has_in);
-    pr32_noin_flags_kernel<<<grid_for(V, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(g, has_in, fz, fi);
+    pr32_noin_flags_kernel<<<grid_for(V, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(g, s.has_in, fz, fi);
     if ((rc = device_scan(h, fz, pz, V, false)) || (rc = device_scan(h, fi, pi, V, false)))
         return rc;
     uint32_t tail[4] = {0, 0, 0, 0}; /* last flag and position of each list */
@@ -5203,16 +5652,12 @@ static int pr32_state(wedge_graph* h)
     WEDGE_CHECK(cudaMemcpyAsync(&tail[2], fi + (V - 1), 4, cudaMemcpyDeviceToHost, st));
     WEDGE_CHECK(cudaMemcpyAsync(&tail[3], pi + (V - 1), 4, cudaMemcpyDeviceToHost, st));
     WEDGE_CHECK(cudaStreamSynchronize(st));
-    s.pnsplit = nsplit[0];
-    s.pnwide = nsplit[1];
     s.nz = tail[0] + tail[1];
     s.ni = tail[2] + tail[3];
     if ((rc = dalloc(h, &s.zlist, (uint64_t)s.nz + 1, true)) || (rc = dalloc(h, &s.ilist, (uint64_t)s.ni + 1, true)))
         return rc;
     compact_flags_kernel<<<grid_for(V, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(fz, pz, V, s.zlist);
     compact_flags_kernel<<<grid_for(V, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(fi, pi, V, s.ilist);
-    cudaFreeAsync(d_cnt, st);
-    cudaFreeAsync(has_in, st);
     cudaFreeAsync(fz, st);
     cudaFreeAsync(fi, st);
     cudaFreeAsync(pz, st);
@@ -5223,41 +5668,38 @@ static int pr32_state(wedge_graph* h)
 }
 
 // state arrays of one application (allocated on first use, reused by later runs)
-// Split lists of the 512-edge SSSP pull's tiles (destinations spanning tiles:
-// short ones from the front, long ones from the back) and their per-tile
-// partial minima
+// the 512-edge SSSP pull's split lists and their per-tile partial minima
 static int sssp_split_state(wedge_graph* h)
 {
-    DevGraph& g = h->g;
     DevState& s = h->s;
-    cudaStream_t st = h->stream;
-    const uint32_t cap = (uint32_t)h->num_sms * 8u;
-    int rc;
-    s.pT = (uint32_t)(g.Epad / SSSP_TILE);
-    if ((rc = dalloc(h, &s.psplit_k, (uint64_t)s.pT + 1, true)) || (rc = dalloc(h, &s.psplit_t0, (uint64_t)s.pT + 1, true)) ||
-        (rc = dalloc(h, &s.psplit_t1, (uint64_t)s.pT + 1, true)) || (rc = dalloc(h, &s.shead, (uint64_t)s.pT + 1, true)) ||
-        (rc = dalloc(h, &s.stail, (uint64_t)s.pT + 1, true)))
+    const int rc = split_state(h, SSSP_TILE);
+    if (rc)
         return rc;
-    unsigned int* d_cnt = nullptr;
-    WEDGE_CHECK(cudaMallocAsync((void**)&d_cnt, 2 * sizeof(unsigned int), st));
-    WEDGE_CHECK(cudaMemsetAsync(d_cnt, 0, 2 * sizeof(unsigned int), st));
-    if (g.Vne)
-        split_kernel<<<grid_for(g.Vne, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(g.dst_off, g.Vne, s.pT, SSSP_TILE, s.psplit_k,
-                                                                               s.psplit_t0, s.psplit_t1, d_cnt);
-    WEDGE_CHECK(cudaGetLastError());
-    unsigned int n[2] = {0, 0};
-    WEDGE_CHECK(cudaMemcpyAsync(n, d_cnt, sizeof(n), cudaMemcpyDeviceToHost, st));
-    WEDGE_CHECK(cudaStreamSynchronize(st));
-    cudaFreeAsync(d_cnt, st);
-    s.pnsplit = n[0];
-    s.pnwide = n[1];
-    return WEDGE_OK;
+    const int r1 = dalloc(h, &s.shead, (uint64_t)s.pT + 1, true);
+    return r1 ? r1 : dalloc(h, &s.stail, (uint64_t)s.pT + 1, true);
 }
 
 // The traversal loops run their Wedge iterations in sparse_loop_kernel where
 // the CSRI holds destinations (and the vertices' out-degrees are its lists'
 // lengths); the phase API and chunk frontiers take the separate launches.
 static bool fused_loop(const wedge_graph* h) { return h->g.csr && !h->g.shard && h->g.E != 0; }
+
+// the hub cache of pr_loop_kernel: the pull's, within what its staged sums leave
+template <bool F64>
+static int pr_loop_hub(wedge_graph* h)
+{
+    cudaFuncAttributes fa;
+    WEDGE_CHECK(cudaFuncGetAttributes(&fa, pr_loop_kernel<F64>));
+    int optin = 0;
+    WEDGE_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
+    const int stage = (int)pr_stage_bytes<F64>(), room = optin - (int)fa.sharedSizeBytes;
+    if (room < stage)
+        return WEDGE_ERR_UNSUPPORTED;
+    const uint32_t most = (uint32_t)(room - stage) & ~15u;
+    h->loop_hub = h->hub_bytes < most ? h->hub_bytes : most;
+    WEDGE_CHECK(cudaFuncSetAttribute(pr_loop_kernel<F64>, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
+    return WEDGE_OK;
+}
 
 static int ensure_state(wedge_graph* h, int app, int precision)
 {
@@ -5291,9 +5733,13 @@ static int ensure_state(wedge_graph* h, int app, int precision)
     } else if (app == WEDGE_APP_PR) {
         if ((rc = dalloc(h, &s.acc, V, true)) || (rc = dalloc(h, &s.inv_od, V, true)))
             return rc;
+        /* no pull writes the sums of vertices without in-edges */
+        WEDGE_CHECK(cudaMemsetAsync(s.acc, 0, (V ? V : 1) * sizeof(double), h->stream));
         pr_inv_outdeg_kernel<<<grid_for(V, AUX_THREADS, (uint32_t)h->num_sms * 8u), AUX_THREADS, 0, h->stream>>>(g, s.inv_od);
         WEDGE_CHECK(cudaGetLastError());
-        if ((rc = dalloc(h, &s.rank, V, true)) || (rc = dalloc(h, &s.head_part, (uint64_t)g.T + 1, true)) ||
+        s.rstride = (V + 31) & ~31ull;
+        if ((rc = dalloc(h, &s.rank, 2 * s.rstride, true)) || (rc = dalloc(h, &s.pmass, 2ull * h->pull_grid + 8, true)) ||
+            (rc = has_in_state(h)) || (rc = split_state(h, 32u * PrPrec<true>::epl)) || (rc = dalloc(h, &s.head_part, (uint64_t)g.T + 1, true)) ||
             (rc = dalloc(h, &s.tail_part, (uint64_t)g.T + 1, true)))
             return rc;
     } else {
@@ -5353,6 +5799,8 @@ static int ensure_state(wedge_graph* h, int app, int precision)
         }
     }
     if ((rc = (app == WEDGE_APP_PR && precision == WEDGE_PREC_FP32C) ? pr32_setup_hub(h) : setup_hub(h, app, precision)))
+        return rc;
+    if (app == WEDGE_APP_PR && (rc = precision == WEDGE_PREC_FP32C ? pr_loop_hub<false>(h) : pr_loop_hub<true>(h)))
         return rc;
     h->built_app = app;
     h->last_precision = precision;
@@ -5572,6 +6020,8 @@ static void cc_finalize(wedge_graph* h)
 static int result_state(wedge_graph* h, DevState* out)
 {
     *out = h->s;
+    if (h->pr_flip) /* an odd number of FP64 PageRank iterations in pr_loop_kernel */
+        out->rank += h->s.rstride;
     if (h->last_app == WEDGE_APP_CC && h->cc_pending) {
         WEDGE_CHECK(cudaMemsetAsync(h->s.cc_best, 0xFF, h->g.V * sizeof(uint32_t), h->stream));
         cc_best_kernel<<<aux_grid(h, h->g.V), AUX_THREADS, 0, h->stream>>>(h->g, h->s.prop32, h->s.cc_best);
@@ -5827,57 +6277,41 @@ static void launch_pr32_iso(wedge_graph* h)
     pr32_iso_kernel<<<aux_grid(h, h->s.ni), AUX_THREADS, 0, h->stream>>>(h->g, h->s);
 }
 
-// Captures one PageRank iteration (pull, ordered merge, vertex phase) as the
-// body of a device-side while loop on Ctrl::iter < Ctrl::max_iter.  The
-// kernels hold the state by value, so the capture is keyed on the damping
-// factor (the precision is part of the state, whose rebuild drops it).
-static int build_pr_graph(wedge_graph* h)
+// The compensated-FP32 form runs in one launch below this many in-edges, R-MAT
+// scale 24: there the separate kernels' pull, which has more registers for its
+// 16 gathers, is as fast (16.7 against 16.8 ms for 20 iterations; scale 22: 4.5
+// against 3.7, scale 26, 30 iterations: 99.5 against 106).  FP64 always does
+// (scale 24, 8 iterations: 16.9 against 10.0 ms).
+constexpr uint64_t PR32_LOOP_EDGES = 1ull << 28;
+
+// A whole PageRank in one launch (pr_loop_kernel): one block per SM, fewer on
+// graphs that leave most of them without work.  The control block starts at zero.
+static int launch_pr_loop(wedge_graph* h, uint32_t iters)
 {
-    uint64_t key;
-    memcpy(&key, &h->s.damping, sizeof(key));
-    if (h->pr_exec && h->pr_key == key)
-        return WEDGE_OK;
-    if (h->pr_exec) {
-        cudaGraphExecDestroy(h->pr_exec);
-        h->pr_exec = nullptr;
-    }
-    const DevGraph& g = h->g;
-    cudaGraph_t graph;
-    WEDGE_CHECK(cudaGraphCreate(&graph, 0));
-    cudaGraphConditionalHandle handle;
-    WEDGE_CHECK(cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault));
-    cudaGraphNodeParams cparams = {};
-    cparams.type = cudaGraphNodeTypeConditional;
-    cparams.conditional.handle = handle;
-    cparams.conditional.type = cudaGraphCondTypeWhile;
-    cparams.conditional.size = 1;
-    cudaGraphNode_t cnode;
-    WEDGE_CHECK(cudaGraphAddNode(&cnode, graph, nullptr, nullptr, 0, &cparams));
-    cudaGraph_t body = cparams.conditional.phGraph_out[0];
-    const cudaStream_t run_stream = h->stream; /* captured on the handle's own stream */
-    h->stream = h->own_stream;
-    WEDGE_CHECK(cudaStreamBeginCaptureToGraph(h->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    if (h->s.precision == WEDGE_PREC_FP32C) {
-        launch_pr32_iteration(h);
-    } else {
-        launch_pull(h, WEDGE_APP_PR);
-        pr_finish_kernel<<<finish_grid(h, g), AUX_THREADS, 0, h->stream>>>(g, h->s, h->pull_grid, counters(h));
-        launch_pr_total(h);
-        pr_vertex_kernel<<<aux_grid(h, g.V), AUX_THREADS, 0, h->stream>>>(g, h->s);
-    }
-    pr_loop_cond_kernel<<<1, 1, 0, h->stream>>>(h->s, handle);
-    cudaGraph_t captured;
-    const cudaError_t ce = cudaStreamEndCapture(h->stream, &captured);
-    h->stream = run_stream;
-    WEDGE_CHECK(ce);
-    WEDGE_CHECK(cudaGraphInstantiate(&h->pr_exec, graph, 0));
-    cudaGraphDestroy(graph);
-    h->pr_key = key;
+    const bool f64 = h->s.precision != WEDGE_PREC_FP32C;
+    const uint64_t want = h->g.E / 2048u + 8u;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((uint32_t)(want < (uint64_t)h->num_sms ? want : (uint64_t)h->num_sms));
+    cfg.blockDim = dim3(PULL_THREADS);
+    cfg.dynamicSmemBytes = h->loop_hub + (f64 ? pr_stage_bytes<true>() : pr_stage_bytes<false>());
+    cfg.stream = h->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    DevState s = h->s;
+    s.hub_bytes = h->loop_hub;
+    WEDGE_CHECK(cudaMemsetAsync(s.ctrl, 0, sizeof(Ctrl), h->stream));
+    if (f64)
+        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, pr_loop_kernel<true>, h->g, s, iters));
+    else
+        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, pr_loop_kernel<false>, h->g, s, iters));
     return WEDGE_OK;
 }
 
 // The statistics of the PageRank run that just ran on h->stream (waits for it)
-static int pr_stats(wedge_graph* h, uint32_t iters, bool use_graph, bool timing, double t_pull, double t_vertex,
+static int pr_stats(wedge_graph* h, uint32_t iters, bool loop, bool timing, double t_pull, double t_vertex,
                     wedge_stats_t* st)
 {
     Ctrl c;
@@ -5899,8 +6333,8 @@ static int pr_stats(wedge_graph* h, uint32_t iters, bool use_graph, bool timing,
         st->edges_scanned = c.edges_scanned;
         st->tiles_scanned = c.tiles_scanned;
         st->pull_launches = c.pull_launches;
-        /* init (+ total), the iterations (+ the loop condition), the sums (+ isolated vertices) */
-        st->kernel_launches = c32 ? 5ull + (use_graph ? 4ull : 3ull) * iters : 3ull + (use_graph ? 5ull : 4ull) * iters;
+        /* one launch, or: init (+ total), the iterations, the sums (+ isolated vertices) */
+        st->kernel_launches = loop ? 1ull : c32 ? 5ull + 3ull * iters : 3ull + 4ull * iters;
         st->pr_sum = c.pr_sum;
     }
     if (c.error)
@@ -5916,22 +6350,22 @@ static int run_pr(wedge_graph* h, const wedge_params_t* p, wedge_stats_t* st, bo
     h->s.precision = (uint32_t)p->precision;
     const uint32_t vgrid = aux_grid(h, g.V);
     const uint32_t fgrid = finish_grid(h, g);
-    const bool use_graph = (p->flags & WEDGE_FLAG_GRAPH) != 0 && !timing && p->num_iterations > 0;
-    if (use_graph) {
-        int rc = build_pr_graph(h);
-        if (rc)
-            return rc;
-    }
+    const bool loop = !timing && p->num_iterations > 0 && g.E != 0 && !g.shard &&
+                      (h->s.precision != WEDGE_PREC_FP32C || g.E < PR32_LOOP_EDGES);
     const bool c32 = h->s.precision == WEDGE_PREC_FP32C;
     double t_pull = 0, t_vertex = 0;
     WEDGE_CHECK(cudaEventRecord(h->ev[0], h->stream));
-    if (c32)
+    h->pr_flip = loop && !c32 ? (int)(p->num_iterations & 1u) : 0;
+    if (loop) {
+        int rc = launch_pr_loop(h, p->num_iterations);
+        if (rc)
+            return rc;
+    } else if (c32) {
         launch_pr32_init(h, p->num_iterations);
-    else
+    } else {
         pr_init_kernel<<<vgrid, AUX_THREADS, 0, h->stream>>>(g, h->s, p->num_iterations);
-    if (use_graph)
-        WEDGE_CHECK(cudaGraphLaunch(h->pr_exec, h->stream));
-    for (uint32_t it = 0; !use_graph && it < p->num_iterations; ++it) {
+    }
+    for (uint32_t it = 0; !loop && it < p->num_iterations; ++it) {
         if (timing)
             WEDGE_CHECK(cudaEventRecord(h->ev[2], h->stream));
         if (c32)
@@ -5964,21 +6398,23 @@ static int run_pr(wedge_graph* h, const wedge_params_t* p, wedge_stats_t* st, bo
             }
         }
     }
-    if (c32)
+    if (c32 && !loop)
         launch_pr32_iso(h); /* vertices with neither in- nor out-edges, once */
     WEDGE_CHECK(cudaEventRecord(h->ev[1], h->stream));
-    double* sums = pr_sums(h);
-    pr_sum_kernel<<<vgrid, AUX_THREADS, 0, h->stream>>>(g, h->s, sums);
-    pr_sum_final_kernel<<<1, 32, 0, h->stream>>>(h->s, sums, vgrid);
+    if (!loop) {
+        double* sums = pr_sums(h);
+        pr_sum_kernel<<<vgrid, AUX_THREADS, 0, h->stream>>>(g, h->s, sums);
+        pr_sum_final_kernel<<<1, 32, 0, h->stream>>>(h->s, sums, vgrid);
+    }
     WEDGE_CHECK(cudaGetLastError());
     h->last_app = WEDGE_APP_PR;
     if (!wait && !timing) {
         h->pend_app = WEDGE_APP_PR;
         h->pend_iters = p->num_iterations;
-        h->pend_launches = use_graph ? 1u : 0u; /* the launch count formula's graph term */
+        h->pend_launches = loop ? 1u : 0u; /* which launch count formula */
         return WEDGE_OK;
     }
-    return pr_stats(h, p->num_iterations, use_graph, timing, t_pull, t_vertex, st);
+    return pr_stats(h, p->num_iterations, loop, timing, t_pull, t_vertex, st);
 }
 
 }  // namespace wedge
@@ -6276,6 +6712,11 @@ int wedge_cuda_run_phase(wedge_graph_t* g, int app, int phase, const wedge_param
     if ((rc = ensure_state(g, app, params->precision)))
         return rc;
     const DevGraph& dg = g->g;
+    if (app == WEDGE_APP_PR && g->pr_flip) { /* the phases keep FP64 ranks in the first buffer */
+        WEDGE_CHECK(cudaMemcpyAsync(g->s.rank, g->s.rank + g->s.rstride, dg.V * sizeof(double), cudaMemcpyDeviceToDevice,
+                                    g->stream));
+        g->pr_flip = 0;
+    }
     g->s.damping = params->damping > 0.0 ? params->damping : 0.875;
     g->s.precision = (uint32_t)params->precision;
     const uint32_t vgrid = aux_grid(g, dg.V);
@@ -6550,10 +6991,6 @@ int wedge_cuda_set_scheduler(wedge_graph_t* g, const float* blob, uint64_t count
         g->graph_exec = nullptr;
         g->graph_app = -1;
     }
-    if (g->pr_exec) {
-        cudaGraphExecDestroy(g->pr_exec);
-        g->pr_exec = nullptr;
-    }
     return WEDGE_OK;
 }
 
@@ -6644,8 +7081,10 @@ __global__ void noalloc_prepare_kernel(const unsigned long long* dst_off, uint32
 __global__ void noalloc_finish_kernel(DevGraph g, DevState s)
 {
     NoAllocScratch* sc = &g_noalloc_scratch;
-    merge_splits(g, s.acc, sc->split_k, sc->split_t0, sc->split_t1, sc->nsplit[0], sc->nsplit[1], g.T,
-                 [&](uint32_t t) { return sc->tail_part[t]; }, [&](uint32_t t) { return sc->head_part[t]; });
+    merge_splits(sc->split_k, sc->split_t0, sc->split_t1, sc->nsplit[0], sc->nsplit[1], g.T,
+                 blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x,
+                 [&](uint32_t t) { return sc->tail_part[t]; }, [&](uint32_t t) { return sc->head_part[t]; },
+                 [&](uint32_t k, double x) { s.acc[g.dst_ident ? k : g.dst_id[k]] = x; });
 }
 
 static int noalloc_setup(int dev, NoAllocScratch** sc, uint32_t* grid)

@@ -134,6 +134,7 @@ struct DevGraph {
     uint32_t sym;              // every edge's reverse is an edge too: CC propagates engine ids (see cc_best_kernel)
     uint32_t csr;              // csri holds destinations (Epad < 2^32), else chunk ids
     double wmean;              // mean weight (0: none)
+    uint32_t Vout, Viso;       // vertices with out-edges (ids [0, Vout)); vertices without any edge
     uint32_t shard;            // a destination-range shard (wedge_cuda_load_shard)
     const uint32_t* src;
     const unsigned long long* w;
@@ -168,7 +169,7 @@ struct DevState {
     uint32_t narrow_lim;           // distances the 32-bit copy holds: below this (2^32-1, or a smaller test limit)
     uint32_t wo;                   // SSSP dense pulls run over the weight-ordered in-edges (sssp_wo_kernel)
     uint2* wo_items;               // (compressed destination, first in-edge) left to sssp_wo_long_kernel
-    double* rank;                  // PageRank FP64: rank / outdegree'
+    double* rank;                  // [2][rstride] PageRank FP64: rank / outdegree'; the second buffer is pr_loop_kernel's
     double* acc;                   // PageRank accumulators (graph_vertex_accumulators)
     double* inv_od;                // PageRank 1 / outdegree' (outdegree, or N for dangling vertices)
     double* head_part;             // [T] partial sum of a split destination ending in tile t
@@ -176,7 +177,8 @@ struct DevState {
     // compensated-FP32 PageRank (WEDGE_PREC_FP32C): see pr32_pull_kernel
     float* rank32;                 // [2][rstride] rank / outdegree', double-buffered by iteration parity
     float* inv32;                  // [V] 1 / outdegree' in FP32, negative for a dangling vertex (-1/N)
-    uint64_t rstride;              // floats between the two rank buffers (V rounded up to 32)
+    uint64_t rstride;              // ranks between the two rank buffers (V rounded up to 32)
+    uint32_t* has_in;              // V-bit: vertices with in-edges
     uint32_t* zlist;               // vertices without in-edges and with out-edges (their rank is the same constant)
     uint32_t* ilist;               // vertices without in-edges or out-edges (written once, after the last iteration)
     uint32_t nz, ni;
@@ -189,7 +191,8 @@ struct DevState {
     unsigned long long* shead;     // SSSP 512-edge pull: [pT] minimum of a split destination ending in tile t
     unsigned long long* stail;     // [pT] minimum of a split destination continuing past tile t (the split lists
                                    // psplit_* are those of the 512-edge tiles)
-    double* pmass;                 // per-block partial sums of the non-dangling ranks (the next total rank)
+    double* pmass;                 // per-block partial sums of the non-dangling ranks (the next total rank);
+                                   // pr_loop_kernel: pairs with the dangling ones'
     float* ovf_sum;                // [Vne] sums of the destinations in ovf_list, by compressed destination
     uint32_t* ovf_list;            // complete destinations past the staged slots of their tile (tile order)
     uint32_t novf;
@@ -268,8 +271,8 @@ struct wedge_graph {
     double* iter_wedge_ms;
     int last_timing;
     cudaGraphExec_t graph_exec;        // captured traversal
-    cudaGraphExec_t pr_exec;           // captured PageRank iterations
-    uint64_t pr_key;                   // (iterations, precision) of pr_exec
+    uint32_t loop_hub;                 // pr_loop_kernel's hub cache, bytes
+    int pr_flip;                       // the FP64 ranks are in the second buffer
     int graph_app;
     int graph_key;
     int cc_pending;                    // CC labels are engine ids (symmetric graph, not yet converted)
