@@ -207,3 +207,39 @@ def test_pagerank_in_one_launch(engine_lib, iterations, degrees):
         g.run_phase(W.APP_PR, W.PHASE_VERTEX_PR, p)
         more = plain_pagerank(V, s.astype(np.int64), d.astype(np.int64), iterations + 1, 0.85)
         assert np.abs(g.read_results().view(np.float64) - more).sum() <= 1e-13 * np.abs(more).sum()
+
+
+@pytest.mark.parametrize("n", [1, 4, 5, 31, 33, 64, 65, 127, 128, 129, 513, 577, 9001])
+@pytest.mark.parametrize("weights", ["bytes", "words", "f64"])
+def test_batched_pulls(engine_lib, n, weights):
+    """out- and in-lists around the batched kernel's sizes (lists of 128 out-edges
+    and pieces of the longer ones, chunks of 4 listed vertices, groups of 32
+    destinations of up to 64 in-edges, pieces of 512), all pulls sparse, all dense and mixed"""
+    W = engine_lib
+    V, s, d, w = fans(n, "random", n)
+    kind = W.WEIGHTS_U64
+    if weights == "words":
+        w = w * np.uint64(1 << 20)
+    elif weights == "f64":
+        w, kind = (w.astype(np.float64) / 8.0).view(np.uint64), W.WEIGHTS_F64
+    with W.Graph.from_edges(V, s, d, w, kind) as g:
+        queries = [(0, app, root) for app in (W.APP_SSSP, W.APP_BFS) for root in (0, 1, n, V - 1)]
+        expect = []
+        for _, app, root in queries:
+            g.run(app, W.Params(root=root, sched=W.SCHED_DENSE))
+            expect.append(g.read_results().copy())
+        if weights == "bytes":
+            assert np.array_equal(expect[0], bellman_ford(V, s.astype(np.int64), d.astype(np.int64), w, 0))
+        with W.Batch([g], queries) as b:
+            for threshold_pct in (1, 20, 100):
+                b.run(W.BatchTuning(threshold_pct=threshold_pct))
+                for i, (_, app, root) in enumerate(queries):
+                    got = b.read_result(i)
+                    if app == W.APP_SSSP:
+                        assert np.array_equal(got, expect[i]), (threshold_pct, root)
+                    else:  # the targets' parents may be any middle vertex that was reached
+                        none = np.uint64(0xFFFFFFFFFFFFFFFF)
+                        assert np.array_equal(got == none, expect[i] == none)
+                        assert np.array_equal(got[:n + 1], expect[i][:n + 1])
+                        tail = got[n + 1:][got[n + 1:] != none].astype(np.int64)
+                        assert np.all((tail == root) | ((tail >= 1) & (tail <= n)))
