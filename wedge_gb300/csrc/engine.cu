@@ -107,6 +107,14 @@ static void free_state(wedge_graph* h)
     h->pr_flip = 0;
 }
 
+static void load_scratch_free(wedge_graph* h)
+{
+    if (h->tscratch)
+        cudaFree(h->tscratch);
+    h->tscratch = nullptr;
+    h->tsize = h->tused = 0;
+}
+
 void free_handle(wedge_graph* h)
 {
     if (!h)
@@ -116,6 +124,7 @@ void free_handle(wedge_graph* h)
     if (h->xstream)
         cudaStreamSynchronize(h->xstream);
     free_state(h);
+    load_scratch_free(h);
     for (int i = 0; i < h->nallocs; ++i)
         cudaFree(h->allocs[i]);
     for (int i = 0; i < 8; ++i)
@@ -149,6 +158,40 @@ static int dalloc(wedge_graph* h, T** p, uint64_t count, bool state = false)
     if (e != cudaSuccess)
         return cuda_status(e);
     return state ? track_state(h, *p) : track(h, *p);
+}
+
+// The load's temporary arrays.  Small graphs take them from one block, as a
+// stack (all work is on one stream, so what a released array held is read
+// before its place is written again); others, and what does not fit, from the
+// stream's pool, which gives its memory back at every synchronisation and has to
+// map it again after it: weighted R-MAT loads of scales 12, 16 and 20 took 0.91,
+// 1.42 and 5.3 ms with the pool alone, 0.79, 1.35 and 4.9 with the block.
+// LOAD_SCRATCH_EDGES (edges and vertices) bounds the block (1.6 GB); beyond it
+// the kernels' time hides the mapping.
+constexpr uint64_t LOAD_SCRATCH_EDGES = 1ull << 25;
+
+template <class T>
+static cudaError_t talloc(wedge_graph* h, T** p, uint64_t bytes)
+{
+    const uint64_t need = ((bytes ? bytes : 1) + 255) & ~255ull;
+    if (h->tscratch && h->tused + need <= h->tsize) {
+        *p = (T*)(h->tscratch + h->tused);
+        h->tused += need;
+        return cudaSuccess;
+    }
+    return cudaMallocAsync((void**)p, bytes ? bytes : 1, h->stream);
+}
+
+// releases an array; the block's place comes back with trelease
+static void tfree(wedge_graph* h, void* p)
+{
+    if (!h->tscratch || (unsigned char*)p < h->tscratch || (unsigned char*)p >= h->tscratch + h->tsize)
+        cudaFreeAsync(p, h->stream);
+}
+
+static void trelease(wedge_graph* h, uint64_t mark)
+{
+    h->tused = mark;
 }
 
 static uint32_t grid_for(uint64_t work, uint32_t threads, uint32_t cap)
@@ -428,10 +471,12 @@ static int device_scan(wedge_graph* h, const InT* in, OutT* out, uint64_t n, boo
     else
         WEDGE_CHECK(cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, (long long)n, h->stream));
     void* tmp = nullptr;
-    WEDGE_CHECK(cudaMallocAsync(&tmp, bytes, h->stream));
+    const uint64_t mark = h->tused;
+    WEDGE_CHECK(talloc(h, &tmp, bytes));
     cudaError_t e = inclusive ? cub::DeviceScan::InclusiveSum(tmp, bytes, in, out, (long long)n, h->stream)
                               : cub::DeviceScan::ExclusiveSum(tmp, bytes, in, out, (long long)n, h->stream);
-    cudaFreeAsync(tmp, h->stream);
+    tfree(h, tmp);
+    trelease(h, mark);
     WEDGE_CHECK(e);
     return WEDGE_OK;
 }
@@ -550,11 +595,12 @@ static int relabel_by_degree(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d
     int rc;
     if ((rc = dalloc(h, new2old, V)) || (rc = dalloc(h, old2new, V)))
         return rc;
+    const uint64_t mark = h->tused;
     uint32_t* deg = nullptr;
     unsigned long long *vk = nullptr, *vk2 = nullptr;
-    WEDGE_CHECK(cudaMallocAsync((void**)&deg, V * sizeof(uint32_t), st));
-    WEDGE_CHECK(cudaMallocAsync((void**)&vk, V * sizeof(unsigned long long), st));
-    WEDGE_CHECK(cudaMallocAsync((void**)&vk2, V * sizeof(unsigned long long), st));
+    WEDGE_CHECK(talloc(h, &deg, V * sizeof(uint32_t)));
+    WEDGE_CHECK(talloc(h, &vk, V * sizeof(unsigned long long)));
+    WEDGE_CHECK(talloc(h, &vk2, V * sizeof(unsigned long long)));
     if (global_outdeg) { /* a shard: the whole graph's degrees, so every shard numbers vertices alike */
         WEDGE_CHECK(cudaMemcpyAsync(deg, global_outdeg, V * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
     } else {
@@ -569,15 +615,16 @@ static int relabel_by_degree(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d
         /* by the degree alone: the sort is stable, and the keys start in id order */
         WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(nullptr, tb, db, (long long)V, 32, 64, st));
         void* tmp = nullptr;
-        WEDGE_CHECK(cudaMallocAsync(&tmp, tb ? tb : 1, st));
+        WEDGE_CHECK(talloc(h, &tmp, tb));
         WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tb, db, (long long)V, 32, 64, st));
-        cudaFreeAsync(tmp, st);
+        tfree(h, tmp);
         permutation_kernel<<<grid_for(V, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(db.Current(), V, *new2old, *old2new);
     }
     permute_degrees_kernel<<<grid_for(V, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(deg, *new2old, V, outdeg);
-    cudaFreeAsync(deg, st);
-    cudaFreeAsync(vk, st);
-    cudaFreeAsync(vk2, st);
+    tfree(h, deg);
+    tfree(h, vk);
+    tfree(h, vk2);
+    trelease(h, mark);
     if (E == 0)
         return WEDGE_OK;
     int vbits = 1;
@@ -586,25 +633,27 @@ static int relabel_by_degree(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d
     const bool in_key = byte_weights && 2 * vbits + 8 <= 64;
     const uint64_t Epad = (E + MAX_TILE_E - 1) / MAX_TILE_E * MAX_TILE_E;
     unsigned long long *ek = nullptr, *ek2 = nullptr, *w2 = nullptr;
-    WEDGE_CHECK(cudaMallocAsync((void**)&ek, E * sizeof(unsigned long long), st));
-    WEDGE_CHECK(cudaMallocAsync((void**)&ek2, E * sizeof(unsigned long long), st));
+    WEDGE_CHECK(talloc(h, &ek, E * sizeof(unsigned long long)));
+    WEDGE_CHECK(talloc(h, &ek2, E * sizeof(unsigned long long)));
     const uint32_t grid = grid_for(E, AUX_THREADS, cap);
     relabel_edges_kernel<<<grid, AUX_THREADS, 0, st>>>(d_src, d_dst, in_key ? d_w : nullptr, E, *old2new, vbits, ek);
     cub::DoubleBuffer<unsigned long long> kb(ek, ek2);
     size_t tb = 0;
     void* tmp = nullptr;
+    uint64_t sort_mark = h->tused;
     if (d_w && !in_key) {
-        WEDGE_CHECK(cudaMallocAsync((void**)&w2, E * sizeof(unsigned long long), st));
+        WEDGE_CHECK(talloc(h, &w2, E * sizeof(unsigned long long)));
+        sort_mark = h->tused;
         cub::DoubleBuffer<unsigned long long> vb(d_w, w2);
         WEDGE_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, tb, kb, vb, (long long)E, 0, 2 * vbits, st));
-        WEDGE_CHECK(cudaMallocAsync(&tmp, tb ? tb : 1, st));
+        WEDGE_CHECK(talloc(h, &tmp, tb));
         WEDGE_CHECK(cub::DeviceRadixSort::SortPairs(tmp, tb, kb, vb, (long long)E, 0, 2 * vbits, st));
         if (vb.Current() != d_w)
             WEDGE_CHECK(cudaMemcpyAsync(d_w, vb.Current(), E * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, st));
     } else {
         const int b0 = in_key ? 8 : 0;
         WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(nullptr, tb, kb, (long long)E, b0, b0 + 2 * vbits, st));
-        WEDGE_CHECK(cudaMallocAsync(&tmp, tb ? tb : 1, st));
+        WEDGE_CHECK(talloc(h, &tmp, tb));
         WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tb, kb, (long long)E, b0, b0 + 2 * vbits, st));
     }
     if (in_key && (rc = dalloc(h, w8, Epad)))
@@ -612,14 +661,16 @@ static int relabel_by_degree(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d
     unpack_edges_kernel<<<grid, AUX_THREADS, 0, st>>>(kb.Current(), E, vbits, d_src, d_dst, *w8);
     if (in_key)
         WEDGE_CHECK(cudaMemsetAsync(*w8 + E, 0, Epad - E, st));
-    cudaFreeAsync(tmp, st);
+    tfree(h, tmp);
+    trelease(h, sort_mark);
     if (in_key && !global_outdeg && Epad < (1ull << 32)) { /* 32-bit in-edge positions */
         if (dalloc(h, wsrc, Epad) == WEDGE_OK && dalloc(h, ww8, Epad) == WEDGE_OK) {
             weight_key_kernel<<<grid, AUX_THREADS, 0, st>>>(kb.Current(), E, vbits);
             WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(nullptr, tb, kb, (long long)E, vbits, 2 * vbits + 8, st));
-            WEDGE_CHECK(cudaMallocAsync(&tmp, tb ? tb : 1, st));
+            WEDGE_CHECK(talloc(h, &tmp, tb));
             WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tb, kb, (long long)E, vbits, 2 * vbits + 8, st));
-            cudaFreeAsync(tmp, st);
+            tfree(h, tmp);
+            trelease(h, sort_mark);
             weight_unpack_kernel<<<grid_for(Epad, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(kb.Current(), E, Epad, vbits,
                                                                                          *wsrc, *ww8);
         } else {
@@ -639,22 +690,23 @@ static int relabel_by_degree(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d
             WEDGE_CHECK(cudaMemcpyAsync(*cw, d_w, E * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, st));
             cub::DoubleBuffer<unsigned long long> vb(*cw, w2);
             WEDGE_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, tb, kb, vb, (long long)E, s0, s0 + vbits, st));
-            WEDGE_CHECK(cudaMallocAsync(&tmp, tb ? tb : 1, st));
+            WEDGE_CHECK(talloc(h, &tmp, tb));
             WEDGE_CHECK(cub::DeviceRadixSort::SortPairs(tmp, tb, kb, vb, (long long)E, s0, s0 + vbits, st));
             if (vb.Current() != *cw)
                 WEDGE_CHECK(cudaMemcpyAsync(*cw, vb.Current(), E * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, st));
         } else {
             WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(nullptr, tb, kb, (long long)E, s0, s0 + vbits, st));
-            WEDGE_CHECK(cudaMallocAsync(&tmp, tb ? tb : 1, st));
+            WEDGE_CHECK(talloc(h, &tmp, tb));
             WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tb, kb, (long long)E, s0, s0 + vbits, st));
         }
-        cudaFreeAsync(tmp, st);
+        tfree(h, tmp);
         csr_unpack_kernel<<<grid, AUX_THREADS, 0, st>>>(kb.Current(), E, shift, wshift, *csri, *cw8);
     }
-    cudaFreeAsync(ek, st);
-    cudaFreeAsync(ek2, st);
+    tfree(h, ek);
+    tfree(h, ek2);
     if (w2)
-        cudaFreeAsync(w2, st);
+        tfree(h, w2);
+    trelease(h, mark);
     WEDGE_CHECK(cudaGetLastError());
     return WEDGE_OK;
 }
@@ -682,9 +734,18 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
     g.w = d_w;
     const uint32_t cap = (uint32_t)h->num_sms * 16u;
 
+    if (E + V <= LOAD_SCRATCH_EDGES) { /* two key arrays, a sort's work space, wide weights; then the scans' */
+        h->tsize = (E + V) * (d_w ? 24u : 16u) + 24u * V + E + (4ull << 20);
+        h->tused = 0;
+        if (cudaMalloc((void**)&h->tscratch, h->tsize) != cudaSuccess) {
+            cudaGetLastError();
+            h->tscratch = nullptr;
+        }
+    }
+
     // input errors and the largest uint64 weight
     unsigned long long *d_chk = nullptr, chk[3] = {0ull, 0ull, 0ull};
-    WEDGE_CHECK(cudaMallocAsync((void**)&d_chk, sizeof(chk), st));
+    WEDGE_CHECK(talloc(h, &d_chk, sizeof(chk)));
     WEDGE_CHECK(cudaMemsetAsync(d_chk, 0, sizeof(chk), st));
     if (E)
         validate_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, d_dst, E, V, grouped,
@@ -694,7 +755,7 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
                                                                                  d_chk + 1);
     WEDGE_CHECK(cudaMemcpyAsync(chk, d_chk, sizeof(chk), cudaMemcpyDeviceToHost, st));
     WEDGE_CHECK(cudaStreamSynchronize(st));
-    cudaFreeAsync(d_chk, st);
+    tfree(h, d_chk);
     // weights in one byte each where every uint64 weight is below 256: the pulls
     // stream 1 byte per in-edge instead of 8
     const bool byte_weights = E && d_w && weight_kind == WEDGE_WEIGHTS_U64 && chk[1] < 256ull;
@@ -739,7 +800,7 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
 
     // compressed destinations
     uint32_t* kidx = nullptr;
-    WEDGE_CHECK(cudaMallocAsync((void**)&kidx, (E ? E : 1) * sizeof(uint32_t), st));
+    WEDGE_CHECK(talloc(h, &kidx, (E ? E : 1) * sizeof(uint32_t)));
     uint32_t Vne = 0;
     if (E) {
         head_flag_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_dst, E, kidx);
@@ -763,18 +824,18 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
     }
     tile_index_kernel<<<grid_for((uint64_t)g.T + 1, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(kidx, E, g.T, Vne,
                                                                                                tile_dst0, dst_off);
-    cudaFreeAsync(kidx, st);
+    tfree(h, kidx);
 
     // CSRI offsets: the out-degrees' prefix sums (a shard's CSRI indexes its own in-edges)
     uint32_t* own = outdeg;
     if (d_global_outdeg) {
-        WEDGE_CHECK(cudaMallocAsync((void**)&own, V * sizeof(uint32_t), st));
+        WEDGE_CHECK(talloc(h, &own, V * sizeof(uint32_t)));
         WEDGE_CHECK(cudaMemsetAsync(own, 0, V * sizeof(uint32_t), st));
         if (E)
             outdeg_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, E, own);
     }
     unsigned long long* wide = nullptr;
-    WEDGE_CHECK(cudaMallocAsync((void**)&wide, (V + 1) * sizeof(unsigned long long), st));
+    WEDGE_CHECK(talloc(h, &wide, (V + 1) * sizeof(unsigned long long)));
     widen_kernel<<<grid_for(V, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(own, wide, V);
     WEDGE_CHECK(cudaMemsetAsync(wide + V, 0, sizeof(unsigned long long), st));
     if ((rc = device_scan(h, wide, csri_off, V + 1, false)))
@@ -783,9 +844,9 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
         WEDGE_CHECK(cudaMemcpyAsync(wide, csri_off, (V + 1) * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, st));
         csri_fill_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, E, wide, csri);
     }
-    cudaFreeAsync(wide, st);
+    tfree(h, wide);
     if (own != outdeg)
-        cudaFreeAsync(own, st);
+        tfree(h, own);
 
     // symmetry (CC's label space); inv stays: a vertex's compressed destination
     unsigned int h_asym = 1u;
@@ -794,7 +855,7 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
         unsigned int* d_asym = nullptr; /* [0] an edge without its reverse, [1] the searches are needed */
         if ((rc = dalloc(h, &inv, V)))
             return rc;
-        WEDGE_CHECK(cudaMallocAsync((void**)&d_asym, 2 * sizeof(unsigned int), st));
+        WEDGE_CHECK(talloc(h, &d_asym, 2 * sizeof(unsigned int)));
         WEDGE_CHECK(cudaMemsetAsync(d_asym, 0, sizeof(unsigned int), st));
         WEDGE_CHECK(cudaMemsetAsync(d_asym + 1, chunks ? 0xFF : 0, sizeof(unsigned int), st));
         WEDGE_CHECK(cudaMemsetAsync(inv, 0xFF, V * sizeof(uint32_t), st));
@@ -804,7 +865,7 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
                                                                                      Vne, E, d_asym + 1);
         sym_check_kernel<<<grid_for(E, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, d_dst, E, inv, dst_off, d_asym);
         WEDGE_CHECK(cudaMemcpyAsync(&h_asym, d_asym, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
-        cudaFreeAsync(d_asym, st);
+        tfree(h, d_asym);
     }
     cudaFreeAsync(d_dst, st);
 
@@ -822,7 +883,7 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
     if ((rc = dalloc(h, &split_k, g.T)) || (rc = dalloc(h, &split_t0, g.T)) || (rc = dalloc(h, &split_t1, g.T)))
         return rc;
     unsigned int* d_cnt = nullptr;
-    WEDGE_CHECK(cudaMallocAsync((void**)&d_cnt, 4 * sizeof(unsigned int), st));
+    WEDGE_CHECK(talloc(h, &d_cnt, 4 * sizeof(unsigned int)));
     WEDGE_CHECK(cudaMemsetAsync(d_cnt, 0, 4 * sizeof(unsigned int), st));
     if (Vne)
         split_kernel<<<grid_for(Vne, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(dst_off, Vne, g.T, TILE, split_k, split_t0,
@@ -838,7 +899,7 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
     if (g.Epad > E)
         pad_kernel<<<1, 128, 0, st>>>(d_src, d_w, E, g.Epad);
     WEDGE_CHECK(cudaStreamSynchronize(st));
-    cudaFreeAsync(d_cnt, st);
+    tfree(h, d_cnt);
     WEDGE_CHECK(cudaGetLastError());
     g.nsplit = nsplit[0];
     g.nwide = nsplit[1];
@@ -862,6 +923,7 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
     g.split_k = split_k;
     g.split_t0 = split_t0;
     g.split_t1 = split_t1;
+    load_scratch_free(h);
 
     return compute_grids(h);
 }

@@ -260,6 +260,8 @@ struct wedge_graph {
     uint32_t hub_bytes;                // the hub cache's bytes
     uint32_t pull_smem;                // dynamic shared memory of the tile pulls (hub cache + staged minima)
     float* net;                        // device copy of the scheduler network (wedge_cuda_set_scheduler)
+    unsigned char* tscratch;           // the load's temporary arrays (small graphs; null otherwise and after the load)
+    uint64_t tsize, tused;
     // allocations owned by the handle
     void* allocs[40];
     int nallocs;
