@@ -243,3 +243,34 @@ def test_batched_pulls(engine_lib, n, weights):
                         assert np.array_equal(got[:n + 1], expect[i][:n + 1])
                         tail = got[n + 1:][got[n + 1:] != none].astype(np.int64)
                         assert np.all((tail == root) | ((tail >= 1) & (tail <= n)))
+
+
+@pytest.mark.parametrize("late", [0, 1, 2, 15, 40])
+@pytest.mark.parametrize("n", [1, 31, 33, 64, 300])
+def test_first_sources(engine_lib, monkeypatch, n, late):
+    """dense pulls that probe n destinations, each settled by its first source or by
+    the one after `late` others (within the probe window and past it), where the
+    launches run apart from the loop of small graphs"""
+    W = engine_lib
+    monkeypatch.setenv("WEDGE_CSRI_CHUNKS", "1")
+    # 0 -> 1 -> n destinations; `late` vertices that nothing reaches, of more out-edges, point at all of them too
+    V = 2 + n + late + 70
+    dests, others, extra = np.arange(2, 2 + n), np.arange(2 + n, 2 + n + late), np.arange(2 + n + late, V)
+    s = np.concatenate([[0], np.full(n, 1), np.repeat(others, n + 70)])
+    d = np.concatenate([[1], dests, np.tile(np.concatenate([dests, extra]), late)])
+    order = np.lexsort((s, d))
+    s, d = s[order].astype(np.uint32), d[order].astype(np.uint32)
+    none = np.uint64(0xFFFFFFFFFFFFFFFF)
+    parents = np.full(V, none)
+    parents[1], parents[dests] = 0, 1  # the root itself reads as without a parent
+    for flags in (0, W.FLAG_GRAPH):
+        with W.Graph.from_edges(V, s, d) as g:
+            g.run(W.APP_BFS, W.Params(root=0, sched=W.SCHED_DENSE, flags=flags))
+            assert np.array_equal(g.read_results(), parents)
+            g.run(W.APP_CC, W.Params(sched=W.SCHED_DENSE, flags=flags))
+            assert np.array_equal(g.read_results().view(np.float64), least_labels(V, s, d))
+        both = np.lexsort((np.concatenate([s, d]), np.concatenate([d, s])))
+        s2, d2 = np.concatenate([s, d])[both], np.concatenate([d, s])[both]
+        with W.Graph.from_edges(V, s2, d2) as g:
+            g.run(W.APP_CC, W.Params(sched=W.SCHED_DENSE, flags=flags))
+            assert np.array_equal(g.read_results().view(np.float64), least_labels(V, s2, d2))

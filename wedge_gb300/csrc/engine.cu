@@ -453,6 +453,13 @@ __global__ void narrow_weights_kernel(const unsigned long long* w, uint64_t E, u
         w8[e] = (uint8_t)w[e];
 }
 
+// the first (least) source of every destination
+__global__ void first_source_kernel(const uint32_t* src, const unsigned long long* dst_off, uint32_t Vne, uint32_t* first_src)
+{
+    for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < Vne; k += (uint64_t)gridDim.x * blockDim.x)
+        first_src[k] = src[dst_off[k]];
+}
+
 __global__ void pad_kernel(uint32_t* src, unsigned long long* w, uint64_t E, uint64_t Epad)
 {
     for (uint64_t e = E + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < Epad; e += (uint64_t)gridDim.x * blockDim.x) {
@@ -879,7 +886,12 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
         dst_start_kernel<<<grid_for(Vne, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(dst_off, Vne, dst_start);
 
     // destinations whose in-edges span tiles (PageRank fixup list)
-    uint32_t *split_k, *split_t0, *split_t1;
+    uint32_t *split_k, *split_t0, *split_t1, *first_src;
+    if ((rc = dalloc(h, &first_src, Vne)))
+        return rc;
+    if (Vne)
+        first_source_kernel<<<grid_for(Vne, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, dst_off, Vne, first_src);
+    g.first_src = first_src;
     if ((rc = dalloc(h, &split_k, g.T)) || (rc = dalloc(h, &split_t0, g.T)) || (rc = dalloc(h, &split_t1, g.T)))
         return rc;
     unsigned int* d_cnt = nullptr;
@@ -2340,6 +2352,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
     constexpr uint32_t TILE_E = 32u * EPL;
     __shared__ unsigned long long sh_cnt[WARPS][NCNT];
     __shared__ unsigned int sh_deg[3];
+    __shared__ uint32_t sh_late[WARPS][64];
     Ctrl* c = s.ctrl;
     if (c->done)
         return;
@@ -2376,6 +2389,45 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
         const uint32_t same = __match_any_sync(FULL, dw);
         if (dw != NONE32 && (uint32_t)(__ffs(same) - 1) == (uint32_t)lane)
             ++occ;
+    };
+
+    // Destinations whose first source does not settle them wait in the warp's
+    // buffer; late(n) goes on with the last n of them, one per lane.  Called by
+    // all lanes.
+    uint32_t kept = 0u;
+    uint32_t* my_late = sh_late[wib];
+    auto defer = [&](bool on, uint32_t k, auto late) {
+        const uint32_t m = __ballot_sync(FULL, on);
+        if (!m)
+            return;
+        if (on)
+            my_late[kept + (uint32_t)__popc(m & ((1u << lane) - 1u))] = k;
+        kept += (uint32_t)__popc(m);
+        __syncwarp();
+        if (kept >= 32u)
+            late(32u);
+    };
+    auto take = [&](uint32_t n) { /* lanes below n: a destination */
+        kept -= n;
+        const uint32_t k = (uint32_t)lane < n ? my_late[kept + (uint32_t)lane] : 0u;
+        __syncwarp();
+        return k;
+    };
+    // the changed destination d into the pull's output and the counters (a late one)
+    auto changed = [&](uint32_t d) {
+        const uint32_t o = g.outdeg[d];
+        occ += atomicOr(&nxt[d >> 5], 1u << (d & 31u)) == 0u ? 1u : 0u;
+        mass += o;
+        ++act;
+        return o;
+    };
+    auto count_degrees = [&](bool on, uint32_t od) {
+#pragma unroll
+        for (uint32_t b = 0; b < 3u; ++b) {
+            const uint32_t nb = __popc(__ballot_sync(FULL, on && degree_bucket(od) == b));
+            if (lane == 0 && nb)
+                atomicAdd(&sh_deg[b], nb);
+        }
     };
 
     // bitmap marks of tiles [ta, tb] (one lane)
@@ -2438,29 +2490,19 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
         const uint32_t kb = hubs ? 0u : s.hub_k, ke = hubs ? s.hub_k : g.Vne;
         const uint32_t hn = s.hub_n;
         const uint32_t nthr = gridDim.x * blockDim.x;
-        // the next group's offsets are loaded while this one is processed
-        unsigned long long plo = 0ull, phi = 0ull;
-        auto prefetch = [&](uint32_t b) {
-            const uint32_t kk = b + (uint32_t)lane;
-            if (kk < ke) {
-                plo = g.dst_off[kk];
-                phi = g.dst_off[kk + 1u];
-            }
-        };
-        prefetch(kb + gw * 32u);
-        for (uint32_t base = kb + gw * 32u; base < ke; base += nthr) {
-            const uint32_t k = base + (uint32_t)lane;
-            const unsigned long long lo = plo, hi = phi;
-            prefetch(base + nthr);
-            bool chg = false, zero = false;
-            uint32_t d = 0u, od = 0u;
-            if (k < ke) {
-                d = g.dst_ident ? k : g.dst_id[k];
+        auto late = [&](uint32_t n) { /* a hub source whose label is not 0 came first */
+            const bool on = (uint32_t)lane < n;
+            const uint32_t k = take(n);
+            bool chg = false;
+            uint32_t od = 0u;
+            if (on) {
+                const uint32_t d = g.dst_ident ? k : g.dst_id[k];
+                const unsigned long long lo = g.dst_off[k], hi = g.dst_off[k + 1u];
                 uint32_t m = d;
                 unsigned long long e = lo;
                 while (e < hi) {
                     const uint32_t x = g.src[e++];
-                    if (hubs || x >= hn) {
+                    if (x >= hn) {
                         m = x < m ? x : m;
                         break;
                     }
@@ -2471,21 +2513,47 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
                 }
                 edges += e - lo;
                 chg = m < d;
-                zero = chg && m == 0u;
                 if (chg) {
                     s.prop32[d] = m; /* the destination's only writer */
-                    od = g.outdeg[d];
+                    if (m == 0u)
+                        atomicOr(&s.vis_c[k >> 5], 1u << (k & 31u)); /* label 0 is final */
+                    od = changed(d);
+                }
+            }
+            count_degrees(chg, od);
+        };
+        // the next group's first sources are loaded while this one is processed
+        uint32_t px = 0u;
+        auto prefetch = [&](uint32_t b) {
+            const uint32_t kk = b + (uint32_t)lane;
+            if (kk < ke)
+                px = g.first_src[kk];
+        };
+        prefetch(kb + gw * 32u);
+        for (uint32_t base = kb + gw * 32u; base < ke; base += nthr) {
+            const uint32_t k = base + (uint32_t)lane;
+            const uint32_t x = px;
+            prefetch(base + nthr);
+            bool chg = false, zero = false, more = false;
+            uint32_t d = 0u, od = 0u;
+            if (k < ke) {
+                d = g.dst_ident ? k : g.dst_id[k];
+                od = g.outdeg[d];
+                const uint32_t l = hubs || x >= hn ? x : s.prop32[x];
+                more = !hubs && x < hn && l != 0u;
+                if (!more) {
+                    ++edges;
+                    chg = l < d;
+                    zero = chg && l == 0u;
+                }
+                if (chg) {
+                    s.prop32[d] = l; /* the destination's only writer */
                     mass += od;
                     ++act;
                 }
             }
             dsts += (uint64_t)__popc(__ballot_sync(FULL, k < ke));
-#pragma unroll
-            for (uint32_t b = 0; b < 3u; ++b) {
-                const uint32_t nb = __popc(__ballot_sync(FULL, chg && degree_bucket(od) == b));
-                if (lane == 0 && nb)
-                    atomicAdd(&sh_deg[b], nb);
-            }
+            count_degrees(chg, od);
             if (g.dst_ident) { /* d = k: the lanes' bits fall in two words at most */
                 const uint32_t w0 = base >> 5;
                 const bool in0 = (k >> 5) == w0;
@@ -2511,7 +2579,10 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
                     atomicOr(&s.vis_c[k >> 5], 1u << (k & 31u));
                 count_words(chg ? d >> 5 : NONE32);
             }
+            defer(more, k, late);
         }
+        if (kept)
+            late(kept);
     }
     if (APP == WEDGE_APP_BFS && cand) {
         // A Wedge pull over the candidates the last build listed (unvisited
@@ -2570,34 +2641,21 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
         // without a hit has no parent this iteration (the frontier is fixed
         // during a pull); one with sources left marks the tiles holding them in
         // tile_need, the only tiles the tile pull (the next launch) walks.
+        // 93% of the first dense pull's destinations at R-MAT scale 24 are settled
+        // by their first source, read from an array of its own: 4 bytes each in
+        // order, where the offset and the sector of the list took 40.
         const uint32_t nthr = gridDim.x * blockDim.x;
-        // the next group's visited word and offsets are loaded while this one is
-        // probed (each group's vis_c word belongs to its warp alone)
-        uint32_t pv = 0u;
-        unsigned long long plo = 0ull, phi = 0ull;
-        auto prefetch = [&](uint32_t b) {
-            const uint32_t kk = b + (uint32_t)lane;
-            if (b < g.Vne)
-                pv = s.vis_c[b >> 5];
-            if (kk < g.Vne) {
-                plo = g.dst_off[kk];
-                phi = g.dst_off[kk + 1u];
-            }
-        };
-        prefetch(gw * 32u);
-        for (uint32_t base = gw * 32u; base < g.Vne; base += nthr) {
-            const uint32_t k = base + (uint32_t)lane; /* base is a multiple of 32: one vis_c word */
-            const uint32_t vw = pv;
-            const unsigned long long lo = plo, hi = phi;
-            prefetch(base + nthr);
-            const bool todo = k < g.Vne && !((vw >> lane) & 1u);
+        auto late = [&](uint32_t n) {
+            const bool on = (uint32_t)lane < n;
+            const uint32_t k = take(n);
             bool hit = false;
-            uint32_t od = 0u, dw = NONE32;
+            uint32_t od = 0u;
             uint32_t ta = 1u, tb = 0u; /* tiles of a destination left unvisited (none: ta > tb) */
-            if (todo) {
+            if (on) {
                 const uint32_t d = g.dst_ident ? k : g.dst_id[k];
+                const unsigned long long lo = g.dst_off[k], hi = g.dst_off[k + 1u];
                 const unsigned long long lim = hi - lo > pwin ? lo + pwin : hi;
-                unsigned long long e = lo;
+                unsigned long long e = lo + (pwin ? 1ull : 0ull); /* the first source is not in the frontier */
                 uint32_t par = NONE32;
                 while (e < lim) {
                     const uint32_t x = g.src[e++];
@@ -2614,10 +2672,40 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
                     // sources past the window remain: the tile pull reads the tiles holding them
                     if (lim < hi)
                         need_tiles((uint32_t)(lim / TILE_E), tb);
-                }
-                if (hit) {
+                } else {
                     s.prop32[d] = par; /* the destination's only writer in this launch */
-                    od = g.outdeg[d];
+                    atomicOr(&s.vis_c[k >> 5], 1u << (k & 31u));
+                    od = changed(d);
+                }
+            }
+            mark_open(ta, tb);
+            count_degrees(hit, od);
+        };
+        // the next group's visited word and first sources are loaded while this one
+        // is probed (a group's vis_c word is its warp's alone)
+        uint32_t pv = 0u, px = 0u;
+        auto prefetch = [&](uint32_t b) {
+            const uint32_t kk = b + (uint32_t)lane;
+            if (b < g.Vne)
+                pv = s.vis_c[b >> 5];
+            if (kk < g.Vne)
+                px = g.first_src[kk];
+        };
+        prefetch(gw * 32u);
+        for (uint32_t base = gw * 32u; base < g.Vne; base += nthr) {
+            const uint32_t k = base + (uint32_t)lane; /* base is a multiple of 32: one vis_c word */
+            const uint32_t vw = pv, x = px;
+            prefetch(base + nthr);
+            const bool todo = k < g.Vne && !((vw >> lane) & 1u);
+            bool hit = false;
+            uint32_t od = 0u, dw = NONE32;
+            if (todo) {
+                const uint32_t d = g.dst_ident ? k : g.dst_id[k];
+                od = g.outdeg[d];
+                hit = pwin && (ld_ro_u32(cur + (x >> 5)) >> (x & 31u)) & 1u;
+                if (hit) {
+                    s.prop32[d] = x; /* the destination's only writer in this launch */
+                    ++edges;
                     mass += od;
                     ++act;
                     if (!g.dst_ident) {
@@ -2626,22 +2714,19 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
                     }
                 }
             }
-            mark_open(ta, tb);
             count_words(dw);
             dsts += (uint64_t)__popc(__ballot_sync(FULL, todo));
-#pragma unroll
-            for (uint32_t b = 0; b < 3u; ++b) {
-                const uint32_t nb = __popc(__ballot_sync(FULL, hit && degree_bucket(od) == b));
-                if (lane == 0 && nb)
-                    atomicAdd(&sh_deg[b], nb);
-            }
+            count_degrees(hit, od);
             const uint32_t hits = __ballot_sync(FULL, hit);
             if (lane == 0 && hits) {
                 atomicOr(&s.vis_c[base >> 5], hits);
                 if (g.dst_ident)
                     set_word(base >> 5, hits); /* d = k */
             }
+            defer(todo && !hit, k, late);
         }
+        if (kept)
+            late(kept);
     }
     if (APP == WEDGE_APP_CC && cand && phase == PHASE_DST_A) {
         // A Wedge pull over the candidates the last build listed (unfinished
@@ -2703,32 +2788,15 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
         // marks its tiles for the tile pull (the next two launches), which walks
         // only those.
         const uint32_t nthr = gridDim.x * blockDim.x;
-        // the next group's finished word and offsets are loaded while this one
-        // is probed (each group's vis_c word belongs to its warp alone)
-        uint32_t pv = 0u;
-        unsigned long long plo = 0ull, phi = 0ull;
-        auto prefetch = [&](uint32_t b) {
-            const uint32_t kk = b + (uint32_t)lane;
-            if (b < g.Vne)
-                pv = s.vis_c[b >> 5];
-            if (kk < g.Vne) {
-                plo = g.dst_off[kk];
-                phi = g.dst_off[kk + 1u];
-            }
-        };
-        prefetch(gw * 32u);
-        for (uint32_t base = gw * 32u; base < g.Vne; base += nthr) {
-            const uint32_t k = base + (uint32_t)lane; /* base is a multiple of 32: one vis_c word */
-            const uint32_t vw = pv;
-            const unsigned long long lo = plo, hi = phi;
-            prefetch(base + nthr);
-            const bool todo = k < g.Vne && !((vw >> lane) & 1u);
-            bool chg = false, zero = false;
-            uint32_t dw = NONE32;
-            uint32_t d = 0u, od = 0u;
+        auto late = [&](uint32_t n) {
+            const bool on = (uint32_t)lane < n;
+            const uint32_t k = take(n);
+            bool chg = false;
+            uint32_t od = 0u;
             uint32_t ta = 1u, tb = 0u;
-            if (todo) {
-                d = g.dst_ident ? k : g.dst_id[k];
+            if (on) {
+                const uint32_t d = g.dst_ident ? k : g.dst_id[k];
+                const unsigned long long lo = g.dst_off[k], hi = g.dst_off[k + 1u];
                 const unsigned long long lim = hi - lo > pwin ? lo + pwin : hi;
                 const uint32_t cv = s.prop32[d];
                 uint32_t m = cv;
@@ -2744,8 +2812,46 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
                 if (whole && m < cv) {
                     s.prop32[d] = m; /* the destination's only writer in this launch */
                     chg = true;
-                    zero = m == 0u;
-                    od = g.outdeg[d];
+                    if (m == 0u)
+                        atomicOr(&s.vis_c[k >> 5], 1u << (k & 31u)); /* label 0 is final */
+                    od = changed(d);
+                }
+                if (!whole)
+                    need_tiles((uint32_t)(lo / TILE_E), (uint32_t)((hi - 1u) / TILE_E));
+                if (!chg || m != 0u) {
+                    ta = (uint32_t)(lo / TILE_E);
+                    tb = (uint32_t)((hi - 1u) / TILE_E);
+                }
+            }
+            mark_open(ta, tb);
+            count_degrees(chg, od);
+        };
+        // the next group's finished word and first sources are loaded while this one
+        // is probed (a group's vis_c word is its warp's alone)
+        uint32_t pv = 0u, px = 0u;
+        auto prefetch = [&](uint32_t b) {
+            const uint32_t kk = b + (uint32_t)lane;
+            if (b < g.Vne)
+                pv = s.vis_c[b >> 5];
+            if (kk < g.Vne)
+                px = g.first_src[kk];
+        };
+        prefetch(gw * 32u);
+        for (uint32_t base = gw * 32u; base < g.Vne; base += nthr) {
+            const uint32_t k = base + (uint32_t)lane; /* base is a multiple of 32: one vis_c word */
+            const uint32_t vw = pv, x = px;
+            prefetch(base + nthr);
+            const bool todo = k < g.Vne && !((vw >> lane) & 1u);
+            bool chg = false;
+            uint32_t dw = NONE32, od = 0u;
+            if (todo) {
+                const uint32_t d = g.dst_ident ? k : g.dst_id[k];
+                od = g.outdeg[d];
+                const uint32_t cv = s.prop32[d];
+                chg = pwin && s.prop32[x] == 0u && cv != 0u; /* label 0 is final */
+                if (chg) {
+                    s.prop32[d] = 0u; /* the destination's only writer in this launch */
+                    ++edges;
                     mass += od;
                     ++act;
                     if (!g.dst_ident) {
@@ -2753,30 +2859,20 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
                         dw = d >> 5;
                     }
                 }
-                if (!whole)
-                    need_tiles((uint32_t)(lo / TILE_E), (uint32_t)((hi - 1u) / TILE_E));
-                if (!zero) {
-                    ta = (uint32_t)(lo / TILE_E);
-                    tb = (uint32_t)((hi - 1u) / TILE_E);
-                }
             }
-            mark_open(ta, tb);
             count_words(dw);
             dsts += (uint64_t)__popc(__ballot_sync(FULL, todo));
-#pragma unroll
-            for (uint32_t b = 0; b < 3u; ++b) {
-                const uint32_t nb = __popc(__ballot_sync(FULL, chg && degree_bucket(od) == b));
-                if (lane == 0 && nb)
-                    atomicAdd(&sh_deg[b], nb);
-            }
-            const uint32_t chgs = __ballot_sync(FULL, chg), zeros = __ballot_sync(FULL, zero);
-            if (lane == 0) {
-                if (zeros)
-                    atomicOr(&s.vis_c[base >> 5], zeros); /* label 0 is final */
-                if (chgs && g.dst_ident)
+            count_degrees(chg, od);
+            const uint32_t chgs = __ballot_sync(FULL, chg);
+            if (lane == 0 && chgs) {
+                atomicOr(&s.vis_c[base >> 5], chgs);
+                if (g.dst_ident)
                     set_word(base >> 5, chgs); /* d = k */
             }
+            defer(todo && !chg, k, late);
         }
+        if (kept)
+            late(kept);
     }
     mass = warp_sum_u64(mass);
     edges = warp_sum_u64(edges);

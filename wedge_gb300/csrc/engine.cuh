@@ -10,6 +10,7 @@
 //   dst_id[Vne]    vertex id of compressed destination k (only vertices with
 //                  in-degree > 0 are listed, ascending)
 //   dst_off[Vne+1] first edge of compressed destination k
+//   first_src[Vne] its first source, src[dst_off[k]]
 //   dst_start[Epad/32] one bit per in-edge: the first in-edge of its destination
 //   tile_dst0[T+1] compressed destination owning edge 128*t (Vne where that
 //                  edge is padding); pull tiles of 32*EPL edges index it with a stride
@@ -139,6 +140,7 @@ struct DevGraph {
     const uint32_t* src;
     const unsigned long long* w;
     const uint8_t* w8;         // the same weights in one byte each, when every weight is a uint64 below 256
+    const uint32_t* first_src; // [Vne] the first source of every destination
     const uint32_t* wsrc;      // [Epad] with byte-wide weights: every destination's sources by ascending weight
     const uint8_t* ww8;        // [Epad] and those weights (dst_off holds for both orders); or null
     const uint32_t* dst_id;
