@@ -3454,7 +3454,7 @@ __global__ void init_kernel(DevGraph g, DevState s, uint32_t app, uint32_t topen
             // execution_cc.c:77: labels are vertex ids -- the caller's, or on a
             // symmetric graph the engine's, converted when the labels converge
             s.prop32[v] = g.sym ? (uint32_t)v : g.new2old[v];
-            if (s.cc_best)
+            if (s.cc_best && (v < g.Vne || !g.dst_ident))
                 s.cc_best[v] = NONE32;
         }
         else {
@@ -3512,17 +3512,10 @@ __global__ void init_root_kernel(DevGraph g, DevState s, uint32_t app, uint64_t 
     if (app == WEDGE_APP_BFS || app == WEDGE_APP_CC) {
         // BFS: the root is visited; CC: the vertex whose id is label 0 holds the least label already
         const uint32_t done = (app == WEDGE_APP_BFS) ? (uint32_t)root : g.sym ? 0u : g.old2new[0];
-        if (tid == 0 && g.Vne) { /* its compressed index: dst_id ascends */
-            uint32_t lo = 0, hi = g.Vne;
-            while (lo < hi) {
-                const uint32_t mid = lo + (hi - lo) / 2u;
-                if (g.dst_id[mid] < done)
-                    lo = mid + 1u;
-                else
-                    hi = mid;
-            }
-            if (lo < g.Vne && g.dst_id[lo] == done)
-                atomicOr(&s.vis_c[lo >> 5], 1u << (lo & 31u));
+        if (tid == 0 && g.Vne) { /* its compressed index, if it has in-edges */
+            const uint32_t k = g.dst_ident ? done : g.dst_index[done];
+            if (k < g.Vne)
+                atomicOr(&s.vis_c[k >> 5], 1u << (k & 31u));
         }
     }
     if (tid == 0) {
@@ -3845,13 +3838,23 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
             if (!loop)
                 continue;
             uint32_t busy = __ballot_sync(FULL, word != 0u);
-            while (busy) { /* one word's vertices a round */
-                const int l = __ffs(busy) - 1;
-                busy &= busy - 1u;
-                const uint32_t w = __shfl_sync(FULL, word, l);
-                const uint32_t v = __shfl_sync(FULL, i, l) * 32u + (uint32_t)lane;
-                const bool on = (w >> lane) & 1u;
-                append(on, v, on ? g.outdeg[v] : 0u);
+            while (busy) { /* four words' vertices a round: their out-degrees are loaded together */
+                uint32_t v[4], od[4];
+                bool on[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int l = busy ? __ffs(busy) - 1 : 0;
+                    const uint32_t w = __shfl_sync(FULL, word, l);
+                    v[u] = __shfl_sync(FULL, i, l) * 32u + (uint32_t)lane;
+                    on[u] = busy && ((w >> lane) & 1u);
+                    busy &= busy - 1u;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    od[u] = on[u] ? g.outdeg[v[u]] : 0u;
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    append(on[u], v[u], od[u]);
             }
         }
         if (s.tile_need)
@@ -4328,8 +4331,12 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
 // phase_edge_pull_cc.c).  best[r] = min over the component of new2old[v], with
 // best preset to NONE32.  Label 0 (the component of engine vertex 0, the
 // highest-degree vertex: the giant component) is reduced per block first;
-// other components are small and take one global atomic per vertex.
-__global__ void cc_best_kernel(DevGraph g, const uint32_t* label, uint32_t* best)
+// other components are small and take one global atomic per vertex.  Only the
+// first n vertices are looked at: the isolated ones (from Vne on where dst_ident,
+// about half of an R-MAT graph) keep their own id.  Bound by the memory traffic,
+// 16 bytes per thread and access: 37 + 44 us for the two kernels at scale 24
+// over every vertex, 4 bytes each, CC_NOW us so.
+__global__ void cc_best_kernel(DevGraph g, const uint32_t* label, uint32_t* best, uint64_t n)
 {
     __shared__ uint32_t best0;
     if (threadIdx.x == 0)
@@ -4337,13 +4344,22 @@ __global__ void cc_best_kernel(DevGraph g, const uint32_t* label, uint32_t* best
     __syncthreads();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     uint32_t m0 = NONE32;
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < g.V; v += stride) {
-        const uint32_t r = label[v], o = g.new2old[v];
+    auto one = [&](uint32_t r, uint32_t o) {
         if (r == 0u)
             m0 = o < m0 ? o : m0;
         else
             atomicMin(&best[r], o);
+    };
+    const uint64_t quads = n / 4u, tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    for (uint64_t i = tid; i < quads; i += stride) {
+        const uint4 r = reinterpret_cast<const uint4*>(label)[i], o = reinterpret_cast<const uint4*>(g.new2old)[i];
+        one(r.x, o.x);
+        one(r.y, o.y);
+        one(r.z, o.z);
+        one(r.w, o.w);
     }
+    if (tid < n - 4u * quads)
+        one(label[4u * quads + tid], g.new2old[4u * quads + tid]);
     m0 = __reduce_min_sync(FULL, m0);
     if ((threadIdx.x & 31) == 0 && m0 != NONE32)
         atomicMin(&best0, m0);
@@ -4352,11 +4368,28 @@ __global__ void cc_best_kernel(DevGraph g, const uint32_t* label, uint32_t* best
         atomicMin(&best[0], best0);
 }
 
-// label[v] = best[label[v]]: the caller-id labels
-__global__ void cc_apply_kernel(DevGraph g, uint32_t* label, const uint32_t* best)
+// label[v] = best[label[v]]: the caller-id labels; an isolated vertex's is its own id
+__global__ void cc_apply_kernel(DevGraph g, uint32_t* label, const uint32_t* best, uint64_t n)
 {
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < g.V; v += (uint64_t)gridDim.x * blockDim.x)
-        label[v] = best[label[v]];
+    const uint64_t quads = g.V / 4u, tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    const uint32_t b0 = best[0];
+    for (uint64_t i = tid; i < quads; i += (uint64_t)gridDim.x * blockDim.x) {
+        uint4 r;
+        if (4u * i >= n) {
+            r = reinterpret_cast<const uint4*>(g.new2old)[i];
+        } else {
+            r = reinterpret_cast<const uint4*>(label)[i];
+            r.x = r.x ? best[r.x] : b0;
+            r.y = r.y ? (4u * i + 1u < n ? best[r.y] : g.new2old[4u * i + 1u]) : b0;
+            r.z = r.z ? (4u * i + 2u < n ? best[r.z] : g.new2old[4u * i + 2u]) : b0;
+            r.w = r.w ? (4u * i + 3u < n ? best[r.w] : g.new2old[4u * i + 3u]) : b0;
+        }
+        reinterpret_cast<uint4*>(label)[i] = r;
+    }
+    if (tid < g.V - 4u * quads) {
+        const uint64_t v = 4u * quads + tid;
+        label[v] = v < n ? best[label[v]] : g.new2old[v];
+    }
 }
 
 /* ------------------------------------------------------------- PageRank */
@@ -6167,8 +6200,9 @@ static void launch_init(wedge_graph* h, int app, uint64_t root, uint32_t sched, 
 // place (2 launches; best was preset by init_kernel)
 static void cc_finalize(wedge_graph* h)
 {
-    cc_best_kernel<<<aux_grid(h, h->g.V), AUX_THREADS, 0, h->stream>>>(h->g, h->s.prop32, h->s.cc_best);
-    cc_apply_kernel<<<aux_grid(h, h->g.V), AUX_THREADS, 0, h->stream>>>(h->g, h->s.prop32, h->s.cc_best);
+    const uint64_t n = h->g.dst_ident ? (uint64_t)h->g.Vne : h->g.V;
+    cc_best_kernel<<<aux_grid(h, n / 4 + 4), AUX_THREADS, 0, h->stream>>>(h->g, h->s.prop32, h->s.cc_best, n);
+    cc_apply_kernel<<<aux_grid(h, h->g.V / 4 + 4), AUX_THREADS, 0, h->stream>>>(h->g, h->s.prop32, h->s.cc_best, n);
     h->cc_pending = 0;
 }
 
@@ -6182,7 +6216,7 @@ static int result_state(wedge_graph* h, DevState* out)
         out->rank += h->s.rstride;
     if (h->last_app == WEDGE_APP_CC && h->cc_pending) {
         WEDGE_CHECK(cudaMemsetAsync(h->s.cc_best, 0xFF, h->g.V * sizeof(uint32_t), h->stream));
-        cc_best_kernel<<<aux_grid(h, h->g.V), AUX_THREADS, 0, h->stream>>>(h->g, h->s.prop32, h->s.cc_best);
+        cc_best_kernel<<<aux_grid(h, h->g.V), AUX_THREADS, 0, h->stream>>>(h->g, h->s.prop32, h->s.cc_best, h->g.V);
         out->cc_map = h->s.cc_best;
     }
     return WEDGE_OK;
