@@ -2343,7 +2343,12 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
 // pull over engine-id labels (launch A: the hub destinations, launch B: the
 // rest).  Latency-bound chains of a few dependent loads: 32 registers, two
 // 1024-thread blocks per SM, so twice the warps of the tile pull are in
-// flight.  block_cnt as pull_kernel's.
+// flight.  Most destinations are settled by their first source, which
+// first_src holds in order: 4 bytes each instead of an offset and a sector of
+// the list.  The others wait until a warp has 32 of them, so that their longer
+// chains hold up no settled ones.  R-MAT scale 24: CC's two dense pulls 102 and
+// 80 us before, 57 and 53 so; a BFS's 124 and 57, 104 and 47 (16% of its first
+// pull's destinations go on past the first source).  block_cnt as pull_kernel's.
 template <int APP, int EPL>
 __global__ void __launch_bounds__(PULL_THREADS, 2)
     dst_kernel(DevGraph g, DevState s, unsigned long long* block_cnt, uint32_t phase)
@@ -3838,7 +3843,10 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
             if (!loop)
                 continue;
             uint32_t busy = __ballot_sync(FULL, word != 0u);
-            while (busy) { /* four words' vertices a round: their out-degrees are loaded together */
+            while (busy) {
+                /* four words' vertices a round, their out-degrees loaded together: the
+                   chain of one word a round took 25 us of a scale-24 BFS's last Wedge
+                   iterations (131 -> 105 us with 1.15 M vertices listed) */
                 uint32_t v[4], od[4];
                 bool on[4];
 #pragma unroll
@@ -4335,7 +4343,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
 // first n vertices are looked at: the isolated ones (from Vne on where dst_ident,
 // about half of an R-MAT graph) keep their own id.  Bound by the memory traffic,
 // 16 bytes per thread and access: 37 + 44 us for the two kernels at scale 24
-// over every vertex, 4 bytes each, CC_NOW us so.
+// over every vertex, 4 bytes each, 17 + 23 so.
 __global__ void cc_best_kernel(DevGraph g, const uint32_t* label, uint32_t* best, uint64_t n)
 {
     __shared__ uint32_t best0;
