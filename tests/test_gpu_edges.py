@@ -274,3 +274,33 @@ def test_first_sources(engine_lib, monkeypatch, n, late):
         with W.Graph.from_edges(V, s2, d2) as g:
             g.run(W.APP_CC, W.Params(sched=W.SCHED_DENSE, flags=flags))
             assert np.array_equal(g.read_results().view(np.float64), least_labels(V, s2, d2))
+
+
+@pytest.mark.parametrize("limit", [None, 300])
+@pytest.mark.parametrize("weights", ["bytes", "zeros", "equal", "steep"])
+def test_bounded_weight_ordered_pulls(engine_lib, weights, limit):
+    """several dense pulls in a row with a bound from the vertices the last one
+    changed, Wedge iterations run as such pulls, and short tails after them, on a
+    graph too large for the loop of small ones; a chain keeps a few vertices
+    changing, and some sums pass a 32-bit limit"""
+    W = engine_lib
+    rng = np.random.default_rng(len(weights))
+    V, n = 60_001, 1_250_000
+    s = np.minimum((V * rng.random(n) ** 3).astype(np.int64), V - 2)
+    d = np.minimum((V * rng.random(n) ** 2).astype(np.int64), V - 2)
+    chain = rng.permutation(V - 1)[:300]
+    s, d = np.concatenate([s, chain[:-1]]), np.concatenate([d, chain[1:]])
+    w = {"bytes": rng.integers(0, 256, len(s)), "zeros": rng.integers(0, 256, len(s)) * (rng.random(len(s)) < 0.3),
+         "equal": np.full(len(s), 7), "steep": np.minimum(255, s % 256 + 1)}[weights].astype(np.int64)
+    w[-299:] = 1
+    order = np.lexsort((s, d))
+    s, d, w = s[order].astype(np.uint32), d[order].astype(np.uint32), w[order].astype(np.uint64)
+    root = int(s[0])
+    expect = bellman_ford(V, s, d, w, root)
+    with W.Graph.from_edges(V, s, d, w) as g:
+        g.set_knob("sssp_narrow", limit)
+        for sched in (W.SCHED_PLAIN, W.SCHED_DENSE, W.SCHED_FILTERED, W.SCHED_WEDGE):
+            for flags in (0, W.FLAG_GRAPH, W.FLAG_TIMING):
+                for threshold_pct in (1, 20, 100):
+                    g.run(W.APP_SSSP, W.Params(root=root, sched=sched, flags=flags, threshold_pct=threshold_pct))
+                    assert np.array_equal(g.read_results(), expect), (sched, flags, threshold_pct)

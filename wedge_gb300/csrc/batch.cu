@@ -39,7 +39,7 @@ constexpr int BT = 256;                       // threads per persistent block
 constexpr uint32_t BATCH_MAX_ROUNDS = 1u << 20; // iteration cap of the slowest query
 constexpr uint32_t PUSH_CHUNK = 4;              // listed vertices per item
 constexpr uint32_t PUSH_PIECE = 128;            // out-edges of a long list per item
-constexpr uint32_t WO_GROUP = 64;               // in-edges of the longest destination a group of 32 pulls
+constexpr uint32_t WO_GROUP = WO_MANY;          // in-edges of the longest destination a group of 32 pulls
 constexpr uint32_t WO_PIECE = 512;              // in-edges per item of the longer ones
 constexpr uint32_t SWEEP = 1024;                // bitmap words per clearing piece
 
@@ -53,6 +53,8 @@ struct BGraph {
     const uint8_t* w8;           // byte-wide weights, or null
     const uint32_t* wsrc;        // weight-ordered sources and weights, or null
     const uint8_t* ww8;
+    const uint32_t* wo_src;      // every destination's first weight-ordered source (bit 31: its only one)
+    const uint16_t* wo_w;        // and first two weights
     const uint2* wo_long;        // (destination, first in-edge) pieces of the destinations past WO_GROUP in-edges
     uint32_t nlong;
     const uint32_t* outdeg;
@@ -81,6 +83,7 @@ struct BCtl {
     unsigned long long mass;
     uint32_t nlist[3]; // by iteration modulo 3
     uint32_t nitem[3];
+    unsigned long long fmin, next_fmin; // SSSP: no vertex the last (this) iteration changed is nearer
     uint32_t items; // work items of the next pull
     uint32_t mode;
     uint32_t iter;
@@ -419,7 +422,8 @@ __device__ void pull_tile(const BArgs& a, uint32_t q, uint32_t t, unsigned long 
 // listing in stages, so that the four chains are in flight together.  BFS: an
 // unvisited destination takes the vertex as its parent; SSSP: min-plus.
 __device__ __forceinline__ void push4(const BQuery& qq, BCtl& c, const BGraph& G, const bool (&on)[4],
-                                      const unsigned long long (&x)[4], const uint32_t (&e)[4], unsigned long long& mass)
+                                      const unsigned long long (&x)[4], const uint32_t (&e)[4], unsigned long long& mass,
+                                      unsigned long long& least)
 {
     uint32_t* nxt = qq.front[(c.iter + 1u) % 3u];
     const bool bfs = qq.app == WEDGE_APP_BFS, f64 = G.weight_kind == WEDGE_WEIGHTS_F64;
@@ -447,8 +451,11 @@ __device__ __forceinline__ void push4(const BQuery& qq, BCtl& c, const BGraph& G
             p[u] = bfs ? atomicCAS(&qq.prop[d[u]], NONE64, nd[u]) : atomicMin(&qq.prop[d[u]], nd[u]);
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < 4; ++u) {
         low[u] = low[u] && (bfs ? p[u] == NONE64 : nd[u] < p[u]);
+        if (low[u])
+            least = min(least, nd[u]);
+    }
     if (!__any_sync(FULL, low[0] || low[1] || low[2] || low[3]))
         return;
     uint32_t o[4], od[4];
@@ -475,7 +482,7 @@ __device__ __forceinline__ unsigned long long push_value(const BQuery& qq, uint3
 }
 
 // one PUSH_PIECE of a long out-list
-__device__ void push_piece(const BArgs& a, uint32_t q, uint2 it, unsigned long long& mass)
+__device__ void push_piece(const BArgs& a, uint32_t q, uint2 it, unsigned long long& mass, unsigned long long& least)
 {
     const int lane = threadIdx.x & 31;
     const BQuery& qq = a.q[q];
@@ -493,7 +500,7 @@ __device__ void push_piece(const BArgs& a, uint32_t q, uint2 it, unsigned long l
             e[u] = t + 32u * u + (uint32_t)lane;
             on[u] = e[u] < hi;
         }
-        push4(qq, c, G, on, x, e, mass);
+        push4(qq, c, G, on, x, e, mass, least);
     }
 }
 
@@ -503,7 +510,8 @@ struct PushShared {
     unsigned long long val[PUSH_CHUNK];
 };
 
-__device__ void push_chunk(const BArgs& a, uint32_t q, uint32_t i0, uint32_t n, PushShared& sh, unsigned long long& mass)
+__device__ void push_chunk(const BArgs& a, uint32_t q, uint32_t i0, uint32_t n, PushShared& sh, unsigned long long& mass,
+                           unsigned long long& least)
 {
     const int lane = threadIdx.x & 31;
     const BQuery& qq = a.q[q];
@@ -546,15 +554,24 @@ __device__ void push_chunk(const BArgs& a, uint32_t q, uint32_t i0, uint32_t n, 
             e[u] = sh.beg[o] + t;
             x[u] = sh.val[o];
         }
-        push4(qq, c, G, on, x, e, mass);
+        push4(qq, c, G, on, x, e, mass, least);
     }
+}
+
+// the weights that may lower a distance: below this.  After a pull only the
+// vertices it changed matter to the next; none of them, and none it lowers in
+// turn, is nearer than fmin.
+__device__ __forceinline__ unsigned long long wo_limit(unsigned long long dist, unsigned long long fmin)
+{
+    return dist > fmin ? dist - fmin : 0ull;
 }
 
 // four weight-ordered in-edges at position p (a multiple of 4), of which those
 // in [lo, hi) are the destination's; returns the weight of position p + 3
 __device__ __forceinline__ uint32_t wo_step(const BQuery& qq, const BGraph& G, uint32_t p, uint32_t lo, uint32_t hi,
-                                            unsigned long long& dist)
+                                            unsigned long long fmin, unsigned long long& dist)
 {
+    const unsigned long long lim = wo_limit(dist, fmin);
     const uint32_t ww = ld_ro_u32(reinterpret_cast<const uint32_t*>(G.ww8 + p));
     const uint4 xs = __ldg(reinterpret_cast<const uint4*>(G.wsrc + p));
     const uint32_t x[4] = {xs.x, xs.y, xs.z, xs.w};
@@ -562,7 +579,7 @@ __device__ __forceinline__ uint32_t wo_step(const BQuery& qq, const BGraph& G, u
 #pragma unroll
     for (uint32_t j = 0; j < 4; ++j) {
         const uint32_t w = (ww >> (8 * j)) & 0xFFu;
-        y[j] = (p + j >= lo && p + j < hi && w < dist) ? qq.prop[x[j]] : NONE64;
+        y[j] = (p + j >= lo && p + j < hi && w < lim) ? qq.prop[x[j]] : NONE64;
     }
 #pragma unroll
     for (uint32_t j = 0; j < 4; ++j)
@@ -574,17 +591,17 @@ __device__ __forceinline__ uint32_t wo_step(const BQuery& qq, const BGraph& G, u
 // weight-ordered in-edges [p, hi) by the warp, 128 a step, up to the first
 // weight that cannot lower dist (p a multiple of 4; all warp-uniform)
 __device__ __forceinline__ unsigned long long wo_run(const BQuery& qq, const BGraph& G, uint32_t p, uint32_t hi,
-                                                     unsigned long long dist)
+                                                     unsigned long long fmin, unsigned long long dist)
 {
     const int lane = threadIdx.x & 31;
     const uint32_t lo = p;
     for (; p < hi; p += 128u) {
         const uint32_t at = p + 4u * (uint32_t)lane;
-        const uint32_t last = at < hi ? wo_step(qq, G, at, lo, hi, dist) : 0xFFFFFFFFu;
+        const uint32_t last = at < hi ? wo_step(qq, G, at, lo, hi, fmin, dist) : 0xFFFFFFFFu;
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1)
             dist = min(dist, __shfl_xor_sync(FULL, dist, d));
-        if (__shfl_sync(FULL, last, 31) >= dist)
+        if (__shfl_sync(FULL, last, 31) >= wo_limit(dist, fmin))
             break;
     }
     return dist;
@@ -595,32 +612,41 @@ __device__ __forceinline__ unsigned long long wo_run(const BQuery& qq, const BGr
 // holds up 31 others (groups of up to 32, 64, 128 and 256 in-edges took 4.4,
 // 3.7, 3.8 and 3.6 ms on the 32 SSSPs of phase_pull's comment, 2.06, 1.72, 1.80
 // and 2.09 ms on 16 over graphs of scales 16 to 20).
-__device__ void wo_group(const BArgs& a, uint32_t q, uint32_t group, unsigned long long& mass)
+__device__ void wo_group(const BArgs& a, uint32_t q, uint32_t group, unsigned long long& mass, unsigned long long& least)
 {
     const int lane = threadIdx.x & 31;
     const BQuery& qq = a.q[q];
     BCtl& c = a.ctl[q];
     const BGraph& G = a.graphs[qq.graph];
     const uint32_t k = group * 32u + (uint32_t)lane;
-    uint32_t lo = 0u, hi = 0u, d = 0u;
-    if (k < G.Vne) {
-        lo = (uint32_t)G.dst_off[k];
-        hi = (uint32_t)G.dst_off[k + 1u];
+    const unsigned long long fmin = c.fmin;
+    unsigned long long before = 0ull, dist = 0ull;
+    uint32_t d = 0u;
+    bool more = false;
+    if (k < G.Vne) { /* the first in-edge and the second's weight settle most */
+        const uint32_t x = G.wo_src[k], w = G.wo_w[k];
         d = G.dst_id[k];
+        before = dist = qq.prop[d];
+        if (!(x & WO_MANY_BIT) && (w & 0xFFu) < wo_limit(dist, fmin)) { /* the long ones are left to their pieces */
+            const unsigned long long y = qq.prop[x & WO_ID_BITS];
+            if (y != NONE64)
+                dist = min(dist, y + (w & 0xFFu));
+            more = !(x & WO_ONLY_BIT) && (w >> 8) < wo_limit(dist, fmin);
+        }
     }
-    const bool mine = hi - lo <= WO_GROUP && hi != lo;
-    const unsigned long long before = mine ? qq.prop[d] : 0ull;
-    unsigned long long dist = before;
-    bool more = mine;
-    for (uint32_t p = lo & ~3u; more; ) {
-        const uint32_t last = wo_step(qq, G, p, lo, hi, dist);
-        p += 4u;
-        more = p < hi && last < dist;
+    if (more) {
+        const uint32_t lo = (uint32_t)G.dst_off[k], hi = (uint32_t)G.dst_off[k + 1u];
+        for (uint32_t p = lo & ~3u; more;) {
+            const uint32_t last = wo_step(qq, G, p, lo, hi, fmin, dist);
+            p += 4u;
+            more = p < hi && last < wo_limit(dist, fmin);
+        }
     }
     const bool low = dist < before;
     uint32_t od = 0u;
     if (low) { /* the destination's only writer in this pull */
         qq.prop[d] = dist;
+        least = min(least, dist);
         atomicOr(&qq.front[(c.iter + 1u) % 3u][d >> 5], 1u << (d & 31u));
         od = G.outdeg[d];
         mass += od;
@@ -629,7 +655,7 @@ __device__ void wo_group(const BArgs& a, uint32_t q, uint32_t group, unsigned lo
 }
 
 // a piece of a destination with many in-edges; the pieces combine with atomicMin
-__device__ void wo_piece(const BArgs& a, uint32_t q, uint2 it, unsigned long long& mass)
+__device__ void wo_piece(const BArgs& a, uint32_t q, uint2 it, unsigned long long& mass, unsigned long long& least)
 {
     const BQuery& qq = a.q[q];
     BCtl& c = a.ctl[q];
@@ -637,6 +663,7 @@ __device__ void wo_piece(const BArgs& a, uint32_t q, uint2 it, unsigned long lon
     const uint32_t d = G.dst_id[it.x], end = (uint32_t)G.dst_off[it.x + 1u];
     const uint32_t hi = end - it.y > WO_PIECE ? it.y + WO_PIECE : end;
     const unsigned long long before = __shfl_sync(FULL, qq.prop[d], 0);
+    const unsigned long long fmin = c.fmin;
     unsigned long long dist = before;
     /* the piece's first in-edges up to a multiple of 4, on lane 0 */
     const uint32_t p = min(hi, (it.y + 3u) & ~3u);
@@ -644,15 +671,16 @@ __device__ void wo_piece(const BArgs& a, uint32_t q, uint2 it, unsigned long lon
     if (p != it.y) {
         uint32_t stop = 0u;
         if ((threadIdx.x & 31) == 0) {
-            wo_step(qq, G, it.y & ~3u, it.y, p, dist);
-            stop = G.ww8[p - 1u] >= dist ? 1u : 0u;
+            wo_step(qq, G, it.y & ~3u, it.y, p, fmin, dist);
+            stop = G.ww8[p - 1u] >= wo_limit(dist, fmin) ? 1u : 0u;
         }
         dist = __shfl_sync(FULL, dist, 0);
         go = __shfl_sync(FULL, stop, 0) == 0u;
     }
     if (go)
-        dist = wo_run(qq, G, p, hi, dist);
+        dist = wo_run(qq, G, p, hi, fmin, dist);
     if ((threadIdx.x & 31) == 0 && dist < before && dist < atomicMin(&qq.prop[d], dist)) {
+        least = min(least, dist);
         const uint32_t b = 1u << (d & 31u);
         if (!(atomicOr(&qq.front[(c.iter + 1u) % 3u][d >> 5], b) & b)) {
             const uint32_t od = G.outdeg[d];
@@ -676,9 +704,9 @@ __device__ __forceinline__ uint32_t wo_spread(uint32_t i, uint32_t n)
 // the sources; lists, out-edges, distances, claims) and by how evenly they
 // spread: items are kept short, and a warp takes fewer of them towards the
 // queue's end.  32 SSSPs over 8 graphs (scales 12 to 20, 177 M in-edges in
-// all): 3.6 ms in 15 rounds, 13.3 with 256-edge tiles that streamed every
-// in-edge of a dense pull; 16 BFS and 16 SSSP over scales 13 to 16: 0.64 ms,
-// 2.8 before.
+// all): 3.1 ms in 16 rounds (3.6 without wo_limit's bound and the first in-edges
+// in arrays of their own), 13.3 with 256-edge tiles that streamed every in-edge
+// of a dense pull; 16 BFS and 16 SSSP over scales 13 to 16: 0.61 ms, 2.8 before.
 __device__ void phase_pull(const BArgs& a)
 {
     __shared__ uint32_t heads_all[BT / 32];
@@ -701,7 +729,7 @@ __device__ void phase_pull(const BArgs& a)
         }
     }
     const unsigned long long total = a.pull_off[a.Q];
-    unsigned long long pulled = 0, mass = 0;
+    unsigned long long pulled = 0, mass = 0, least = NONE64;
     uint32_t q = 0;
     auto settle = [&]() { /* the mass of the items of query q so far */
         if (__any_sync(FULL, mass != 0ull)) {
@@ -711,7 +739,15 @@ __device__ void phase_pull(const BArgs& a)
             if (lane == 0)
                 atomicAdd(&a.ctl[q].mass, mass);
         }
+        if (__any_sync(FULL, least != NONE64) && a.graphs[a.q[q].graph].wsrc) {
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1)
+                least = min(least, __shfl_xor_sync(FULL, least, d));
+            if (lane == 0 && least < *(volatile unsigned long long*)&a.ctl[q].next_fmin)
+                atomicMin(&a.ctl[q].next_fmin, least);
+        }
         mass = 0ull;
+        least = NONE64;
     };
     const unsigned long long warps = 2ull * ((gridDim.x * blockDim.x) >> 5);
     unsigned long long base = 0;
@@ -738,15 +774,15 @@ __device__ void phase_pull(const BArgs& a)
                 if (qq.app != WEDGE_APP_SSSP || !G.wsrc)
                     pull_tile(a, q, local, mass); /* tiles of BTILE_CH chunks */
                 else if (local < G.nlong)
-                    wo_piece(a, q, G.wo_long[local], mass);
+                    wo_piece(a, q, G.wo_long[local], mass, least);
                 else
-                    wo_group(a, q, wo_spread(local - G.nlong, groups), mass);
+                    wo_group(a, q, wo_spread(local - G.nlong, groups), mass, least);
             } else if (G.push) {
                 const uint32_t ni = c.nitem[c.iter % 3u];
                 if (local < ni)
-                    push_piece(a, q, qq.items[c.iter & 1u][local], mass);
+                    push_piece(a, q, qq.items[c.iter & 1u][local], mass, least);
                 else
-                    push_chunk(a, q, (local - ni) * PUSH_CHUNK, c.nlist[c.iter % 3u], push_sh, mass);
+                    push_chunk(a, q, (local - ni) * PUSH_CHUNK, c.nlist[c.iter % 3u], push_sh, mass, least);
             } else {
                 const uint32_t ch = qq.chunk_list[local];
                 pull_chunk(a, q, ch, heads, mass);
@@ -785,6 +821,8 @@ __device__ void phase_decide(const BArgs& a)
         c.iter += 1u;
         const unsigned long long m = c.mass;
         c.mass = 0ull;
+        c.fmin = c.next_fmin;
+        c.next_fmin = NONE64;
         if (m == 0ull || c.iter >= a.max_rounds) { /* execution_bfs.c:239-251 */
             c.done = 1u;
             continue;
@@ -888,6 +926,8 @@ __global__ void batch_seed_kernel(BArgs a)
         const uint32_t r = G.old2new[root_in];
         c.root = r;
         c.mass = 0ull;
+        c.fmin = 0ull;
+        c.next_fmin = NONE64;
         c.iter = 0u;
         c.done = G.E == 0ull ? 1u : 0u;
         qq.prop[r] = (qq.app == WEDGE_APP_BFS) ? (unsigned long long)r : 0ull;
@@ -1083,6 +1123,8 @@ extern "C" int wedge_cuda_batch_create(wedge_graph_t* const* graphs, uint32_t nu
         G.push = g.csr;
         G.wsrc = g.csr ? g.wsrc : nullptr;
         G.ww8 = g.ww8;
+        G.wo_src = g.wo_src;
+        G.wo_w = g.wo_w;
         if (!g.csr)
             b->chunks = 1u;
         if (g.V > b->maxV)

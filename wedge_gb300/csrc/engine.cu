@@ -460,6 +460,20 @@ __global__ void first_source_kernel(const uint32_t* src, const unsigned long lon
         first_src[k] = src[dst_off[k]];
 }
 
+// the first weight-ordered source of every destination, with the bits that tell
+// how many it has, and its first two weights
+__global__ void wo_first_kernel(const uint32_t* wsrc, const uint8_t* ww8, const unsigned long long* dst_off, uint32_t Vne,
+                                uint32_t* wo_src, uint16_t* wo_w)
+{
+    for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < Vne; k += (uint64_t)gridDim.x * blockDim.x) {
+        const unsigned long long lo = dst_off[k];
+        const unsigned long long n = dst_off[k + 1] - lo;
+        const bool only = n == 1ull;
+        wo_src[k] = wsrc[lo] | (only ? WO_ONLY_BIT : 0u) | (n > WO_MANY ? WO_MANY_BIT : 0u);
+        wo_w[k] = (uint16_t)(ww8[lo] | (only ? 0xFF00u : (uint32_t)ww8[lo + 1] << 8));
+    }
+}
+
 __global__ void pad_kernel(uint32_t* src, unsigned long long* w, uint64_t E, uint64_t Epad)
 {
     for (uint64_t e = E + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < Epad; e += (uint64_t)gridDim.x * blockDim.x) {
@@ -892,6 +906,19 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
     if (Vne)
         first_source_kernel<<<grid_for(Vne, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(d_src, dst_off, Vne, first_src);
     g.first_src = first_src;
+    if (g.wsrc) {
+        uint32_t* wo_src = nullptr;
+        uint16_t* wo_w = nullptr;
+        if (dalloc(h, &wo_src, Vne) == WEDGE_OK && dalloc(h, &wo_w, Vne) == WEDGE_OK) {
+            wo_first_kernel<<<grid_for(Vne, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(g.wsrc, g.ww8, dst_off, Vne, wo_src, wo_w);
+            g.wo_src = wo_src;
+            g.wo_w = wo_w;
+        } else {
+            cudaGetLastError(); /* no room, as above */
+            g.wsrc = nullptr;
+            g.ww8 = nullptr;
+        }
+    }
     if ((rc = dalloc(h, &split_k, g.T)) || (rc = dalloc(h, &split_t0, g.T)) || (rc = dalloc(h, &split_t1, g.T)))
         return rc;
     unsigned int* d_cnt = nullptr;
@@ -1187,7 +1214,7 @@ __device__ __forceinline__ void dist32_put(const DevState& s, uint32_t v, unsign
 // the weight-ordered kernels run this pull: dense and filtered pulls while every distance fits the 32-bit copy
 __device__ __forceinline__ bool sssp_wo_runs(const DevState& s, const Ctrl* c)
 {
-    return s.wo && c->mode != MODE_WEDGE && !c->narrow_ovf;
+    return s.wo && (c->mode != MODE_WEDGE || c->heavy) && !c->narrow_ovf;
 }
 
 // The Wedge pull of SSSP over the out-edges: every vertex the last pull
@@ -1330,13 +1357,15 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
     Ctrl* c = s.ctrl;
     if (c->done)
         return;
-    const uint32_t mode = c->mode;
+    const uint32_t mode = APP == WEDGE_APP_SSSP && c->heavy ? (uint32_t)MODE_DENSE : c->mode;
     if (phase == PHASE_REST && mode == MODE_WEDGE) {
         // a Wedge pull runs whole in the first launch: this one only reports zeros
         if (threadIdx.x < NCNT)
             block_cnt[NCNT * blockIdx.x + threadIdx.x] = 0ull;
         return;
     }
+    if (APP == WEDGE_APP_SSSP && s.wo && !sssp_wo_runs(s, c) && blockIdx.x == 0 && threadIdx.x == 0)
+        c->fmin[c->parity == 2u ? 0u : c->parity + 1u] = 0u; /* this pull keeps no bound */
     if (APP == WEDGE_APP_SSSP && mode == MODE_WEDGE && s.push) {
         sssp_push_pull(g, s, c, block_cnt);
         return;
@@ -2082,18 +2111,30 @@ __global__ void sssp_split_kernel(DevGraph g, DevState s, unsigned long long* bl
 }
 
 // SSSP dense and source-filtered pulls over weight-ordered in-edges, 32-bit
-// sums.  Distances are not negative, so an in-edge whose weight alone is not
+// sums.  After a pull every in-edge of a vertex that the pull did not change
+// has been relaxed or could not lower its destination, so only the changed
+// vertices matter to the next one; none of them, and no vertex it lowers, has a
+// distance below Ctrl::fmin.  An in-edge whose weight and fmin together are not
 // below its destination's distance cannot lower it, and neither can the ones
 // after it: a destination reads its in-edges by ascending weight and stops at
 // the first such weight.  On R-MAT graphs with weights 1..255 the first dense
-// pull reads 15% of the in-edges and the later ones 5-6% (scales 20 and 22),
-// where a tile pull streams and gathers them all: 4.95 / 4.90 / 4.64 ms for
-// the three dense pulls at scale 26 before.  Bound by the latency of a
-// destination's chain (offsets, distance, weights and sources, distances of
-// the sources): one destination per lane, four in-edges a step (one word of
-// weights, one 128-bit load of sources, up to four gathers in flight), 64
-// warps per SM.  A destination that has not stopped after SSSP_WO_WINDOW
-// in-edges leaves the others to sssp_wo_long_kernel, in pieces of
+// pull reads 15% of the in-edges and the later ones 6, 4, 3 and 2% (scale 20;
+// fmin rises by about 1 a pull, and 5% without it), where a tile pull streams
+// and gathers them all: 4.95 / 4.90 / 4.64 ms for the three dense pulls at
+// scale 26 before.
+//
+// Bound by the latency of a destination's chain (offsets, distance, weights and
+// sources, distances of the sources) and by the sectors its short list takes
+// from memory.  So the first source and the first two weights of every
+// destination lie in arrays of their own (6 bytes in order, where offset,
+// weights and sources took three sectors): one destination per lane, most are
+// settled there (27% in the first pull, 60 to 90% in the later ones).  The
+// others wait until the warp has 32 of them and go on, four in-edges a step
+// (one word of weights, one 128-bit load of sources, up to four gathers in
+// flight), 64 warps per SM.  Scale 26: the four pulls read 66, 34, 21 and 12 M
+// in-edges, 86, 46, 41 and 41 M without the bound; the SSSP takes 3.18 ms, 3.72
+// without the bound and the arrays.  A destination that has not stopped after
+// SSSP_WO_WINDOW in-edges leaves the others to sssp_wo_long_kernel, in pieces of
 // SSSP_WO_PIECE up to the first weight that cannot lower it.
 //
 // A sum at or above the 32-bit copy's limit that would have lowered its
@@ -2109,16 +2150,23 @@ struct WoStep {
     bool dropped;     // a sum past the limit would have lowered dist
 };
 
-__device__ __forceinline__ WoStep sssp_wo_step(const DevGraph& g, const DevState& s, const uint32_t* filter, uint32_t p,
-                                               uint32_t lo, uint32_t hi, uint32_t& dist, uint32_t& edges)
+// the weights that may lower a distance: below this
+__device__ __forceinline__ uint32_t sssp_wo_limit(uint32_t dist, uint32_t fmin)
 {
+    return dist > fmin ? dist - fmin : 0u;
+}
+
+__device__ __forceinline__ WoStep sssp_wo_step(const DevGraph& g, const DevState& s, const uint32_t* filter, uint32_t p,
+                                               uint32_t lo, uint32_t hi, uint32_t fmin, uint32_t& dist, uint32_t& edges)
+{
+    const uint32_t lim = sssp_wo_limit(dist, fmin);
     const uint32_t ww = ld_ro_u32(reinterpret_cast<const uint32_t*>(g.ww8 + p));
     const uint4 xs = __ldg(reinterpret_cast<const uint4*>(g.wsrc + p));
     const uint32_t x[4] = {xs.x, xs.y, xs.z, xs.w};
     uint32_t y[4];
 #pragma unroll
     for (uint32_t j = 0; j < 4; ++j) {
-        bool on = p + j >= lo && p + j < hi && ((ww >> (8 * j)) & 0xFFu) < dist;
+        bool on = p + j >= lo && p + j < hi && ((ww >> (8 * j)) & 0xFFu) < lim;
         edges += on ? 1u : 0u;
         if (filter && on)
             on = (ld_ro_u32(filter + (x[j] >> 5)) >> (x[j] & 31u)) & 1u; /* changed by the previous pull */
@@ -2141,6 +2189,14 @@ __device__ __forceinline__ WoStep sssp_wo_step(const DevGraph& g, const DevState
     r.dropped = r.dropped && m == NONE32;
     dist = m;
     return r;
+}
+
+// the least distance a warp's lanes gave, into the next frontier's bound
+__device__ __forceinline__ void sssp_wo_least(Ctrl* c, uint32_t least)
+{
+    least = __reduce_min_sync(FULL, least);
+    if ((threadIdx.x & 31) == 0 && least != NONE32)
+        atomicMin(&c->fmin[c->parity == 2u ? 0u : c->parity + 1u], least);
 }
 
 // a block's counters, per lane in 32 bits except the mass (in-edge positions fit 32 bits here)
@@ -2167,6 +2223,7 @@ __device__ __forceinline__ void sssp_wo_counters(unsigned long long* block_cnt, 
 __global__ void __launch_bounds__(PULL_THREADS, 2) sssp_wo_kernel(DevGraph g, DevState s, unsigned long long* block_cnt)
 {
     __shared__ uint32_t runs; /* one answer per block: another block may set Ctrl::narrow_ovf meanwhile */
+    __shared__ uint32_t sh_late[PULL_THREADS / 32][64];
     Ctrl* c = s.ctrl;
     if (c->done)
         return;
@@ -2182,48 +2239,70 @@ __global__ void __launch_bounds__(PULL_THREADS, 2) sssp_wo_kernel(DevGraph g, De
     const uint32_t nthr = gridDim.x * blockDim.x;
     const uint32_t* filter = c->mode == MODE_FILTERED ? cur_front(s, c->parity) : nullptr;
     uint32_t* nxt = next_front(s, c->parity);
+    const uint32_t fmin = c->fmin[c->parity];
+    uint32_t* my_late = sh_late[threadIdx.x >> 5];
     unsigned long long mass = 0;
     uint32_t edges = 0, dsts = 0, act = 0, occ = 0, deg[3] = {0u, 0u, 0u};
+    uint32_t kept = 0u, least = NONE32;
     bool dropped = false;
-    // the next group's offsets and vertices are loaded while this one is pulled
-    uint32_t plo = 0u, phi = 0u, pd = 0u;
-    auto prefetch = [&](uint32_t b) {
-        const uint32_t kk = b + (uint32_t)lane;
-        if (kk < g.Vne) {
-            plo = (uint32_t)g.dst_off[kk];
-            phi = (uint32_t)g.dst_off[kk + 1u];
-            pd = g.dst_ident ? kk : g.dst_id[kk];
+    // destination d, lowered to dist (chg): its only writer in this launch; called by all lanes
+    auto settle = [&](bool chg, uint32_t d, uint32_t dist, bool waited) {
+        uint32_t word = NONE32;
+        if (chg) {
+            s.dist32[d] = dist;
+            s.prop64[d] = dist;
+            least = min(least, dist);
+            const uint32_t od = g.outdeg[d];
+            word = d >> 5;
+            mass += od;
+            ++act;
+            const uint32_t bk = degree_bucket(od);
+#pragma unroll
+            for (uint32_t b = 0; b < 3u; ++b)
+                deg[b] += bk == b ? 1u : 0u;
+        }
+        // frontier bits: one atomicOr per distinct word of the 32 destinations
+        const uint32_t grp = __match_any_sync(FULL, word);
+        const uint32_t bits = __reduce_or_sync(grp, chg ? 1u << (d & 31u) : 0u);
+        if (chg && (uint32_t)lane == (uint32_t)(__ffs(grp) - 1)) {
+            if (waited) { /* its word may have been counted with the group's others */
+                occ += atomicOr(&nxt[word], bits) == 0u ? 1u : 0u;
+            } else {
+                atomicOr(&nxt[word], bits);
+                ++occ;
+            }
         }
     };
-    const uint32_t b0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
-    prefetch(b0);
-    for (uint32_t base = b0; base < g.Vne; base += nthr) {
-        const uint32_t k = base + (uint32_t)lane;
-        const uint32_t lo = plo, hi = phi, d = pd;
-        prefetch(base + nthr);
-        const bool mine = k < g.Vne;
+    // the last n destinations that wait, from their first in-edge on
+    auto late = [&](uint32_t n) {
+        kept -= n;
+        const bool on = (uint32_t)lane < n;
+        const uint32_t k = on ? my_late[kept + (uint32_t)lane] : 0u;
+        __syncwarp();
         bool chg = false;
-        uint32_t npiece = 0u, rest = 0u;
-        uint32_t word = NONE32, od = 0u;
-        if (mine) {
-            ++dsts;
+        uint32_t npiece = 0u, rest = 0u, d = 0u, dist = 0u;
+        if (on) {
+            const uint32_t lo = (uint32_t)g.dst_off[k], hi = (uint32_t)g.dst_off[k + 1u];
+            d = g.dst_ident ? k : g.dst_id[k];
             const uint32_t before = s.dist32[d];
-            uint32_t dist = before, p = lo & ~3u;
+            uint32_t p = lo & ~3u;
             bool more = true;
+            dist = before;
             do {
-                const WoStep r = sssp_wo_step(g, s, filter, p, lo, hi, dist, edges);
+                const WoStep r = sssp_wo_step(g, s, filter, p, lo, hi, fmin, dist, edges);
                 dropped = dropped || r.dropped;
                 p += 4u;
-                more = p < hi && r.last < dist;
+                more = p < hi && r.last < sssp_wo_limit(dist, fmin);
             } while (more && p - lo < SSSP_WO_WINDOW);
             if (more) {
                 rest = p;
                 uint32_t end = hi;
                 if (hi - p > SSSP_WO_PIECE) { /* first weight that cannot lower the destination */
+                    const uint32_t lim = sssp_wo_limit(dist, fmin);
                     uint32_t a = p;
                     while (a < end) {
                         const uint32_t mid = a + (end - a) / 2u;
-                        if (g.ww8[mid] < dist)
+                        if (g.ww8[mid] < lim)
                             a = mid + 1u;
                         else
                             end = mid;
@@ -2232,26 +2311,8 @@ __global__ void __launch_bounds__(PULL_THREADS, 2) sssp_wo_kernel(DevGraph g, De
                 npiece = (end - p + SSSP_WO_PIECE - 1u) / SSSP_WO_PIECE;
             }
             chg = dist < before;
-            if (chg) { /* the destination's only writer in this launch */
-                s.dist32[d] = dist;
-                s.prop64[d] = dist;
-                od = g.outdeg[d];
-                word = d >> 5;
-                mass += od;
-                ++act;
-                const uint32_t bk = degree_bucket(od);
-#pragma unroll
-                for (uint32_t b = 0; b < 3u; ++b)
-                    deg[b] += bk == b ? 1u : 0u;
-            }
         }
-        // frontier bits: one atomicOr per distinct word of the 32 destinations
-        const uint32_t grp = __match_any_sync(FULL, word);
-        const uint32_t bits = __reduce_or_sync(grp, chg ? 1u << (d & 31u) : 0u);
-        if (chg && (uint32_t)lane == (uint32_t)(__ffs(grp) - 1)) {
-            atomicOr(&nxt[word], bits);
-            ++occ;
-        }
+        settle(chg, d, dist, true);
         if (__any_sync(FULL, npiece != 0u)) {
             uint32_t incl = npiece;
 #pragma unroll
@@ -2267,7 +2328,62 @@ __global__ void __launch_bounds__(PULL_THREADS, 2) sssp_wo_kernel(DevGraph g, De
             for (uint32_t i = 0; i < npiece; ++i)
                 s.wo_items[at + i] = make_uint2(k, rest + i * SSSP_WO_PIECE);
         }
+    };
+    // the next group's first in-edges are loaded while this one is pulled
+    uint32_t px = 0u, pw = 0u;
+    auto prefetch = [&](uint32_t b) {
+        const uint32_t kk = b + (uint32_t)lane;
+        if (kk < g.Vne) {
+            px = g.wo_src[kk];
+            pw = g.wo_w[kk];
+        }
+    };
+    const uint32_t b0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
+    prefetch(b0);
+    for (uint32_t base = b0; base < g.Vne; base += nthr) {
+        const uint32_t k = base + (uint32_t)lane;
+        const uint32_t x = px & WO_ID_BITS, w = pw & 0xFFu, w2 = pw >> 8;
+        const bool only = px & WO_ONLY_BIT;
+        prefetch(base + nthr);
+        bool chg = false, more = false;
+        uint32_t d = 0u, dist = 0u;
+        if (k < g.Vne) {
+            d = g.dst_ident ? k : g.dst_id[k];
+            ++dsts;
+            const uint32_t before = s.dist32[d];
+            dist = before;
+            if (w < sssp_wo_limit(before, fmin)) {
+                uint32_t y = NONE32;
+                bool over = false;
+                if (!filter || ((ld_ro_u32(filter + (x >> 5)) >> (x & 31u)) & 1u)) /* changed by the previous pull */
+                    y = ld_gather_u32(s.dist32 + x);
+                if (y != NONE32) {
+                    const uint32_t sum = y + w; /* phase_edge_pull_sssp.c:136-137 */
+                    over = sum < y || sum >= s.narrow_lim;
+                    dist = over ? dist : min(dist, sum);
+                }
+                more = !only && w2 < sssp_wo_limit(dist, fmin);
+                if (!more) { /* one that waits starts again */
+                    ++edges;
+                    dropped = dropped || (over && dist == NONE32);
+                    chg = dist < before;
+                }
+            }
+        }
+        settle(chg, d, dist, false);
+        const uint32_t m = __ballot_sync(FULL, more);
+        if (m) {
+            if (more)
+                my_late[kept + (uint32_t)__popc(m & ((1u << lane) - 1u))] = k;
+            kept += (uint32_t)__popc(m);
+            __syncwarp();
+            if (kept >= 32u)
+                late(32u);
+        }
     }
+    if (kept)
+        late(kept);
+    sssp_wo_least(c, least);
     if (dropped) {
         atomicOr(&c->narrow_ovf, 1u);
         atomicOr(&c->ovf_redo, 1u);
@@ -2294,6 +2410,8 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
     const int lane = threadIdx.x & 31;
     const uint32_t* filter = c->mode == MODE_FILTERED ? cur_front(s, c->parity) : nullptr;
     uint32_t* nxt = next_front(s, c->parity);
+    const uint32_t fmin = c->fmin[c->parity];
+    uint32_t least = NONE32;
     unsigned long long mass = 0;
     uint32_t edges = 0, act = 0, occ = 0, deg[3] = {0u, 0u, 0u};
     bool dropped = false;
@@ -2309,14 +2427,15 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
             const uint32_t q = p + 4u * (uint32_t)lane;
             WoStep r{0xFFFFFFFFu, false};
             if (q < hi)
-                r = sssp_wo_step(g, s, filter, q, it.y, hi, dist, edges);
+                r = sssp_wo_step(g, s, filter, q, it.y, hi, fmin, dist, edges);
             dropped = dropped || r.dropped;
             dist = __reduce_min_sync(FULL, dist);
-            if (__shfl_sync(FULL, r.last, 31) >= dist)
+            if (__shfl_sync(FULL, r.last, 31) >= sssp_wo_limit(dist, fmin))
                 break; /* the step's largest weight; past the end: none */
         }
         if (lane == 0 && dist < before && dist < atomicMin(&s.dist32[d], dist)) {
             atomicMin(&s.prop64[d], (unsigned long long)dist);
+            least = min(least, dist);
             const uint32_t b = 1u << (d & 31u);
             const uint32_t o = atomicOr(&nxt[d >> 5], b);
             occ += o == 0u ? 1u : 0u;
@@ -2331,6 +2450,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
             }
         }
     }
+    sssp_wo_least(c, least);
     if (dropped) {
         atomicOr(&c->narrow_ovf, 1u);
         atomicOr(&c->ovf_redo, 1u);
@@ -3106,6 +3226,7 @@ __device__ __forceinline__ void decide_block(const DevGraph& g, DevState& s, Ctr
         c->tiles = 0u;
         c->items = 0u;
         c->alist_n = 0u;
+        c->heavy = 0u;
         go = 0u;
         // SSSP: a pull dropped 32-bit sums that reached the copy's limit; the
         // next pull is dense and 64-bit, and relaxes every in-edge again
@@ -3555,6 +3676,9 @@ __global__ void init_root_kernel(DevGraph g, DevState s, uint32_t app, uint64_t 
         c->narrow_ovf = 0;
         c->ovf_redo = 0;
         c->bodies = 0;
+        c->heavy = 0u;
+        for (int i = 0; i < 3; ++i)
+            c->fmin[i] = 0u;
         loop_reset(c);
         if (app == WEDGE_APP_CC) {
             c->last_mass = g.E;
@@ -3625,6 +3749,12 @@ constexpr unsigned long long NEAR_MASS = 1ull << 16;
 constexpr double NEAR_STEP = 1.0;
 constexpr uint32_t NEAR_ITER = 16;
 constexpr uint32_t BARRIER_TRIES = 1u << 22;
+// A Wedge iteration whose vertices have more than WO_HEAVY out-edges per
+// destination of the graph runs as a weight-ordered pull (117 M of 1.07 G at
+// scale 26, below the 20% that make an iteration dense: 1.0 ms relaxed one by
+// one, 0.4 as a pull).  The whole SSSP at scales 26, 22 and 20: 3.20, 0.62 and
+// 0.44 ms; with 1: 3.19, 0.63, 0.44; with 4: 3.19, 0.72, 0.44; never: 3.82 at 26.
+constexpr uint32_t WO_HEAVY = 2;
 enum : uint32_t { ERR_BARRIER_TIMEOUT = 4u };
 
 // all blocks of a cooperative launch; false when it did not complete within
@@ -3740,6 +3870,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
         uint32_t release, nfar;                             /* far lists begun; vertices of the one whose turn it is */
     } so;
     __shared__ unsigned long long sh_far[2];
+    __shared__ uint32_t sh_least;
     Ctrl* c = s.ctrl;
     if (c->done)
         return;
@@ -3751,7 +3882,12 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
     uint32_t mode = c->mode, parity = c->parity, iter = c->iter;
     const uint32_t sched = c->sched, max_iter = c->max_iter, probe_iter = c->probe_iter, probe_mode = c->probe_mode;
     const unsigned long long thr = c->threshold;
-    const bool loop = small != 0u || mode == MODE_WEDGE;
+    // SSSP: whether a Wedge iteration over `mass` out-edges is better a weight-ordered pull
+    const bool may_pull = APP == WEDGE_APP_SSSP && s.wo && small == 0u && max_steps > 1u &&
+                          (sched == WEDGE_SCHED_PLAIN || sched == WEDGE_SCHED_LEARNED);
+    auto heavy = [&](unsigned long long mass) { return may_pull && mass > WO_HEAVY * (unsigned long long)g.Vne; };
+    const bool pull_now = mode == MODE_WEDGE && heavy(c->mass);
+    const bool loop = small != 0u || (mode == MODE_WEDGE && !pull_now);
     const bool f64 = g.weight_kind == WEDGE_WEIGHTS_F64;
     uint32_t* my_buf = sh_buf[wib];
     uint32_t* my_pre = sh_pre[wib];
@@ -3868,6 +4004,11 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
         if (s.tile_need)
             for (uint32_t i = tid; i < g.T / 32u + 2u; i += nthr)
                 s.tile_need[i] = 0u;
+        if (APP == WEDGE_APP_SSSP && tid == 0u) {
+            c->fmin[(parity + 1u) % 3u] = NONE32; /* of the frontier the next pull writes */
+            if (pull_now)
+                c->heavy = 1u;
+        }
         if (!loop)
             return;
         flush();
@@ -3934,7 +4075,13 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
         const bool narrow = APP == WEDGE_APP_SSSP && s.dist32 && !sh_n[2];
         unsigned long long mass = 0, degs = 0; /* degs: activated vertices per out-degree bucket 0..2, 21 bits each */
         uint32_t edges = 0, act = 0, occ = 0, dsts = 0;
+        uint32_t least32 = NONE32; /* SSSP with weight-ordered pulls: the least distance given */
         if (tid == 0u) { /* counters no block reads any more */
+            if (APP == WEDGE_APP_SSSP) {
+                c->fmin[(parity + 2u) % 3u] = NONE32;
+                if (sorting) /* waiting vertices join the frontier of a dense pull: no bound */
+                    c->fmin[(parity + 1u) % 3u] = 0u;
+            }
             c->ln[(step + 2u) % 3u] = 0u;
             c->li[(step + 2u) % 3u] = 0u;
             if (sorting && so.nfar)
@@ -4077,6 +4224,8 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
                 od[u] = 0u;
                 wait[u] = FAR && low[u] && (unsigned long long)nd[u] > bound;
                 if (low[u]) {
+                    if constexpr (APP == WEDGE_APP_SSSP && !FAR)
+                        least32 = min(least32, (uint32_t)min((unsigned long long)nd[u], (unsigned long long)NONE32 - 1ull));
                     o[u] = atomicOr(&(wait[u] ? s.far : nxt)[d[u] >> 5], 1u << (d[u] & 31u));
                     od[u] = g.outdeg[d[u]];
                     if (APP == WEDGE_APP_BFS || (APP == WEDGE_APP_CC && x[u] == 0u)) { /* visited; label 0 is final */
@@ -4244,6 +4393,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
         if (threadIdx.x == 32) {
             sh_far[0] = NONE64;
             sh_far[1] = 0ull;
+            sh_least = NONE32;
         }
         __syncthreads();
         if (__any_sync(FULL, (edges | dsts) != 0u)) {
@@ -4256,6 +4406,11 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
                 for (uint32_t j = 0; j < NCNT; ++j)
                     if (v[j])
                         atomicAdd(&sh_acc[j], v[j]);
+            if (APP == WEDGE_APP_SSSP && !sorting) {
+                least32 = __reduce_min_sync(FULL, least32);
+                if (lane == 0 && least32 != NONE32)
+                    atomicMin(&sh_least, least32);
+            }
             if (sorting) {
                 far_mass = warp_sum_u64(far_mass);
                 for (int q = 16; q > 0; q >>= 1)
@@ -4269,6 +4424,8 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
         __syncthreads();
         if (threadIdx.x < NCNT && sh_acc[threadIdx.x])
             atomicAdd(&c->lacc[a][threadIdx.x], sh_acc[threadIdx.x]);
+        if (APP == WEDGE_APP_SSSP && threadIdx.x == 64 && sh_least != NONE32)
+            atomicMin(&c->fmin[(parity + 1u) % 3u], sh_least);
         if (sorting && threadIdx.x == 32) {
             if (sh_far[0] != NONE64)
                 atomicMin(&c->lmin[a], sh_far[0]);
@@ -4298,9 +4455,10 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
         for (uint32_t j = 0; j < NCNT; ++j)
             cnt[j] = sh_acc[j];
         const NextPull next = next_pull(sched, cnt[CNT_MASS], false, iter + 1u, max_iter, thr, probe_iter, probe_mode);
+        const bool pull_next = APP == WEDGE_APP_SSSP && !(sorting && so.release + so.waiting != 0ull) && heavy(cnt[CNT_MASS]);
         if (scribe)
             book.note(g, s, (uint32_t)APP, cnt, next, mode, iter);
-        if (scribe && (next.done || step + 1u == max_steps || (!small && next.mode != MODE_WEDGE) ||
+        if (scribe && (next.done || step + 1u == max_steps || (!small && next.mode != MODE_WEDGE) || pull_next ||
                        sched == WEDGE_SCHED_LEARNED))
             book.close(c, cnt[CNT_MASS], next, iter + 1u, (parity + 1u) % 3u);
         if (!next.done && sched == WEDGE_SCHED_LEARNED && s.net && blockIdx.x + 1u == gridDim.x)
@@ -4313,7 +4471,9 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
                 return;
             mode = *(volatile unsigned int*)&c->mode;
         }
-        const bool leave = step + 1u == max_steps || (!small && mode != MODE_WEDGE);
+        if (scribe && pull_next && !next.done)
+            c->heavy = 1u; /* the pull that follows this launch */
+        const bool leave = step + 1u == max_steps || (!small && mode != MODE_WEDGE) || pull_next;
         if (!next.done && leave && (APP == WEDGE_APP_BFS || (sorting && so.release + so.waiting != 0ull))) {
             /* another launch takes over: the waiting vertices join the frontier */
             uint32_t* fr = s.front + parity * s.front_stride; /* this iteration's bitmap */
@@ -6877,6 +7037,7 @@ int wedge_cuda_shard_state(wedge_graph_t* g, int which, void* host, uint64_t byt
         return WEDGE_ERR_ARG;
     if (import) {
         WEDGE_CHECK(cudaMemcpyAsync(dev, host, need, cudaMemcpyHostToDevice, g->stream));
+        WEDGE_CHECK(cudaMemsetAsync(g->s.ctrl->fmin, 0, sizeof(g->s.ctrl->fmin), g->stream));
         if (which == WEDGE_SHARD_PROPS && g->s.dist32) {
             narrow_copy_kernel<<<grid_for(g->g.V, AUX_THREADS, (uint32_t)g->num_sms * 8u), AUX_THREADS, 0, g->stream>>>(
                 g->g, g->s);

@@ -6,7 +6,8 @@
 //   w[Epad]        64-bit weight words (SSSP only; uint64 or IEEE double), or
 //   w8[Epad]       one byte each where every uint64 weight is below 256; then also
 //   wsrc[Epad], ww8[Epad]  sources and weights once more, each destination's by
-//                  ascending weight (the SSSP dense pulls)
+//                  ascending weight (the SSSP dense pulls); wo_src[Vne], wo_w[Vne]
+//                  the first of each and the first two weights
 //   dst_id[Vne]    vertex id of compressed destination k (only vertices with
 //                  in-degree > 0 are listed, ascending)
 //   dst_off[Vne+1] first edge of compressed destination k
@@ -35,6 +36,11 @@ namespace wedge {
 constexpr uint32_t TILE = 128;          // granularity of the tile index (tile_dst0)
 constexpr uint32_t MAX_TILE_E = 512;    // largest pull tile; E is padded to a multiple of it
 constexpr uint32_t CHUNK = 32;
+// DevGraph::wo_src: beside byte weights an id has 28 bits at most
+constexpr uint32_t WO_ID_BITS = 0x0FFFFFFFu;
+constexpr uint32_t WO_ONLY_BIT = 1u << 31;  // the destination's only in-edge
+constexpr uint32_t WO_MANY_BIT = 1u << 30;  // a destination of more than WO_MANY in-edges
+constexpr uint32_t WO_MANY = 64;
 constexpr uint32_t CHUNKS_PER_TILE = TILE / CHUNK;        // 4
 constexpr uint32_t TILES_PER_WORD = 32 / CHUNKS_PER_TILE;  // 8 tiles per 32-bit chunk-bitmap word
 constexpr uint32_t REGION_WORDS = 32;                      // chunk-bitmap words per summary bit
@@ -115,6 +121,8 @@ struct Ctrl {
                                        // pull is dense (64-bit) and the traversal does not stop before it
     unsigned int bodies;               // rounds of the fused traversal loop
     unsigned int bar;                  // sparse_loop_kernel: grid-barrier arrivals, and per step modulo 3
+    unsigned int heavy;                // SSSP: the Wedge iteration at hand runs as a weight-ordered pull
+    unsigned int fmin[3];              // SSSP: no distance in the frontier bitmap of that number is below (dense pulls)
     unsigned int ln[3], li[3];         // vertices and items listed for it,
     unsigned long long lacc[3][NCNT];  // its counters; SSSP: the least distance it sorted out and by how many
     unsigned long long lmin[3], lfar[3]; // out-edges it changed the waiting ones; by far list modulo 3:
@@ -140,6 +148,8 @@ struct DevGraph {
     const uint32_t* src;
     const unsigned long long* w;
     const uint8_t* w8;         // the same weights in one byte each, when every weight is a uint64 below 256
+    const uint32_t* wo_src;    // with wsrc: [Vne] every destination's first weight-ordered source (and WO_*_BIT)
+    const uint16_t* wo_w;      // and first two weights (the second above)
     const uint32_t* first_src; // [Vne] the first source of every destination
     const uint32_t* wsrc;      // [Epad] with byte-wide weights: every destination's sources by ascending weight
     const uint8_t* ww8;        // [Epad] and those weights (dst_off holds for both orders); or null
