@@ -154,6 +154,12 @@ static int dalloc(wedge_graph* h, T** p, uint64_t count, bool state = false)
 {
     *p = nullptr;
     const size_t bytes = (size_t)(count ? count : 1) * sizeof(T);
+    const uint64_t need = ((uint64_t)bytes + 255) & ~255ull;
+    if (!state && h->slab && h->slab_used + need <= h->slab_size) {
+        *p = (T*)(h->slab + h->slab_used);
+        h->slab_used += need;
+        return WEDGE_OK;
+    }
     cudaError_t e = cudaMalloc((void**)p, bytes);
     if (e != cudaSuccess)
         return cuda_status(e);
@@ -169,6 +175,9 @@ static int dalloc(wedge_graph* h, T** p, uint64_t count, bool state = false)
 // LOAD_SCRATCH_EDGES (edges and vertices) bounds the block (1.6 GB); beyond it
 // the kernels' time hides the mapping.
 constexpr uint64_t LOAD_SCRATCH_EDGES = 1ull << 25;
+// Up to this many edges and vertices a graph's own arrays, twenty of them, lie
+// in one block too (100 MB at most, 5% of it unused)
+constexpr uint64_t SLAB_EDGES = 1ull << 22;
 
 template <class T>
 static cudaError_t talloc(wedge_graph* h, T** p, uint64_t bytes)
@@ -755,6 +764,17 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
     g.w = d_w;
     const uint32_t cap = (uint32_t)h->num_sms * 16u;
 
+    if (E + V <= SLAB_EDGES) { /* the arrays below, at most (a slot each rounded up) */
+        const uint64_t vne = E < V ? E : V;
+        const uint64_t size = (d_w ? 14u : 5u) * g.Epad + 16ull * g.T + 24ull * V + 26ull * vne + 32u * 256u;
+        unsigned char* slab = nullptr;
+        const int rc = dalloc(h, &slab, size);
+        if (rc)
+            return rc;
+        h->slab = slab;
+        h->slab_size = size;
+        h->slab_used = 0;
+    }
     if (E + V <= LOAD_SCRATCH_EDGES) { /* two key arrays, a sort's work space, wide weights; then the scans' */
         h->tsize = (E + V) * (d_w ? 24u : 16u) + 24u * V + E + (4ull << 20);
         h->tused = 0;
@@ -955,7 +975,7 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
     g.csri = csri;
     g.csr = chunks ? 0u : 1u;
     g.dst_index = g.dst_ident ? nullptr : inv;
-    if (g.dst_ident && inv) {
+    if (g.dst_ident && inv && !h->slab) {
         untrack(h, inv);
         cudaFree(inv);
     }

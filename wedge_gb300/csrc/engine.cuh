@@ -274,6 +274,8 @@ struct wedge_graph {
     float* net;                        // device copy of the scheduler network (wedge_cuda_set_scheduler)
     unsigned char* tscratch;           // the load's temporary arrays (small graphs; null otherwise and after the load)
     uint64_t tsize, tused;
+    unsigned char* slab;               // a small graph's arrays (tracked as one allocation; null otherwise)
+    uint64_t slab_size, slab_used;
     // allocations owned by the handle
     void* allocs[40];
     int nallocs;
