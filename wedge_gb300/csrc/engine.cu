@@ -769,12 +769,13 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
         const uint64_t vne = E < V ? E : V;
         const uint64_t size = (d_w ? 14u : 5u) * g.Epad + 16ull * g.T + 24ull * V + 26ull * vne + 32u * 256u;
         unsigned char* slab = nullptr;
-        const int rc = dalloc(h, &slab, size);
-        if (rc)
-            return rc;
-        h->slab = slab;
-        h->slab_size = size;
-        h->slab_used = 0;
+        if (dalloc(h, &slab, size) == WEDGE_OK) {
+            h->slab = slab;
+            h->slab_size = size;
+            h->slab_used = 0;
+        } else {
+            cudaGetLastError(); /* one by one, as far as the memory goes */
+        }
     }
     if (E + V <= LOAD_SCRATCH_EDGES) { /* two key arrays, a sort's work space, wide weights; then the scans' */
         h->tsize = (E + V) * (d_w ? 24u : 16u) + 24u * V + E + (4ull << 20);
