@@ -304,3 +304,30 @@ def test_bounded_weight_ordered_pulls(engine_lib, weights, limit):
                 for threshold_pct in (1, 20, 100):
                     g.run(W.APP_SSSP, W.Params(root=root, sched=sched, flags=flags, threshold_pct=threshold_pct))
                     assert np.array_equal(g.read_results(), expect), (sched, flags, threshold_pct)
+
+
+@pytest.mark.parametrize("n", [100_000, 300_001])
+def test_heavy_wedge_iterations(engine_lib, n):
+    """BFS and CC with a frontier of many vertices of one out-edge each, below the
+    dense threshold: too few and enough of them to run as a dense pull"""
+    W = engine_lib
+    rng = np.random.default_rng(n)
+    middle, target = np.arange(1, n + 1), np.arange(n + 1, 2 * n + 1)
+    V = 2 * n + 1001
+    # 0 -> n vertices -> one more each, and edges among 1000 others that count towards the threshold
+    s = np.concatenate([np.zeros(n, np.int64), middle, 2 * n + 1 + rng.integers(0, 1000, 3_000_000)])
+    d = np.concatenate([middle, rng.permutation(target), 2 * n + 1 + rng.integers(0, 1000, 3_000_000)])
+    order = np.lexsort((s, d))
+    s, d = s[order], d[order]
+    parents = np.full(V, np.uint64(0xFFFFFFFFFFFFFFFF))
+    reached = (d <= 2 * n)
+    parents[d[reached]] = s[reached]
+    labels = least_labels(V, s, d)
+    with W.Graph.from_edges(V, s.astype(np.uint32), d.astype(np.uint32)) as g:
+        for sched in (W.SCHED_PLAIN, W.SCHED_WEDGE, W.SCHED_DENSE):
+            for flags in (0, W.FLAG_GRAPH, W.FLAG_TIMING):
+                st = g.run(W.APP_BFS, W.Params(root=0, sched=sched, flags=flags))
+                assert st["iterations"] == 2  # the targets have no out-edges
+                assert np.array_equal(g.read_results(), parents), (sched, flags)
+                g.run(W.APP_CC, W.Params(sched=sched, flags=flags))
+                assert np.array_equal(g.read_results().view(np.float64), labels), (sched, flags)

@@ -8,6 +8,9 @@
 //   pull_kernel<PR>           phase_edge_pull_pr.c:28-116
 //   pr_finish_kernel          phases.c:71-114 (ordered merge) + phases.c:37-46 (total rank)
 //   pr_vertex_kernel          phase_vertex_pr.c:26-77
+//   sparse_loop_kernel        the Wedge iterations of execution_{bfs,cc,sssp}.c:122-365 in one launch
+//   sssp_wo_kernel            phase_edge_pull_sssp.c:57-170 over weight-ordered in-edges
+//   pr_loop_kernel            execution_pr.c:396-486 in one launch
 //   collect_kernel            wedge.c:63-155 (walk of the active-vertex bitmap)
 //   wedge_build_kernel        wedge.c:37-46 (CSRI walk setting frontier bits)
 //   decide_kernel             execution_*.c driver loop: mass reduce, dense/Wedge choice, convergence
@@ -1379,7 +1382,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
     Ctrl* c = s.ctrl;
     if (c->done)
         return;
-    const uint32_t mode = APP == WEDGE_APP_SSSP && c->heavy ? (uint32_t)MODE_DENSE : c->mode;
+    const uint32_t mode = c->mode == MODE_WEDGE && c->heavy ? (uint32_t)MODE_DENSE : c->mode;
     if (phase == PHASE_REST && mode == MODE_WEDGE) {
         // a Wedge pull runs whole in the first launch: this one only reports zeros
         if (threadIdx.x < NCNT)
@@ -2503,7 +2506,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
     Ctrl* c = s.ctrl;
     if (c->done)
         return;
-    const uint32_t mode = c->mode;
+    const uint32_t mode = c->mode == MODE_WEDGE && c->heavy ? (uint32_t)MODE_DENSE : c->mode;
     // CC on a symmetric graph propagates engine ids; before its first pull every
     // label is its vertex's own id
     const bool ident0 = APP == WEDGE_APP_CC && g.sym != 0u && c->iter == 0u;
@@ -3249,6 +3252,7 @@ __device__ __forceinline__ void decide_block(const DevGraph& g, DevState& s, Ctr
         c->items = 0u;
         c->alist_n = 0u;
         c->heavy = 0u;
+        c->last_act = cnt[CNT_ACT];
         go = 0u;
         // SSSP: a pull dropped 32-bit sums that reached the copy's limit; the
         // next pull is dense and 64-bit, and relaxes every in-edge again
@@ -3699,6 +3703,7 @@ __global__ void init_root_kernel(DevGraph g, DevState s, uint32_t app, uint64_t 
         c->ovf_redo = 0;
         c->bodies = 0;
         c->heavy = 0u;
+        c->last_act = 1ull;
         for (int i = 0; i < 3; ++i)
             c->fmin[i] = 0u;
         loop_reset(c);
@@ -3777,6 +3782,13 @@ constexpr uint32_t BARRIER_TRIES = 1u << 22;
 // one, 0.4 as a pull).  The whole SSSP at scales 26, 22 and 20: 3.20, 0.62 and
 // 0.44 ms; with 1: 3.19, 0.63, 0.44; with 4: 3.19, 0.72, 0.44; never: 3.82 at 26.
 constexpr uint32_t WO_HEAVY = 2;
+// BFS and CC: a listed vertex takes about 75 ps and an out-edge 8 (all blocks
+// together), a dense pull's probe about 5 ps per destination of the graph and
+// 15 us for its launches; in units of 5 ps.  R-MAT scales 24 and 26, BFS with the
+// rule 0.338 and 0.856 ms, without it 0.367 and 0.976; CC at 24: 0.300 and 0.350.
+// Half or twice the first two costs: 0.368 or 0.335 and 0.855 for BFS, 0.326 for
+// CC, and twice loses 4% on CC at scale 21 (0.139 -> 0.147).
+constexpr uint32_t HEAVY_VERT = 14, HEAVY_EDGE = 2, HEAVY_FIXED = 3u << 20;
 enum : uint32_t { ERR_BARRIER_TIMEOUT = 4u };
 
 // all blocks of a cooperative launch; false when it did not complete within
@@ -3853,13 +3865,14 @@ struct LoopBook {
     }
 
     // into the control block: before another launch or block reads it
-    __device__ void close(Ctrl* c, unsigned long long mass, const NextPull& next, uint32_t iter, uint32_t parity) const
+    __device__ void close(Ctrl* c, unsigned long long mass, unsigned long long act, const NextPull& next, uint32_t iter, uint32_t parity) const
     {
         c->edges_scanned = edges;
         c->dsts_scanned = dsts;
         c->activated = activated;
         c->last_mass = mass;
         c->mass = mass;
+        c->last_act = act;
         c->wedge_iters = wedge_iters;
         c->pull_launches = pull_launches;
         c->iter = iter;
@@ -3904,11 +3917,15 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
     uint32_t mode = c->mode, parity = c->parity, iter = c->iter;
     const uint32_t sched = c->sched, max_iter = c->max_iter, probe_iter = c->probe_iter, probe_mode = c->probe_mode;
     const unsigned long long thr = c->threshold;
-    // SSSP: whether a Wedge iteration over `mass` out-edges is better a weight-ordered pull
-    const bool may_pull = APP == WEDGE_APP_SSSP && s.wo && small == 0u && max_steps > 1u &&
+    // whether a Wedge iteration over `act` vertices of `mass` out-edges is better a dense pull
+    const bool may_pull = (APP != WEDGE_APP_SSSP || s.wo) && small == 0u && max_steps > 1u &&
                           (sched == WEDGE_SCHED_PLAIN || sched == WEDGE_SCHED_LEARNED);
-    auto heavy = [&](unsigned long long mass) { return may_pull && mass > WO_HEAVY * (unsigned long long)g.Vne; };
-    const bool pull_now = mode == MODE_WEDGE && heavy(c->mass);
+    auto heavy = [&](unsigned long long mass, unsigned long long act) {
+        const unsigned long long vne = g.Vne;
+        return may_pull && (APP == WEDGE_APP_SSSP ? mass > WO_HEAVY * vne
+                                                  : HEAVY_VERT * act + HEAVY_EDGE * mass > vne + HEAVY_FIXED);
+    };
+    const bool pull_now = mode == MODE_WEDGE && iter != 0u && heavy(c->mass, c->last_act);
     const bool loop = small != 0u || (mode == MODE_WEDGE && !pull_now);
     const bool f64 = g.weight_kind == WEDGE_WEIGHTS_F64;
     uint32_t* my_buf = sh_buf[wib];
@@ -4026,8 +4043,9 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
         if (s.tile_need)
             for (uint32_t i = tid; i < g.T / 32u + 2u; i += nthr)
                 s.tile_need[i] = 0u;
-        if (APP == WEDGE_APP_SSSP && tid == 0u) {
-            c->fmin[(parity + 1u) % 3u] = NONE32; /* of the frontier the next pull writes */
+        if (tid == 0u) {
+            if (APP == WEDGE_APP_SSSP)
+                c->fmin[(parity + 1u) % 3u] = NONE32; /* of the frontier the next pull writes */
             if (pull_now)
                 c->heavy = 1u;
         }
@@ -4477,12 +4495,12 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
         for (uint32_t j = 0; j < NCNT; ++j)
             cnt[j] = sh_acc[j];
         const NextPull next = next_pull(sched, cnt[CNT_MASS], false, iter + 1u, max_iter, thr, probe_iter, probe_mode);
-        const bool pull_next = APP == WEDGE_APP_SSSP && !(sorting && so.release + so.waiting != 0ull) && heavy(cnt[CNT_MASS]);
+        const bool pull_next = !(sorting && so.release + so.waiting != 0ull) && heavy(cnt[CNT_MASS], cnt[CNT_ACT]);
         if (scribe)
             book.note(g, s, (uint32_t)APP, cnt, next, mode, iter);
         if (scribe && (next.done || step + 1u == max_steps || (!small && next.mode != MODE_WEDGE) || pull_next ||
                        sched == WEDGE_SCHED_LEARNED))
-            book.close(c, cnt[CNT_MASS], next, iter + 1u, (parity + 1u) % 3u);
+            book.close(c, cnt[CNT_MASS], cnt[CNT_ACT], next, iter + 1u, (parity + 1u) % 3u);
         if (!next.done && sched == WEDGE_SCHED_LEARNED && s.net && blockIdx.x + 1u == gridDim.x)
             ask_network(s, c, (uint32_t)APP, iter + 1u);
         mode = next.mode;
