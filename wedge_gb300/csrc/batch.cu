@@ -1094,7 +1094,7 @@ extern "C" int wedge_cuda_batch_create(wedge_graph_t* const* graphs, uint32_t nu
     b->device = dev;
     b->Q = num_queries;
     b->G = num_graphs;
-    b->qallocs = (void**)calloc((size_t)num_queries + 2 * (size_t)num_graphs + 1, sizeof(void*)); /* one block per query, two arrays per graph */
+    b->qallocs = (void**)calloc((size_t)num_graphs + 3, sizeof(void*)); /* an array per graph, the lists, the queries */
     b->h_graphs = (BGraph*)calloc(num_graphs, sizeof(BGraph));
     b->h_queries = (BQuery*)calloc(num_queries, sizeof(BQuery));
     int rc = WEDGE_OK;
@@ -1151,24 +1151,32 @@ extern "C" int wedge_cuda_batch_create(wedge_graph_t* const* graphs, uint32_t nu
     uint32_t* h_long = (uint32_t*)calloc(num_graphs, sizeof(uint32_t));
     if (!h_long)
         return fail(WEDGE_ERR_OOM);
+    uint2* lists = nullptr; /* one after the other */
     for (int pass = 0; pass < 2 && !rc; ++pass) {
-        cudaMemsetAsync(d_long, 0, num_graphs * sizeof(uint32_t), b->stream);
+        if (cudaMemsetAsync(d_long, 0, num_graphs * sizeof(uint32_t), b->stream) != cudaSuccess)
+            rc = WEDGE_ERR_CUDA;
+        uint64_t at = 0;
         for (uint32_t i = 0; i < num_graphs && !rc; ++i) {
             BGraph& G = b->h_graphs[i];
-            uint2* list = nullptr;
             if (!G.wsrc || (pass && !h_long[i]))
                 continue;
-            if (pass && (rc = balloc(b, &list, h_long[i], true)))
-                break;
-            batch_wo_long_kernel<<<bgrid(G.Vne, 256, (uint32_t)b->num_sms * 8), 256, 0, b->stream>>>(G.dst_off, G.Vne, d_long + i,
-                                                                                                    list);
-            G.wo_long = list;
-            G.nlong = pass ? h_long[i] : 0u;
+            G.wo_long = lists + at;
+            G.nlong = h_long[i];
+            at += h_long[i];
+            batch_wo_long_kernel<<<bgrid(G.Vne, 256, (uint32_t)b->num_sms * 8), 256, 0, b->stream>>>(
+                G.dst_off, G.Vne, d_long + i, pass ? lists + (at - h_long[i]) : nullptr);
         }
-        if (!rc && (cudaMemcpyAsync(h_long, d_long, num_graphs * sizeof(uint32_t), cudaMemcpyDeviceToHost, b->stream) !=
-                        cudaSuccess ||
-                    cudaStreamSynchronize(b->stream) != cudaSuccess))
+        if (pass || rc)
+            break;
+        if (cudaMemcpyAsync(h_long, d_long, num_graphs * sizeof(uint32_t), cudaMemcpyDeviceToHost, b->stream) != cudaSuccess ||
+            cudaStreamSynchronize(b->stream) != cudaSuccess) {
             rc = WEDGE_ERR_CUDA;
+            break;
+        }
+        for (uint32_t i = 0; i < num_graphs; ++i)
+            at += h_long[i];
+        if (!at || (rc = balloc(b, &lists, at, true)))
+            break;
     }
     free(h_long);
     if (rc)
@@ -1176,37 +1184,41 @@ extern "C" int wedge_cuda_batch_create(wedge_graph_t* const* graphs, uint32_t nu
     uint32_t* h_sweep = (uint32_t*)calloc((size_t)num_queries + 1, sizeof(uint32_t));
     if (!h_sweep)
         return fail(WEDGE_ERR_OOM);
-    for (uint32_t i = 0; i < num_queries && !rc; ++i) {
-        const BGraph& G = b->h_graphs[queries[i].graph];
-        BQuery& q = b->h_queries[i];
-        q.graph = queries[i].graph;
-        q.app = (uint32_t)queries[i].app;
-        q.root_in = queries[i].root < G.V ? (uint32_t)queries[i].root : 0u;
-        const uint64_t words = (G.V + 31) / 32 + 1, chunks = G.push ? 0 : (uint64_t)G.nchunks,
-                       nitems = G.push ? G.E / (PUSH_PIECE / 2u) + 1 : 0;
-        h_sweep[i + 1] = h_sweep[i] + (uint32_t)((words + SWEEP - 1) / SWEEP);
-        // a query's arrays in one block, each on a 256-byte boundary
-        uint64_t size = 0;
-        auto place = [&](uint64_t bytes) {
-            const uint64_t at = size;
-            size += (bytes + 255) & ~255ull;
-            return at;
-        };
-        const uint64_t at_prop = place(8 * G.V), at_front = place(3 * ((4 * words + 255) & ~255ull)), at_l0 = place(4 * G.V),
-                       at_l1 = place(4 * G.V), at_bits = place(4 * (chunks / 32 + 1)), at_list = place(4 * chunks),
-                       at_i0 = place(8 * nitems), at_i1 = place(8 * nitems);
-        unsigned char* base = nullptr;
-        if ((rc = balloc(b, &base, size, true)))
+    unsigned char* base = nullptr; /* all queries' arrays, each on a 256-byte boundary */
+    uint64_t size = 0;
+    for (int pass = 0; pass < 2 && !rc; ++pass) {
+        if (pass && (rc = balloc(b, &base, size, true)))
             break;
-        q.prop = (unsigned long long*)(base + at_prop);
-        for (uint32_t f = 0; f < 3; ++f)
-            q.front[f] = (uint32_t*)(base + at_front + f * ((4 * words + 255) & ~255ull));
-        q.list[0] = (uint32_t*)(base + at_l0);
-        q.list[1] = (uint32_t*)(base + at_l1);
-        q.chunk_bits = (uint32_t*)(base + at_bits);
-        q.chunk_list = (uint32_t*)(base + at_list);
-        q.items[0] = (uint2*)(base + at_i0);
-        q.items[1] = (uint2*)(base + at_i1);
+        size = 0;
+        for (uint32_t i = 0; i < num_queries; ++i) {
+            const BGraph& G = b->h_graphs[queries[i].graph];
+            BQuery& q = b->h_queries[i];
+            q.graph = queries[i].graph;
+            q.app = (uint32_t)queries[i].app;
+            q.root_in = queries[i].root < G.V ? (uint32_t)queries[i].root : 0u;
+            const uint64_t words = (G.V + 31) / 32 + 1, chunks = G.push ? 0 : (uint64_t)G.nchunks,
+                           nitems = G.push ? G.E / (PUSH_PIECE / 2u) + 1 : 0;
+            h_sweep[i + 1] = h_sweep[i] + (uint32_t)((words + SWEEP - 1) / SWEEP);
+            auto place = [&](uint64_t bytes) {
+                const uint64_t at = size;
+                size += (bytes + 255) & ~255ull;
+                return at;
+            };
+            const uint64_t at_prop = place(8 * G.V), at_front = place(3 * ((4 * words + 255) & ~255ull)), at_l0 = place(4 * G.V),
+                           at_l1 = place(4 * G.V), at_bits = place(4 * (chunks / 32 + 1)), at_list = place(4 * chunks),
+                           at_i0 = place(8 * nitems), at_i1 = place(8 * nitems);
+            if (!pass)
+                continue;
+            q.prop = (unsigned long long*)(base + at_prop);
+            for (uint32_t f = 0; f < 3; ++f)
+                q.front[f] = (uint32_t*)(base + at_front + f * ((4 * words + 255) & ~255ull));
+            q.list[0] = (uint32_t*)(base + at_l0);
+            q.list[1] = (uint32_t*)(base + at_l1);
+            q.chunk_bits = (uint32_t*)(base + at_bits);
+            q.chunk_list = (uint32_t*)(base + at_list);
+            q.items[0] = (uint2*)(base + at_i0);
+            q.items[1] = (uint2*)(base + at_i1);
+        }
     }
     if (!rc && !(rc = balloc(b, &b->d_graphs, num_graphs, false)) && !(rc = balloc(b, &b->d_queries, num_queries, false)) &&
         !(rc = balloc(b, &b->d_ctl, num_queries, false)) && !(rc = balloc(b, &b->d_sh, 1, false)) &&
