@@ -289,7 +289,7 @@ def _roofline(W, suite, peak):
         else:
             ms = sum(r["pull_ms"] for r in log)
             byts = sum(pull_bytes(a, r, V) for r in log)
-            out[a] = {"kernel": "dst_kernel + pull_kernel" if a in ("bfs", "cc") else "pull_kernel",
+            out[a] = {"kernel": "dst_kernel + pull_kernel" if a in ("bfs", "cc") else "sparse_loop_kernel + sssp_wo_kernel",
                       "iterations": len(log), "pull_ms": round(ms, 4), "algorithmic_bytes": int(byts),
                       "modes": [r["mode"] for r in log], "edges_scanned": int(sum(r["edges_scanned"] for r in log))}
         ach = byts / (ms / 1e3) / 1e9 if ms > 0 else 0.0
