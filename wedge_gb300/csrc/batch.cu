@@ -5,10 +5,11 @@
 //   pull    warps take items from the work queue, across all queries.  Sparse
 //           pulls relax the out-edges of the vertices the last iteration changed
 //           (items of PUSH_CHUNK listed vertices, whose out-edges are spread over
-//           the lanes, and PUSH_PIECE-edge pieces of long lists); dense SSSP
-//           pulls read weight-ordered in-edges up to the first weight that cannot
-//           lower the destination (items of 32 destinations, and WO_PIECE-edge
-//           pieces of the ones with more in-edges); other dense pulls take tiles
+//           the lanes, and PUSH_PIECE-edge pieces of long lists); dense pulls
+//           take 32 destinations, and WO_PIECE-edge pieces of the ones with more
+//           in-edges: BFS the first source in the frontier, SSSP weight-ordered
+//           in-edges up to the first weight that cannot lower the destination;
+//           graphs without byte weights (SSSP) or with chunk ids take tiles
 //           of 256 in-edges.  Changed vertices are listed as they change, and the
 //           bitmap the next round writes is cleared.
 //   decide  (block 0) per query: done when no mass changed, else the plain rule
@@ -55,6 +56,7 @@ struct BGraph {
     const uint8_t* ww8;
     const uint32_t* wo_src;      // every destination's first weight-ordered source (bit 31: its only one)
     const uint16_t* wo_w;        // and first two weights
+    const uint32_t* first_src;   // every destination's first source
     const uint2* wo_long;        // (destination, first in-edge) pieces of the destinations past WO_GROUP in-edges
     uint32_t nlong;
     const uint32_t* outdeg;
@@ -690,6 +692,91 @@ __device__ void wo_piece(const BArgs& a, uint32_t q, uint2 it, unsigned long lon
     }
 }
 
+// dense pulls by destinations (and pieces of the long ones) instead of tiles
+__device__ __forceinline__ bool by_destination(const BGraph& G, uint32_t app)
+{
+    return app == WEDGE_APP_BFS ? G.push != 0u : G.wsrc != nullptr;
+}
+
+// A dense BFS pull's item: 32 destinations, one per lane.  An unvisited one
+// takes its first source in the frontier; for most that is the first of all,
+// which first_src holds in order.  A destination's pieces and its lane claim it
+// by compare-and-swap.
+__device__ void bfs_group(const BArgs& a, uint32_t q, uint32_t group, unsigned long long& mass)
+{
+    const int lane = threadIdx.x & 31;
+    const BQuery& qq = a.q[q];
+    BCtl& c = a.ctl[q];
+    const BGraph& G = a.graphs[qq.graph];
+    const uint32_t k = group * 32u + (uint32_t)lane;
+    const uint32_t* cur = qq.front[c.iter % 3u];
+    uint32_t d = 0u, par = NONE32, od = 0u;
+    if (k < G.Vne) {
+        d = G.dst_id[k];
+        const uint32_t x = G.first_src[k];
+        if (qq.prop[d] == NONE64) {
+            if ((cur[x >> 5] >> (x & 31u)) & 1u) {
+                par = x;
+            } else {
+                const uint32_t lo = (uint32_t)G.dst_off[k], hi = (uint32_t)G.dst_off[k + 1u];
+                if (hi - lo <= WO_GROUP) /* the others are left to their pieces */
+                    for (uint32_t p = lo & ~3u; p < hi && par == NONE32; p += 4u) {
+                        const uint4 xs = __ldg(reinterpret_cast<const uint4*>(G.src + p));
+                        const uint32_t y[4] = {xs.x, xs.y, xs.z, xs.w};
+                        uint32_t w[4];
+#pragma unroll
+                        for (uint32_t j = 0; j < 4; ++j)
+                            w[j] = p + j > lo && p + j < hi ? cur[y[j] >> 5] : 0u;
+#pragma unroll
+                        for (int j = 3; j >= 0; --j)
+                            if ((w[j] >> (y[j] & 31u)) & 1u)
+                                par = y[j];
+                    }
+            }
+        }
+    }
+    const bool hit = par != NONE32 && atomicCAS(&qq.prop[d], NONE64, (unsigned long long)par) == NONE64;
+    if (hit) {
+        atomicOr(&qq.front[(c.iter + 1u) % 3u][d >> 5], 1u << (d & 31u));
+        od = G.outdeg[d];
+        mass += od;
+    }
+    list_warp(qq, c, G, hit, d, od);
+}
+
+// a piece of a destination with many in-edges: the first source in the frontier
+__device__ void bfs_piece(const BArgs& a, uint32_t q, uint2 it, unsigned long long& mass)
+{
+    const int lane = threadIdx.x & 31;
+    const BQuery& qq = a.q[q];
+    BCtl& c = a.ctl[q];
+    const BGraph& G = a.graphs[qq.graph];
+    const uint32_t d = G.dst_id[it.x], end = (uint32_t)G.dst_off[it.x + 1u];
+    if (__shfl_sync(FULL, qq.prop[d], 0) != NONE64)
+        return;
+    const uint32_t* cur = qq.front[c.iter % 3u];
+    const uint32_t hi = end - it.y > WO_PIECE ? it.y + WO_PIECE : end;
+    for (uint32_t p = it.y; p < hi; p += 32u) {
+        const uint32_t e = p + (uint32_t)lane;
+        uint32_t x = 0u;
+        bool on = false;
+        if (e < hi) {
+            x = G.src[e];
+            on = (cur[x >> 5] >> (x & 31u)) & 1u;
+        }
+        const uint32_t m = __ballot_sync(FULL, on);
+        if (m) {
+            if (lane == __ffs(m) - 1 && atomicCAS(&qq.prop[d], NONE64, (unsigned long long)x) == NONE64) {
+                const uint32_t od = G.outdeg[d];
+                atomicOr(&qq.front[(c.iter + 1u) % 3u][d >> 5], 1u << (d & 31u));
+                list_one(qq, c, G, d, od);
+                mass += od;
+            }
+            return;
+        }
+    }
+}
+
 // The order of the groups in the queue: in-degrees fall with the destination
 // number, and a warp takes up to 32 items at a time, so consecutive items are
 // groups far apart (32 neighbouring hub groups kept one warp busy for 900 us of
@@ -706,7 +793,8 @@ __device__ __forceinline__ uint32_t wo_spread(uint32_t i, uint32_t n)
 // queue's end.  32 SSSPs over 8 graphs (scales 12 to 20, 177 M in-edges in
 // all): 3.1 ms in 16 rounds (3.6 without wo_limit's bound and the first in-edges
 // in arrays of their own), 13.3 with 256-edge tiles that streamed every in-edge
-// of a dense pull; 16 BFS and 16 SSSP over scales 13 to 16: 0.61 ms, 2.8 before.
+// of a dense pull; 16 BFS over scales 16 to 20: 0.61 ms, 1.5 in tiles; 16 BFS
+// and 16 SSSP over scales 13 to 16: 0.55 ms, 2.8 before.
 __device__ void phase_pull(const BArgs& a)
 {
     __shared__ uint32_t heads_all[BT / 32];
@@ -771,8 +859,12 @@ __device__ void phase_pull(const BArgs& a)
             const BGraph& G = a.graphs[qq.graph];
             if (c.mode != MODE_WEDGE) {
                 const uint32_t groups = (G.Vne + 31u) / 32u;
-                if (qq.app != WEDGE_APP_SSSP || !G.wsrc)
+                if (!by_destination(G, qq.app))
                     pull_tile(a, q, local, mass); /* tiles of BTILE_CH chunks */
+                else if (qq.app == WEDGE_APP_BFS && local < G.nlong)
+                    bfs_piece(a, q, G.wo_long[local], mass);
+                else if (qq.app == WEDGE_APP_BFS)
+                    bfs_group(a, q, wo_spread(local - G.nlong, groups), mass);
                 else if (local < G.nlong)
                     wo_piece(a, q, G.wo_long[local], mass, least);
                 else
@@ -802,7 +894,7 @@ __device__ void phase_pull(const BArgs& a)
 __device__ __forceinline__ uint32_t pull_items(const BGraph& G, const BQuery& qq, const BCtl& c)
 {
     if (c.mode == MODE_DENSE) {
-        if (qq.app == WEDGE_APP_SSSP && G.wsrc)
+        if (by_destination(G, qq.app))
             return (G.Vne + 31u) / 32u + G.nlong;
         return (G.nchunks + BTILE_CH - 1u) / BTILE_CH;
     }
@@ -1124,6 +1216,7 @@ extern "C" int wedge_cuda_batch_create(wedge_graph_t* const* graphs, uint32_t nu
         G.wsrc = g.csr ? g.wsrc : nullptr;
         G.ww8 = g.ww8;
         G.wo_src = g.wo_src;
+        G.first_src = g.first_src;
         G.wo_w = g.wo_w;
         if (!g.csr)
             b->chunks = 1u;
@@ -1144,7 +1237,7 @@ extern "C" int wedge_cuda_batch_create(wedge_graph_t* const* graphs, uint32_t nu
         G.chunk_dst0 = cd;
         batch_chunk_index_kernel<<<bgrid((uint64_t)G.nchunks + 1, 256, (uint32_t)b->num_sms * 8), 256, 0, b->stream>>>(G, cd);
     }
-    // pieces of the destinations with many in-edges (dense SSSP pulls): all graphs' counts, then their lists
+    // pieces of the destinations with many in-edges (dense pulls): all graphs' counts, then their lists
     uint32_t* d_long = nullptr;
     if ((rc = balloc(b, &d_long, num_graphs, false)))
         return fail(rc);
@@ -1158,7 +1251,7 @@ extern "C" int wedge_cuda_batch_create(wedge_graph_t* const* graphs, uint32_t nu
         uint64_t at = 0;
         for (uint32_t i = 0; i < num_graphs && !rc; ++i) {
             BGraph& G = b->h_graphs[i];
-            if (!G.wsrc || (pass && !h_long[i]))
+            if (!G.push || (pass && !h_long[i]))
                 continue;
             G.wo_long = lists + at;
             G.nlong = h_long[i];
