@@ -43,7 +43,7 @@ ENGINE_SPACE = {
     "sssp": {"hub_bytes": HUB_CHOICES, "sssp_tile": (256, 512), "sssp_narrow": (0, 1)},
     "pr": {"hub_bytes": HUB_CHOICES},
 }
-GRID = {"threshold_pct": (10, 20, 40), "grab": (2, 8, 32), "blocks_per_sm": (1, 2, 4), "split": (8, 32, 128)}
+GRID = {"threshold_pct": (2, 5, 10, 20, 40), "grab": (2, 8, 32), "blocks_per_sm": (1, 2, 4), "split": (8, 32, 128)}
 
 
 def load_tuning(path: str = DEFAULT_TUNING):
