@@ -331,3 +331,80 @@ def test_heavy_wedge_iterations(engine_lib, n):
                 assert np.array_equal(g.read_results(), parents), (sched, flags)
                 g.run(W.APP_CC, W.Params(sched=sched, flags=flags))
                 assert np.array_equal(g.read_results().view(np.float64), labels), (sched, flags)
+
+
+def sorted_again_and_again(filler, seed):
+    """An SSSP whose far vertices become near and far again under a bound that falls: a
+    path from 0 with fans of out-edges on it.  D (past the first 16 iterations) sets
+    the first bound and leaves A, behind a long edge, beyond it; A is released and
+    lowers the targets T, which have no out-edges, past the second bound; B lowers
+    them below it; R ends the sorting with its fewer out-edges; C lowers T past the
+    third bound, which is the least.  Returns the edges and the vertices of T."""
+    T, path = 70_000, 40
+    a, v0 = path + 1, path + 2  # vertices 0..path, A, then T and others that only receive
+    junk = v0 + T
+    V = junk + 40
+    fan = {14: (20_000, 1), 15: (66_000, 1), 22: (20_000, 1)}  # path vertex -> out-edges to the others, weight
+    parts = [(np.arange(path), np.arange(1, path + 1), np.ones(path, np.int64))]
+    for p, (n, w) in fan.items():
+        parts.append((np.full(n, p), junk + np.arange(n) % 40, np.full(n, w)))
+    parts.append(([15], [a], [10_000_000]))
+    for p, w in ((a, 4_000_000), (20, 5_000_000), (23, 4_000_000)):
+        parts.append((np.full(T, p), v0 + np.arange(T), np.full(T, w)))
+    rng = np.random.default_rng(seed)
+    parts.append((junk + rng.integers(0, 20, filler), junk + 20 + rng.integers(0, 20, filler), rng.integers(0, 2, filler)))
+    s, d, w = (np.concatenate([p[i] for p in parts]).astype(np.int64) for i in range(3))
+    order = np.lexsort((s, d))
+    return V, s[order], d[order], w[order], np.arange(v0, v0 + T)
+
+
+def real_distances(V, src, dst, w, root):
+    """least path sums in doubles, in the order of the path; inf = unreached"""
+    dist = np.full(V, np.inf)
+    dist[root] = 0.0
+    while True:
+        new = dist.copy()
+        np.minimum.at(new, dst, dist[src] + w)
+        if np.array_equal(new, dist):
+            return dist
+        dist = new
+
+
+@pytest.mark.parametrize("places", [None, 1, 64, 70_000])
+@pytest.mark.parametrize("filler", [100_000, 1_200_000])
+@pytest.mark.parametrize("weights", ["words", "f64"])
+def test_far_list_holds_a_vertex_once(engine_lib, monkeypatch, weights, filler, places):
+    """vertices that are sorted out again and again, also with a list that fills up,
+    in one launch (100,000 more edges) and apart from the dense pulls"""
+    W = engine_lib
+    if places is not None:
+        monkeypatch.setenv("WEDGE_FAR_LIST", str(places))
+    V, s, d, w, _ = sorted_again_and_again(filler, 1)
+    if weights == "f64":
+        expect, words, kind = real_distances(V, s, d, w + 0.25, 0).view(np.uint64), (w + 0.25).view(np.uint64), W.WEIGHTS_F64
+    else:
+        expect, words, kind = bellman_ford(V, s, d, w, 0), w.astype(np.uint64), W.WEIGHTS_U64
+    with W.Graph.from_edges(V, s.astype(np.uint32), d.astype(np.uint32), words, kind) as g:
+        for sched in (W.SCHED_PLAIN, W.SCHED_WEDGE):
+            for flags in (0, W.FLAG_GRAPH):
+                g.run(W.APP_SSSP, W.Params(sched=sched, flags=flags))
+                assert np.array_equal(g.read_results(), expect), (sched, flags)
+
+
+@pytest.mark.parametrize("places", [None, 1, 1000])
+def test_far_list_of_a_grid(engine_lib, monkeypatch, places):
+    """the same on a grid with random pairs, against plain arithmetic"""
+    W = engine_lib
+    if places is not None:
+        monkeypatch.setenv("WEDGE_FAR_LIST", str(places))
+    side, rng = 700, np.random.default_rng(8)
+    v = np.arange(side * side).reshape(side, side)
+    s = np.concatenate([v[:, :-1].ravel(), v[:, 1:].ravel(), v[:-1].ravel(), v[1:].ravel(), rng.integers(0, side * side, 9000)])
+    d = np.concatenate([v[:, 1:].ravel(), v[:, :-1].ravel(), v[1:].ravel(), v[:-1].ravel(), rng.integers(0, side * side, 9000)])
+    order = np.lexsort((s, d))
+    s, d, w = s[order], d[order], rng.integers(0, 100_000, len(s))
+    expect = bellman_ford(side * side, s, d, w, 0)
+    with W.Graph.from_edges(side * side, s.astype(np.uint32), d.astype(np.uint32), w.astype(np.uint64)) as g:
+        for flags in (0, W.FLAG_GRAPH):
+            g.run(W.APP_SSSP, W.Params(flags=flags))
+            assert np.array_equal(g.read_results(), expect), flags

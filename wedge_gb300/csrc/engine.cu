@@ -3151,10 +3151,11 @@ __device__ __forceinline__ void log_iteration(DevState& s, Ctrl* c, const unsign
 __device__ __forceinline__ void loop_reset(Ctrl* c)
 {
     c->bar = 0u;
+    c->lall[0] = c->lall[1] = 0u;
     for (int i = 0; i < 3; ++i) {
         c->ln[i] = 0u;
         c->li[i] = 0u;
-        c->lf[i] = 0u;
+        c->lf[i] = c->lput[i] = 0u;
         c->lmin[i] = NONE64;
         c->lfar[i] = 0ull;
         for (uint32_t j = 0; j < NCNT; ++j)
@@ -3765,7 +3766,12 @@ __global__ void init_root_kernel(DevGraph g, DevState s, uint32_t app, uint64_t 
 // relaxed once or twice instead of 13 times (4096^2 grid: 78 M out-edges
 // relaxed for 1.9 G; 16.1 -> 6.6 ms.  Steps of 1/2, 2 and 4 mean weights: 7.4,
 // 6.9, 9.1 ms; masses of 2^14, 2^17, 2^18: 6.8, 6.6, 7.1 ms).  Before a dense
-// pull the waiting vertices join the frontier bitmap.
+// pull the waiting vertices join the frontier bitmap.  A far bit per vertex keeps
+// it from being listed twice while it waits.  One that becomes near loses the bit
+// and leaves its entry, so a new list begins wherever the bound may fall; within
+// one list and iteration a vertex that changes several times, far and near in
+// turn, can still leave more entries than one.  What a list has no room for is
+// found by its bits.
 //
 // Graphs of at most LOOP_SMALL_EDGES in-edges run whole in the launch: there a
 // dense iteration is no more work than a Wedge one, and the launches were all
@@ -3897,14 +3903,16 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
     __shared__ val_t sh_val[WARPS][32];
     __shared__ uint32_t sh_fbuf[APP == WEDGE_APP_SSSP ? WARPS : 1][LOOP_BUF]; /* for the far list */
     __shared__ unsigned long long sh_acc[NCNT];
-    __shared__ uint32_t sh_ok, sh_n[4];
+    __shared__ uint32_t sh_ok, sh_n[3];
     // SSSP: what every block knows of the sorting-out, computed by thread 0
     __shared__ struct {
         unsigned long long bound, listed, waiting, far_min; /* far_min: the least distance waiting (none waiting: the
                                                                least one the last iteration changed) */
         uint32_t release, nfar;                             /* far lists begun; vertices of the one whose turn it is */
+        uint32_t begun, overrun;                            /* this iteration begins one; that one did not hold all */
+        unsigned long long held;                            /* entries of the present one */
     } so;
-    __shared__ unsigned long long sh_far[2];
+    __shared__ unsigned long long sh_far[3];
     __shared__ uint32_t sh_least;
     Ctrl* c = s.ctrl;
     if (c->done)
@@ -3940,6 +3948,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
         so.far_min = NONE64;
         so.release = 0u;
         so.nfar = 0u;
+        so.held = 0ull;
     }
     uint32_t* out_list = s.alist;
     uint2* out_items = s.items;
@@ -4065,11 +4074,10 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
     for (uint32_t step = 0;; ++step) {
         const uint32_t a = step % 3u, b = (step + 1u) % 3u;
         /* one warp of the block reads what all blocks read at once */
-        if (threadIdx.x < 4)
+        if (threadIdx.x < 3)
             sh_n[threadIdx.x] = __ldcg(threadIdx.x == 0   ? &c->ln[a]
                                        : threadIdx.x == 1 ? &c->li[a]
-                                       : threadIdx.x == 2 ? &c->narrow_ovf
-                                                          : &c->lf[APP == WEDGE_APP_SSSP ? so.release % 3u : 0u]);
+                                                          : &c->narrow_ovf);
         __syncthreads();
         const uint32_t n = sh_n[0], ni = sh_n[1];
         /* from one iteration before distances may be sorted out: that one finds the least */
@@ -4087,20 +4095,39 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
                 const bool now = iter >= NEAR_ITER && mode == MODE_WEDGE && so.listed > NEAR_MASS;
                 if (!now)
                     so.bound = NONE64; /* every vertex is near */
-                so.nfar = 0u;
-                if (so.waiting != 0ull && (!now || so.listed - so.waiting < NEAR_MASS)) {
-                    so.nfar = sh_n[3];
-                    ++so.release; /* from here on far vertices go to the other buffer */
+                so.nfar = so.begun = so.overrun = 0u;
+                if (so.waiting != 0ull && (!now || so.listed - so.waiting < NEAR_MASS || so.held > s.far_cap)) {
+                    so.nfar = (uint32_t)min(so.held, (unsigned long long)s.far_cap);
+                    so.overrun = so.held > s.far_cap ? 1u : 0u;
+                    so.begun = 1u; /* from here on far vertices go to the other buffer */
                     if (now)
                         so.bound = beyond(max(so.bound, so.far_min));
                     so.far_min = NONE64;
                 } else if (so.waiting == 0ull) {
+                    /* the list holds vertices that became near, and ones without out-edges: nothing to
+                       read, but under a bound that falls they could be listed once more behind it */
+                    so.begun = so.held ? 1u : 0u;
                     if (now && so.bound == NONE64 && so.far_min != NONE64)
                         so.bound = beyond(so.far_min);
                     so.far_min = NONE64;
                 }
+                if (so.begun) {
+                    ++so.release;
+                    so.held = 0ull;
+                }
             }
             __syncthreads();
+            if (so.overrun) { /* the list anew, from the waiting vertices' bits */
+                uint32_t* all = s.far_list + ((so.release & 1u) ? 0ull : s.alist_stride);
+                for (uint32_t i = tid; i < nwords; i += nthr)
+                    for (uint32_t w = s.far[i]; w; w &= w - 1u)
+                        all[atomicAdd(&c->lall[step & 1u], 1u)] = i * 32u + (uint32_t)(__ffs(w) - 1);
+                if (!grid_barrier(c, target, &sh_ok))
+                    return;
+                if (threadIdx.x == 0)
+                    so.nfar = __ldcg(&c->lall[step & 1u]);
+                __syncthreads();
+            }
         }
         const uint32_t half = step & 1u;
         const uint32_t* list = s.alist + (half ? s.alist_stride : 0ull);
@@ -4124,10 +4151,12 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
             }
             c->ln[(step + 2u) % 3u] = 0u;
             c->li[(step + 2u) % 3u] = 0u;
-            if (sorting && so.nfar)
+            if (sorting && so.begun)
                 c->lf[(so.release + 1u) % 3u] = 0u;
+            c->lall[(step + 1u) & 1u] = 0u;
             c->lmin[b] = NONE64;
             c->lfar[b] = 0ull;
+            c->lput[b] = 0u;
         }
         if (blockIdx.x == 0 && threadIdx.x < NCNT)
             c->lacc[b][threadIdx.x] = 0ull;
@@ -4135,6 +4164,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
             old[i] = 0u;
 
         unsigned long long far_mass = 0ull, least = NONE64; /* sorting: change of the waiting out-edges, least distance */
+        uint32_t far_put = 0u;                              /* and entries of the far list, on lane 0 */
         auto work = [&](auto tag) {
         constexpr bool FAR = decltype(tag)::value;
         const unsigned long long bound = FAR ? so.bound : NONE64;
@@ -4146,11 +4176,14 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
         auto flush_far = [&]() {
             __syncwarp();
             uint32_t at = 0u;
-            if (lane == 0)
+            if (lane == 0) {
                 at = atomicAdd(&c->lf[release % 3u], far_kept);
+                far_put += far_kept;
+            }
             at = __shfl_sync(FULL, at, 0);
             for (uint32_t q = (uint32_t)lane; q < far_kept; q += 32u)
-                far_dst[at + q] = sh_fbuf[APP == WEDGE_APP_SSSP ? wib : 0][q];
+                if (at + q < s.far_cap) /* past it: the far bit alone says that the vertex waits */
+                    far_dst[at + q] = sh_fbuf[APP == WEDGE_APP_SSSP ? wib : 0][q];
             far_kept = 0u;
             __syncwarp();
         };
@@ -4432,7 +4465,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
             sh_acc[threadIdx.x] = 0ull;
         if (threadIdx.x == 32) {
             sh_far[0] = NONE64;
-            sh_far[1] = 0ull;
+            sh_far[1] = sh_far[2] = 0ull;
             sh_least = NONE32;
         }
         __syncthreads();
@@ -4459,6 +4492,8 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
                     atomicAdd(&sh_far[1], far_mass); /* modulo 2^64: it may be negative */
                 if (lane == 0 && least != NONE64)
                     atomicMin(&sh_far[0], least);
+                if (far_put)
+                    atomicAdd(&sh_far[2], (unsigned long long)far_put);
             }
         }
         __syncthreads();
@@ -4471,19 +4506,22 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
                 atomicMin(&c->lmin[a], sh_far[0]);
             if (sh_far[1])
                 atomicAdd(&c->lfar[a], sh_far[1]);
+            if (sh_far[2])
+                atomicAdd(&c->lput[a], (unsigned int)sh_far[2]);
         }
         if (!grid_barrier(c, target, &sh_ok))
             return;
         // the decision, the same in every block; block 0 writes it down
         if (threadIdx.x < NCNT)
             sh_acc[threadIdx.x] = __ldcg(&c->lacc[a][threadIdx.x]);
-        if (sorting && threadIdx.x >= 32 && threadIdx.x < 34)
-            sh_far[threadIdx.x - 32] = __ldcg(threadIdx.x == 32 ? &c->lmin[a] : &c->lfar[a]);
+        if (sorting && threadIdx.x >= 32 && threadIdx.x < 35)
+            sh_far[threadIdx.x - 32] = threadIdx.x == 34 ? __ldcg(&c->lput[a]) : __ldcg(threadIdx.x == 32 ? &c->lmin[a] : &c->lfar[a]);
         __syncthreads();
         if (APP == WEDGE_APP_SSSP && threadIdx.x == 0) {
             if (sorting) { /* the waiting vertices are active too */
                 so.far_min = min(so.far_min, sh_far[0]);
                 so.waiting += sh_far[1];
+                so.held += sh_far[2]; /* from sums, as above: Ctrl::lf goes on counting while slower blocks read */
                 sh_acc[CNT_MASS] += so.waiting;
             }
             so.listed = sh_acc[CNT_MASS];
@@ -6100,6 +6138,15 @@ static int pr_loop_hub(wedge_graph* h)
     return WEDGE_OK;
 }
 
+// entries that a far list of sparse_loop_kernel takes: one per vertex (WEDGE_FAR_LIST: fewer, to test a full list)
+static uint32_t far_entries(uint64_t V)
+{
+    const char* e = getenv("WEDGE_FAR_LIST");
+    char* end = nullptr;
+    const uint64_t n = e ? strtoull(e, &end, 10) : 0u;
+    return (uint32_t)(n && end && *end == '\0' && n < V + 1 ? n : V + 1);
+}
+
 static int ensure_state(wedge_graph* h, int app, int precision)
 {
     if (h->built_app == app && (app != WEDGE_APP_PR || h->last_precision == precision))
@@ -6164,6 +6211,7 @@ static int ensure_state(wedge_graph* h, int app, int precision)
         s.front_stride = nwords;
         s.alist_stride = V + 1;
         s.item_stride = g.E / (LOOP_LONG / 2u) + 2;
+        s.far_cap = far_entries(V);
         const uint64_t build_items = V + g.E / PIECE + 2, loop_items = fused_loop(h) ? 2 * s.item_stride : 0;
         const uint64_t nitems = build_items > loop_items ? build_items : loop_items;
         if ((rc = dalloc(h, &s.front, 3 * nwords, true)) ||

@@ -127,7 +127,8 @@ struct Ctrl {
     unsigned int ln[3], li[3];         // vertices and items listed for it,
     unsigned long long lacc[3][NCNT];  // its counters; SSSP: the least distance it sorted out and by how many
     unsigned long long lmin[3], lfar[3]; // out-edges it changed the waiting ones; by far list modulo 3:
-    unsigned int lf[3];                // vertices listed
+    unsigned int lf[3];                // vertices listed; by step modulo 2: found by their far bits; by
+    unsigned int lall[2], lput[3];     // step modulo 3: listed in the far list at hand
     double pr_total;                   // sum of all accumulators (phase_vertex_pr.c:161); compensated FP32:
                                        // the total the next iteration uses
     double pr_prev;                    // compensated FP32: the total the last iteration used
@@ -226,7 +227,8 @@ struct DevState {
     uint32_t* alist;               // vertices the last pull activated: Wedge build, or two buffers alist_stride apart
     uint64_t alist_stride, item_stride;
     uint32_t* far;                 // V-bit, SSSP: changed vertices that wait (sparse_loop_kernel), and
-    uint32_t* far_list;            // two lists of them alist_stride apart
+    uint32_t* far_list;            // two lists of them alist_stride apart, of
+    uint32_t far_cap;              // entries
     uint32_t* cc_best;             // CC on a symmetric graph: least caller id of the component a label represents
     const uint32_t* cc_map;        // results only: CC labels are looked up here (engine ids not yet converted)
     Ctrl* ctrl;
