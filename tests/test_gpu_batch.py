@@ -8,7 +8,7 @@ import os
 import numpy as np
 import pytest
 
-from helpers import check_bfs_sorted, levels_from_parents
+from helpers import UNREACHED, check_bfs_sorted, levels_from_parents
 
 pytestmark = pytest.mark.gpu
 THREADS = os.cpu_count() or 8
@@ -116,3 +116,48 @@ def test_full_workload_64_graphs(W, O):
         _check(b, want)
     for g in graphs:
         g.close()
+
+
+@pytest.mark.parametrize("chunks", [0, 1])
+@pytest.mark.parametrize("own", [1, 127, 128, 129, 700])
+def test_batch_of_shards(W, monkeypatch, chunks, own):
+    """queries over destination-range shards: a vertex's out-degree is the whole
+    graph's, its out-list the shard's part of it (`own` of 40,000 edges here)"""
+    from helpers import check_bfs
+
+    monkeypatch.setenv("WEDGE_CSRI_CHUNKS", str(chunks))
+    rng = np.random.default_rng(own)
+    V = 2000
+    # the shard of destinations [0, 1000): 0 and `own` hubs point at them, the rest of their edges goes elsewhere
+    hubs = np.arange(1, 6)
+    s = np.concatenate([[0] * 5, np.repeat(hubs, own), rng.integers(0, 1000, 3000)])
+    d = np.concatenate([hubs, rng.integers(0, 1000, 5 * own), rng.integers(0, 1000, 3000)])
+    order = np.lexsort((s, d))
+    s, d = s[order].astype(np.uint32), d[order].astype(np.uint32)
+    w = rng.integers(1, 256, len(s)).astype(np.uint64)
+    outdeg = np.bincount(s, minlength=V).astype(np.uint64)
+    outdeg[:6] += 40_000
+    fw = (w.astype(np.float64) / 4.0).view(np.uint64)
+    with W.Graph.shard(V, s, d, outdeg, len(s) + 240_000, w) as g, \
+            W.Graph.shard(V, s, d, outdeg, len(s) + 240_000, fw, W.WEIGHTS_F64) as gf:
+        queries = [(i, app, root) for i in (0, 1) for app in (W.APP_SSSP, W.APP_BFS) for root in (0, 1, 500)]
+        with W.Batch([g, gf], queries) as b:
+            for threshold_pct in (1, 100):
+                b.run(W.BatchTuning(threshold_pct=threshold_pct))
+                for q, (i, app, root) in enumerate(queries):
+                    got = b.read_result(q)
+                    if app == W.APP_BFS:
+                        check_bfs(got, V, s, d, root)
+                        continue
+                    dist = np.full(V, np.inf)
+                    dist[root] = 0.0
+                    wt = fw.view(np.float64) if i else w.astype(np.float64)
+                    while True:  # exact: small whole numbers and quarters
+                        new = dist.copy()
+                        np.minimum.at(new, d, dist[s] + wt)
+                        if np.array_equal(new, dist):
+                            break
+                        dist = new
+                    none = np.isinf(dist)
+                    expect = dist.view(np.uint64) if i else np.where(none, UNREACHED, np.where(none, 0.0, dist).astype(np.uint64))
+                    assert np.array_equal(got, expect), (i, root, threshold_pct)

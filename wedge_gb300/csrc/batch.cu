@@ -69,6 +69,7 @@ struct BGraph {
     uint64_t V, E;
     uint32_t Vne, nchunks, weight_kind;
     uint32_t push;               // sparse pulls relax out-edges (CSRI of destinations)
+    uint32_t shard;              // outdeg are the whole graph's, longer than the out-lists
 };
 
 struct BQuery {
@@ -235,12 +236,19 @@ __device__ void phase_prefix(const BArgs& a)
 }
 
 // ---------------------------------------------------------------- pull
+// how many of vertex v's od out-edges the graph holds (a shard: those to its own destinations)
+__device__ __forceinline__ uint32_t list_length(const BGraph& G, uint32_t v, uint32_t od)
+{
+    return G.shard ? (uint32_t)(G.csri_off[v + 1u] - G.csri_off[v]) : od;
+}
+
 // vertex v of out-degree od into the next iteration's list, or its items; one lane
 __device__ __forceinline__ void list_one(const BQuery& qq, BCtl& c, const BGraph& G, uint32_t v, uint32_t od)
 {
     const uint32_t nx = (c.iter + 1u) % 3u, buf = (c.iter + 1u) & 1u;
-    if (G.push && od > PUSH_PIECE) {
-        const uint32_t np = (od + PUSH_PIECE - 1u) / PUSH_PIECE;
+    const uint32_t len = G.push ? list_length(G, v, od) : 0u;
+    if (len > PUSH_PIECE) {
+        const uint32_t np = (len + PUSH_PIECE - 1u) / PUSH_PIECE;
         const uint32_t at = atomicAdd(&c.nitem[nx], np);
         for (uint32_t j = 0; j < np; ++j)
             qq.items[buf][at + j] = make_uint2(v, j);
@@ -253,7 +261,7 @@ __device__ __forceinline__ void list_one(const BQuery& qq, BCtl& c, const BGraph
 __device__ __forceinline__ void list_warp(const BQuery& qq, BCtl& c, const BGraph& G, bool on, uint32_t v, uint32_t od)
 {
     const int lane = threadIdx.x & 31;
-    const bool shrt = on && od <= PUSH_PIECE;
+    const bool shrt = on && (od <= PUSH_PIECE || list_length(G, v, od) <= PUSH_PIECE);
     const uint32_t m = __ballot_sync(FULL, shrt);
     if (m) {
         uint32_t at = 0u;
@@ -1029,8 +1037,9 @@ __global__ void batch_seed_kernel(BArgs a)
             c.nitem[j] = 0u;
         }
         const uint32_t od = G.outdeg[r];
-        if (G.push && od > PUSH_PIECE) {
-            c.nitem[0] = (od + PUSH_PIECE - 1u) / PUSH_PIECE;
+        const uint32_t len = G.push ? list_length(G, r, od) : 0u;
+        if (len > PUSH_PIECE) {
+            c.nitem[0] = (len + PUSH_PIECE - 1u) / PUSH_PIECE;
             for (uint32_t j = 0; j < c.nitem[0]; ++j)
                 qq.items[0][j] = make_uint2(r, j);
         } else {
@@ -1213,6 +1222,7 @@ extern "C" int wedge_cuda_batch_create(wedge_graph_t* const* graphs, uint32_t nu
         G.cw8 = g.cw8;
         G.cw = g.cw;
         G.push = g.csr;
+        G.shard = g.shard;
         G.wsrc = g.csr ? g.wsrc : nullptr;
         G.ww8 = g.ww8;
         G.wo_src = g.wo_src;
