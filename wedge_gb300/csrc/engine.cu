@@ -2175,12 +2175,6 @@ struct WoStep {
     bool dropped;     // a sum past the limit would have lowered dist
 };
 
-// the weights that may lower a distance: below this
-__device__ __forceinline__ uint32_t sssp_wo_limit(uint32_t dist, uint32_t fmin)
-{
-    return dist > fmin ? dist - fmin : 0u;
-}
-
 __device__ __forceinline__ WoStep sssp_wo_step(const DevGraph& g, const DevState& s, const uint32_t* filter, uint32_t p,
                                                uint32_t lo, uint32_t hi, uint32_t fmin, uint32_t& dist, uint32_t& edges)
 {

@@ -283,6 +283,14 @@ __device__ __forceinline__ uint32_t pos_dst(const TileGeo<EPL>& tg, int i)
     return tg.k0 + tg.before + __popc(tg.nib_inner & ((2u << i) - 1u));
 }
 
+// The byte weights that may lower a 32-bit distance where no source is nearer
+// than fmin: below this.  An unreached destination (NONE32) takes every weight:
+// a sum past 32 bits does not lower it, but has to be seen (Ctrl::narrow_ovf).
+__host__ __device__ __forceinline__ uint32_t sssp_wo_limit(uint32_t dist, uint32_t fmin)
+{
+    return dist == NONE32 ? 256u : dist > fmin ? dist - fmin : 0u;
+}
+
 // (value, compensation) pair for the FP32 compensated PageRank sums
 struct F2 {
     float s, c;
