@@ -107,7 +107,8 @@ typedef struct wedge_params {
     double damping;           /* PageRank damping; 0 selects the reference's 0.875 (include/constants.h:39) */
     int32_t precision;        /* enum wedge_precision (PageRank only) */
     int32_t sched;            /* enum wedge_sched */
-    uint32_t max_iterations;  /* cap for BFS/CC/SSSP; 0 = |V| + 1 */
+    uint32_t max_iterations;  /* cap for BFS/CC/SSSP; 0 = |V| + 1, beside which a long SSSP may take iterations over
+                                 the nearest of its changed vertices alone (given a cap it takes none) */
     uint32_t flags;           /* WEDGE_FLAG_* */
     uint32_t probe_iter;      /* WEDGE_SCHED_PROBE: the iteration whose strategy is forced */
     int32_t probe_mode;       /* WEDGE_SCHED_PROBE: its enum wedge_mode */

@@ -408,3 +408,51 @@ def test_far_list_of_a_grid(engine_lib, monkeypatch, places):
         for flags in (0, W.FLAG_GRAPH):
             g.run(W.APP_SSSP, W.Params(flags=flags))
             assert np.array_equal(g.read_results(), expect), flags
+
+
+def rounds_of_all_changed(V, src, dst, w, root):
+    """distances, and the iterations in which every vertex changed by the last one relaxes its out-edges"""
+    dist = np.full(V, 1 << 62, np.int64)
+    dist[root] = 0
+    n = 0
+    while True:
+        new = dist.copy()
+        reached = dist[src] < 1 << 62
+        np.minimum.at(new, dst[reached], dist[src[reached]] + w[reached])
+        if np.array_equal(new, dist):
+            return np.where(dist >= 1 << 62, np.uint64(0xFFFFFFFFFFFFFFFF), dist.astype(np.uint64)), n
+        dist, n = new, n + 1
+
+
+@pytest.mark.parametrize("graph", ["grid", "steps"])
+def test_iteration_caps_of_long_sssp(engine_lib, graph):
+    """a cap that suffices when every changed vertex is visited at once suffices, and
+    one that does not is kept to; no cap is |V| + 1, which always suffices: "steps" is
+    a path whose shortcuts change nearly all vertices in nearly |V| iterations"""
+    W = engine_lib
+    rng = np.random.default_rng(3)
+    if graph == "grid":
+        side = 700
+        V = side * side
+        v = np.arange(V).reshape(side, side)
+        s = np.concatenate([v[:, :-1].ravel(), v[:, 1:].ravel(), v[:-1].ravel(), v[1:].ravel(), rng.integers(0, V, 9000)])
+        d = np.concatenate([v[:, 1:].ravel(), v[:, :-1].ravel(), v[1:].ravel(), v[:-1].ravel(), rng.integers(0, V, 9000)])
+        w = rng.integers(1, 100_000, len(s))
+    else:
+        V = 120
+        i, j = np.triu_indices(V, 1)
+        copies = 200  # 1.4 M edges, most of them parallel
+        s, d = np.repeat(i, copies), np.repeat(j, copies)
+        w = np.repeat(np.where(j == i + 1, 1, 300 * (j - i)), copies)
+    order = np.lexsort((s, d))
+    s, d, w = s[order], d[order], w[order].astype(np.int64)
+    expect, rounds = rounds_of_all_changed(V, s, d, w, 0)
+    with W.Graph.from_edges(V, s.astype(np.uint32), d.astype(np.uint32), w.astype(np.uint64)) as g:
+        for sched in (W.SCHED_PLAIN, W.SCHED_WEDGE):
+            for flags in (0, W.FLAG_GRAPH):
+                for cap in (0, rounds + 1):
+                    st = g.run(W.APP_SSSP, W.Params(sched=sched, flags=flags, max_iterations=cap))
+                    assert cap == 0 or st["iterations"] <= cap
+                    assert np.array_equal(g.read_results(), expect), (sched, flags, cap)
+                st = g.run(W.APP_SSSP, W.Params(sched=sched, flags=flags, max_iterations=30), allow_not_converged=True)
+                assert st["iterations"] == 30, (sched, flags)

@@ -3253,7 +3253,7 @@ __device__ __forceinline__ void decide_block(const DevGraph& g, DevState& s, Ctr
         // next pull is dense and 64-bit, and relaxes every in-edge again
         const bool redo = c->ovf_redo != 0u;
         c->ovf_redo = 0u;
-        const NextPull n = next_pull(c->sched, m, redo, c->iter, c->max_iter, c->threshold, c->probe_iter, c->probe_mode);
+        const NextPull n = next_pull(c->sched, m, redo, c->iter, c->max_iter + c->near_iters, c->threshold, c->probe_iter, c->probe_mode);
         if (n.done) {
             c->done = 1u;
             c->not_converged = n.capped ? 1u : 0u;
@@ -3652,7 +3652,8 @@ __global__ void init_kernel(DevGraph g, DevState s, uint32_t app, uint32_t topen
 // root activation (execution_bfs.c:110-117, execution_sssp.c:83-88) and the
 // control block
 __global__ void init_root_kernel(DevGraph g, DevState s, uint32_t app, uint64_t root_in, uint32_t sched,
-                                 unsigned long long thr, uint32_t max_iter, uint32_t probe_iter, uint32_t probe_mode)
+                                 unsigned long long thr, uint32_t max_iter, uint32_t probe_iter, uint32_t probe_mode,
+                                 uint32_t near_first)
 {
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t root = g.old2new[root_in]; /* the caller's id -> relabelled id */
@@ -3683,6 +3684,8 @@ __global__ void init_root_kernel(DevGraph g, DevState s, uint32_t app, uint64_t 
         c->done = 0;
         c->not_converged = 0;
         c->max_iter = max_iter;
+        c->near_first = near_first;
+        c->near_iters = 0;
         c->sched = sched;
         c->parity = 0;
         c->loop = 1;
@@ -3766,6 +3769,12 @@ __global__ void init_root_kernel(DevGraph g, DevState s, uint32_t app, uint64_t 
 // one list and iteration a vertex that changes several times, far and near in
 // turn, can still leave more entries than one.  What a list has no room for is
 // found by its bits.
+//
+// Sorting out takes more iterations than visiting every changed vertex at once
+// (4096^2 grid: 160 to 300 for 158), so a run whose caller gave a cap does without
+// it.  With the default cap, |V| + 1, the iterations that left vertices waiting
+// are not counted, up to as many again: in the others every vertex that changed
+// since it was last visited is, so |V| of them suffice as ever.
 //
 // Graphs of at most LOOP_SMALL_EDGES in-edges run whole in the launch: there a
 // dense iteration is no more work than a Wedge one, and the launches were all
@@ -3865,8 +3874,10 @@ struct LoopBook {
     }
 
     // into the control block: before another launch or block reads it
-    __device__ void close(Ctrl* c, unsigned long long mass, unsigned long long act, const NextPull& next, uint32_t iter, uint32_t parity) const
+    __device__ void close(Ctrl* c, unsigned long long mass, unsigned long long act, const NextPull& next, uint32_t iter, uint32_t parity,
+                          uint32_t extra) const
     {
+        c->near_iters = extra;
         c->edges_scanned = edges;
         c->dsts_scanned = dsts;
         c->activated = activated;
@@ -3905,6 +3916,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
         uint32_t release, nfar;                             /* far lists begun; vertices of the one whose turn it is */
         uint32_t begun, overrun;                            /* this iteration begins one; that one did not hold all */
         unsigned long long held;                            /* entries of the present one */
+        uint32_t from, extra;                               /* the first iteration that sorts out; how many did */
     } so;
     __shared__ unsigned long long sh_far[3];
     __shared__ uint32_t sh_least;
@@ -3943,6 +3955,8 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
         so.release = 0u;
         so.nfar = 0u;
         so.held = 0ull;
+        so.from = c->near_first ? NEAR_ITER : NONE32;
+        so.extra = c->near_iters;
     }
     uint32_t* out_list = s.alist;
     uint2* out_items = s.items;
@@ -4075,7 +4089,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
         __syncthreads();
         const uint32_t n = sh_n[0], ni = sh_n[1];
         /* from one iteration before distances may be sorted out: that one finds the least */
-        const bool sorting = APP == WEDGE_APP_SSSP && iter + 1u >= NEAR_ITER && (so.waiting != 0ull || so.listed > NEAR_MASS / 4u);
+        const bool sorting = APP == WEDGE_APP_SSSP && iter + 1u >= so.from && (so.waiting != 0ull || so.listed > NEAR_MASS / 4u);
         if (APP == WEDGE_APP_SSSP && !sorting && threadIdx.x == 0)
             so.far_min = NONE64;
         if (sorting) {
@@ -4086,7 +4100,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
                             : from + (unsigned long long)(NEAR_STEP * g.wmean);
                     return max(from, to);
                 };
-                const bool now = iter >= NEAR_ITER && mode == MODE_WEDGE && so.listed > NEAR_MASS;
+                const bool now = iter >= NEAR_ITER && mode == MODE_WEDGE && so.listed > NEAR_MASS && so.extra < max_iter;
                 if (!now)
                     so.bound = NONE64; /* every vertex is near */
                 so.nfar = so.begun = so.overrun = 0u;
@@ -4109,6 +4123,8 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
                     ++so.release;
                     so.held = 0ull;
                 }
+                if (so.bound != NONE64 || so.nfar != 0u)
+                    ++so.extra;
             }
             __syncthreads();
             if (so.overrun) { /* the list anew, from the waiting vertices' bits */
@@ -4526,13 +4542,15 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
 #pragma unroll
         for (uint32_t j = 0; j < NCNT; ++j)
             cnt[j] = sh_acc[j];
-        const NextPull next = next_pull(sched, cnt[CNT_MASS], false, iter + 1u, max_iter, thr, probe_iter, probe_mode);
+        const NextPull next = next_pull(sched, cnt[CNT_MASS], false, iter + 1u,
+                                        APP == WEDGE_APP_SSSP ? max_iter + so.extra : max_iter, thr, probe_iter, probe_mode);
         const bool pull_next = !(sorting && so.release + so.waiting != 0ull) && heavy(cnt[CNT_MASS], cnt[CNT_ACT]);
         if (scribe)
             book.note(g, s, (uint32_t)APP, cnt, next, mode, iter);
         if (scribe && (next.done || step + 1u == max_steps || (!small && next.mode != MODE_WEDGE) || pull_next ||
                        sched == WEDGE_SCHED_LEARNED))
-            book.close(c, cnt[CNT_MASS], cnt[CNT_ACT], next, iter + 1u, (parity + 1u) % 3u);
+            book.close(c, cnt[CNT_MASS], cnt[CNT_ACT], next, iter + 1u, (parity + 1u) % 3u,
+                       APP == WEDGE_APP_SSSP ? so.extra : 0u);
         if (!next.done && sched == WEDGE_SCHED_LEARNED && s.net && blockIdx.x + 1u == gridDim.x)
             ask_network(s, c, (uint32_t)APP, iter + 1u);
         mode = next.mode;
@@ -6433,14 +6451,15 @@ static void launch_tail(wedge_graph* h, int app)
 }
 
 static void launch_init(wedge_graph* h, int app, uint64_t root, uint32_t sched, unsigned long long thr, uint32_t max_iter,
-                        uint32_t probe_iter = 0xFFFFFFFFu, uint32_t probe_mode = MODE_DENSE, bool build = true)
+                        uint32_t probe_iter = 0xFFFFFFFFu, uint32_t probe_mode = MODE_DENSE, bool build = true,
+                        bool near_first = false)
 {
     const uint64_t work = h->g.V > h->g.T ? h->g.V : h->g.T;
     const uint32_t tile_e = pull_tile_e(h, app);
     const uint32_t topen = (uint32_t)((h->g.E + tile_e - 1) / tile_e); /* pull tiles holding in-edges */
     init_kernel<<<aux_grid(h, work), AUX_THREADS, 0, h->stream>>>(h->g, h->s, (uint32_t)app, topen);
     init_root_kernel<<<1, 32, 0, h->stream>>>(h->g, h->s, (uint32_t)app, root, sched, thr,
-                                                                           max_iter, probe_iter, probe_mode);
+                                                                           max_iter, probe_iter, probe_mode, near_first ? 1u : 0u);
     h->cc_pending = (app == WEDGE_APP_CC && h->s.cc_best) ? 1 : 0;
     if (build)
         launch_wedge_build(h, h->g, app); /* collect_kernel clears the bitmaps for the first pull */
@@ -6595,7 +6614,8 @@ static int run_traversal(wedge_graph* h, int app, const wedge_params_t* p, wedge
             return rc;
     }
     WEDGE_CHECK(cudaEventRecord(h->ev[0], h->stream));
-    launch_init(h, app, root, (uint32_t)p->sched, thr, (uint32_t)cap, p->probe_iter, (uint32_t)p->probe_mode, !fused);
+    launch_init(h, app, root, (uint32_t)p->sched, thr, (uint32_t)cap, p->probe_iter, (uint32_t)p->probe_mode, !fused,
+                p->max_iterations == 0u);
     launches += 2ull + (fused ? 0ull : build_launches(h)); /* init, root, the Wedge build */
     Ctrl c;
     if (one) {

@@ -104,6 +104,8 @@ struct Ctrl {
     unsigned int done;                 // traversal finished
     unsigned int not_converged;        // iteration cap reached
     unsigned int max_iter;
+    unsigned int near_first;           // SSSP: far vertices may wait (sparse_loop_kernel); iterations
+    unsigned int near_iters;           // in which some did, beyond max_iter
     unsigned int sched;                // enum wedge_sched
     unsigned int parity;               // which of the three frontier bitmaps the next pull reads
     unsigned int loop;                 // 1 while the traversal continues (CUDA-graph loop condition)
