@@ -161,3 +161,31 @@ def test_batch_of_shards(W, monkeypatch, chunks, own):
                     none = np.isinf(dist)
                     expect = dist.view(np.uint64) if i else np.where(none, UNREACHED, np.where(none, 0.0, dist).astype(np.uint64))
                     assert np.array_equal(got, expect), (i, root, threshold_pct)
+
+
+def test_failed_read_leaves_the_buffer(W):
+    """no device memory for the staging of a result: the call says so, and the
+    caller's buffer is as it was; with memory again it is read"""
+    import ctypes
+
+    import torch
+
+    with W.Graph.rmat(22, 1, 3) as g, W.Batch([g], [(0, W.APP_BFS, 0)]) as b:
+        b.run()
+        out = np.full(g.V, 0xABABABABABABABAB, np.uint64)
+        held = []
+        for size in (1 << 30, 1 << 27, 1 << 25):  # the staging takes 32 MB
+            try:
+                while True:
+                    held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+            except torch.OutOfMemoryError:
+                pass
+        read = lambda: W.lib().wedge_cuda_batch_read_result(  # noqa: E731
+            b._h, 0, out.ctypes.data_as(ctypes.c_void_p), ctypes.c_uint64(out.nbytes))
+        rc = read()
+        held.clear()
+        torch.cuda.empty_cache()
+        assert rc != 0 and np.all(out == 0xABABABABABABABAB)
+        assert read() == 0
+        g.run(W.APP_BFS)
+        assert np.array_equal(out == UNREACHED, g.read_results() == UNREACHED)

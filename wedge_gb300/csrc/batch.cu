@@ -1484,7 +1484,6 @@ extern "C" int wedge_cuda_batch_read_result(wedge_batch_t* b, uint32_t query, vo
     if (bytes < 8ull * G.V)
         return WEDGE_ERR_ARG;
     WEDGE_CHECK(cudaSetDevice(b->device));
-    touch_pages(host_props, 8ull * G.V);
     cudaError_t e = cudaSuccess;
     pthread_mutex_lock(&b->xlock);
     if (!b->xbuf) /* kept: an allocation and its release took 180 of a small read's 200 us */
@@ -1493,8 +1492,10 @@ extern "C" int wedge_cuda_batch_read_result(wedge_batch_t* b, uint32_t query, vo
         batch_export_kernel<<<bgrid(G.V, 256, (uint32_t)b->num_sms * 8), 256, 0, b->stream>>>(G, q, b->xbuf);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess)
+    if (e == cudaSuccess) { /* a call that fails leaves the caller's buffer as it is; the pages while the kernel runs */
+        touch_pages(host_props, 8ull * G.V);
         e = cudaMemcpyAsync(host_props, b->xbuf, 8ull * G.V, cudaMemcpyDeviceToHost, b->stream);
+    }
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(b->stream);
     pthread_mutex_unlock(&b->xlock);

@@ -37,8 +37,10 @@ int compute_grids(wedge_graph* h);
 
 int cuda_status(cudaError_t e)
 {
-    if (e == cudaErrorMemoryAllocation)
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError(); /* reported here: the next call's check of its launches is not to find it */
         return WEDGE_ERR_OOM;
+    }
     return WEDGE_ERR_CUDA;
 }
 
