@@ -456,3 +456,55 @@ def test_iteration_caps_of_long_sssp(engine_lib, graph):
                     assert np.array_equal(g.read_results(), expect), (sched, flags, cap)
                 st = g.run(W.APP_SSSP, W.Params(sched=sched, flags=flags, max_iterations=30), allow_not_converged=True)
                 assert st["iterations"] == 30, (sched, flags)
+
+
+@pytest.mark.parametrize("weights", ["none", "bytes", "f64"])
+def test_loads_with_little_memory(engine_lib, weights):
+    """a load takes the optional copies of the in-edges and the out-edges' arrays only
+    where they fit: it succeeds from what the sort of the in-edges needs (the edges
+    and their sort keys, twice, and the vertices' arrays), and says so below it"""
+    import torch
+
+    W = engine_lib
+    rng = np.random.default_rng(1)
+    V, n = 1 << 20, (1 << 23) - 5000
+    s = np.minimum((V * rng.random(n) ** 2).astype(np.int64), V - 1)
+    d = np.sort(np.minimum((V * rng.random(n) ** 3).astype(np.int64), V - 1))
+    s[:2], d[:2] = (0, 1), (0, 0)
+    s, d = s.astype(np.uint32), d.astype(np.uint32)
+    args, app, per_edge = (), W.APP_BFS, 24
+    if weights == "bytes":
+        args, app, per_edge = (rng.integers(0, 256, n).astype(np.uint64),), W.APP_SSSP, 40
+    elif weights == "f64":
+        args, app, per_edge = (rng.random(n).view(np.uint64), W.WEIGHTS_F64), W.APP_SSSP, 40
+    root = int(s[n // 2])
+    need = per_edge * n + 64 * V + (48 << 20)
+    expect = None
+    outcomes = []
+    for room in (need + (1 << 30), need + (96 << 20), need + (48 << 20), need, need // 2, need // 8):
+        torch.cuda.empty_cache()
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        held = torch.empty(free - room, dtype=torch.uint8, device="cuda")
+        try:
+            g = W.Graph.from_edges(V, s, d, *args)
+        except W.WedgeError as e:
+            outcomes.append((room, e.status))
+            g = None
+        del held
+        torch.cuda.empty_cache()
+        if g is not None:
+            with g:
+                g.run(app, W.Params(root=root))
+                got = g.read_results()
+                outcomes.append((room, 0))
+            if expect is None:
+                expect = got
+            if app == W.APP_BFS:  # parents may be others: the same vertices are reached
+                got, expect = got == np.uint64(0xFFFFFFFFFFFFFFFF), expect == np.uint64(0xFFFFFFFFFFFFFFFF) \
+                    if expect.dtype == np.uint64 else expect
+            assert np.array_equal(got, expect), room
+    assert [rc for room, rc in outcomes if room >= need] == [0] * 4, outcomes
+    assert outcomes[-1][1] == W.engine.ERR_OOM, outcomes
+    with W.Graph.from_edges(V, s, d, *args) as g:  # nothing of the failed loads is left
+        g.run(app, W.Params(root=root))

@@ -87,6 +87,18 @@ static void untrack(wedge_graph* h, void* p)
             h->allocs[i] = h->allocs[--h->nallocs];
 }
 
+// gives an array of the handle back (cudaFree waits for the kernels that use it); one of the slab stays there
+template <class T>
+static void give_back(wedge_graph* h, T** p)
+{
+    unsigned char* at = (unsigned char*)*p;
+    if (at && !(h->slab && at >= h->slab && at < h->slab + h->slab_size)) {
+        untrack(h, at);
+        cudaFree(at);
+    }
+    *p = nullptr;
+}
+
 static int track_state(wedge_graph* h, void* p)
 {
     if (h->nstate >= (int)(sizeof(h->state_allocs) / sizeof(h->state_allocs[0])))
@@ -618,8 +630,11 @@ static bool csri_chunks(uint64_t Epad)
 // out-edges: every source's destinations (*csri) and weights (*cw8 or *cw);
 // with radix passes over the source bits alone that is 3-4 passes, where
 // filling them through atomic cursors took as long as nine (R-MAT scale 24).
+// Where the sort of the in-edges fits but these arrays beside its keys do not
+// (12 bytes per in-edge with 64-bit weights), *csri stays null and the graph
+// takes the chunk form; 64-bit words that bytes replace are freed before.
 static int relabel_by_degree(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_src, uint32_t* d_dst,
-                             unsigned long long* d_w, bool byte_weights, uint32_t** new2old, uint32_t** old2new,
+                             unsigned long long*& d_w, bool byte_weights, uint32_t** new2old, uint32_t** old2new,
                              uint8_t** w8, uint32_t** wsrc, uint8_t** ww8, uint32_t** csri, uint8_t** cw8,
                              unsigned long long** cw, uint32_t* outdeg, const uint32_t* global_outdeg)
 {
@@ -699,43 +714,66 @@ static int relabel_by_degree(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d
         WEDGE_CHECK(cudaMemsetAsync(*w8 + E, 0, Epad - E, st));
     tfree(h, tmp);
     trelease(h, sort_mark);
-    if (in_key && !global_outdeg && Epad < (1ull << 32)) { /* 32-bit in-edge positions */
-        if (dalloc(h, wsrc, Epad) == WEDGE_OK && dalloc(h, ww8, Epad) == WEDGE_OK) {
-            weight_key_kernel<<<grid, AUX_THREADS, 0, st>>>(kb.Current(), E, vbits);
-            WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(nullptr, tb, kb, (long long)E, vbits, 2 * vbits + 8, st));
-            WEDGE_CHECK(talloc(h, &tmp, tb));
-            WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tb, kb, (long long)E, vbits, 2 * vbits + 8, st));
-            tfree(h, tmp);
-            trelease(h, sort_mark);
-            weight_unpack_kernel<<<grid_for(Epad, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(kb.Current(), E, Epad, vbits,
-                                                                                         *wsrc, *ww8);
+    if (in_key)
+        give_back(h, &d_w); /* the bytes are read from here on */
+    /* the arrays the out-edges need, and a sort's work space, before the optional weight order */
+    bool csr = !csri_chunks(Epad);
+    void* work = nullptr;
+    if (csr) {
+        cub::DoubleBuffer<unsigned long long> vb(w2, w2);
+        WEDGE_CHECK(d_w ? cub::DeviceRadixSort::SortPairs(nullptr, tb, kb, vb, (long long)E, 0, vbits, st)
+                        : cub::DeviceRadixSort::SortKeys(nullptr, tb, kb, (long long)E, 0, vbits + 8, st)); /* the longer of two */
+        rc = dalloc(h, csri, E);
+        if (!rc && in_key)
+            rc = dalloc(h, cw8, E);
+        if (!rc && d_w)
+            rc = dalloc(h, cw, E);
+        const cudaError_t e = rc ? cudaSuccess : talloc(h, &work, tb);
+        if (rc == WEDGE_ERR_OOM || e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            give_back(h, csri);
+            give_back(h, cw8);
+            give_back(h, cw);
+            csr = false;
+        } else if (rc) {
+            return rc;
         } else {
-            cudaGetLastError(); /* no room: the SSSP pulls go without (one of the two stays the handle's, unused) */
-            *wsrc = nullptr;
-            *ww8 = nullptr;
+            WEDGE_CHECK(e);
         }
     }
-    if (!csri_chunks(Epad)) {
-        if ((rc = dalloc(h, csri, E)) || (in_key && (rc = dalloc(h, cw8, E))) || (d_w && !in_key && (rc = dalloc(h, cw, E))))
+    bool by_weight = false; /* the keys are destination | weight | source */
+    if (csr && in_key && !global_outdeg) {
+        rc = dalloc(h, wsrc, Epad);
+        if (!rc)
+            rc = dalloc(h, ww8, Epad);
+        if (rc == WEDGE_ERR_OOM) { /* no room: the SSSP pulls go without */
+            give_back(h, wsrc);
+            give_back(h, ww8);
+        } else if (rc) {
             return rc;
+        } else {
+            by_weight = true;
+            weight_key_kernel<<<grid, AUX_THREADS, 0, st>>>(kb.Current(), E, vbits);
+            WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(work, tb, kb, (long long)E, vbits, 2 * vbits + 8, st));
+            weight_unpack_kernel<<<grid_for(Epad, AUX_THREADS, cap), AUX_THREADS, 0, st>>>(kb.Current(), E, Epad, vbits,
+                                                                                         *wsrc, *ww8);
+        }
+    }
+    if (csr) {
         /* the keys hold the source in bits [0, vbits) after the weight order, else above the weight byte */
-        const int s0 = (in_key && !*wsrc) ? 8 : 0;
+        const int s0 = (in_key && !by_weight) ? 8 : 0;
         const int shift = in_key ? vbits + 8 : vbits;
-        const int wshift = *wsrc ? vbits : 0;
-        if (d_w && !in_key) {
+        const int wshift = by_weight ? vbits : 0;
+        if (d_w) {
             WEDGE_CHECK(cudaMemcpyAsync(*cw, d_w, E * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, st));
             cub::DoubleBuffer<unsigned long long> vb(*cw, w2);
-            WEDGE_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, tb, kb, vb, (long long)E, s0, s0 + vbits, st));
-            WEDGE_CHECK(talloc(h, &tmp, tb));
-            WEDGE_CHECK(cub::DeviceRadixSort::SortPairs(tmp, tb, kb, vb, (long long)E, s0, s0 + vbits, st));
+            WEDGE_CHECK(cub::DeviceRadixSort::SortPairs(work, tb, kb, vb, (long long)E, s0, s0 + vbits, st));
             if (vb.Current() != *cw)
                 WEDGE_CHECK(cudaMemcpyAsync(*cw, vb.Current(), E * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, st));
         } else {
-            WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(nullptr, tb, kb, (long long)E, s0, s0 + vbits, st));
-            WEDGE_CHECK(talloc(h, &tmp, tb));
-            WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tb, kb, (long long)E, s0, s0 + vbits, st));
+            WEDGE_CHECK(cub::DeviceRadixSort::SortKeys(work, tb, kb, (long long)E, s0, s0 + vbits, st));
         }
-        tfree(h, tmp);
+        tfree(h, work);
         csr_unpack_kernel<<<grid, AUX_THREADS, 0, st>>>(kb.Current(), E, shift, wshift, *csri, *cw8);
     }
     tfree(h, ek);
@@ -788,6 +826,9 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
         if (cudaMalloc((void**)&h->tscratch, h->tsize) != cudaSuccess) {
             cudaGetLastError();
             h->tscratch = nullptr;
+            unsigned char* slab = h->slab; /* arrays that come later are not to take the sort's memory */
+            h->slab = nullptr;
+            give_back(h, &slab);
         }
     }
 
@@ -830,11 +871,8 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
         g.cw = cw;
         g.new2old = n2o;
         g.old2new = o2n;
-        if (w8) { /* the 64-bit words are not read any more */
-            WEDGE_CHECK(cudaStreamSynchronize(st));
-            untrack(h, d_w);
-            cudaFree(d_w);
-            g.w = d_w = nullptr;
+        if (w8) {
+            g.w = nullptr; /* relabel_by_degree gave them back */
         } else if (byte_weights) {
             if ((rc = dalloc(h, &w8, g.Epad)))
                 return rc;
@@ -861,7 +899,7 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
     g.Vne = Vne;
     uint32_t *dst_id, *tile_dst0;
     unsigned long long *dst_off, *csri_off;
-    const bool chunks = csri_chunks(g.Epad);
+    const bool chunks = csri_chunks(g.Epad) || (E && !csri); /* or the out-edges' arrays did not fit */
     int rc;
     if ((rc = dalloc(h, &dst_id, Vne)) || (rc = dalloc(h, &dst_off, (uint64_t)Vne + 1)) ||
         (rc = dalloc(h, &tile_dst0, (uint64_t)g.T + 1)) || (rc = dalloc(h, &csri_off, V + 1)) ||
@@ -941,7 +979,11 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
             g.wo_src = wo_src;
             g.wo_w = wo_w;
         } else {
-            cudaGetLastError(); /* no room, as above */
+            uint32_t* wsrc = const_cast<uint32_t*>(g.wsrc);
+            uint8_t* ww8 = const_cast<uint8_t*>(g.ww8);
+            give_back(h, &wsrc); /* no room, as above */
+            give_back(h, &ww8);
+            give_back(h, &wo_src);
             g.wsrc = nullptr;
             g.ww8 = nullptr;
         }
