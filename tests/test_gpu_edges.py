@@ -508,3 +508,29 @@ def test_loads_with_little_memory(engine_lib, weights):
     assert outcomes[-1][1] == W.engine.ERR_OOM, outcomes
     with W.Graph.from_edges(V, s, d, *args) as g:  # nothing of the failed loads is left
         g.run(app, W.Params(root=root))
+
+
+@pytest.mark.parametrize("symmetric", [False, True])
+@pytest.mark.parametrize("n", [900, 40_000])
+def test_asked_strategies_of_small_graphs(engine_lib, n, symmetric):
+    """a strategy that a caller asks for is the one that runs, on a graph of any size
+    (dense pulls are launches of their own, Wedge iterations share one), and the
+    results are the plain rule's"""
+    W = engine_lib
+    rng = np.random.default_rng(n)
+    V = n // 2
+    s, d = rng.integers(0, V, n), (V * rng.random(n) ** 2).astype(np.int64)
+    if symmetric:
+        s, d = np.concatenate([s, d]), np.concatenate([d, s])
+    order = np.lexsort((s, d))
+    s, d = s[order].astype(np.uint32), d[order].astype(np.uint32)
+    w = rng.integers(0, 256, len(s)).astype(np.uint64)
+    check_traversals(W, V, s, d, w, (W.SCHED_PLAIN, W.SCHED_DENSE, W.SCHED_WEDGE, W.SCHED_FILTERED), (0, W.FLAG_GRAPH))
+    with W.Graph.from_edges(V, s, d, w) as g:
+        for app in (W.APP_BFS, W.APP_CC, W.APP_SSSP):
+            launches = {}
+            for sched in (W.SCHED_PLAIN, W.SCHED_DENSE, W.SCHED_FILTERED):
+                st = g.run(app, W.Params(sched=sched, flags=W.FLAG_GRAPH))
+                launches[sched] = st["kernel_launches"]
+            # preparation (2), the loop, CC's labels (2); else a dense iteration's pulls and decision as well
+            assert launches[W.SCHED_PLAIN] <= 5 < min(launches[W.SCHED_DENSE], launches[W.SCHED_FILTERED]), launches

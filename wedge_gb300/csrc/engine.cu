@@ -3820,9 +3820,10 @@ __global__ void init_root_kernel(DevGraph g, DevState s, uint32_t app, uint64_t 
 // are not counted, up to as many again: in the others every vertex that changed
 // since it was last visited is, so |V| of them suffice as ever.
 //
-// Graphs of at most LOOP_SMALL_EDGES in-edges run whole in the launch: there a
-// dense iteration is no more work than a Wedge one, and the launches were all
-// the time (BFS at scale 12: 182 us).
+// Graphs of at most LOOP_SMALL_EDGES in-edges run whole in the launch under the
+// plain rule: there a dense iteration is no more work than a Wedge one, and the
+// launches were all the time (BFS at scale 12: 182 us).  A caller that asks for a
+// strategy, or for the network's choice of one, gets that strategy's kernels.
 constexpr uint32_t LOOP_LONG = 128;   // out-edges of one vertex a warp takes at once: one round of four per lane
 constexpr uint32_t LOOP_BUF = 96;     // listed vertices a warp keeps in shared memory (each list)
 constexpr unsigned long long NEAR_MASS = 1ull << 16;
@@ -6456,11 +6457,11 @@ static void launch_decide(wedge_graph* h, int app, bool fused, bool captured = f
 
 // whole traversals in one launch up to this many in-edges
 constexpr uint64_t LOOP_SMALL_EDGES = 1ull << 20;
-static bool small_loop(const wedge_graph* h) { return h->g.E <= LOOP_SMALL_EDGES; }
+static bool small_loop(const wedge_graph* h, int sched) { return h->g.E <= LOOP_SMALL_EDGES && sched == WEDGE_SCHED_PLAIN; }
 
 // one block per SM, fewer on graphs that leave most of them without work (a
 // barrier of few blocks is faster)
-static int launch_sparse_loop(wedge_graph* h, int app, uint32_t max_steps)
+static int launch_sparse_loop(wedge_graph* h, int app, bool whole, uint32_t max_steps)
 {
     const uint64_t want = h->g.E / 2048u + 8u;
     cudaLaunchConfig_t cfg = {};
@@ -6472,7 +6473,7 @@ static int launch_sparse_loop(wedge_graph* h, int app, uint32_t max_steps)
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    const uint32_t small = small_loop(h) ? 1u : 0u;
+    const uint32_t small = whole ? 1u : 0u;
     switch (app) {
     case WEDGE_APP_BFS:
         WEDGE_CHECK(cudaLaunchKernelEx(&cfg, sparse_loop_kernel<WEDGE_APP_BFS>, h->g, h->s, small, max_steps));
@@ -6577,7 +6578,7 @@ static int build_graph(wedge_graph* h, int app)
     WEDGE_CHECK(cudaStreamBeginCaptureToGraph(h->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
     int rc = WEDGE_OK;
     if (fused_loop(h)) { /* Wedge iterations, a dense pull, the decision and the loop condition */
-        rc = launch_sparse_loop(h, app, 0xFFFFFFFFu);
+        rc = launch_sparse_loop(h, app, false, 0xFFFFFFFFu);
         launch_pull(h, app);
         launch_decide(h, app, true, true, handle);
     } else {
@@ -6648,7 +6649,8 @@ static int run_traversal(wedge_graph* h, int app, const wedge_params_t* p, wedge
         cap = 0x7fffffffull;
     const bool timing = (p->flags & WEDGE_FLAG_TIMING) != 0;
     const bool fused = fused_loop(h);
-    const bool one = fused && small_loop(h) && !timing; /* the whole traversal in one launch */
+    const bool small = fused && small_loop(h, p->sched);
+    const bool one = small && !timing; /* the whole traversal in one launch */
     const bool use_graph = (p->flags & WEDGE_FLAG_GRAPH) != 0 && !timing && !one;
     uint64_t launches = 0;
     double t_pull_dense = 0, t_pull_wedge = 0, t_wedge = 0;
@@ -6663,7 +6665,7 @@ static int run_traversal(wedge_graph* h, int app, const wedge_params_t* p, wedge
     launches += 2ull + (fused ? 0ull : build_launches(h)); /* init, root, the Wedge build */
     Ctrl c;
     if (one) {
-        int rc = launch_sparse_loop(h, app, 0xFFFFFFFFu);
+        int rc = launch_sparse_loop(h, app, true, 0xFFFFFFFFu);
         if (rc)
             return rc;
         launches += 1ull;
@@ -6677,9 +6679,9 @@ static int run_traversal(wedge_graph* h, int app, const wedge_params_t* p, wedge
             if (c.done)
                 break;
             const uint32_t mode = c.mode;
-            const bool sparse = fused && (mode == MODE_WEDGE || small_loop(h));
+            const bool sparse = fused && (mode == MODE_WEDGE || small);
             WEDGE_CHECK(cudaEventRecord(h->ev[2], h->stream));
-            if (fused && (rc = launch_sparse_loop(h, app, 1u))) /* one Wedge iteration, or the bitmaps' clearing */
+            if (fused && (rc = launch_sparse_loop(h, app, small, 1u))) /* one Wedge iteration, or the bitmaps' clearing */
                 return rc;
             if (!sparse)
                 launch_pull(h, app);
@@ -6711,7 +6713,7 @@ static int run_traversal(wedge_graph* h, int app, const wedge_params_t* p, wedge
         for (;;) {
             for (int b = 0; b < 3; ++b) {
                 if (fused) {
-                    int rc = launch_sparse_loop(h, app, 0xFFFFFFFFu);
+                    int rc = launch_sparse_loop(h, app, false, 0xFFFFFFFFu);
                     if (rc)
                         return rc;
                 }
