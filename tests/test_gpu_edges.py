@@ -534,3 +534,26 @@ def test_asked_strategies_of_small_graphs(engine_lib, n, symmetric):
                 launches[sched] = st["kernel_launches"]
             # preparation (2), the loop, CC's labels (2); else a dense iteration's pulls and decision as well
             assert launches[W.SCHED_PLAIN] <= 5 < min(launches[W.SCHED_DENSE], launches[W.SCHED_FILTERED]), launches
+
+
+@pytest.mark.parametrize("n", [100_000, 300_001])
+def test_log_says_which_pulls_ran(engine_lib, n):
+    """the iterations' log of timed, captured and host-driven runs: a frontier too large
+    for its out-edges one by one is a dense pull in all of them, and reads as one"""
+    W = engine_lib
+    rng = np.random.default_rng(n)
+    V = 2 * n + 1001
+    s = np.concatenate([np.zeros(n, np.int64), np.arange(1, n + 1), 2 * n + 1 + rng.integers(0, 1000, 3_000_000)])
+    d = np.concatenate([np.arange(1, n + 1), n + 1 + rng.permutation(n), 2 * n + 1 + rng.integers(0, 1000, 3_000_000)])
+    order = np.lexsort((s, d))
+    with W.Graph.from_edges(V, s[order].astype(np.uint32), d[order].astype(np.uint32)) as g:
+        logs = []
+        for flags in (0, W.FLAG_GRAPH, W.FLAG_TIMING):
+            st = g.run(W.APP_BFS, W.Params(root=0, flags=flags))
+            log = g.iteration_log()
+            assert [r["mode"] for r in log] == [W.MODE_WEDGE, W.MODE_DENSE if n > 200_000 else W.MODE_WEDGE]
+            assert st["wedge_iterations"] == sum(r["used_wedge"] for r in log) == sum(r["mode"] == W.MODE_WEDGE for r in log)
+            logs.append([(r["mode"], r["active_edges"], r["changed_mass"], r["vertices_activated"]) for r in log])
+            if flags == W.FLAG_TIMING:
+                assert all(r["pull_ms"] > 0.0 for r in log)
+        assert logs[0] == logs[1] == logs[2]

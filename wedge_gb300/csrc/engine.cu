@@ -1283,7 +1283,7 @@ __device__ __forceinline__ void dist32_put(const DevState& s, uint32_t v, unsign
 // the weight-ordered kernels run this pull: dense and filtered pulls while every distance fits the 32-bit copy
 __device__ __forceinline__ bool sssp_wo_runs(const DevState& s, const Ctrl* c)
 {
-    return s.wo && (c->mode != MODE_WEDGE || c->heavy) && !c->narrow_ovf;
+    return s.wo && c->mode != MODE_WEDGE && !c->narrow_ovf;
 }
 
 // The Wedge pull of SSSP over the out-edges: every vertex the last pull
@@ -1426,7 +1426,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
     Ctrl* c = s.ctrl;
     if (c->done)
         return;
-    const uint32_t mode = c->mode == MODE_WEDGE && c->heavy ? (uint32_t)MODE_DENSE : c->mode;
+    const uint32_t mode = c->mode;
     if (phase == PHASE_REST && mode == MODE_WEDGE) {
         // a Wedge pull runs whole in the first launch: this one only reports zeros
         if (threadIdx.x < NCNT)
@@ -2544,7 +2544,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
     Ctrl* c = s.ctrl;
     if (c->done)
         return;
-    const uint32_t mode = c->mode == MODE_WEDGE && c->heavy ? (uint32_t)MODE_DENSE : c->mode;
+    const uint32_t mode = c->mode;
     // CC on a symmetric graph propagates engine ids; before its first pull every
     // label is its vertex's own id
     const bool ident0 = APP == WEDGE_APP_CC && g.sym != 0u && c->iter == 0u;
@@ -3088,9 +3088,34 @@ __global__ void __launch_bounds__(PULL_THREADS, 2)
     }
 }
 
+// The loops whose Wedge iterations sparse_loop_kernel runs take a dense pull
+// below the threshold too, where it is cheaper than the frontier's out-edges.
+// SSSP: more than HEAVY_SSSP out-edges per destination of the graph relaxed one
+// by one cost more than a weight-ordered pull (117 M of 1.07 G at scale 26: 1.0
+// ms against 0.4).  The whole SSSP at scales 26, 22 and 20: 3.20, 0.62 and 0.44
+// ms; with 1: 3.19, 0.63, 0.44; with 4: 3.19, 0.72, 0.44; never: 3.82 at 26.
+constexpr uint32_t HEAVY_SSSP = 2;
+// BFS and CC: a listed vertex takes about 75 ps and an out-edge 8 (all blocks
+// together), a dense pull's probe about 5 ps per destination of the graph and
+// 15 us for its launches; in units of 5 ps.  R-MAT scales 24 and 26, BFS with the
+// rule 0.338 and 0.856 ms, without it 0.367 and 0.976; CC at 24: 0.300 and 0.350.
+// Half or twice the first two costs: 0.368 or 0.335 and 0.855 for BFS, 0.326 for
+// CC, and twice loses 4% on CC at scale 21 (0.139 -> 0.147).
+constexpr uint32_t HEAVY_VERT = 14, HEAVY_EDGE = 2, HEAVY_FIXED = 3u << 20;
+
+// whether `act` vertices of `mass` out-edges are better a dense pull
+__device__ __forceinline__ bool heavy_frontier(const DevGraph& g, const DevState& s, uint32_t app, unsigned long long mass,
+                                               unsigned long long act)
+{
+    const unsigned long long vne = g.Vne;
+    return app == WEDGE_APP_SSSP ? s.wo && mass > HEAVY_SSSP * vne
+                                 : HEAVY_VERT * act + HEAVY_EDGE * mass > vne + HEAVY_FIXED;
+}
+
 // the fixed schedules; WEDGE_SCHED_LEARNED and WEDGE_SCHED_PROBE fall back to
 // the plain rule here (decide_kernel overrides it where they apply)
-__device__ __forceinline__ uint32_t choose_mode(uint32_t sched, unsigned long long mass, unsigned long long thr)
+__device__ __forceinline__ uint32_t choose_mode(uint32_t sched, unsigned long long mass, unsigned long long thr,
+                                                bool heavy = false)
 {
     if (sched == WEDGE_SCHED_DENSE)
         return MODE_DENSE;
@@ -3098,7 +3123,7 @@ __device__ __forceinline__ uint32_t choose_mode(uint32_t sched, unsigned long lo
         return MODE_WEDGE;
     if (sched == WEDGE_SCHED_FILTERED)
         return MODE_FILTERED;
-    return mass > thr ? MODE_DENSE : MODE_WEDGE; /* execution_bfs.c:141 */
+    return mass > thr || heavy ? MODE_DENSE : MODE_WEDGE; /* execution_bfs.c:141 */
 }
 
 // Scheduler features of the next iteration, from the pull just finished (its
@@ -3214,7 +3239,7 @@ struct NextPull {
 
 __device__ __forceinline__ NextPull next_pull(uint32_t sched, unsigned long long mass, bool redo, uint32_t iter,
                                               uint32_t max_iter, unsigned long long thr, uint32_t probe_iter,
-                                              uint32_t probe_mode)
+                                              uint32_t probe_mode, bool heavy)
 {
     NextPull n{false, false, MODE_DENSE};
     if (mass == 0ull && !redo) {
@@ -3222,7 +3247,7 @@ __device__ __forceinline__ NextPull next_pull(uint32_t sched, unsigned long long
     } else if (iter >= max_iter) {
         n.done = n.capped = true;
     } else if (!redo) {
-        n.mode = choose_mode(sched, mass, thr);
+        n.mode = choose_mode(sched, mass, thr, heavy);
         if (sched == WEDGE_SCHED_PROBE && iter == probe_iter)
             n.mode = probe_mode;
     }
@@ -3273,7 +3298,7 @@ __device__ __forceinline__ void ask_network(DevState& s, Ctrl* c, uint32_t app, 
 // The control block after a pull whose reduced counters are cnt (one block, all
 // threads): the iteration's record, convergence and the next pull.
 __device__ __forceinline__ void decide_block(const DevGraph& g, DevState& s, Ctrl* c, uint32_t app,
-                                             const unsigned long long (&cnt)[NCNT], uint32_t pull_launches)
+                                             const unsigned long long (&cnt)[NCNT], uint32_t pull_launches, bool fused)
 {
     __shared__ float feat[NF];
     __shared__ uint32_t go;
@@ -3290,14 +3315,13 @@ __device__ __forceinline__ void decide_block(const DevGraph& g, DevState& s, Ctr
         c->tiles = 0u;
         c->items = 0u;
         c->alist_n = 0u;
-        c->heavy = 0u;
-        c->last_act = cnt[CNT_ACT];
         go = 0u;
         // SSSP: a pull dropped 32-bit sums that reached the copy's limit; the
         // next pull is dense and 64-bit, and relaxes every in-edge again
         const bool redo = c->ovf_redo != 0u;
         c->ovf_redo = 0u;
-        const NextPull n = next_pull(c->sched, m, redo, c->iter, c->max_iter + c->near_iters, c->threshold, c->probe_iter, c->probe_mode);
+        const NextPull n = next_pull(c->sched, m, redo, c->iter, c->max_iter + c->near_iters, c->threshold, c->probe_iter,
+                                     c->probe_mode, fused && heavy_frontier(g, s, app, m, cnt[CNT_ACT]));
         if (n.done) {
             c->done = 1u;
             c->not_converged = n.capped ? 1u : 0u;
@@ -3334,7 +3358,7 @@ __global__ void decide_kernel(DevGraph g, DevState s, const unsigned long long* 
             s.summary[i] = 0u; /* the pull has cleared every chunk word it walked */
         unsigned long long cnt[NCNT];
         reduce_counters(block_cnt, nblocks, cnt);
-        decide_block(g, s, c, app, cnt, s.wo ? SSSP_WO_LAUNCHES : pull_launches_of((int)app));
+        decide_block(g, s, c, app, cnt, s.wo ? SSSP_WO_LAUNCHES : pull_launches_of((int)app), fused != 0u);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -3744,8 +3768,6 @@ __global__ void init_root_kernel(DevGraph g, DevState s, uint32_t app, uint64_t 
         c->narrow_ovf = 0;
         c->ovf_redo = 0;
         c->bodies = 0;
-        c->heavy = 0u;
-        c->last_act = 1ull;
         for (int i = 0; i < 3; ++i)
             c->fmin[i] = 0u;
         loop_reset(c);
@@ -3830,19 +3852,6 @@ constexpr unsigned long long NEAR_MASS = 1ull << 16;
 constexpr double NEAR_STEP = 1.0;
 constexpr uint32_t NEAR_ITER = 16;
 constexpr uint32_t BARRIER_TRIES = 1u << 22;
-// A Wedge iteration whose vertices have more than WO_HEAVY out-edges per
-// destination of the graph runs as a weight-ordered pull (117 M of 1.07 G at
-// scale 26, below the 20% that make an iteration dense: 1.0 ms relaxed one by
-// one, 0.4 as a pull).  The whole SSSP at scales 26, 22 and 20: 3.20, 0.62 and
-// 0.44 ms; with 1: 3.19, 0.63, 0.44; with 4: 3.19, 0.72, 0.44; never: 3.82 at 26.
-constexpr uint32_t WO_HEAVY = 2;
-// BFS and CC: a listed vertex takes about 75 ps and an out-edge 8 (all blocks
-// together), a dense pull's probe about 5 ps per destination of the graph and
-// 15 us for its launches; in units of 5 ps.  R-MAT scales 24 and 26, BFS with the
-// rule 0.338 and 0.856 ms, without it 0.367 and 0.976; CC at 24: 0.300 and 0.350.
-// Half or twice the first two costs: 0.368 or 0.335 and 0.855 for BFS, 0.326 for
-// CC, and twice loses 4% on CC at scale 21 (0.139 -> 0.147).
-constexpr uint32_t HEAVY_VERT = 14, HEAVY_EDGE = 2, HEAVY_FIXED = 3u << 20;
 enum : uint32_t { ERR_BARRIER_TIMEOUT = 4u };
 
 // all blocks of a cooperative launch; false when it did not complete within
@@ -3919,7 +3928,7 @@ struct LoopBook {
     }
 
     // into the control block: before another launch or block reads it
-    __device__ void close(Ctrl* c, unsigned long long mass, unsigned long long act, const NextPull& next, uint32_t iter, uint32_t parity,
+    __device__ void close(Ctrl* c, unsigned long long mass, const NextPull& next, uint32_t iter, uint32_t parity,
                           uint32_t extra) const
     {
         c->near_iters = extra;
@@ -3928,7 +3937,6 @@ struct LoopBook {
         c->activated = activated;
         c->last_mass = mass;
         c->mass = mass;
-        c->last_act = act;
         c->wedge_iters = wedge_iters;
         c->pull_launches = pull_launches;
         c->iter = iter;
@@ -3976,16 +3984,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
     uint32_t mode = c->mode, parity = c->parity, iter = c->iter;
     const uint32_t sched = c->sched, max_iter = c->max_iter, probe_iter = c->probe_iter, probe_mode = c->probe_mode;
     const unsigned long long thr = c->threshold;
-    // whether a Wedge iteration over `act` vertices of `mass` out-edges is better a dense pull
-    const bool may_pull = (APP != WEDGE_APP_SSSP || s.wo) && small == 0u && max_steps > 1u &&
-                          (sched == WEDGE_SCHED_PLAIN || sched == WEDGE_SCHED_LEARNED);
-    auto heavy = [&](unsigned long long mass, unsigned long long act) {
-        const unsigned long long vne = g.Vne;
-        return may_pull && (APP == WEDGE_APP_SSSP ? mass > WO_HEAVY * vne
-                                                  : HEAVY_VERT * act + HEAVY_EDGE * mass > vne + HEAVY_FIXED);
-    };
-    const bool pull_now = mode == MODE_WEDGE && iter != 0u && heavy(c->mass, c->last_act);
-    const bool loop = small != 0u || (mode == MODE_WEDGE && !pull_now);
+    const bool loop = small != 0u || mode == MODE_WEDGE;
     const bool f64 = g.weight_kind == WEDGE_WEIGHTS_F64;
     uint32_t* my_buf = sh_buf[wib];
     uint32_t* my_pre = sh_pre[wib];
@@ -4105,12 +4104,8 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
         if (s.tile_need)
             for (uint32_t i = tid; i < g.T / 32u + 2u; i += nthr)
                 s.tile_need[i] = 0u;
-        if (tid == 0u) {
-            if (APP == WEDGE_APP_SSSP)
-                c->fmin[(parity + 1u) % 3u] = NONE32; /* of the frontier the next pull writes */
-            if (pull_now)
-                c->heavy = 1u;
-        }
+        if (APP == WEDGE_APP_SSSP && tid == 0u)
+            c->fmin[(parity + 1u) % 3u] = NONE32; /* of the frontier the next pull writes */
         if (!loop)
             return;
         flush();
@@ -4587,14 +4582,16 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
 #pragma unroll
         for (uint32_t j = 0; j < NCNT; ++j)
             cnt[j] = sh_acc[j];
+        /* far vertices wait for their turn, not for a dense pull */
+        const bool pull_next = small == 0u && !(sorting && so.release + so.waiting != 0ull) &&
+                               heavy_frontier(g, s, (uint32_t)APP, cnt[CNT_MASS], cnt[CNT_ACT]);
         const NextPull next = next_pull(sched, cnt[CNT_MASS], false, iter + 1u,
-                                        APP == WEDGE_APP_SSSP ? max_iter + so.extra : max_iter, thr, probe_iter, probe_mode);
-        const bool pull_next = !(sorting && so.release + so.waiting != 0ull) && heavy(cnt[CNT_MASS], cnt[CNT_ACT]);
+                                        APP == WEDGE_APP_SSSP ? max_iter + so.extra : max_iter, thr, probe_iter, probe_mode,
+                                        pull_next);
         if (scribe)
             book.note(g, s, (uint32_t)APP, cnt, next, mode, iter);
-        if (scribe && (next.done || step + 1u == max_steps || (!small && next.mode != MODE_WEDGE) || pull_next ||
-                       sched == WEDGE_SCHED_LEARNED))
-            book.close(c, cnt[CNT_MASS], cnt[CNT_ACT], next, iter + 1u, (parity + 1u) % 3u,
+        if (scribe && (next.done || step + 1u == max_steps || (!small && next.mode != MODE_WEDGE) || sched == WEDGE_SCHED_LEARNED))
+            book.close(c, cnt[CNT_MASS], next, iter + 1u, (parity + 1u) % 3u,
                        APP == WEDGE_APP_SSSP ? so.extra : 0u);
         if (!next.done && sched == WEDGE_SCHED_LEARNED && s.net && blockIdx.x + 1u == gridDim.x)
             ask_network(s, c, (uint32_t)APP, iter + 1u);
@@ -4606,9 +4603,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
                 return;
             mode = *(volatile unsigned int*)&c->mode;
         }
-        if (scribe && pull_next && !next.done)
-            c->heavy = 1u; /* the pull that follows this launch */
-        const bool leave = step + 1u == max_steps || (!small && mode != MODE_WEDGE) || pull_next;
+        const bool leave = step + 1u == max_steps || (!small && mode != MODE_WEDGE);
         if (!next.done && leave && (APP == WEDGE_APP_BFS || (sorting && so.release + so.waiting != 0ull))) {
             /* another launch takes over: the waiting vertices join the frontier */
             uint32_t* fr = s.front + parity * s.front_stride; /* this iteration's bitmap */

@@ -123,8 +123,6 @@ struct Ctrl {
                                        // pull is dense (64-bit) and the traversal does not stop before it
     unsigned int bodies;               // rounds of the fused traversal loop
     unsigned int bar;                  // sparse_loop_kernel: grid-barrier arrivals, and per step modulo 3
-    unsigned int heavy;                // the Wedge iteration at hand runs as a dense pull
-    unsigned long long last_act;       // vertices the last iteration activated
     unsigned int fmin[3];              // SSSP: no distance in the frontier bitmap of that number is below (dense pulls)
     unsigned int ln[3], li[3];         // vertices and items listed for it,
     unsigned long long lacc[3][NCNT];  // its counters; SSSP: the least distance it sorted out and by how many
