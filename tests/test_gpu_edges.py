@@ -557,3 +557,37 @@ def test_log_says_which_pulls_ran(engine_lib, n):
             if flags == W.FLAG_TIMING:
                 assert all(r["pull_ms"] > 0.0 for r in log)
         assert logs[0] == logs[1] == logs[2]
+
+
+@pytest.mark.parametrize("graph", ["grid", "rmat18", "rmat12"])
+def test_timed_runs_are_the_plain_runs(engine_lib, graph):
+    """a run with per-iteration times takes the kernels that a run without takes: far
+    vertices wait in it, PageRank is one launch, and the times add up to the run's"""
+    W = engine_lib
+    make = {"grid": lambda wk: W.Graph.grid(1500, 0.01, 5, wk), "rmat18": lambda wk: W.Graph.rmat(18, 16, 5, weight_kind=wk),
+            "rmat12": lambda wk: W.Graph.rmat(12, 16, 5, weight_kind=wk)}[graph]
+    with make(W.WEIGHTS_U64) as g:
+        for app in (W.APP_SSSP, W.APP_BFS, W.APP_CC):
+            plain = g.run(app, W.Params(flags=W.FLAG_GRAPH))
+            expect = g.read_results().copy()
+            for _ in range(2):
+                st = g.run(app, W.Params(flags=W.FLAG_TIMING))
+            assert app == W.APP_BFS or np.array_equal(g.read_results(), expect)
+            log = g.iteration_log()
+            assert st["edges_scanned"] <= 1.5 * plain["edges_scanned"] and plain["edges_scanned"] <= 1.5 * st["edges_scanned"]
+            assert len(log) == st["iterations"] and all(r["pull_ms"] >= 0.0 and r["wedge_ms"] >= 0.0 for r in log)
+            total = st["pull_ms_dense"] + st["pull_ms_wedge"] + st["wedge_ms"]
+            assert abs(sum(r["pull_ms"] + r["wedge_ms"] for r in log) - total) < 1e-3 * total
+            assert total < st["running_ms"]
+            if plain["running_ms"] > 1.0:  # the launches around the iterations are little beside them
+                assert total > 0.6 * plain["running_ms"], (total, plain["running_ms"])
+        for prec in (W.PREC_FP64, W.PREC_FP32C):
+            p = dict(num_iterations=7, damping=0.85, precision=prec)
+            plain = g.run(W.APP_PR, W.Params(**p))
+            expect = g.read_results().copy()
+            st = g.run(W.APP_PR, W.Params(flags=W.FLAG_TIMING, **p))
+            assert np.array_equal(g.read_results(), expect)
+            assert st["pull_launches"] == plain["pull_launches"] == 1 and st["kernel_launches"] == 1
+            log = g.iteration_log()
+            assert len(log) == 7 and all(r["pull_ms"] > 0.0 for r in log)
+            assert 0.0 < sum(r["pull_ms"] for r in log) + st["vertex_ms"] < st["running_ms"]

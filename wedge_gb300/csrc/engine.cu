@@ -3226,11 +3226,6 @@ __device__ __forceinline__ void loop_reset(Ctrl* c)
     }
 }
 
-__global__ void loop_reset_kernel(DevState s)
-{
-    loop_reset(s.ctrl);
-}
-
 // what follows a pull that changed `mass` out-edges
 struct NextPull {
     bool done, capped;
@@ -3880,6 +3875,14 @@ __device__ __forceinline__ bool grid_barrier(Ctrl* c, uint32_t& target, uint32_t
     return *ok != 0u;
 }
 
+// the device's clock, for the iterations of a timed run (WEDGE_FLAG_TIMING)
+__device__ __forceinline__ unsigned long long device_ns()
+{
+    unsigned long long ns;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(ns));
+    return ns;
+}
+
 template <bool B>
 struct BoolTag {
     static constexpr bool value = B;
@@ -3903,7 +3906,7 @@ struct LoopBook {
 
     // after iteration `iter`, run in `mode`
     __device__ void note(const DevGraph& g, const DevState& s, uint32_t app, const unsigned long long (&cnt)[NCNT],
-                         const NextPull& next, uint32_t mode, uint32_t iter)
+                         const NextPull& next, uint32_t mode, uint32_t iter, bool timed)
     {
         edges += cnt[CNT_EDGES];
         dsts += cnt[CNT_DSTS];
@@ -3919,6 +3922,8 @@ struct LoopBook {
             r.activated = cnt[CNT_ACT];
             r.mode = mode;
             r.iter = iter;
+            if (timed)
+                r.end_ns = device_ns();
         }
         if (!next.done && iter + 1u < LOG_CAP) {
             sched_features(g, activated, iter + 1u, app, cnt, s.log[iter + 1u].feat);
@@ -3953,7 +3958,7 @@ struct LoopBook {
 
 template <int APP>
 __global__ void __launch_bounds__(PULL_THREADS, 1)
-    sparse_loop_kernel(DevGraph g, DevState s, uint32_t small, uint32_t max_steps)
+    sparse_loop_kernel(DevGraph g, DevState s, uint32_t small, uint32_t timed)
 {
     constexpr int WARPS = PULL_THREADS / 32;
     using val_t = typename CurT<APP>::type;
@@ -4589,8 +4594,8 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
                                         APP == WEDGE_APP_SSSP ? max_iter + so.extra : max_iter, thr, probe_iter, probe_mode,
                                         pull_next);
         if (scribe)
-            book.note(g, s, (uint32_t)APP, cnt, next, mode, iter);
-        if (scribe && (next.done || step + 1u == max_steps || (!small && next.mode != MODE_WEDGE) || sched == WEDGE_SCHED_LEARNED))
+            book.note(g, s, (uint32_t)APP, cnt, next, mode, iter, timed != 0u);
+        if (scribe && (next.done || (!small && next.mode != MODE_WEDGE) || sched == WEDGE_SCHED_LEARNED))
             book.close(c, cnt[CNT_MASS], next, iter + 1u, (parity + 1u) % 3u,
                        APP == WEDGE_APP_SSSP ? so.extra : 0u);
         if (!next.done && sched == WEDGE_SCHED_LEARNED && s.net && blockIdx.x + 1u == gridDim.x)
@@ -4603,7 +4608,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
                 return;
             mode = *(volatile unsigned int*)&c->mode;
         }
-        const bool leave = step + 1u == max_steps || (!small && mode != MODE_WEDGE);
+        const bool leave = !small && mode != MODE_WEDGE;
         if (!next.done && leave && (APP == WEDGE_APP_BFS || (sorting && so.release + so.waiting != 0ull))) {
             /* another launch takes over: the waiting vertices join the frontier */
             uint32_t* fr = s.front + parity * s.front_stride; /* this iteration's bitmap */
@@ -5422,7 +5427,7 @@ __device__ __forceinline__ double ld_rank(const double* p)
 }
 
 template <bool F64>
-__global__ void __launch_bounds__(PULL_THREADS, 1) pr_loop_kernel(DevGraph g, DevState s, uint32_t iters)
+__global__ void __launch_bounds__(PULL_THREADS, 1) pr_loop_kernel(DevGraph g, DevState s, uint32_t iters, uint32_t timed)
 {
     using P = PrPrec<F64>;
     using rank_t = typename P::rank_t;
@@ -5464,6 +5469,8 @@ __global__ void __launch_bounds__(PULL_THREADS, 1) pr_loop_kernel(DevGraph g, De
     if (!grid_barrier(c, target, &sh_ok))
         return;
     const unsigned long long pol = l2_evict_first_policy();
+    if (timed && tid == 0u)
+        c->start_ns = device_ns();
     for (uint32_t it = 0; it < iters; ++it) {
         const rank_t* cur = rank + ((it & 1u) ? stride : 0ull);
         rank_t* nxt = rank + ((it & 1u) ? 0ull : stride);
@@ -5562,6 +5569,8 @@ __global__ void __launch_bounds__(PULL_THREADS, 1) pr_loop_kernel(DevGraph g, De
             atomicAdd(&sh_dsts, dsts);
         if (!grid_barrier(c, target, &sh_ok))
             return;
+        if (timed && tid == 0u && it < LOG_CAP)
+            s.log[it].pull_ns = device_ns();
         // ---- destinations whose in-edges span tiles, in tile order (phases.c:71-114)
         if constexpr (F64) {
             merge_splits(s.psplit_k, s.psplit_t0, s.psplit_t1, s.pnsplit, s.pnwide, s.pT, spread * 32u + (uint32_t)lane, nthr,
@@ -5599,6 +5608,8 @@ __global__ void __launch_bounds__(PULL_THREADS, 1) pr_loop_kernel(DevGraph g, De
         }
         __syncthreads();
         total = sh_part[0];
+        if (timed && tid == 0u && it < LOG_CAP)
+            s.log[it].end_ns = device_ns();
         __syncthreads();
     }
     // vertices with neither in- nor out-edges: the last iteration's constant, once
@@ -6456,7 +6467,7 @@ static bool small_loop(const wedge_graph* h, int sched) { return h->g.E <= LOOP_
 
 // one block per SM, fewer on graphs that leave most of them without work (a
 // barrier of few blocks is faster)
-static int launch_sparse_loop(wedge_graph* h, int app, bool whole, uint32_t max_steps)
+static int launch_sparse_loop(wedge_graph* h, int app, bool whole, bool timed = false)
 {
     const uint64_t want = h->g.E / 2048u + 8u;
     cudaLaunchConfig_t cfg = {};
@@ -6471,13 +6482,13 @@ static int launch_sparse_loop(wedge_graph* h, int app, bool whole, uint32_t max_
     const uint32_t small = whole ? 1u : 0u;
     switch (app) {
     case WEDGE_APP_BFS:
-        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, sparse_loop_kernel<WEDGE_APP_BFS>, h->g, h->s, small, max_steps));
+        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, sparse_loop_kernel<WEDGE_APP_BFS>, h->g, h->s, small, timed ? 1u : 0u));
         break;
     case WEDGE_APP_CC:
-        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, sparse_loop_kernel<WEDGE_APP_CC>, h->g, h->s, small, max_steps));
+        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, sparse_loop_kernel<WEDGE_APP_CC>, h->g, h->s, small, timed ? 1u : 0u));
         break;
     default:
-        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, sparse_loop_kernel<WEDGE_APP_SSSP>, h->g, h->s, small, max_steps));
+        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, sparse_loop_kernel<WEDGE_APP_SSSP>, h->g, h->s, small, timed ? 1u : 0u));
         break;
     }
     return WEDGE_OK;
@@ -6573,7 +6584,7 @@ static int build_graph(wedge_graph* h, int app)
     WEDGE_CHECK(cudaStreamBeginCaptureToGraph(h->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
     int rc = WEDGE_OK;
     if (fused_loop(h)) { /* Wedge iterations, a dense pull, the decision and the loop condition */
-        rc = launch_sparse_loop(h, app, false, 0xFFFFFFFFu);
+        rc = launch_sparse_loop(h, app, false);
         launch_pull(h, app);
         launch_decide(h, app, true, true, handle);
     } else {
@@ -6632,6 +6643,50 @@ static int traversal_stats(wedge_graph* h, int app, uint64_t launches, bool use_
     return WEDGE_OK;
 }
 
+// The times of a timed run's last round, from iteration before.iter to
+// after.iter: the loop's iterations by the clock that it noted (the first with
+// the launch), the pull's and its tail's by their events (ev 2, 5, 3, 4).
+static int note_times(wedge_graph* h, const Ctrl& before, const Ctrl& after, bool fused, bool small, double* dense, double* wedge,
+                      double* tail)
+{
+    float loop_ms = 0, pull_ms = 0, tail_ms = 0;
+    WEDGE_CHECK(cudaEventElapsedTime(&loop_ms, h->ev[2], h->ev[5]));
+    WEDGE_CHECK(cudaEventElapsedTime(&pull_ms, h->ev[5], h->ev[3]));
+    WEDGE_CHECK(cudaEventElapsedTime(&tail_ms, h->ev[3], h->ev[4]));
+    const uint32_t n = after.iter - before.iter;
+    const uint32_t in_loop = !fused ? 0u : small ? n : after.wedge_iters - before.wedge_iters;
+    const uint32_t logged = before.iter >= LOG_CAP ? 0u : n < LOG_CAP - before.iter ? n : LOG_CAP - before.iter;
+    IterRec* r = (IterRec*)malloc((size_t)(logged ? logged : 1u) * sizeof(IterRec));
+    if (!r)
+        return WEDGE_ERR_OOM;
+    const cudaError_t e = cudaMemcpy(r, h->s.log + before.iter, logged * sizeof(IterRec), cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) {
+        free(r);
+        return cuda_status(e);
+    }
+    double rest = loop_ms; /* of the loop's time, for the first of its iterations */
+    for (uint32_t i = logged < in_loop ? logged : in_loop; i-- > 0u;) {
+        const double ms = i ? (double)(r[i].end_ns - r[i - 1u].end_ns) / 1e6 : rest > 0.0 ? rest : 0.0;
+        rest -= ms;
+        h->iter_pull_ms[before.iter + i] = ms;
+        h->iter_wedge_ms[before.iter + i] = 0.0;
+        *(r[i].mode == MODE_WEDGE ? wedge : dense) += ms;
+    }
+    if (in_loop && !logged)
+        *wedge += loop_ms; /* past the log's end */
+    if (n > in_loop) {
+        const double ms = in_loop ? pull_ms : pull_ms + loop_ms;
+        if (logged > in_loop) {
+            h->iter_pull_ms[before.iter + in_loop] = ms;
+            h->iter_wedge_ms[before.iter + in_loop] = tail_ms;
+        }
+        *(!fused && before.mode == MODE_WEDGE ? wedge : dense) += ms;
+        *tail += tail_ms;
+    }
+    free(r);
+    return WEDGE_OK;
+}
+
 // One traversal.  With wait false (graph loop only) the work is queued and the
 // statistics are left to traversal_stats, through wedge_cuda_wait.
 static int run_traversal(wedge_graph* h, int app, const wedge_params_t* p, wedge_stats_t* st, bool wait = true)
@@ -6660,7 +6715,7 @@ static int run_traversal(wedge_graph* h, int app, const wedge_params_t* p, wedge
     launches += 2ull + (fused ? 0ull : build_launches(h)); /* init, root, the Wedge build */
     Ctrl c;
     if (one) {
-        int rc = launch_sparse_loop(h, app, true, 0xFFFFFFFFu);
+        int rc = launch_sparse_loop(h, app, true);
         if (rc)
             return rc;
         launches += 1ull;
@@ -6673,42 +6728,30 @@ static int run_traversal(wedge_graph* h, int app, const wedge_params_t* p, wedge
                 return rc;
             if (c.done)
                 break;
-            const uint32_t mode = c.mode;
-            const bool sparse = fused && (mode == MODE_WEDGE || small);
+            /* a round of the plain run's launches; the loop notes its iterations' ends itself */
             WEDGE_CHECK(cudaEventRecord(h->ev[2], h->stream));
-            if (fused && (rc = launch_sparse_loop(h, app, small, 1u))) /* one Wedge iteration, or the bitmaps' clearing */
+            if (fused && (rc = launch_sparse_loop(h, app, small, true)))
                 return rc;
-            if (!sparse)
+            WEDGE_CHECK(cudaEventRecord(h->ev[5], h->stream));
+            if (!small)
                 launch_pull(h, app);
             WEDGE_CHECK(cudaEventRecord(h->ev[3], h->stream));
-            if (sparse)
-                loop_reset_kernel<<<1, 1, 0, h->stream>>>(h->s);
-            else if (fused)
+            if (!small && fused)
                 launch_decide(h, app, true);
-            else
+            else if (!small)
                 launch_tail(h, app);
             WEDGE_CHECK(cudaEventRecord(h->ev[4], h->stream));
-            launches += sparse ? 2ull : fused ? fused_launches(h, app) : iteration_launches(h, app);
-            WEDGE_CHECK(cudaEventSynchronize(h->ev[4]));
-            float a = 0, b = 0;
-            cudaEventElapsedTime(&a, h->ev[2], h->ev[3]);
-            cudaEventElapsedTime(&b, h->ev[3], h->ev[4]);
-            if (mode != MODE_WEDGE)
-                t_pull_dense += a;
-            else
-                t_pull_wedge += a;
-            t_wedge += b;
-            if (c.iter < LOG_CAP) {
-                h->iter_pull_ms[c.iter] = a;
-                h->iter_wedge_ms[c.iter] = b;
-            }
+            launches += small ? 1ull : fused ? fused_launches(h, app) : iteration_launches(h, app);
+            Ctrl after;
+            if ((rc = read_ctrl(h, &after)) || (rc = note_times(h, c, after, fused, small, &t_pull_dense, &t_pull_wedge, &t_wedge)))
+                return rc;
         }
     } else {
         // speculative batches: kernels are no-ops once Ctrl::done is set
         for (;;) {
             for (int b = 0; b < 3; ++b) {
                 if (fused) {
-                    int rc = launch_sparse_loop(h, app, false, 0xFFFFFFFFu);
+                    int rc = launch_sparse_loop(h, app, false);
                     if (rc)
                         return rc;
                 }
@@ -6789,7 +6832,7 @@ constexpr uint64_t PR32_LOOP_EDGES = 1ull << 28;
 
 // A whole PageRank in one launch (pr_loop_kernel): one block per SM, fewer on
 // graphs that leave most of them without work.  The control block starts at zero.
-static int launch_pr_loop(wedge_graph* h, uint32_t iters)
+static int launch_pr_loop(wedge_graph* h, uint32_t iters, bool timed)
 {
     const bool f64 = h->s.precision != WEDGE_PREC_FP32C;
     const uint64_t want = h->g.E / 2048u + 8u;
@@ -6807,9 +6850,9 @@ static int launch_pr_loop(wedge_graph* h, uint32_t iters)
     s.hub_bytes = h->loop_hub;
     WEDGE_CHECK(cudaMemsetAsync(s.ctrl, 0, sizeof(Ctrl), h->stream));
     if (f64)
-        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, pr_loop_kernel<true>, h->g, s, iters));
+        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, pr_loop_kernel<true>, h->g, s, iters, timed ? 1u : 0u));
     else
-        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, pr_loop_kernel<false>, h->g, s, iters));
+        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, pr_loop_kernel<false>, h->g, s, iters, timed ? 1u : 0u));
     return WEDGE_OK;
 }
 
@@ -6845,6 +6888,29 @@ static int pr_stats(wedge_graph* h, uint32_t iters, bool loop, bool timing, doub
     return WEDGE_OK;
 }
 
+// The times of a timed pr_loop_kernel's iterations (waits for it): the pull, and what follows it
+static int pr_loop_times(wedge_graph* h, uint32_t iters, double* pull, double* vertex)
+{
+    Ctrl c;
+    const int rc = read_ctrl(h, &c);
+    if (rc)
+        return rc;
+    const uint32_t n = iters < LOG_CAP ? iters : LOG_CAP;
+    IterRec* r = (IterRec*)malloc(n * sizeof(IterRec));
+    if (!r)
+        return WEDGE_ERR_OOM;
+    const cudaError_t e = cudaMemcpy(r, h->s.log, n * sizeof(IterRec), cudaMemcpyDeviceToHost);
+    for (uint32_t i = 0; i < n && e == cudaSuccess; ++i) {
+        const unsigned long long from = i ? r[i - 1u].end_ns : c.start_ns;
+        h->iter_pull_ms[i] = (double)(r[i].pull_ns - from) / 1e6;
+        h->iter_wedge_ms[i] = 0.0;
+        *pull += h->iter_pull_ms[i];
+        *vertex += (double)(r[i].end_ns - r[i].pull_ns) / 1e6;
+    }
+    free(r);
+    return e == cudaSuccess ? WEDGE_OK : cuda_status(e);
+}
+
 static int run_pr(wedge_graph* h, const wedge_params_t* p, wedge_stats_t* st, bool wait = true)
 {
     const DevGraph& g = h->g;
@@ -6853,14 +6919,14 @@ static int run_pr(wedge_graph* h, const wedge_params_t* p, wedge_stats_t* st, bo
     h->s.precision = (uint32_t)p->precision;
     const uint32_t vgrid = aux_grid(h, g.V);
     const uint32_t fgrid = finish_grid(h, g);
-    const bool loop = !timing && p->num_iterations > 0 && g.E != 0 && !g.shard &&
+    const bool loop = p->num_iterations > 0 && g.E != 0 && !g.shard &&
                       (h->s.precision != WEDGE_PREC_FP32C || g.E < PR32_LOOP_EDGES);
     const bool c32 = h->s.precision == WEDGE_PREC_FP32C;
     double t_pull = 0, t_vertex = 0;
     WEDGE_CHECK(cudaEventRecord(h->ev[0], h->stream));
     h->pr_flip = loop && !c32 ? (int)(p->num_iterations & 1u) : 0;
     if (loop) {
-        int rc = launch_pr_loop(h, p->num_iterations);
+        int rc = launch_pr_loop(h, p->num_iterations, timing);
         if (rc)
             return rc;
     } else if (c32) {
@@ -6904,6 +6970,11 @@ static int run_pr(wedge_graph* h, const wedge_params_t* p, wedge_stats_t* st, bo
     if (c32 && !loop)
         launch_pr32_iso(h); /* vertices with neither in- nor out-edges, once */
     WEDGE_CHECK(cudaEventRecord(h->ev[1], h->stream));
+    if (loop && timing) {
+        const int rc = pr_loop_times(h, p->num_iterations, &t_pull, &t_vertex);
+        if (rc)
+            return rc;
+    }
     if (!loop) {
         double* sums = pr_sums(h);
         pr_sum_kernel<<<vgrid, AUX_THREADS, 0, h->stream>>>(g, h->s, sums);

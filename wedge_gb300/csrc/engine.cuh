@@ -82,6 +82,7 @@ struct IterRec {
     float feat[16];                // scheduler features this iteration's mode was chosen on
     unsigned int learned;          // 1 if the scheduler network chose the mode
     unsigned int pad;
+    unsigned long long pull_ns, end_ns; // timed runs of the loop kernels: when it ended (PageRank: its pull, before)
 };
 
 // Device control block of one traversal; read and written only by the
@@ -129,6 +130,7 @@ struct Ctrl {
     unsigned long long lmin[3], lfar[3]; // out-edges it changed the waiting ones; by far list modulo 3:
     unsigned int lf[3];                // vertices listed; by step modulo 2: found by their far bits; by
     unsigned int lall[2], lput[3];     // step modulo 3: listed in the far list at hand
+    unsigned long long start_ns;       // timed pr_loop_kernel: when its first iteration began
     double pr_total;                   // sum of all accumulators (phase_vertex_pr.c:161); compensated FP32:
                                        // the total the next iteration uses
     double pr_prev;                    // compensated FP32: the total the last iteration used

@@ -174,7 +174,11 @@ def load(path: str = DEFAULT_NET) -> np.ndarray:
 # ---------------------------------------------------------------- training set
 # scale 26 with another seed than the benchmark's, so that graphs of its size
 # lie inside the trained feature range (a feature outside it keeps the plain rule)
+# Few iterations of a graph have strategies that differ by more than the noise
+# (SSSP's last dense pulls, BFS's and CC's first sparse ones), so every scale is
+# there several times.
 TRAIN_RMAT = [(18, 16, 11), (20, 16, 12), (22, 16, 13), (24, 16, 14), (20, 8, 15), (22, 32, 16), (26, 16, 6)]
+TRAIN_RMAT += [(s, ef, 100 * s + ef) for s in (18, 19, 20, 21, 22, 23, 24) for ef in (8, 12, 16, 24)]
 EVAL_RMAT = [(19, 16, 21), (21, 16, 22), (23, 16, 23)]
 # the workload the metric is quoted on: R-MAT scale 26, edge factor 16, seed 5 (held out)
 C5_RMAT = [(26, 16, 5)]
