@@ -591,3 +591,19 @@ def test_timed_runs_are_the_plain_runs(engine_lib, graph):
             log = g.iteration_log()
             assert len(log) == 7 and all(r["pull_ms"] > 0.0 for r in log)
             assert 0.0 < sum(r["pull_ms"] for r in log) + st["vertex_ms"] < st["running_ms"]
+
+
+def test_captured_loops_without_cooperative_launches(engine_lib, monkeypatch):
+    """under MPS a captured loop's iterations are separate launches: the results are the
+    host-driven loop's, and so are those of small graphs, which are no captured loop"""
+    W = engine_lib
+    monkeypatch.setenv("WEDGE_MPS", "1")
+    rng = np.random.default_rng(12)
+    for n in (60_000, 1_200_000):
+        V = n // 8
+        s, d = (V * rng.random(n) ** 2).astype(np.int64), (V * rng.random(n) ** 2).astype(np.int64)
+        s, d = np.concatenate([s, np.arange(200)]), np.concatenate([d, np.arange(1, 201)])
+        order = np.lexsort((s, d))
+        w = rng.integers(0, 256, len(s)).astype(np.uint64)
+        check_traversals(W, V, s[order].astype(np.uint32), d[order].astype(np.uint32), w,
+                         (W.SCHED_PLAIN, W.SCHED_WEDGE, W.SCHED_FILTERED), (0, W.FLAG_GRAPH, W.FLAG_TIMING))

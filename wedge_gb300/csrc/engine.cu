@@ -57,6 +57,13 @@ int new_handle(wedge_graph** out)
     h->pend_app = -1;
     WEDGE_CHECK(cudaGetDevice(&h->device));
     WEDGE_CHECK(cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->device));
+    /* a captured loop must not hold a cooperative launch under MPS (WEDGE_MPS=1: as if it were in use) */
+    const char* mps = getenv("WEDGE_MPS");
+    if (cudaDeviceGetAttribute(&h->mps, cudaDevAttrMpsEnabled, h->device) != cudaSuccess) {
+        cudaGetLastError();
+        h->mps = 0;
+    }
+    h->mps = h->mps || (mps && mps[0] == '1') ? 1 : 0;
     WEDGE_CHECK(cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking));
     h->stream = h->own_stream;
     for (int i = 0; i < 8; ++i)
@@ -6558,7 +6565,7 @@ __global__ void loop_cond_kernel(DevState s, cudaGraphConditionalHandle handle)
     cudaGraphSetConditional(handle, s.ctrl->loop);
 }
 
-static int build_graph(wedge_graph* h, int app)
+static int build_graph(wedge_graph* h, int app, bool fused)
 {
     if (h->graph_exec && h->graph_app == app)
         return WEDGE_OK;
@@ -6583,7 +6590,7 @@ static int build_graph(wedge_graph* h, int app)
     h->stream = h->own_stream;
     WEDGE_CHECK(cudaStreamBeginCaptureToGraph(h->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
     int rc = WEDGE_OK;
-    if (fused_loop(h)) { /* Wedge iterations, a dense pull, the decision and the loop condition */
+    if (fused) { /* Wedge iterations, a dense pull, the decision and the loop condition */
         rc = launch_sparse_loop(h, app, false);
         launch_pull(h, app);
         launch_decide(h, app, true, true, handle);
@@ -6698,14 +6705,14 @@ static int run_traversal(wedge_graph* h, int app, const wedge_params_t* p, wedge
     if (cap > 0x7fffffffull)
         cap = 0x7fffffffull;
     const bool timing = (p->flags & WEDGE_FLAG_TIMING) != 0;
-    const bool fused = fused_loop(h);
-    const bool small = fused && small_loop(h, p->sched);
+    const bool small = fused_loop(h) && small_loop(h, p->sched);
     const bool one = small && !timing; /* the whole traversal in one launch */
     const bool use_graph = (p->flags & WEDGE_FLAG_GRAPH) != 0 && !timing && !one;
+    const bool fused = fused_loop(h) && !(use_graph && h->mps); /* else an iteration's launches apart */
     uint64_t launches = 0;
     double t_pull_dense = 0, t_pull_wedge = 0, t_wedge = 0;
     if (use_graph) {
-        int rc = build_graph(h, app);
+        int rc = build_graph(h, app, fused);
         if (rc)
             return rc;
     }

@@ -267,6 +267,7 @@ struct wedge_graph {
     uint32_t pend_iters;
     int device;
     int num_sms;
+    int mps;                           // the device is shared through MPS
     int weight_kind;
     int built_app;                     // app whose state arrays are sized (-1 none)
     int last_app;                      // app of the last run (for read_results)
