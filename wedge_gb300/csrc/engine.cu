@@ -119,6 +119,7 @@ static void free_state(wedge_graph* h)
     for (int i = 0; i < h->nstate; ++i)
         cudaFree(h->state_allocs[i]);
     h->nstate = 0;
+    h->sblock = nullptr;
     memset(&h->s, 0, sizeof(h->s));
     h->s.net = h->net; /* the scheduler network outlives the state arrays */
     h->built_app = -1;
@@ -182,6 +183,11 @@ static int dalloc(wedge_graph* h, T** p, uint64_t count, bool state = false)
     if (!state && h->slab && h->slab_used + need <= h->slab_size) {
         *p = (T*)(h->slab + h->slab_used);
         h->slab_used += need;
+        return WEDGE_OK;
+    }
+    if (state && h->sblock && h->sblock_used + need <= h->sblock_size) {
+        *p = (T*)(h->sblock + h->sblock_used);
+        h->sblock_used += need;
         return WEDGE_OK;
     }
     cudaError_t e = cudaMalloc((void**)p, bytes);
@@ -5444,7 +5450,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1) pr_loop_kernel(DevGraph g, De
     __shared__ unsigned long long hub_bar;
     __shared__ double sh_part[PULL_THREADS / 32];
     __shared__ typename P::K sh_k; /* one thread's FP64 divisions: this GPU's FP64 units are slow */
-    __shared__ uint32_t sh_ok, sh_dsts;
+    __shared__ uint32_t sh_ok, sh_dsts, sh_splits[2]; /* FP64: short and long split destinations */
     extern __shared__ __align__(16) unsigned char pr_smem[];
     Ctrl* c = s.ctrl;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -5462,6 +5468,11 @@ __global__ void __launch_bounds__(PULL_THREADS, 1) pr_loop_kernel(DevGraph g, De
     uint32_t target = 0u, phase = 0u;
     if (threadIdx.x == 0) {
         sh_dsts = 0u;
+        if constexpr (F64) {
+            const unsigned long long n = *s.pcount;
+            sh_splits[0] = (uint32_t)n;
+            sh_splits[1] = (uint32_t)(n >> 32);
+        }
         if (hub_bytes)
             mbar_init(&hub_bar, 1u);
     }
@@ -5580,7 +5591,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1) pr_loop_kernel(DevGraph g, De
             s.log[it].pull_ns = device_ns();
         // ---- destinations whose in-edges span tiles, in tile order (phases.c:71-114)
         if constexpr (F64) {
-            merge_splits(s.psplit_k, s.psplit_t0, s.psplit_t1, s.pnsplit, s.pnwide, s.pT, spread * 32u + (uint32_t)lane, nthr,
+            merge_splits(s.psplit_k, s.psplit_t0, s.psplit_t1, sh_splits[0], sh_splits[1], s.pT, spread * 32u + (uint32_t)lane, nthr,
                          [&](uint32_t tt) { return s.tail_part[tt]; }, [&](uint32_t tt) { return s.head_part[tt]; },
                          [&](uint32_t k, double x) { put(g.dst_ident ? k : g.dst_id[k], P::rank(K, x)); });
         } else {
@@ -6052,8 +6063,9 @@ static int pr32_setup_hub(wedge_graph* h)
 }
 
 // Split lists of tiles of tile_e in-edges (destinations spanning tiles: short
-// ones from the front, long ones from the back)
-static int split_state(wedge_graph* h, uint32_t tile_e)
+// ones from the front, long ones from the back).  Their counts stay on the
+// device (DevState::pcount), and come to the host where launches need them.
+static int split_state(wedge_graph* h, uint32_t tile_e, bool on_host = true)
 {
     DevGraph& g = h->g;
     DevState& s = h->s;
@@ -6061,23 +6073,28 @@ static int split_state(wedge_graph* h, uint32_t tile_e)
     const uint32_t cap = (uint32_t)h->num_sms * 8u;
     int rc;
     s.pT = (uint32_t)(g.Epad / tile_e);
-    if ((rc = dalloc(h, &s.psplit_k, (uint64_t)s.pT + 1, true)) || (rc = dalloc(h, &s.psplit_t0, (uint64_t)s.pT + 1, true)) ||
-        (rc = dalloc(h, &s.psplit_t1, (uint64_t)s.pT + 1, true)))
+    const uint64_t n = (uint64_t)s.pT + 1;
+    unsigned long long* flag = nullptr; /* then the places; the last one is the counts */
+    unsigned char* tmp = nullptr;
+    size_t bytes = 0;
+    WEDGE_CHECK(cub::DeviceScan::ExclusiveSum(nullptr, bytes, flag, flag, (long long)n, st));
+    if ((rc = dalloc(h, &s.psplit_k, n, true)) || (rc = dalloc(h, &s.psplit_t0, n, true)) || (rc = dalloc(h, &s.psplit_t1, n, true)) ||
+        (rc = dalloc(h, &flag, n, true)) || (rc = dalloc(h, &tmp, bytes, true)))
         return rc;
-    unsigned long long *flag = nullptr, n = 0ull;
-    WEDGE_CHECK(cudaMallocAsync((void**)&flag, ((uint64_t)s.pT + 1) * sizeof(unsigned long long), st));
-    const uint32_t grid = grid_for((uint64_t)s.pT + 1, AUX_THREADS, cap);
+    const uint32_t grid = grid_for(n, AUX_THREADS, cap);
     split_flag_kernel<<<grid, AUX_THREADS, 0, st>>>(g.tile_dst0, g.dst_off, s.pT, g.E, tile_e, flag);
-    if ((rc = device_scan(h, flag, flag, (uint64_t)s.pT + 1, false)))
-        return rc;
+    WEDGE_CHECK(cub::DeviceScan::ExclusiveSum(tmp, bytes, flag, flag, (long long)n, st));
     split_fill_kernel<<<grid, AUX_THREADS, 0, st>>>(g.tile_dst0, g.dst_off, s.pT, g.E, tile_e, flag, s.psplit_k, s.psplit_t0,
                                                    s.psplit_t1);
     WEDGE_CHECK(cudaGetLastError());
-    WEDGE_CHECK(cudaMemcpyAsync(&n, flag + s.pT, sizeof(n), cudaMemcpyDeviceToHost, st));
-    WEDGE_CHECK(cudaStreamSynchronize(st));
-    cudaFreeAsync(flag, st);
-    s.pnsplit = (uint32_t)n;
-    s.pnwide = (uint32_t)(n >> 32);
+    s.pcount = flag + s.pT;
+    if (on_host) {
+        unsigned long long c = 0ull;
+        WEDGE_CHECK(cudaMemcpyAsync(&c, s.pcount, sizeof(c), cudaMemcpyDeviceToHost, st));
+        WEDGE_CHECK(cudaStreamSynchronize(st));
+        s.pnsplit = (uint32_t)c;
+        s.pnwide = (uint32_t)(c >> 32);
+    }
     return WEDGE_OK;
 }
 
@@ -6232,8 +6249,25 @@ static int ensure_state(wedge_graph* h, int app, int precision)
     double* bp;
     // [grid] block sums | [counter_slots * NCNT] block counters | [aux grid] PageRank-sum partials
     const uint64_t slots = counter_slots(h);
-    if ((rc = dalloc(h, &ctrl, 1, true)) ||
-        (rc = dalloc(h, &bp, grid + slots * NCNT + (uint64_t)h->num_sms * 8 + 8, true)) ||
+    const uint64_t bps = grid + slots * NCNT + (uint64_t)h->num_sms * 8 + 8;
+    s.rstride = (V + 31) & ~31ull; /* PageRank */
+    if (app == WEDGE_APP_PR && precision != WEDGE_PREC_FP32C) {
+        /* all arrays in one block, if it fits: one by one, and with a wait for the split lists' counts,
+           a first run of one iteration took 332 us at scale 12 and 487 at 16, 245 and 280 so */
+        const uint64_t tiles = g.Epad / (32u * PrPrec<true>::epl) + 1;
+        const uint64_t size = sizeof(Ctrl) + 8 * bps + LOG_CAP * sizeof(IterRec) + 16 * V + 16 * s.rstride + 16 * grid +
+                              4 * nwords + 20 * tiles + (tiles >> 3) + 16ull * (g.T + 1) + (64u << 10);
+        unsigned char* block = nullptr;
+        rc = dalloc(h, &block, size, true);
+        if (rc == WEDGE_OK) {
+            h->sblock = block;
+            h->sblock_size = size;
+            h->sblock_used = 0;
+        } else if (rc != WEDGE_ERR_OOM) {
+            return rc;
+        }
+    }
+    if ((rc = dalloc(h, &ctrl, 1, true)) || (rc = dalloc(h, &bp, bps, true)) ||
         (rc = dalloc(h, &s.log, LOG_CAP, true)))
         return rc;
     WEDGE_CHECK(cudaMemset(ctrl, 0, sizeof(Ctrl)));
@@ -6253,9 +6287,8 @@ static int ensure_state(wedge_graph* h, int app, int precision)
         WEDGE_CHECK(cudaMemsetAsync(s.acc, 0, (V ? V : 1) * sizeof(double), h->stream));
         pr_inv_outdeg_kernel<<<grid_for(V, AUX_THREADS, (uint32_t)h->num_sms * 8u), AUX_THREADS, 0, h->stream>>>(g, s.inv_od);
         WEDGE_CHECK(cudaGetLastError());
-        s.rstride = (V + 31) & ~31ull;
         if ((rc = dalloc(h, &s.rank, 2 * s.rstride, true)) || (rc = dalloc(h, &s.pmass, 2ull * h->pull_grid + 8, true)) ||
-            (rc = has_in_state(h)) || (rc = split_state(h, 32u * PrPrec<true>::epl)) || (rc = dalloc(h, &s.head_part, (uint64_t)g.T + 1, true)) ||
+            (rc = has_in_state(h)) || (rc = split_state(h, 32u * PrPrec<true>::epl, false)) || (rc = dalloc(h, &s.head_part, (uint64_t)g.T + 1, true)) ||
             (rc = dalloc(h, &s.tail_part, (uint64_t)g.T + 1, true)))
             return rc;
     } else {

@@ -201,6 +201,7 @@ struct DevState {
     uint32_t* psplit_k;            // destinations spanning pull tiles (PR32_TILE in-edges): short ones from the
     uint32_t* psplit_t0;           // front (pnsplit), long ones from the back (pnwide; entry pT-1-j)
     uint32_t* psplit_t1;
+    const unsigned long long* pcount; // pnwide << 32 | pnsplit
     uint32_t pnsplit, pnwide, pT;
     float2* phead;                 // [pT] (sum, compensation) of a split destination ending in tile t
     float2* ptail;                 // [pT] (sum, compensation) of a split destination continuing past tile t
@@ -282,6 +283,8 @@ struct wedge_graph {
     uint64_t tsize, tused;
     unsigned char* slab;               // a small graph's arrays (tracked as one allocation; null otherwise)
     uint64_t slab_size, slab_used;
+    unsigned char* sblock;             // several of the state's arrays (tracked as one allocation; null otherwise)
+    uint64_t sblock_size, sblock_used;
     // allocations owned by the handle
     void* allocs[40];
     int nallocs;
