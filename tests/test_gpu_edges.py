@@ -607,3 +607,28 @@ def test_captured_loops_without_cooperative_launches(engine_lib, monkeypatch):
         w = rng.integers(0, 256, len(s)).astype(np.uint64)
         check_traversals(W, V, s[order].astype(np.uint32), d[order].astype(np.uint32), w,
                          (W.SCHED_PLAIN, W.SCHED_WEDGE, W.SCHED_FILTERED), (0, W.FLAG_GRAPH, W.FLAG_TIMING))
+
+
+@pytest.mark.parametrize("iterations", [1, 2, 7])
+def test_vertex_phase_after_a_pagerank(engine_lib, iterations):
+    """the vertex phase alone after a run works on the run's last sums: the same ranks
+    with the same damping, that iteration's with another"""
+    W = engine_lib
+    rng = np.random.default_rng(iterations)
+    V, n = 3000, 40_000
+    s, d = (V * rng.random(n) ** 3).astype(np.int64), np.sort((V * rng.random(n) ** 2).astype(np.int64))
+    s[-1], s, d = V - 5, s.astype(np.uint32), d.astype(np.uint32)
+    outdeg = np.bincount(s, minlength=V).astype(np.float64)
+    outdeg[outdeg == 0] = V
+    before = plain_pagerank(V, s.astype(np.int64), d.astype(np.int64), iterations - 1, 0.85)
+    acc = np.zeros(V, np.longdouble)
+    np.add.at(acc, d, before.astype(np.longdouble)[s])
+    with W.Graph.from_edges(V, s, d) as g:
+        g.run(W.APP_PR, W.Params(num_iterations=iterations, damping=0.85))
+        ran = g.read_results().view(np.float64).copy()
+        for damping in (0.85, 0.6, 0.85):
+            g.run_phase(W.APP_PR, W.PHASE_VERTEX_PR, W.Params(damping=damping))
+            got = g.read_results().view(np.float64)
+            expect = (((acc + (1.0 - acc.sum()) / V) * damping + (1.0 - damping) / V) / outdeg).astype(np.float64)
+            assert np.abs(got - expect).sum() <= 1e-13 * np.abs(expect).sum(), damping
+        assert np.abs(got - ran).sum() <= 1e-13 * np.abs(ran).sum()

@@ -129,7 +129,7 @@ static void free_state(wedge_graph* h)
         h->graph_exec = nullptr;
         h->graph_app = -1;
     }
-    h->pr_flip = 0;
+    h->pr_flip = h->pr_sums_due = 0;
 }
 
 static void load_scratch_free(wedge_graph* h)
@@ -6965,6 +6965,7 @@ static int run_pr(wedge_graph* h, const wedge_params_t* p, wedge_stats_t* st, bo
     double t_pull = 0, t_vertex = 0;
     WEDGE_CHECK(cudaEventRecord(h->ev[0], h->stream));
     h->pr_flip = loop && !c32 ? (int)(p->num_iterations & 1u) : 0;
+    h->pr_sums_due = loop && !c32 ? 1 : 0;
     if (loop) {
         int rc = launch_pr_loop(h, p->num_iterations, timing);
         if (rc)
@@ -7327,13 +7328,25 @@ int wedge_cuda_run_phase(wedge_graph_t* g, int app, int phase, const wedge_param
     if ((rc = ensure_state(g, app, params->precision)))
         return rc;
     const DevGraph& dg = g->g;
+    g->s.damping = params->damping > 0.0 ? params->damping : 0.875;
+    g->s.precision = (uint32_t)params->precision;
+    if (app == WEDGE_APP_PR && g->pr_sums_due && phase == WEDGE_PHASE_VERTEX_PR) {
+        /* the vertex phase again after a run in one launch, which keeps no sums: those of its last
+           iteration, from the ranks before it in the other buffer */
+        double* rank = g->s.rank;
+        if (!g->pr_flip)
+            g->s.rank += g->s.rstride;
+        launch_pull(g, app);
+        pr_finish_kernel<<<finish_grid(g, dg), AUX_THREADS, 0, g->stream>>>(dg, g->s, g->pull_grid, counters(g));
+        launch_pr_total(g);
+        g->s.rank = rank;
+    }
+    g->pr_sums_due = 0;
     if (app == WEDGE_APP_PR && g->pr_flip) { /* the phases keep FP64 ranks in the first buffer */
         WEDGE_CHECK(cudaMemcpyAsync(g->s.rank, g->s.rank + g->s.rstride, dg.V * sizeof(double), cudaMemcpyDeviceToDevice,
                                     g->stream));
         g->pr_flip = 0;
     }
-    g->s.damping = params->damping > 0.0 ? params->damping : 0.875;
-    g->s.precision = (uint32_t)params->precision;
     const uint32_t vgrid = aux_grid(g, dg.V);
     Ctrl c;
     switch (phase) {

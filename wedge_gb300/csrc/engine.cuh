@@ -298,6 +298,7 @@ struct wedge_graph {
     cudaGraphExec_t graph_exec;        // captured traversal
     uint32_t loop_hub;                 // pr_loop_kernel's hub cache, bytes
     int pr_flip;                       // the FP64 ranks are in the second buffer
+    int pr_sums_due;                   // DevState::acc does not hold the last run's sums
     int graph_app;
     int graph_key;
     int cc_pending;                    // CC labels are engine ids (symmetric graph, not yet converted)
