@@ -555,21 +555,14 @@ def sub_records(W, S, blob, args, peak):
 
 
 def _batch_record(W):
-    import json as _json
-
     import numpy as np
+    from wedge_gb300 import autotune
     from wedge_gb300 import batch as B
 
     params = B.graph_params()
     queries = B.queries(params)
     graphs = B.load_graphs(params)
-    tuning = None
-    try:
-        with open(os.path.join(ROOT, "wedge_gb300", "data", "batch_tuning.json")) as f:
-            best = _json.load(f)["best"]
-        tuning = W.BatchTuning(best["threshold_pct"], best["grab"], best["blocks_per_sm"], best["split"])
-    except Exception:
-        pass
+    tuning = autotune.load_tuning()
     with W.Batch(graphs, queries) as b:
         b.run(tuning, W.FLAG_GRAPH)
         ts = [b.run(tuning, W.FLAG_GRAPH)["running_ms"] for _ in range(3)]

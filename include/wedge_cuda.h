@@ -262,7 +262,8 @@ int wedge_cuda_set_stream(wedge_graph_t* g, void* stream);
  * gone.  Out-of-range values return WEDGE_ERR_ARG. */
 enum wedge_knob {
     WEDGE_KNOB_HUB_BYTES = 0,    /* shared-memory hub cache of the pulls, bytes: 0 (none) .. 196608, multiple
-                                    of 16 (WEDGE_HUB_BYTES; default 65536); the device's limit applies */
+                                    of 16 (WEDGE_HUB_BYTES; default 65536); the device's limit applies.  SSSP
+                                    over weight-ordered in-edges has none */
     WEDGE_KNOB_PROBE_EDGES = 1,  /* BFS/CC per-destination probe window, in-edges: 1 .. 4096
                                     (WEDGE_PROBE_EDGES; default 16) */
     WEDGE_KNOB_SSSP_TILE = 2,    /* SSSP dense pulls: 512 or 256 (WEDGE_SSSP_TILES512=1/0).  512: over
@@ -355,9 +356,9 @@ int wedge_mlp_train(float* blob, const float* X, const float* Y, const float* M,
 /* No counterpart in the reference, which runs one query per process.  Many
  * BFS and SSSP queries over many graphs run together in one persistent
  * cooperative kernel: every iteration of every unfinished query is split into
- * 32-edge chunks on one device work queue, and the Wedge frontiers of all
- * queries are built in the same pass, so small and large queries share the
- * GPU.  Results equal those of wedge_cuda_run on each query alone. */
+ * short work items on one device queue, and the vertices that change are listed
+ * for the next in the same pass, so small and large queries share the GPU.
+ * Results equal those of wedge_cuda_run on each query alone. */
 typedef struct wedge_query {
     uint32_t graph;           /* index into the batch's graph array */
     int32_t app;              /* WEDGE_APP_BFS or WEDGE_APP_SSSP (SSSP needs a weighted graph) */
@@ -366,10 +367,11 @@ typedef struct wedge_query {
 
 typedef struct wedge_batch_tuning {
     uint32_t threshold_pct;   /* dense pull iff active out-edge mass > t% of the query's edges (0: 20) */
-    uint32_t grab;            /* 32-edge chunks a warp takes from the queue at a time (0: 8) */
+    uint32_t grab;            /* work items (listed vertices, pieces of lists, groups of destinations, tiles or
+                                 chunks) a warp takes from the queue at a time at most (0: 8) */
     uint32_t blocks_per_sm;   /* persistent blocks per SM, at most the occupancy limit (0: that limit) */
-    uint32_t split;           /* out-degree above which the Wedge build expands a vertex with the whole
-                                 warp instead of one lane (0: 32) */
+    uint32_t split;           /* chunk frontiers (beyond 2^32 in-edges): out-degree above which the build expands
+                                 a vertex with the whole warp instead of one lane (0: 32); not read otherwise */
 } wedge_batch_tuning_t;
 
 typedef struct wedge_batch_stats {

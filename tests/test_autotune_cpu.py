@@ -65,3 +65,12 @@ def test_knob_names_match_the_header():
     for name, k in W.KNOB_NAMES.items():
         assert f"WEDGE_KNOB_{name.upper()} = {k}," in text
     assert W.KNOB_DEFAULT == np.iinfo(np.uint64).max
+
+
+def test_combinations_that_cannot_differ_are_timed_once():
+    g = FakeGraph(lambda k: 4.0 if A.weight_ordered_alike(k).get("hub_bytes") is None else 5.0 + k["hub_bytes"] / 1e6)
+    space = A.ENGINE_SPACE["sssp"]
+    default, best, results = A.tune_engine(g, W.APP_SSSP, None, space, reps=2, log=lambda *_: None, alike=A.weight_ordered_alike)
+    assert len(results) == 3 * len(space["hub_bytes"]) + 1
+    assert sum(r["sssp_tile"] == 512 and r["sssp_narrow"] == 1 for r in results) == 1
+    assert best["ms"] == 4.0 and "split" not in A.GRID and A.load_tuning() is not None

@@ -1,12 +1,12 @@
 """Autotuners: the batched multi-query kernel and the single-query engine.
 
-Batched kernel.  The persistent kernel has four knobs (wedge_batch_tuning_t):
-the dense/Wedge threshold of each query's next pull, how many 32-edge chunks a
-warp takes from the work queue at a time, how many persistent blocks run per
-SM, and the out-degree above which the Wedge build expands a vertex with a
-whole warp instead of one lane.  The tuner times every combination of a small
-grid on the workload (captured CUDA graph, CUDA events, median of repeats) and
-keeps the fastest; the table goes to data/batch_tuning.json.
+Batched kernel.  The tuner times three knobs of wedge_batch_tuning_t: the
+dense/Wedge threshold of each query's next pull, how many work items a warp
+takes from the queue at a time at most, and how many persistent blocks run per
+SM.  (The fourth, split, is read on graphs beyond 2^32 in-edges only, whose
+frontiers are chunks.)  It times every combination of a small grid on the
+workload (captured CUDA graph, CUDA events, median of repeats) and keeps the
+fastest; the table goes to data/batch_tuning.json.
 
 Single-query engine.  Each application's launches have the knobs of
 wedge_cuda_set_knob: the shared-memory hub cache's bytes (what the pulls
@@ -43,7 +43,15 @@ ENGINE_SPACE = {
     "sssp": {"hub_bytes": HUB_CHOICES, "sssp_tile": (256, 512), "sssp_narrow": (0, 1)},
     "pr": {"hub_bytes": HUB_CHOICES},
 }
-GRID = {"threshold_pct": (2, 5, 10, 20, 40), "grab": (2, 8, 32), "blocks_per_sm": (1, 2, 4), "split": (8, 32, 128)}
+GRID = {"threshold_pct": (2, 5, 10, 20, 40), "grab": (2, 8, 32), "blocks_per_sm": (1, 2, 4)}
+
+
+def weight_ordered_alike(cfg: dict) -> dict:
+    """the knobs that matter of an SSSP configuration on a graph with byte weights: its
+    weight-ordered pulls (512-edge tiles asked for, 32-bit distances) use no hub cache"""
+    if cfg.get("sssp_tile") == 512 and cfg.get("sssp_narrow") == 1:
+        return {k: v for k, v in cfg.items() if k != "hub_bytes"}
+    return cfg
 
 
 def load_tuning(path: str = DEFAULT_TUNING):
@@ -75,10 +83,10 @@ def _median_ms(g: W.Graph, app: int, params: W.Params, reps: int) -> float:
     return float(np.median([g.run(app, params)["running_ms"] for _ in range(reps)]))
 
 
-def tune_engine(g: W.Graph, app: int, params: W.Params, space: dict, reps: int = 5, log=print):
+def tune_engine(g: W.Graph, app: int, params: W.Params, space: dict, reps: int = 5, log=print, alike=None):
     """every combination of the knobs in space on one handle; returns (default, best, results),
     each result {knob: value, ..., "ms": median Running Time}; the knobs go back to their
-    defaults afterwards"""
+    defaults afterwards.  alike: what matters of a combination; one of those with the same is timed"""
     keys = list(space)
     for k in keys:
         g.set_knob(k, None)
@@ -86,6 +94,8 @@ def tune_engine(g: W.Graph, app: int, params: W.Params, space: dict, reps: int =
     results = []
     for values in itertools.product(*(space[k] for k in keys)):
         cfg = dict(zip(keys, values))
+        if alike and any(alike(cfg) == alike({k: r[k] for k in keys}) for r in results):
+            continue
         for k, v in cfg.items():
             g.set_knob(k, v)
         results.append({**cfg, "ms": _median_ms(g, app, params, reps)})
@@ -139,7 +149,8 @@ def engine_main(a):
                          "30 PageRank iterations (compensated FP32)",
              "scale": scale, "edge_factor": ef, "reps": a.reps, "apps": {}}
     for name, (g, app, params) in apps.items():
-        default, best, results = tune_engine(g, app, params, ENGINE_SPACE[name], a.reps)
+        default, best, results = tune_engine(g, app, params, ENGINE_SPACE[name], a.reps,
+                                             alike=weight_ordered_alike if name == "sssp" else None)
         table["apps"][name] = {"default": default, "best": best, "speedup_vs_default": default["ms"] / best["ms"],
                                "results": results}
         g.close()
