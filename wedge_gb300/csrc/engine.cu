@@ -200,8 +200,9 @@ static int dalloc(wedge_graph* h, T** p, uint64_t count, bool state = false)
 // stack (all work is on one stream, so what a released array held is read
 // before its place is written again); others, and what does not fit, from the
 // stream's pool, which gives its memory back at every synchronisation and has to
-// map it again after it: weighted R-MAT loads of scales 12, 16 and 20 took 0.91,
-// 1.42 and 5.3 ms with the pool alone, 0.79, 1.35 and 4.9 with the block.
+// map it again after it: weighted R-MAT graphs of scales 12, 16 and 20 took 1.14,
+// 1.96 and 6.4 ms to generate, build and close with the pool alone, 1.08, 1.92
+// and 6.3 with the block, 1.12, 1.58 and 5.4 with the arrays' block below too.
 // LOAD_SCRATCH_EDGES (edges and vertices) bounds the block (1.6 GB); beyond it
 // the kernels' time hides the mapping.
 constexpr uint64_t LOAD_SCRATCH_EDGES = 1ull << 25;
@@ -3833,7 +3834,8 @@ __global__ void init_root_kernel(DevGraph g, DevState s, uint32_t app, uint64_t 
 // cleared while no block reads it).  Every block takes the iteration's
 // decision for itself from the summed counters; the last one writes it down.
 // A long SSSP (past NEAR_ITER iterations: grids and roads; an R-MAT graph takes
-// 10-15 and would only take more) visits the near vertices first: while its
+// 10-15 and would only take more: 3 to 10% with FP64 weights from iteration 8 on;
+// the 1001^2 grid takes 1.00 ms from 8 or 16 on, 1.12 from 32 on) visits the near vertices first: while its
 // changed vertices have more than NEAR_MASS out-edges (fewer cost no more than
 // the barrier), those whose distance is above a bound wait in a far list.
 // When the near ones have fewer, the bound rises by NEAR_STEP mean weights, at
@@ -3857,8 +3859,12 @@ __global__ void init_root_kernel(DevGraph g, DevState s, uint32_t app, uint64_t 
 //
 // Graphs of at most LOOP_SMALL_EDGES in-edges run whole in the launch under the
 // plain rule: there a dense iteration is no more work than a Wedge one, and the
-// launches were all the time (BFS at scale 12: 182 us).  A caller that asks for a
-// strategy, or for the network's choice of one, gets that strategy's kernels.
+// launches were all the time (BFS at scale 12: 182 us).  R-MAT graphs whole and
+// with the dense iterations apart, BFS and SSSP: 2^18 in-edges 64 and 176 us for
+// 101 and 271, 2^20 85 and 252 for 106 and 337, 2^21 98 and 279 for 108 and 320,
+// 2^22 143 and 388 for 117 and 333; a dense iteration's out-edges cost more from
+// there on.  A caller that asks for a strategy, or for the network's choice of
+// one, gets that strategy's kernels.
 constexpr uint32_t LOOP_LONG = 128;   // out-edges of one vertex a warp takes at once: one round of four per lane
 constexpr uint32_t LOOP_BUF = 96;     // listed vertices a warp keeps in shared memory (each list)
 constexpr unsigned long long NEAR_MASS = 1ull << 16;
@@ -4729,8 +4735,7 @@ __global__ void pr_inv_outdeg_kernel(DevGraph g, double* inv_od)
     }
 }
 
-// execution_initialize_pr (execution_pr.c:380-392); max_iter bounds the
-// captured iteration loop
+// execution_initialize_pr (execution_pr.c:380-392); max_iter: the iterations asked for
 __global__ void pr_init_kernel(DevGraph g, DevState s, uint32_t max_iter)
 {
     const double invN = __ddiv_rn(1.0, (double)g.V);
@@ -6428,7 +6433,6 @@ static void launch_pull(wedge_graph* h, int app)
     }
 }
 
-// kernels one iteration launches: the pull(s) and the five of the tail
 // the Wedge build's launches: collect, expand, build (not for SSSP over
 // out-edges), compact (chunk frontiers only)
 static uint64_t build_launches(const wedge_graph* h)
