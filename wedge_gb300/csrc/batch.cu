@@ -59,7 +59,7 @@ struct BGraph {
     const uint32_t* first_src;   // every destination's first source
     const uint2* wo_long;        // (destination, first in-edge) pieces of the destinations past WO_GROUP in-edges
     uint32_t nlong;
-    const uint32_t* outdeg;
+    const uint32_t* outdeg;      // with push: the out-lists' lengths (a shard's are shorter than its out-degrees)
     const unsigned long long* csri_off;
     const uint32_t* csri;
     const uint8_t* cw8;          // out-edge weights (push): byte-wide, or
@@ -69,7 +69,6 @@ struct BGraph {
     uint64_t V, E;
     uint32_t Vne, nchunks, weight_kind;
     uint32_t push;               // sparse pulls relax out-edges (CSRI of destinations)
-    uint32_t shard;              // outdeg are the whole graph's, longer than the out-lists
 };
 
 struct BQuery {
@@ -236,19 +235,12 @@ __device__ void phase_prefix(const BArgs& a)
 }
 
 // ---------------------------------------------------------------- pull
-// how many of vertex v's od out-edges the graph holds (a shard: those to its own destinations)
-__device__ __forceinline__ uint32_t list_length(const BGraph& G, uint32_t v, uint32_t od)
-{
-    return G.shard ? (uint32_t)(G.csri_off[v + 1u] - G.csri_off[v]) : od;
-}
-
 // vertex v of out-degree od into the next iteration's list, or its items; one lane
 __device__ __forceinline__ void list_one(const BQuery& qq, BCtl& c, const BGraph& G, uint32_t v, uint32_t od)
 {
     const uint32_t nx = (c.iter + 1u) % 3u, buf = (c.iter + 1u) & 1u;
-    const uint32_t len = G.push ? list_length(G, v, od) : 0u;
-    if (len > PUSH_PIECE) {
-        const uint32_t np = (len + PUSH_PIECE - 1u) / PUSH_PIECE;
+    if (G.push && od > PUSH_PIECE) {
+        const uint32_t np = (od + PUSH_PIECE - 1u) / PUSH_PIECE;
         const uint32_t at = atomicAdd(&c.nitem[nx], np);
         for (uint32_t j = 0; j < np; ++j)
             qq.items[buf][at + j] = make_uint2(v, j);
@@ -261,7 +253,7 @@ __device__ __forceinline__ void list_one(const BQuery& qq, BCtl& c, const BGraph
 __device__ __forceinline__ void list_warp(const BQuery& qq, BCtl& c, const BGraph& G, bool on, uint32_t v, uint32_t od)
 {
     const int lane = threadIdx.x & 31;
-    const bool shrt = on && (od <= PUSH_PIECE || list_length(G, v, od) <= PUSH_PIECE);
+    const bool shrt = on && od <= PUSH_PIECE;
     const uint32_t m = __ballot_sync(FULL, shrt);
     if (m) {
         uint32_t at = 0u;
@@ -1037,9 +1029,8 @@ __global__ void batch_seed_kernel(BArgs a)
             c.nitem[j] = 0u;
         }
         const uint32_t od = G.outdeg[r];
-        const uint32_t len = G.push ? list_length(G, r, od) : 0u;
-        if (len > PUSH_PIECE) {
-            c.nitem[0] = (len + PUSH_PIECE - 1u) / PUSH_PIECE;
+        if (G.push && od > PUSH_PIECE) {
+            c.nitem[0] = (od + PUSH_PIECE - 1u) / PUSH_PIECE;
             for (uint32_t j = 0; j < c.nitem[0]; ++j)
                 qq.items[0][j] = make_uint2(r, j);
         } else {
@@ -1078,6 +1069,13 @@ __global__ void batch_wo_long_kernel(const unsigned long long* dst_off, uint32_t
         for (uint32_t j = 0; out && j < np; ++j)
             out[at + j] = make_uint2(k, lo + j * WO_PIECE);
     }
+}
+
+// the lengths of a shard's out-lists
+__global__ void batch_list_length_kernel(const unsigned long long* off, uint64_t V, uint32_t* len)
+{
+    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x)
+        len[v] = (uint32_t)(off[v + 1] - off[v]);
 }
 
 __global__ void batch_export_kernel(BGraph G, BQuery qq, unsigned long long* out)
@@ -1195,7 +1193,7 @@ extern "C" int wedge_cuda_batch_create(wedge_graph_t* const* graphs, uint32_t nu
     b->device = dev;
     b->Q = num_queries;
     b->G = num_graphs;
-    b->qallocs = (void**)calloc((size_t)num_graphs + 3, sizeof(void*)); /* an array per graph, the lists, the queries */
+    b->qallocs = (void**)calloc(2 * (size_t)num_graphs + 3, sizeof(void*)); /* two arrays per graph, the lists, the queries */
     b->h_graphs = (BGraph*)calloc(num_graphs, sizeof(BGraph));
     b->h_queries = (BQuery*)calloc(num_queries, sizeof(BQuery));
     int rc = WEDGE_OK;
@@ -1222,7 +1220,6 @@ extern "C" int wedge_cuda_batch_create(wedge_graph_t* const* graphs, uint32_t nu
         G.cw8 = g.cw8;
         G.cw = g.cw;
         G.push = g.csr;
-        G.shard = g.shard;
         G.wsrc = g.csr ? g.wsrc : nullptr;
         G.ww8 = g.ww8;
         G.wo_src = g.wo_src;
@@ -1245,6 +1242,13 @@ extern "C" int wedge_cuda_batch_create(wedge_graph_t* const* graphs, uint32_t nu
         if ((rc = balloc(b, &cd, (uint64_t)G.nchunks + 1, true)))
             return fail(rc);
         G.chunk_dst0 = cd;
+        if (g.shard && g.csr) {
+            uint32_t* len = nullptr;
+            if ((rc = balloc(b, &len, g.V, true)))
+                return fail(rc);
+            batch_list_length_kernel<<<bgrid(g.V, 256, (uint32_t)b->num_sms * 8), 256, 0, b->stream>>>(g.csri_off, g.V, len);
+            G.outdeg = len;
+        }
         batch_chunk_index_kernel<<<bgrid((uint64_t)G.nchunks + 1, 256, (uint32_t)b->num_sms * 8), 256, 0, b->stream>>>(G, cd);
     }
     // pieces of the destinations with many in-edges (dense pulls): all graphs' counts, then their lists
