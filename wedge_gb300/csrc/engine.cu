@@ -208,10 +208,11 @@ static int dalloc(wedge_graph* h, T** p, uint64_t count, bool state = false)
 constexpr uint64_t LOAD_SCRATCH_EDGES = 1ull << 25;
 // Up to this many edges and vertices a graph's own arrays, twenty of them, lie
 // in one block too: loading a scale-20 graph from memory, BFS, read and close
-// 6.57 ms with 2^22, 6.08 with 2^25.  The block is as large as the arrays where
-// every vertex has in-edges (1 GB at most, 0.8 GB unweighted, with about as many
-// vertices as edges; R-MAT scale 20, edge factor 16: 250 and 110 MB); 22 or 16
-// bytes are unused for each that has none, 1 byte per edge with byte weights.
+// 6.57 ms with 2^22, 6.08 with 2^25.  The block is somewhat larger than the arrays
+// where every vertex has in-edges: 1.1 GB at most, 0.9 GB unweighted, with as many
+// vertices as edges (R-MAT scale 20, edge factor 16: 290 and 140 MB, of which 60
+// and 30 are not used).  Cut to their size, 1 to 2 bytes per edge and 4 to 10 per
+// vertex less, the batch of 512 queries over 64 graphs took 17.0 ms for 16.7.
 constexpr uint64_t SLAB_EDGES = 1ull << 25;
 
 template <class T>
@@ -827,9 +828,7 @@ int build_from_device_edges(wedge_graph* h, uint64_t V, uint64_t E, uint32_t* d_
 
     if (E + V <= SLAB_EDGES) { /* the arrays below, at most (a slot each rounded up) */
         const uint64_t vne = E < V ? E : V;
-        /* per edge: destination starts, out-edges; weights in the three orders or wide ones */
-        const uint64_t edges = g.Epad / 8 + (d_w ? 12u : 4u) * g.Epad;
-        const uint64_t size = edges + 16ull * g.T + 24ull * V + (d_w ? 22u : 16u) * vne + 32u * 256u;
+        const uint64_t size = (d_w ? 14u : 5u) * g.Epad + 16ull * g.T + 24ull * V + 26ull * vne + 32u * 256u;
         unsigned char* slab = nullptr;
         if (dalloc(h, &slab, size) == WEDGE_OK) {
             h->slab = slab;
