@@ -632,3 +632,20 @@ def test_vertex_phase_after_a_pagerank(engine_lib, iterations):
             expect = (((acc + (1.0 - acc.sum()) / V) * damping + (1.0 - damping) / V) / outdeg).astype(np.float64)
             assert np.abs(got - expect).sum() <= 1e-13 * np.abs(expect).sum(), damping
         assert np.abs(got - ran).sum() <= 1e-13 * np.abs(ran).sum()
+
+
+def test_timed_runs_past_the_log(engine_lib):
+    """more iterations than the log keeps: the kept ones have their own times, the
+    others' are in the totals"""
+    W = engine_lib
+    V = 6001
+    s, d = np.arange(V - 1, dtype=np.uint32), np.arange(1, V, dtype=np.uint32)
+    with W.Graph.from_edges(V, s, d) as g:
+        for app, p in ((W.APP_BFS, {}), (W.APP_PR, dict(num_iterations=6000))):
+            for _ in range(2):
+                st = g.run(app, W.Params(flags=W.FLAG_TIMING, **p))
+            times = np.array([r["pull_ms"] for r in g.iteration_log()])
+            total = st["pull_ms_dense"] + st["pull_ms_wedge"] + st["vertex_ms"]
+            assert st["iterations"] == 6000 and len(times) == 4096
+            assert times.min() > 0.0 and times[0] < 50 * np.median(times)
+            assert 0.8 * st["running_ms"] < total <= st["running_ms"] and total > 1.3 * times.sum()

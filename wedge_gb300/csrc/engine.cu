@@ -4004,6 +4004,8 @@ __global__ void __launch_bounds__(PULL_THREADS, 1)
     Ctrl* c = s.ctrl;
     if (c->done)
         return;
+    if (timed && blockIdx.x == 0 && threadIdx.x == 0)
+        c->start_ns = device_ns();
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
     const uint32_t nw = nthr >> 5;
@@ -5639,6 +5641,8 @@ __global__ void __launch_bounds__(PULL_THREADS, 1) pr_loop_kernel(DevGraph g, De
             s.log[it].end_ns = device_ns();
         __syncthreads();
     }
+    if (timed && tid == 0u)
+        c->end_ns = device_ns();
     // vertices with neither in- nor out-edges: the last iteration's constant, once
     if (threadIdx.x == 0)
         sh_k = P::constants(g, s, before);
@@ -6692,8 +6696,9 @@ static int traversal_stats(wedge_graph* h, int app, uint64_t launches, bool use_
 }
 
 // The times of a timed run's last round, from iteration before.iter to
-// after.iter: the loop's iterations by the clock that it noted (the first with
-// the launch), the pull's and its tail's by their events (ev 2, 5, 3, 4).
+// after.iter: the loop's iterations by the clock that it noted (what the launch
+// took beyond the logged ones counts as Wedge pulls where the log was full), the
+// pull's and its tail's by their events (ev 2, 5, 3, 4).
 static int note_times(wedge_graph* h, const Ctrl& before, const Ctrl& after, bool fused, bool small, double* dense, double* wedge,
                       double* tail)
 {
@@ -6712,16 +6717,17 @@ static int note_times(wedge_graph* h, const Ctrl& before, const Ctrl& after, boo
         free(r);
         return cuda_status(e);
     }
-    double rest = loop_ms; /* of the loop's time, for the first of its iterations */
-    for (uint32_t i = logged < in_loop ? logged : in_loop; i-- > 0u;) {
-        const double ms = i ? (double)(r[i].end_ns - r[i - 1u].end_ns) / 1e6 : rest > 0.0 ? rest : 0.0;
+    double rest = loop_ms; /* of the loop's time, for the iterations past the log's end */
+    const uint32_t both = logged < in_loop ? logged : in_loop;
+    for (uint32_t i = 0; i < both; ++i) {
+        const double ms = (double)(r[i].end_ns - (i ? r[i - 1u].end_ns : after.start_ns)) / 1e6;
         rest -= ms;
         h->iter_pull_ms[before.iter + i] = ms;
         h->iter_wedge_ms[before.iter + i] = 0.0;
         *(r[i].mode == MODE_WEDGE ? wedge : dense) += ms;
     }
-    if (in_loop && !logged)
-        *wedge += loop_ms; /* past the log's end */
+    if (both < in_loop && rest > 0.0)
+        *wedge += rest;
     if (n > in_loop) {
         const double ms = in_loop ? pull_ms : pull_ms + loop_ms;
         if (logged > in_loop) {
@@ -6954,6 +6960,11 @@ static int pr_loop_times(wedge_graph* h, uint32_t iters, double* pull, double* v
         h->iter_wedge_ms[i] = 0.0;
         *pull += h->iter_pull_ms[i];
         *vertex += (double)(r[i].end_ns - r[i].pull_ns) / 1e6;
+    }
+    if (iters > n) { /* past the log's end: in the proportion of the ones in it */
+        const double all = (double)(c.end_ns - c.start_ns) / 1e6 / (*pull + *vertex);
+        *pull *= all;
+        *vertex *= all;
     }
     free(r);
     return e == cudaSuccess ? WEDGE_OK : cuda_status(e);

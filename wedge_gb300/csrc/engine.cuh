@@ -130,7 +130,8 @@ struct Ctrl {
     unsigned long long lmin[3], lfar[3]; // out-edges it changed the waiting ones; by far list modulo 3:
     unsigned int lf[3];                // vertices listed; by step modulo 2: found by their far bits; by
     unsigned int lall[2], lput[3];     // step modulo 3: listed in the far list at hand
-    unsigned long long start_ns;       // timed pr_loop_kernel: when its first iteration began
+    unsigned long long start_ns, end_ns; // timed runs of the loop kernels: when the first iteration began,
+                                       // when the last one ended (PageRank)
     double pr_total;                   // sum of all accumulators (phase_vertex_pr.c:161); compensated FP32:
                                        // the total the next iteration uses
     double pr_prev;                    // compensated FP32: the total the last iteration used
