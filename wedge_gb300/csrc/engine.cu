@@ -5450,8 +5450,8 @@ __device__ __forceinline__ double ld_rank(const double* p)
     return r;
 }
 
-template <bool F64>
-__global__ void __launch_bounds__(PULL_THREADS, 1) pr_loop_kernel(DevGraph g, DevState s, uint32_t iters, uint32_t timed)
+template <bool F64, bool TIMED>
+__global__ void __launch_bounds__(PULL_THREADS, 1) pr_loop_kernel(DevGraph g, DevState s, uint32_t iters)
 {
     using P = PrPrec<F64>;
     using rank_t = typename P::rank_t;
@@ -5498,7 +5498,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1) pr_loop_kernel(DevGraph g, De
     if (!grid_barrier(c, target, &sh_ok))
         return;
     const unsigned long long pol = l2_evict_first_policy();
-    if (timed && tid == 0u)
+    if (TIMED && tid == 0u)
         c->start_ns = device_ns();
     for (uint32_t it = 0; it < iters; ++it) {
         const rank_t* cur = rank + ((it & 1u) ? stride : 0ull);
@@ -5598,7 +5598,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 1) pr_loop_kernel(DevGraph g, De
             atomicAdd(&sh_dsts, dsts);
         if (!grid_barrier(c, target, &sh_ok))
             return;
-        if (timed && tid == 0u && it < LOG_CAP)
+        if (TIMED && tid == 0u && it < LOG_CAP)
             s.log[it].pull_ns = device_ns();
         // ---- destinations whose in-edges span tiles, in tile order (phases.c:71-114)
         if constexpr (F64) {
@@ -5637,11 +5637,11 @@ __global__ void __launch_bounds__(PULL_THREADS, 1) pr_loop_kernel(DevGraph g, De
         }
         __syncthreads();
         total = sh_part[0];
-        if (timed && tid == 0u && it < LOG_CAP)
+        if (TIMED && tid == 0u && it < LOG_CAP)
             s.log[it].end_ns = device_ns();
         __syncthreads();
     }
-    if (timed && tid == 0u)
+    if (TIMED && tid == 0u)
         c->end_ns = device_ns();
     // vertices with neither in- nor out-edges: the last iteration's constant, once
     if (threadIdx.x == 0)
@@ -6226,7 +6226,7 @@ template <bool F64>
 static int pr_loop_hub(wedge_graph* h)
 {
     cudaFuncAttributes fa;
-    WEDGE_CHECK(cudaFuncGetAttributes(&fa, pr_loop_kernel<F64>));
+    WEDGE_CHECK(cudaFuncGetAttributes(&fa, pr_loop_kernel<F64, false>));
     int optin = 0;
     WEDGE_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
     const int stage = (int)pr_stage_bytes<F64>(), room = optin - (int)fa.sharedSizeBytes;
@@ -6234,7 +6234,8 @@ static int pr_loop_hub(wedge_graph* h)
         return WEDGE_ERR_UNSUPPORTED;
     const uint32_t most = (uint32_t)(room - stage) & ~15u;
     h->loop_hub = h->hub_bytes < most ? h->hub_bytes : most;
-    WEDGE_CHECK(cudaFuncSetAttribute(pr_loop_kernel<F64>, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
+    WEDGE_CHECK(cudaFuncSetAttribute(pr_loop_kernel<F64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
+    WEDGE_CHECK(cudaFuncSetAttribute(pr_loop_kernel<F64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
     return WEDGE_OK;
 }
 
@@ -6903,10 +6904,14 @@ static int launch_pr_loop(wedge_graph* h, uint32_t iters, bool timed)
     DevState s = h->s;
     s.hub_bytes = h->loop_hub;
     WEDGE_CHECK(cudaMemsetAsync(s.ctrl, 0, sizeof(Ctrl), h->stream));
-    if (f64)
-        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, pr_loop_kernel<true>, h->g, s, iters, timed ? 1u : 0u));
+    if (f64 && timed)
+        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, pr_loop_kernel<true, true>, h->g, s, iters));
+    else if (f64)
+        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, pr_loop_kernel<true, false>, h->g, s, iters));
+    else if (timed)
+        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, pr_loop_kernel<false, true>, h->g, s, iters));
     else
-        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, pr_loop_kernel<false>, h->g, s, iters, timed ? 1u : 0u));
+        WEDGE_CHECK(cudaLaunchKernelEx(&cfg, pr_loop_kernel<false, false>, h->g, s, iters));
     return WEDGE_OK;
 }
 
